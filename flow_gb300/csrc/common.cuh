@@ -32,15 +32,18 @@ constexpr double kCT = 0.3;
 //                             double: bit order = value order)
 //   [7] mesh power-of-two     1 when every mesh spacing is a power of two
 //                             (formed on the device at the start of a step)
-//   [8] moving tiles          the fused step's count of first-sweep tiles
-//                             it did not skip (uint64), read with dt
-//   [9 ...]                   per-block partials (2 doubles per block, at
+//   [8] minimum at rest       the CFL minimum over the shock-heating tiles
+//                             the next step need not visit (as [6])
+//   [9 .. 12] tile counts     lengths of the next step's tile lists (uint32,
+//                             128- and 127-column tiles of 2, 4, 8, 16 rows)
+//   [13 ...]                  per-block partials (2 doubles per block, at
 //                             most kMaxReduceBlocks blocks)
 //   [kRaQFlags ...]           the fused step's tile flags, when the array
 //                             is large enough to hold them: per-tile CFL
 //                             minima, then the viscous-stress, mass-flux and
-//                             velocity flags and the two halves of the
-//                             sweeps' skip marks (fused.cu, fill_mesh_args)
+//                             velocity flags, the two halves of the sweeps'
+//                             skip marks and the tile lists (fused.cu,
+//                             fill_mesh_args)
 enum : int {
   kRaDt = 0,
   kRaDtH = 1,
@@ -50,8 +53,9 @@ enum : int {
   kRaStatus = 5,
   kRaMinBits = 6,
   kRaMeshPow2 = 7,
-  kRaMoving = 8,
-  kRaPartial = 9,
+  kRaRestMin = 8,
+  kRaTileCounts = 9,
+  kRaPartial = 13,
 };
 constexpr int kMaxReduceBlocks = 1024;
 constexpr int kRaQFlags = kRaPartial + 2 * kMaxReduceBlocks;

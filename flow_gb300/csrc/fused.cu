@@ -2,6 +2,7 @@
 // solve_hydro_2d, and the mixed form gb300_mixed_solve): one kernel launch per
 // phase, each CTA running one tile function of fused_tiles.cuh.
 #include <array>
+#include <cmath>
 #include <cstddef>
 
 #include "../../include/flow_gb300.h"
@@ -31,7 +32,7 @@ __device__ __forceinline__ void pdl_trigger() {
 // step.  The tiles then skip their own spacing tests (block_mesh_pow2).
 constexpr int kPow2Threads = 1024;
 // It also clears the CFL minimum slot and the block ticket for the step's
-// Lagrangian kernels, and the count of moving first-sweep tiles.
+// Lagrangian kernels.
 __global__ void __launch_bounds__(kPow2Threads)
     k_mesh_pow2(int nx, int ny, const double* celldx, const double* edgedx,
                 const double* celldy, const double* edgedy, unsigned long long* flag,
@@ -41,7 +42,6 @@ __global__ void __launch_bounds__(kPow2Threads)
   if (threadIdx.x == 0) {
     *reinterpret_cast<unsigned long long*>(ra + kRaTicket) = 0ull;
     *reinterpret_cast<unsigned long long*>(ra + kRaMinBits) = ~0ull;
-    *reinterpret_cast<unsigned long long*>(ra + kRaMoving) = 0ull;
   }
   // Every test is made (no short circuit), so that a thread's loads are
   // independent and in flight together.
@@ -58,7 +58,24 @@ __global__ void __launch_bounds__(kPow2Threads)
   if (threadIdx.x == 0) *flag = ok ? 1ull : 0ull;
 }
 
-template <typename R, bool kFl>
+// How a kernel of the step runs: without flags (a mesh too small for them),
+// with flags over its whole grid, or with flags over the listed tiles.  Two
+// instantiations for the latter, as the tile of a block is uniform to the
+// compiler only when it comes from blockIdx (the mixed form's pairs took 2%
+// longer over a whole mesh with the choice made at run time).
+enum : int { kNoFlags = 0, kWhole = 1, kListed = 2 };
+template <int kMd, typename R>
+__device__ __forceinline__ bool block_tile(const StepArgs<R>& a, int& bx, int& by) {
+  if constexpr (kMd == kListed) {
+    return listed_tile(a, (int)blockIdx.x, bx, by);
+  } else {
+    bx = blockIdx.x;
+    by = blockIdx.y;
+    return true;
+  }
+}
+
+template <typename R, int kMd>
 __global__ void __launch_bounds__(kCols) k_lag_pressure(const StepArgs<R> a) {
   pdl_wait();
   pdl_trigger();
@@ -66,39 +83,55 @@ __global__ void __launch_bounds__(kCols) k_lag_pressure(const StepArgs<R> a) {
   // of the shock-heating kernel (three kernels later, which waits for it).
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
     *reinterpret_cast<unsigned long long*>(a.ra + kRaTicket) = 0ull;
-    *a.min_slot = ~0ull;
-    if (a.moving) *a.moving = 0ull;
+    // (and starts the minimum from the tiles the step does not visit), and
+    // what the step's last kernel accumulates.
+    *a.min_slot = a.from_rest_min ? *a.rest_min : ~0ull;
+    if constexpr (kMd != kNoFlags) {
+      *a.rest_min = ~0ull;
+#pragma unroll
+      for (int k = kRaTileCounts; k < kRaPartial; ++k) {
+        *reinterpret_cast<unsigned long long*>(a.ra + k) = 0ull;
+      }
+    }
   }
-  tile_lag_pressure<R, kFl>(a, blockIdx.x, blockIdx.y);
+  int bx, by;
+  if (block_tile<kMd>(a, bx, by)) tile_lag_pressure<R, (kMd != kNoFlags)>(a, bx, by);
 }
-// kFlags: the viscous-stress flags (a.qmask) are kept -- the viscosity
+// With flags, the viscous-stress flags (a.qmask) are kept -- the viscosity
 // kernel stores only warp rows with a non-zero stress, and the two kernels
 // after it load only those.
-template <typename R, bool kFlags>
+template <typename R, int kMd>
 __global__ void __launch_bounds__(kCols) k_lag_viscosity(const StepArgs<R> a) {
   pdl_wait();
   pdl_trigger();
-  tile_lag_viscosity<R, kFlags>(a, blockIdx.x, blockIdx.y);
+  int bx, by;
+  if (block_tile<kMd>(a, bx, by)) tile_lag_viscosity<R, (kMd != kNoFlags)>(a, bx, by);
 }
-template <typename R, bool kFlags>
+template <typename R, int kMd>
 __global__ void __launch_bounds__(kCols) k_lag_viscous_accel(const StepArgs<R> a) {
   pdl_wait();
   pdl_trigger();
-  tile_lag_viscous_accel<R, true, kFlags>(a, blockIdx.x, blockIdx.y);
+  int bx, by;
+  if (block_tile<kMd>(a, bx, by)) {
+    tile_lag_viscous_accel<R, true, (kMd != kNoFlags)>(a, bx, by);
+  }
 }
 // Shock heating + CFL minimum; the last block to finish (ticket in
 // reduce_array) applies the dt rule.
-template <typename R, bool kFlags>
+template <typename R, int kMd>
 __global__ void __launch_bounds__(kCols) k_lag_energy_dt(const StepArgs<R> a) {
   __shared__ bool s_last;
   __shared__ unsigned long long s_tile_min;  // the tile's CFL minimum (kFlags)
   pdl_wait();
   pdl_trigger();
-  tile_lag_energy_dt<R, true, kFlags>(a, blockIdx.x, blockIdx.y, kFlags ? &s_tile_min : nullptr);
+  int bx, by;
+  constexpr bool kFlags = kMd != kNoFlags;
+  const bool tile = block_tile<kMd>(a, bx, by);
+  if (tile) tile_lag_energy_dt<R, true, kFlags>(a, bx, by, kFlags ? &s_tile_min : nullptr);
   if (threadIdx.x == 0) {
     // (Thread 0 wrote the minimum it stores here.)
-    if (kFlags && a.cfl_tile) {
-      a.cfl_tile[(size_t)blockIdx.y * a.qm_stride + blockIdx.x] = s_tile_min;
+    if (kFlags && a.cfl_tile && tile) {
+      a.cfl_tile[(size_t)by * a.qm_stride + bx] = s_tile_min;
     }
     __threadfence();
     unsigned long long* ticket = reinterpret_cast<unsigned long long*>(a.ra + kRaTicket);
@@ -111,36 +144,204 @@ __global__ void __launch_bounds__(kCols) k_lag_energy_dt(const StepArgs<R> a) {
     *reinterpret_cast<unsigned long long*>(a.ra + kRaTicket) = 0ull;
   }
 }
-// kFl (sweeps and momentum pairs): the mass-flux flags (a.fxflag, a.fyflag)
-// are kept -- the sweeps store only warps with a non-zero mass flux, and the
+// With flags, the mass-flux flags (a.fxflag, a.fyflag) are kept -- the sweeps store only warps with a non-zero mass flux, and the
 // momentum pairs load only those.
-template <typename R, bool kFirst, bool kFl>
+template <typename R, bool kFirst, int kMd>
 __global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 8 : 7) k_mass_sweep_x(const StepArgs<R> a,
                                                         const SweepArgs<R> s) {
   pdl_wait();
   pdl_trigger();
-  tile_mass_sweep_x<R, kFirst, true, kFl>(a, s, blockIdx.x, blockIdx.y);
+  int bx, by;
+  if (block_tile<kMd>(a, bx, by)) {
+    tile_mass_sweep_x<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by);
+  }
 }
-template <typename R, bool kFirst, bool kFl>
+template <typename R, bool kFirst, int kMd>
 __global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 7 : 6) k_mass_sweep_y(const StepArgs<R> a,
                                                         const SweepArgs<R> s) {
   pdl_wait();
   pdl_trigger();
-  tile_mass_sweep_y<R, kFirst, true, kFl>(a, s, blockIdx.x, blockIdx.y);
+  int bx, by;
+  if (block_tile<kMd>(a, bx, by)) {
+    tile_mass_sweep_y<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by);
+  }
 }
+// ---------------------------------------------------------------------------
+// Tile lists: the tiles the next step has to visit.  A cell in a tile the
+// step's first sweep marked was at rest through the step (StepArgs::rest).  In
+// the next step the flow reaches at most five cells past the cells that were
+// not (one by the pressure jumps, one by the stresses, one by the sweeps'
+// fluxes, two by the momentum fluxes), so a tile with every cell within
+// kReach + pad of it marked (pad: the pressure phase's tiles start pad rows and
+// columns earlier than the others') is left by every kernel of the next step
+// as it is: it would test its flags and return.  On a blast that holds 1% of a
+// 4096^2 mesh such tiles were half of a step (8192 tiles a kernel, 8 or so at
+// once on an SM, about 2.5 us each).
+constexpr int kListHeights = 4;               // tiles of 2, 4, 8 and 16 rows
+constexpr int kListBand = 2 << (kListHeights - 1);
+constexpr int kReach = 6;
+
+struct ListArgs {
+  int nx, ny, pad;
+  const unsigned char* marks;  // this step's skip marks
+  int mark_w, mark_tiles_x, mark_rows;
+  unsigned* next_marks;        // the next step's half, filled with ones here
+  int next_words;
+  int tx[2], bands;            // columns of 128- and 127-wide tiles, 16-row bands
+  int blocks;                  // of each width (0: no lists)
+  unsigned* list[2];           // [heights][tx * bands * 16 / height] each
+  unsigned* counts;            // [2][kListHeights], cleared by the pressure phase
+  // The CFL minimum over this step's shock-heating tiles that are not listed.
+  const unsigned long long* cfl_tile;
+  int cfl_tx, cfl_ty, cfl_rows;
+  unsigned long long* rest_min;
+};
+// First entry of the list of height 2 << h in list[wide].
+__host__ __device__ inline size_t list_offset(int tx, int bands, int h) {
+  size_t o = 0;
+  for (int k = 0; k < h; ++k) o += (size_t)tx * bands * (kListBand / (2 << k));
+  return o;
+}
+
+// The lists, in blocks 0 .. 2 blocks - 1 of kCols threads: eight lanes per
+// 16-row band of a tile column, each of which loads two or three bands of
+// marks (all its loads in flight together) and decides one pair of rows.
+__device__ __forceinline__ void tile_lists(const ListArgs& l, int block) {
+  const int wd = block < l.blocks ? 0 : 1;  // the tile width
+  const int t = (block - wd * l.blocks) * kCols + (int)threadIdx.x;
+  if (wd == 0) {
+    for (int q = t; q < l.next_words; q += l.blocks * kCols) l.next_marks[q] = 0x01010101u;
+  }
+  constexpr int kSub = kListBand / 2;
+  const int lane = threadIdx.x & 31, sub = lane & (kSub - 1), grp = lane & ~(kSub - 1);
+  const int tx = l.tx[wd];
+  const int k = t / kSub;
+  const bool in = k < tx * l.bands;
+  const int by = in ? k / tx : 0, bx = in ? k - by * tx : 0;
+  const int pad = l.pad, D = kReach + pad;
+  const int w = wd ? kCols - 1 : kCols;
+  // The tile's columns and rows (clamped next to the walls: a ghost cell's
+  // mirror source lies within pad of them) with the reach around them: at most
+  // three columns of marks.
+  const int c0 = min(pad + bx * w, l.nx - 2 * pad);
+  const int x0 = (max(c0 - D, pad) - pad) / l.mark_w;
+  const int x1 = (min(c0 + w + D, l.nx - pad) - 1 - pad) / l.mark_w;
+  const int r0 = pad + by * kListBand;
+  const int lo = max(min(r0, l.ny - 2 * pad) - D, pad);
+  const int hi = min(r0 + kListBand + D, l.ny - pad);
+  const int b0 = (lo - pad) / l.mark_rows, b1 = (hi - 1 - pad) / l.mark_rows;
+  // Bit b - b0: band b of marks holds a tile that was not at rest.
+  unsigned long long moved = 0ull;
+  constexpr int kRounds = 3;  // (kListBand + 2 D) / 2 + 1 bands at most, pad <= 4
+  unsigned char m[kRounds][3];
+#pragma unroll
+  for (int q = 0; q < kRounds; ++q) {
+    const int b = b0 + q * kSub + sub;
+    const size_t row = (size_t)min(b, b1) * l.mark_tiles_x;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) m[q][c] = l.marks[row + min(x0 + c, x1)];
+  }
+#pragma unroll
+  for (int q = 0; q < kRounds; ++q) {
+    const bool rest = (m[q][0] & m[q][1] & m[q][2]) != 0 || b0 + q * kSub + sub > b1;
+    const unsigned v = __ballot_sync(0xffffffffu, in && !rest);
+    moved |= (unsigned long long)((v >> grp) & ((1u << kSub) - 1)) << (q * kSub);
+  }
+  for (int q = kRounds * kSub; b0 + q <= b1; ++q) {  // (wide ghost layers)
+    const size_t row = (size_t)(b0 + q) * l.mark_tiles_x;
+    if ((l.marks[row + x0] & l.marks[row + min(x0 + 1, x1)] & l.marks[row + x1]) == 0) {
+      moved |= 1ull << min(q, 63);
+    }
+  }
+  const int s0 = r0 + 2 * sub;
+  const int p0 = (max(min(s0, l.ny - 2 * pad) - D, pad) - pad) / l.mark_rows - b0;
+  const int p1 = (min(s0 + 2 + D, l.ny - pad) - 1 - pad) / l.mark_rows - b0;
+  const unsigned long long window =
+      p0 > 63 ? 1ull << 63 : ((p1 >= 63 ? ~0ull : (1ull << (p1 + 1)) - 1) & ~((1ull << p0) - 1));
+  // The tiles of height 2, then 4, 8 and 16: bit i of act, the group's i-th.
+  unsigned act = (__ballot_sync(0xffffffffu, in && (moved & window) != 0ull) >> grp) &
+                 ((1u << kSub) - 1);
+unsigned acts[kListHeights], all[kListHeights];
+#pragma unroll
+  for (int h = 0; h < kListHeights; ++h) {
+    const int per = kSub >> h;
+    if (h) {
+      unsigned up = 0u;
+      for (int i = 0; i < per; ++i) up |= ((act >> (2 * i)) & 3u) ? 1u << i : 0u;
+      act = up;
+    }
+    acts[h] = act;
+    all[h] = __ballot_sync(0xffffffffu, sub < per && ((act >> sub) & 1u));
+  }
+  // Lane h takes the warp's places in the list of height h (one round trip for
+  // all of them).
+  unsigned base = 0u;
+#pragma unroll
+  for (int h = 0; h < kListHeights; ++h) {
+    if (lane == h) base = (unsigned)__popc(all[h]);
+  }
+  if (base) base = atomicAdd(l.counts + wd * kListHeights + lane, base);
+#pragma unroll
+  for (int h = 0; h < kListHeights; ++h) {
+    const int per = kSub >> h;
+    const bool mine = sub < per && ((acts[h] >> sub) & 1u);
+    const unsigned at = __shfl_sync(0xffffffffu, base, h) + __popc(all[h] & ((1u << lane) - 1));
+    if (mine) {
+      l.list[wd][list_offset(tx, l.bands, h) + at] =
+          ((unsigned)(by * per + sub) << 16) | (unsigned)bx;
+    }
+    if (wd == 0 && l.cfl_rows == (2 << h)) {
+      const int ty = by * per + sub;
+      unsigned long long c = ~0ull;
+      if (in && sub < per && !mine && bx < l.cfl_tx && ty < l.cfl_ty) {
+        c = l.cfl_tile[(size_t)ty * l.cfl_tx + bx];
+      }
+      c = warp_min_u64(c);
+      if (lane == 0 && c != ~0ull) atomicMin(l.rest_min, c);
+    }
+  }
+}
+
 // Momentum pairs (flux fused with its update): x pairs share a row's fluxes
 // through shared memory (127 faces per CTA), y pairs march down columns.
-template <typename R, bool kV, bool kVel, bool kFl>
-__global__ void __launch_bounds__(kCols) k_mom_x(const StepArgs<R> a) {
-  pdl_wait();
-  pdl_trigger();
-  tile_mom_x<R, kV, kVel, true, kFl>(a, blockIdx.x, blockIdx.y);
+// kLists: the step's last pair, whose last 2 l.blocks blocks form the next
+// step's tile lists beside it (the pair reads neither the marks nor the minima
+// they are formed from; on its own the list kernel took 7 to 20 us a step,
+// mostly latency).  Its grid is 1-D.
+template <int kMd, bool kLists, typename R>
+__device__ __forceinline__ bool pair_tile(const StepArgs<R>& a, const ListArgs& l, int& bx,
+                                          int& by) {
+  if constexpr (kLists) {
+    const int k = (int)blockIdx.x, n = (int)gridDim.x - 2 * l.blocks;
+    if (k >= n) {
+      tile_lists(l, k - n);
+      return false;
+    }
+    if constexpr (kMd == kListed) return listed_tile(a, k, bx, by);
+    by = k / a.grid_x;
+    bx = k - by * a.grid_x;
+    return true;
+  } else {
+    return block_tile<kMd>(a, bx, by);
+  }
 }
-template <typename R, bool kV, bool kVel, bool kFl>
-__global__ void __launch_bounds__(kCols) k_mom_y(const StepArgs<R> a) {
+template <typename R, bool kV, bool kVel, int kMd, bool kLists>
+__global__ void __launch_bounds__(kCols) k_mom_x(const StepArgs<R> a, const ListArgs l) {
   pdl_wait();
   pdl_trigger();
-  tile_mom_y<R, kV, kVel, true, kFl>(a, blockIdx.x, blockIdx.y);
+  int bx, by;
+  if (pair_tile<kMd, kLists>(a, l, bx, by)) {
+    tile_mom_x<R, kV, kVel, true, (kMd != kNoFlags)>(a, bx, by);
+  }
+}
+template <typename R, bool kV, bool kVel, int kMd, bool kLists>
+__global__ void __launch_bounds__(kCols) k_mom_y(const StepArgs<R> a, const ListArgs l) {
+  pdl_wait();
+  pdl_trigger();
+  int bx, by;
+  if (pair_tile<kMd, kLists>(a, l, bx, by)) {
+    tile_mom_y<R, kV, kVel, true, (kMd != kNoFlags)>(a, bx, by);
+  }
 }
 
 // The whole Lagrangian phase of the FP64 step in one kernel (lag_fused.cuh):
@@ -283,25 +484,104 @@ void launch_pdl(void (*k)(KArgs...), dim3 grid, cudaStream_t s, Args... args) {
   launch_pdl_block(k, grid, dim3(kCols), s, args...);
 }
 
+// The previous step's tile lists, by tile width (128, 127) and height.
+struct TileLists {
+  bool use = false;
+  const unsigned* list[2][kListHeights] = {};
+  int n[2][kListHeights] = {};
+};
+inline int height_index(int rows) { return rows == 2 ? 0 : rows == 4 ? 1 : rows == 8 ? 2 : 3; }
+// The grid of a kernel over the tiles of `full` (set in a): all of them, or
+// the listed ones.
+template <typename R>
+dim3 tile_grid(StepArgs<R>& a, const TileLists& tl, int narrow, dim3 full) {
+  a.grid_x = (int)full.x;
+  a.grid_y = (int)full.y;
+  if (!tl.use) {
+    a.tiles = nullptr;
+    return full;
+  }
+  const int h = height_index(a.rows);
+  a.tiles = tl.list[narrow][h];
+  a.n_tiles = tl.n[narrow][h];
+  return dim3((unsigned)(a.n_tiles > 0 ? a.n_tiles : 1));
+}
+
 inline dim3 strip_grid(int cols, int rows, int tile_rows, int cols_per_cta = kCols) {
   return dim3((unsigned)((cols + cols_per_cta - 1) / cols_per_cta),
               (unsigned)((rows + tile_rows - 1) / tile_rows));
 }
 
-// x pair for rho_u (kV false): x-faces pad .. nx-pad, 127 per CTA; for rho_v:
-// y-faces pad .. nx-pad-1.  Rows: the faces' rows.
-// Tile heights of the momentum pairs (with and without the velocity
-// update) and of the viscous acceleration: the pairs without a velocity
-// update and the viscous update skip the still tiles (flags) and work only
-// where the flow moves, and shorter tiles there shorten the longest tile's
-// chain of rows, which bounds such a kernel.
-constexpr int kRowsMomVel = 16, kRowsMomFlux = 8, kRowsAccel = 8;
-// Tile heights of the pressure, viscosity and shock-heating kernels, and of
-// the two mass sweeps (whose bands are also the skip marks' bands): a step
-// whose previous step's first sweep skipped at least half of its tiles takes
-// the shorter sweep tiles (the moving tiles' chains of rows bound a sweep
-// there), others the taller ones (less halo work on a field in motion).
-constexpr int kRowsLag = 16, kRowsSweepStill = 8, kRowsSweepMoving = 16;
+// Tile heights of a step, by kernel.  A warp's FP64 instructions issue one per
+// 64 clocks, and depend on one another at that distance too, so a tile takes
+// its rows one after another at about 1 to 3 us a row, and a kernel whose tiles
+// fit the SMs at once takes as long as its longest tile: on a 48x32 mesh
+// 16-row tiles made a step of 345 us with most SMs idle.  The height taken is
+// the one with the least time on the busiest SM,
+//   (rows + kHaloRows) * max(ceil(tiles / SMs), tiles that an SM overlaps):
+// kHaloRows for a tile's first face flux, table set-up and first loads (about
+// a row's time or two); an SM overlaps the tiles whose latencies hide behind
+// one another's, three in the FP64 form (a third of a row's time is FP64
+// issue), six in the mixed form.
+struct StepRows {
+  int lag = 16, energy = 16, accel = 16, sweep = 16, mom_vel = 16, mom_flux = 16;
+};
+// Shortest tiles: with flags, the second sweep's skip test reads the marks one
+// band either side of its own, which hold the two rows it reaches past it.
+constexpr int kMinRowsFlags = 2;
+constexpr int kMaxRowsStep = 16;
+// The shock-heating tiles keep their minima from step to step by tile, so a
+// new height makes that kernel visit the whole mesh once.  It starts at eight
+// rows at most (a run's first step does not know what moves) and stays there
+// while the lists are in use.
+constexpr int kRowsEnergy = 8;
+// The viscous update and the momentum pairs without a velocity update leave
+// tiles without a stress or a mass flux at once, so their longest chain of
+// rows bounds them (4096x2048 moving everywhere: the viscous update takes
+// 196 us with 16 rows, 181 with 8; 2048^2 mixed: a step 556 us, 546 with 8).
+constexpr int kRowsSparse = 8;
+constexpr double kHaloRows = 1.5, kOverlap64 = 3.0, kOverlapMixed = 6.0;
+inline double rows_cost(double tiles, int rows, double overlap) {
+  const double per_sm = ceil(tiles / num_sms());
+  return (rows + kHaloRows) * (per_sm > overlap ? per_sm : overlap);
+}
+// The tiles of each height a step visits: all of a mesh of cols x rows, or
+// counts of the lists (index: height 2 << i).  was: the previous step's
+// height, kept unless another is a fifth cheaper (0: none).
+int pick_rows(int cols, int rows, int cols_per_cta, const unsigned* counts, int min_rows,
+              int was, double overlap) {
+  const double tx = (cols + cols_per_cta - 1) / cols_per_cta;
+  auto cost = [&](int h) {
+    return rows_cost(counts ? (double)counts[height_index(h)] : tx * ((rows + h - 1) / h), h,
+                     overlap);
+  };
+  int best = kMaxRowsStep;
+  for (int h = kMaxRowsStep / 2; h >= min_rows; h /= 2) {
+    if (cost(h) < cost(best)) best = h;
+  }
+  return was >= min_rows && cost(best) > 0.8 * cost(was) ? was : best;
+}
+// counts: the lengths of the tile lists ([2][kListHeights]), or null where
+// the step visits every tile; was: the step before, when this one follows it.
+StepRows pick_step_rows(int nx, int ny, int pad, const unsigned* counts, bool flags,
+                        const StepRows* was, double overlap) {
+  const int w = nx - 2 * pad, h = ny - 2 * pad;
+  const int lo = flags ? kMinRowsFlags : 1;
+  const unsigned* narrow = counts ? counts + kListHeights : nullptr;
+  StepRows r;
+  r.lag = pick_rows(w, h, kCols, counts, lo, was ? was->lag : 0, overlap);
+  r.accel = r.lag > kRowsSparse ? kRowsSparse : r.lag;
+  r.energy = r.lag;
+  if (flags && counts) {
+    r.energy = was->energy <= kRowsEnergy ? was->energy : kRowsEnergy;
+  } else if (flags && !was && r.energy > kRowsEnergy) {
+    r.energy = kRowsEnergy;
+  }
+  r.sweep = pick_rows(w + 1, h, kCols - 1, narrow, lo, was ? was->sweep : 0, overlap);
+  r.mom_vel = r.sweep;
+  r.mom_flux = r.sweep > kRowsSparse ? kRowsSparse : r.sweep;
+  return r;
+}
 template <typename R>
 StepArgs<R> with_rows(const StepArgs<R>& a, int rows) {
   StepArgs<R> b = a;
@@ -309,46 +589,80 @@ StepArgs<R> with_rows(const StepArgs<R>& a, int rows) {
   return b;
 }
 
+// x pair for rho_u (kV false): x-faces pad .. nx-pad, 127 per CTA; for rho_v:
+// y-faces pad .. nx-pad-1.  Rows: the faces' rows.
+// Launches the instantiation of kernel template K (its arguments before the
+// mode and after it) that a step runs.
+#define FLOW_LAUNCH_MODE(md, g, s, args, K, ...)                                       \
+  do {                                                                                 \
+    if ((md) == kNoFlags) launch_pdl(K<__VA_ARGS__, kNoFlags>, g, s, FLOW_UNPACK args); \
+    else if ((md) == kWhole) launch_pdl(K<__VA_ARGS__, kWhole>, g, s, FLOW_UNPACK args); \
+    else launch_pdl(K<__VA_ARGS__, kListed>, g, s, FLOW_UNPACK args);                  \
+  } while (0)
+#define FLOW_UNPACK(...) __VA_ARGS__
+template <typename R>
+int step_mode(const StepArgs<R>& a) {
+  return !a.qmask ? kNoFlags : a.tiles ? kListed : kWhole;
+}
+
 template <typename R, bool kV, bool kVel>
-void launch_mom_x(cudaStream_t s, const StepArgs<R>& a0) {
-  const StepArgs<R> a = with_rows(a0, kVel ? kRowsMomVel : kRowsMomFlux);
+void launch_mom_x(cudaStream_t s, const StepArgs<R>& a0, const StepRows& sr,
+                  const TileLists& tl, const ListArgs& l) {
+  StepArgs<R> a = with_rows(a0, kVel ? sr.mom_vel : sr.mom_flux);
   const int cols = kV ? (a.nx - 2 * a.pad) : (a.nx + 1 - 2 * a.pad);
   const int rows = kV ? (a.ny + 1 - 2 * a.pad) : (a.ny - 2 * a.pad);
-  launch_pdl(a.fxflag ? k_mom_x<R, kV, kVel, true> : k_mom_x<R, kV, kVel, false>,
-             strip_grid(cols, rows, a.rows, kCols - 1), s, a);
+  dim3 g = tile_grid(a, tl, 1, strip_grid(cols, rows, a.rows, kCols - 1));
+  const int md = step_mode(a);
+  if constexpr (kV && !kVel) {  // the step's last pair
+    if (l.blocks) {
+      g = dim3(g.x * g.y + 2 * (unsigned)l.blocks);
+      if (md == kListed) launch_pdl(k_mom_x<R, kV, kVel, kListed, true>, g, s, a, l);
+      else launch_pdl(k_mom_x<R, kV, kVel, kWhole, true>, g, s, a, l);
+      return;
+    }
+  }
+  if (md == kNoFlags) launch_pdl(k_mom_x<R, kV, kVel, kNoFlags, false>, g, s, a, l);
+  else if (md == kWhole) launch_pdl(k_mom_x<R, kV, kVel, kWhole, false>, g, s, a, l);
+  else launch_pdl(k_mom_x<R, kV, kVel, kListed, false>, g, s, a, l);
 }
 template <typename R, bool kV, bool kVel>
-void launch_mom_y(cudaStream_t s, const StepArgs<R>& a0) {
-  const StepArgs<R> a = with_rows(a0, kVel ? kRowsMomVel : kRowsMomFlux);
+void launch_mom_y(cudaStream_t s, const StepArgs<R>& a0, const StepRows& sr,
+                  const TileLists& tl, const ListArgs& l) {
+  StepArgs<R> a = with_rows(a0, kVel ? sr.mom_vel : sr.mom_flux);
   const int cols = kV ? (a.nx - 2 * a.pad) : (a.nx + 1 - 2 * a.pad);
   const int rows = kV ? (a.ny + 1 - 2 * a.pad) : (a.ny - 2 * a.pad);
-  launch_pdl(a.fyflag ? k_mom_y<R, kV, kVel, true> : k_mom_y<R, kV, kVel, false>,
-             strip_grid(cols, rows, a.rows), s, a);
+  dim3 g = tile_grid(a, tl, 0, strip_grid(cols, rows, a.rows));
+  const int md = step_mode(a);
+  if constexpr (kV && !kVel) {  // the step's last pair
+    if (l.blocks) {
+      g = dim3(g.x * g.y + 2 * (unsigned)l.blocks);
+      if (md == kListed) launch_pdl(k_mom_y<R, kV, kVel, kListed, true>, g, s, a, l);
+      else launch_pdl(k_mom_y<R, kV, kVel, kWhole, true>, g, s, a, l);
+      return;
+    }
+  }
+  if (md == kNoFlags) launch_pdl(k_mom_y<R, kV, kVel, kNoFlags, false>, g, s, a, l);
+  else if (md == kWhole) launch_pdl(k_mom_y<R, kV, kVel, kWhole, false>, g, s, a, l);
+  else launch_pdl(k_mom_y<R, kV, kVel, kListed, false>, g, s, a, l);
 }
 
 template <typename R>
-void launch_mass(cudaStream_t s, const StepArgs<R>& a, bool dir_y, bool first,
-                 const SweepArgs<R>& sw) {
+void launch_mass(cudaStream_t s, const StepArgs<R>& a0, bool dir_y, bool first,
+                 const SweepArgs<R>& sw, const TileLists& tl) {
+  StepArgs<R> a = a0;
   const int pad = a.pad;
   if (dir_y) {
-    const bool fl = a.fyflag != nullptr;
-    const dim3 g = strip_grid(a.nx - 2 * pad, a.ny - 2 * pad, a.rows);
-    if (first) {
-      launch_pdl(fl ? k_mass_sweep_y<R, true, true> : k_mass_sweep_y<R, true, false>, g, s, a, sw);
-    } else {
-      launch_pdl(fl ? k_mass_sweep_y<R, false, true> : k_mass_sweep_y<R, false, false>, g, s, a,
-                 sw);
-    }
+    const dim3 g = tile_grid(a, tl, 0, strip_grid(a.nx - 2 * pad, a.ny - 2 * pad, a.rows));
+    const int md = step_mode(a);
+    if (first) FLOW_LAUNCH_MODE(md, g, s, (a, sw), k_mass_sweep_y, R, true);
+    else FLOW_LAUNCH_MODE(md, g, s, (a, sw), k_mass_sweep_y, R, false);
   } else {
-    const bool fl = a.fxflag != nullptr;
     // Faces pad .. nx-pad; every CTA advances 127 columns.
-    const dim3 g = strip_grid(a.nx + 1 - 2 * pad, a.ny - 2 * pad, a.rows, kCols - 1);
-    if (first) {
-      launch_pdl(fl ? k_mass_sweep_x<R, true, true> : k_mass_sweep_x<R, true, false>, g, s, a, sw);
-    } else {
-      launch_pdl(fl ? k_mass_sweep_x<R, false, true> : k_mass_sweep_x<R, false, false>, g, s, a,
-                 sw);
-    }
+    const dim3 g =
+        tile_grid(a, tl, 1, strip_grid(a.nx + 1 - 2 * pad, a.ny - 2 * pad, a.rows, kCols - 1));
+    const int md = step_mode(a);
+    if (first) FLOW_LAUNCH_MODE(md, g, s, (a, sw), k_mass_sweep_x, R, true);
+    else FLOW_LAUNCH_MODE(md, g, s, (a, sw), k_mass_sweep_x, R, false);
   }
 }
 
@@ -368,7 +682,8 @@ inline int apply_blocks(const lagf::LagArgs& l) {
 template <typename R>
 void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
                  const SweepArgs<R>& first, const SweepArgs<R>& second,
-                 StepProfiler& prof, int sweep_rows, bool mesh_known,
+                 StepProfiler& prof, const StepRows& sr, bool mesh_known,
+                 const TileLists& tl, const ListArgs& lists,
                  const lagf::LagArgs* lag = nullptr) {
   const int nx = a.nx, ny = a.ny, pad = a.pad;
   // The whole-mesh spacing test the tiles read (one block, a few
@@ -389,26 +704,29 @@ void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
                      const_cast<double*>(lag->rho_v));
   } else {
     prof.mark("lag_pressure");
-    launch_pdl(a.vflag ? k_lag_pressure<R, true> : k_lag_pressure<R, false>,
-               strip_grid(nx, ny, a.rows), s, a);
-    const bool fl = a.qmask != nullptr;
+    StepArgs<R> al = a;
+    dim3 g = tile_grid(al, tl, 0, strip_grid(nx, ny, a.rows));
+    FLOW_LAUNCH_MODE(step_mode(al), g, s, (al), k_lag_pressure, R);
     prof.mark("lag_viscosity");
-    launch_pdl(fl ? k_lag_viscosity<R, true> : k_lag_viscosity<R, false>,
-               strip_grid(nx - 2 * pad, ny - 2 * pad, a.rows), s, a);
+    g = tile_grid(al, tl, 0, strip_grid(nx - 2 * pad, ny - 2 * pad, a.rows));
+    FLOW_LAUNCH_MODE(step_mode(al), g, s, (al), k_lag_viscosity, R);
     prof.mark("lag_viscous_accel");
-    const StepArgs<R> aa = with_rows(a, kRowsAccel);
-    launch_pdl(fl ? k_lag_viscous_accel<R, true> : k_lag_viscous_accel<R, false>,
-               strip_grid(nx + 1 - 2 * pad, ny + 1 - 2 * pad, aa.rows), s, aa);
+    StepArgs<R> aa = with_rows(a, sr.accel);
+    g = tile_grid(aa, tl, 0, strip_grid(nx + 1 - 2 * pad, ny + 1 - 2 * pad, aa.rows));
+    FLOW_LAUNCH_MODE(step_mode(aa), g, s, (aa), k_lag_viscous_accel, R);
     prof.mark("lag_energy_dt");
-    launch_pdl(fl ? k_lag_energy_dt<R, true> : k_lag_energy_dt<R, false>,
-               strip_grid(nx - 2 * pad, ny - 2 * pad, a.rows), s, a);
+    // (All tiles where the minima of those off the list are not known.)
+    StepArgs<R> ae = with_rows(a, sr.energy);
+    g = tile_grid(ae, a.cfl_known ? tl : TileLists{}, 0,
+                  strip_grid(nx - 2 * pad, ny - 2 * pad, ae.rows));
+    FLOW_LAUNCH_MODE(step_mode(ae), g, s, (ae), k_lag_energy_dt, R);
   }
 
   // The advection phase reads velocity flags only when this step's
   // Lagrangian kernels wrote them (not the one-kernel phase).
   StepArgs<R> ad = a;
   if (lag) ad.vflag = nullptr;
-  const StepArgs<R> as = with_rows(ad, sweep_rows);
+  const StepArgs<R> as = with_rows(ad, sr.sweep);
   const bool x_first = (tt % 2 == 0);
   // With flags, the first sweep marks the tiles it skips (in its own grid);
   // the second reads their cells from the first sweep's input.
@@ -416,49 +734,49 @@ void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
   if (a.skipf) {
     sw1.skip = sw2.skip = a.skipf;
     sw1.skip_tiles_x = sw2.skip_tiles_x = x_first ? a.fx_stride / 4 : a.qm_stride;
-    sw1.skip_bands = sw2.skip_bands = (ny - 2 * pad + sweep_rows - 1) / sweep_rows;
+    sw1.skip_bands = sw2.skip_bands = (ny - 2 * pad + sr.sweep - 1) / sr.sweep;
     sw2.r_alt = first.r_in;
     sw2.e_alt = first.e_in;
     sw2.r_alt_r = first.r_in_r;
     sw2.e_alt_r = first.e_in_r;
   }
   prof.mark(x_first ? "mass_sweep_x" : "mass_sweep_y");
-  launch_mass(s, as, !x_first, true, sw1);
+  launch_mass(s, as, !x_first, true, sw1, tl);
   prof.mark(x_first ? "mass_sweep_y" : "mass_sweep_x");
-  launch_mass(s, as, x_first, false, sw2);
+  launch_mass(s, as, x_first, false, sw2, tl);
 
   // Momentum: each flux fused with its update, in the reference order; the
   // pair that recomputes a velocity comes first in each chain.
   if (tt % 2) {
     prof.mark("mom_uFx");
-    launch_mom_x<R, false, true>(s, ad);
+    launch_mom_x<R, false, true>(s, ad, sr, tl, lists);
     prof.mark("mom_uFy");
-    launch_mom_y<R, false, false>(s, ad);
+    launch_mom_y<R, false, false>(s, ad, sr, tl, lists);
     prof.mark("mom_vFx");
-    launch_mom_x<R, true, true>(s, ad);
+    launch_mom_x<R, true, true>(s, ad, sr, tl, lists);
     prof.mark("mom_vFy");
-    launch_mom_y<R, true, false>(s, ad);
+    launch_mom_y<R, true, false>(s, ad, sr, tl, lists);
   } else {
     prof.mark("mom_uFy");
-    launch_mom_y<R, false, true>(s, ad);
+    launch_mom_y<R, false, true>(s, ad, sr, tl, lists);
     prof.mark("mom_uFx");
-    launch_mom_x<R, false, false>(s, ad);
+    launch_mom_x<R, false, false>(s, ad, sr, tl, lists);
     prof.mark("mom_vFy");
-    launch_mom_y<R, true, true>(s, ad);
+    launch_mom_y<R, true, true>(s, ad, sr, tl, lists);
     prof.mark("mom_vFx");
-    launch_mom_x<R, true, false>(s, ad);
+    launch_mom_x<R, true, false>(s, ad, sr, tl, lists);
   }
 }
 
 int finish_step(cudaStream_t s, Mesh* mesh, double* ra, StepProfiler& prof,
-                const char* where, unsigned long long* moving = nullptr) {
+                const char* where, unsigned* counts) {
   {
     const int st = check_launch(where);
     if (st != GB300_OK) return st;
   }
-  // dt, dt_h (slots 0, 1), the status word (slot 5) and the moving-tile
-  // count (slot 8) in one copy.
-  double head[kRaMoving + 1];
+  // dt, dt_h (slots 0, 1), the status word (slot 5) and the lengths of the
+  // tile lists (slots 9 .. 12) in one copy.
+  double head[kRaPartial];
   cudaMemcpyAsync(head, ra + kRaDt, sizeof(head), cudaMemcpyDeviceToHost, s);
   const cudaError_t err = cudaStreamSynchronize(s);
   if (err != cudaSuccess) {
@@ -472,7 +790,7 @@ int finish_step(cudaStream_t s, Mesh* mesh, double* ra, StepProfiler& prof,
     return record_error(GB300_ERR_TIMEOUT,
                         "%s: a row copy of the Lagrangian kernel did not arrive", where);
   }
-  if (moving) memcpy(moving, &head[kRaMoving], sizeof(*moving));
+  memcpy(counts, &head[kRaTileCounts], 2 * kListHeights * sizeof(unsigned));
   const double pair[2] = {head[kRaDt], head[kRaDtH]};
   mesh->dt = pair[0];
   mesh->dt_h = pair[1];
@@ -489,12 +807,16 @@ int finish_step(cudaStream_t s, Mesh* mesh, double* ra, StepProfiler& prof,
 // ((ny + 1 - 2 pad) x stride), the x mass-flux flags ((ny - 2 pad) x xtiles),
 // the velocity flags (ny x vtiles) and the skip marks of even and odd steps
 // (a step's first sweep writes its own half; the next step reads it while its
-// own first sweep writes the other).
+// own first sweep writes the other), and the tile lists that even and odd steps
+// leave (the step's last kernel forms its own while it reads the previous
+// step's).
 constexpr int kConsTile = 128;  // rows and columns of a conservation tile
 struct FlagLayout {
   bool fits = false;
   int stride = 0, xtiles = 0, vtiles = 0, cons_tx = 0, cons_ty = 0;
-  size_t cfl = 0, cons = 0, q = 0, fy = 0, fx = 0, v = 0, marks = 0, sk_words = 0;
+  int list_tx[2] = {0, 0}, list_bands = 0;
+  size_t cfl = 0, cons = 0, q = 0, fy = 0, fx = 0, v = 0, marks = 0, sk_words = 0, lists = 0,
+         list_words[2] = {0, 0};
 };
 FlagLayout flag_layout(int nx, int ny, int pad) {
   FlagLayout L;
@@ -505,9 +827,8 @@ FlagLayout flag_layout(int nx, int ny, int pad) {
   if (L.stride <= 0 || rows <= 0) return L;
   L.cons_tx = (nx - 2 * pad + kConsTile - 1) / kConsTile;
   L.cons_ty = (int)((rows + kConsTile - 1) / kConsTile);
-  const long long bands = (rows + kRowsLag - 1) / kRowsLag;  // shock-heating tiles
-  const long long sweep_bands = (rows + kRowsSweepStill - 1) / kRowsSweepStill;  // at most
-  L.sk_words = ((size_t)sweep_bands * (L.xtiles > L.stride ? L.xtiles : L.stride) + 3) / 4;
+  const long long bands = (rows + kMinRowsFlags - 1) / kMinRowsFlags;  // tile bands, at most
+  L.sk_words = ((size_t)bands * (L.xtiles > L.stride ? L.xtiles : L.stride) + 3) / 4;
   L.cfl = 0;
   L.cons = L.cfl + 2 * (size_t)bands * L.stride;
   L.q = L.cons + 4 * (size_t)L.cons_tx * L.cons_ty;
@@ -515,7 +836,14 @@ FlagLayout flag_layout(int nx, int ny, int pad) {
   L.fx = L.fy + (size_t)(rows + 1) * L.stride;
   L.v = L.fx + (size_t)rows * L.xtiles;
   L.marks = L.v + (size_t)ny * L.vtiles;
-  const size_t words = L.marks + 2 * L.sk_words;
+  L.lists = L.marks + 2 * L.sk_words;
+  L.list_tx[0] = L.vtiles;
+  L.list_tx[1] = L.xtiles;
+  L.list_bands = (ny + kListBand - 1) / kListBand;
+  for (int w = 0; w < 2; ++w) {
+    L.list_words[w] = list_offset(L.list_tx[w], L.list_bands, kListHeights);
+  }
+  const size_t words = L.lists + 2 * (L.list_words[0] + L.list_words[1]);
   L.fits = (size_t)kRaQFlags * sizeof(double) + words * sizeof(unsigned) <=
            (size_t)nx * ny * sizeof(double);
   return L;
@@ -538,7 +866,7 @@ void fill_mesh_args(StepArgs<R>& a, const Mesh* mesh, int tt, double* ra) {
   a.dt_h = mesh->dt_h;
   a.max_dt = mesh->max_dt;
   a.first_step = (tt == 0);
-  a.rows = kRowsLag;
+  a.rows = kMaxRowsStep;
   a.qmask = nullptr;
   a.qm_stride = 0;
   a.fxflag = nullptr;
@@ -550,7 +878,11 @@ void fill_mesh_args(StepArgs<R>& a, const Mesh* mesh, int tt, double* ra) {
   a.rest = nullptr;
   a.rest_w = a.rest_tiles_x = a.rest_rows = 0;
   a.cfl_tile = nullptr;
-  a.moving = nullptr;
+  a.cfl_known = 0;
+  a.tiles = nullptr;
+  a.n_tiles = a.grid_x = a.grid_y = 0;
+  a.rest_min = reinterpret_cast<unsigned long long*>(ra + kRaRestMin);
+  a.from_rest_min = 0;
   const FlagLayout L = flag_layout(a.nx, a.ny, a.pad);
   if (L.fits) {
     unsigned* base = reinterpret_cast<unsigned*>(ra + kRaQFlags);
@@ -570,8 +902,7 @@ void fill_mesh_args(StepArgs<R>& a, const Mesh* mesh, int tt, double* ra) {
     const bool prev_x_first = ((tt - 1) % 2 == 0);
     a.rest_w = prev_x_first ? kCols - 1 : kCols;
     a.rest_tiles_x = prev_x_first ? L.xtiles : L.stride;
-    a.rest_rows = kRowsSweepMoving;
-    a.moving = reinterpret_cast<unsigned long long*>(ra + kRaMoving);
+    a.rest_rows = kMaxRowsStep;
   }
 }
 
@@ -639,23 +970,28 @@ struct RestRecord {
   const void* e = nullptr;
   const void* ra = nullptr;
   int nx = 0, ny = 0, pad = 0, form = -1, tt = 0;
-  int sweep_rows = 0;                    // the step's sweep tile height
-  unsigned long long tiles = 0;          // its first sweep's tiles
-  unsigned long long moving = ~0ull;     // of which not skipped (read after the step)
+  StepRows rows;                         // the step's tile heights
+  unsigned counts[2 * kListHeights] = {};  // the lengths of the tile lists it left
+  bool listed = false;                   // it left tile lists
+  bool dense = false;                    // the last lists held nearly every tile
   unsigned long long calls = 0;
   bool valid = false;
   bool follows = false;                  // it directly followed a flagged step
 };
 thread_local RestRecord t_rest;
 
+constexpr double kDense = 0.8;
+constexpr int kDensePeriod = 8;
+
 // Keeps a.rest only when this step directly follows the recorded one on the
 // same arrays (and no other mesh call came between), then records this step
-// as the one the next may follow (when it runs with flags).  Returns this
-// step's sweep tile height: the shorter where the previous step's first sweep
-// skipped at least half of its tiles.
+// as the one the next may follow (when it runs with flags).  Sets the step's
+// tile heights and lists: the previous step's lists unless they hold nearly
+// every tile (whose order in the grid is then the better one).
 template <typename R>
-int take_rest(StepArgs<R>& a, int tt, int form, const std::array<const void*, 12>& arrays,
-              bool flagged, const void* rho, const void* e, const void* ra) {
+StepRows take_rest(StepArgs<R>& a, int tt, int form, const std::array<const void*, 12>& arrays,
+                   bool flagged, const void* rho, const void* e, double* ra, TileLists& tl,
+                   ListArgs& la) {
   const unsigned long long calls = mesh_calls();
   const RestRecord& p = t_rest;
   const std::array<const void*, 4> mesh{a.edgedx, a.edgedy, a.celldx, a.celldy};
@@ -663,12 +999,68 @@ int take_rest(StepArgs<R>& a, int tt, int form, const std::array<const void*, 12
                        p.calls + 1 == calls && p.form == form && p.nx == a.nx &&
                        p.ny == a.ny && p.pad == a.pad && p.arrays == arrays && p.mesh == mesh;
   if (follows) {
-    a.rest_rows = p.sweep_rows;
+    a.rest_rows = p.rows.sweep;
   } else {
     a.rest = nullptr;
   }
-  const bool still = follows && p.moving != ~0ull && 2 * p.moving <= p.tiles;
-  const int rows = still ? kRowsSweepStill : kRowsSweepMoving;
+  const FlagLayout L = flag_layout(a.nx, a.ny, a.pad);
+  unsigned* base = reinterpret_cast<unsigned*>(ra + kRaQFlags);
+  // The lists the previous step left, and those this step leaves.
+  const size_t list_half = L.list_words[0] + L.list_words[1];
+  const unsigned* lists = base + L.lists + ((tt + 1) & 1) * list_half;
+  unsigned* out_lists = base + L.lists + (tt & 1) * list_half;
+  // (A list entry holds 16 bits for each tile index.)
+  const bool listed = flagged && L.list_bands * (kListBand / 2) < 0x10000 && L.list_tx[1] < 0x10000;
+  bool use = false, dense = follows && p.dense;
+  if (follows && p.listed) {
+    const double all = (double)L.list_tx[0] * L.list_bands + (double)L.list_tx[1] * L.list_bands;
+    use = p.counts[kListHeights - 1] + p.counts[2 * kListHeights - 1] < kDense * all;
+    dense = !use;
+  }
+  const StepRows rows = pick_step_rows(a.nx, a.ny, a.pad, use ? p.counts : nullptr, flagged,
+                                       follows ? &p.rows : nullptr,
+                                       Prec<R>::kMixed ? kOverlapMixed : kOverlap64);
+  // The per-tile CFL minima are those of tiles of the same height.
+  a.cfl_known = follows && p.rows.energy == rows.energy;
+  a.rows = rows.lag;
+  tl.use = use;
+  if (use) {
+    a.from_rest_min = a.cfl_known;
+    for (int w = 0; w < 2; ++w) {
+      for (int h = 0; h < kListHeights; ++h) {
+        tl.list[w][h] = lists + (w ? L.list_words[0] : 0) + list_offset(L.list_tx[w], L.list_bands, h);
+        tl.n[w][h] = (int)p.counts[w * kListHeights + h];
+      }
+    }
+  }
+  // Where the last lists held nearly every tile the next are formed eight
+  // steps later (10 us a step on a 2048^2 field in motion everywhere).
+  const bool build = listed && (!dense || tt % kDensePeriod == 0);
+  if (build) {
+    const bool x_first = (tt % 2 == 0);
+    la.nx = a.nx;
+    la.ny = a.ny;
+    la.pad = a.pad;
+    la.marks = a.skipf;
+    la.mark_w = x_first ? kCols - 1 : kCols;
+    la.mark_tiles_x = x_first ? L.xtiles : L.stride;
+    la.mark_rows = rows.sweep;
+    la.next_marks = base + L.marks + ((tt + 1) & 1) * L.sk_words;
+    la.next_words = (int)L.sk_words;
+    la.bands = L.list_bands;
+    const int tx = L.list_tx[0] > L.list_tx[1] ? L.list_tx[0] : L.list_tx[1];
+    la.blocks = (int)(((long long)tx * L.list_bands * (kListBand / 2) + kCols - 1) / kCols);
+    for (int w = 0; w < 2; ++w) {
+      la.tx[w] = L.list_tx[w];
+      la.list[w] = out_lists + (w ? L.list_words[0] : 0);
+    }
+    la.counts = reinterpret_cast<unsigned*>(ra + kRaTileCounts);
+    la.cfl_tile = a.cfl_tile;
+    la.cfl_tx = L.stride;
+    la.cfl_rows = rows.energy;
+    la.cfl_ty = (a.ny - 2 * a.pad + rows.energy - 1) / rows.energy;
+    la.rest_min = a.rest_min;
+  }
   RestRecord r;
   r.arrays = arrays;
   r.mesh = mesh;
@@ -680,14 +1072,12 @@ int take_rest(StepArgs<R>& a, int tt, int form, const std::array<const void*, 12
   r.pad = a.pad;
   r.form = form;
   r.tt = tt;
-  r.sweep_rows = rows;
-  const bool x_first = (tt % 2 == 0);
-  const unsigned long long tiles_x =
-      x_first ? (unsigned long long)(a.fx_stride / 4) : (unsigned long long)a.qm_stride;
-  r.tiles = tiles_x * (unsigned long long)((a.ny - 2 * a.pad + rows - 1) / rows);
+  r.rows = rows;
   r.calls = calls;
   r.valid = flagged;
   r.follows = follows;
+  r.listed = build;
+  r.dense = dense;
   t_rest = r;
   return rows;
 }
@@ -847,7 +1237,7 @@ bool tile_conservation(int nx, int ny, int pad, const double* rho, const double*
     c.marks = reinterpret_cast<const unsigned char*>(base + L.marks + (p.tt & 1) * L.sk_words);
     c.mark_w = x_first ? kCols - 1 : kCols;
     c.mark_tiles_x = x_first ? L.xtiles : L.stride;
-    c.mark_rows = p.sweep_rows;
+    c.mark_rows = p.rows.sweep;
   }
   cudaMemsetAsync(ra + kRaTicket, 0, sizeof(double), s);
   k_conservation_tiles<<<(unsigned)c.tiles, kCols, 0, s>>>(c);
@@ -930,16 +1320,16 @@ int fused_solve(Mesh* mesh, int tt, double* P, double* rho, double* rho_old,
       lagp = &lag;
     }
   }
-  const int sweep_rows =
+  TileLists tl;
+  ListArgs la{};
+  const StepRows sr =
       take_rest(a, tt, 0, {P, rho, e, rho_u, rho_v, uF_y, vF_x, uF_x, vF_y, F_x, F_y, reduce_array},
-                a.skipf != nullptr && lagp == nullptr, rho, e, reduce_array);
+                a.skipf != nullptr && lagp == nullptr, rho, e, reduce_array, tl, la);
   StepProfiler prof;
   prof.begin(s);
-  launch_step(s, a, tt, first, second, prof, sweep_rows, a.rest != nullptr, lagp);
-  unsigned long long moving = ~0ull;
-  const int st = finish_step(s, mesh, reduce_array, prof, "solve_hydro_2d (fused)", &moving);
+  launch_step(s, a, tt, first, second, prof, sr, a.rest != nullptr, tl, la, lagp);
+  const int st = finish_step(s, mesh, reduce_array, prof, "solve_hydro_2d (fused)", t_rest.counts);
   if (st != GB300_OK) t_rest.valid = false;
-  t_rest.moving = moving;
   return st;
 }
 
@@ -1002,17 +1392,17 @@ int mixed_solve(Mesh* mesh, int tt, double* rho, double* e, float* rho_u,
                                F(L.s_r32), F(L.s_e32)};
   const SweepArgs<float> second{D(L.s_r), D(L.s_e), F(L.s_r32), F(L.s_e32),
                                 rho, e, a.rho_r, a.e_r};
-  const int sweep_rows =
+  TileLists tl;
+  ListArgs la{};
+  const StepRows sr =
       take_rest(a, tt, 1, {rho, e, rho_u, rho_v, work, reduce_array, nullptr, nullptr, nullptr,
                            nullptr, nullptr, nullptr},
-                a.skipf != nullptr, rho, e, reduce_array);
+                a.skipf != nullptr, rho, e, reduce_array, tl, la);
   StepProfiler prof;
   prof.begin(s);
-  launch_step(s, a, tt, first, second, prof, sweep_rows, a.rest != nullptr);
-  unsigned long long moving = ~0ull;
-  const int st = finish_step(s, mesh, reduce_array, prof, "gb300_mixed_solve", &moving);
+  launch_step(s, a, tt, first, second, prof, sr, a.rest != nullptr, tl, la);
+  const int st = finish_step(s, mesh, reduce_array, prof, "gb300_mixed_solve", t_rest.counts);
   if (st != GB300_OK) t_rest.valid = false;
-  t_rest.moving = moving;
   return st;
 }
 

@@ -125,11 +125,33 @@ struct StepArgs {
   const unsigned char* rest;
   int rest_w, rest_tiles_x, rest_rows;
   // Each shock-heating tile's CFL minimum of the last step it ran (FP64 bit
-  // pattern, word by * qm_stride + bx), set with the flags, or null.
+  // pattern, word by * qm_stride + bx), set with the flags, or null;
+  // cfl_known: that step is the one before, with tiles of this height.
   unsigned long long* cfl_tile;
-  // Count of the first sweep's tiles not skipped this step (flags only).
-  unsigned long long* moving;
+  int cfl_known;
+  // The tiles a kernel of the step visits (single-problem kernels): all of its
+  // grid_x x grid_y grid, one per block of a 2-D launch, when tiles is null;
+  // else the first n_tiles entries (by << 16 | bx) of the list that the
+  // previous step left, one per block of a 1-D launch -- the others hold only
+  // cells at rest, where every kernel of the step would leave what its arrays
+  // and flags hold.
+  const unsigned* tiles;
+  int n_tiles, grid_x, grid_y;
+  // The CFL minimum over the shock-heating tiles off the list (kRaRestMin),
+  // and whether the step starts its own minimum from it.
+  unsigned long long* rest_min;
+  int from_rest_min;
 };
+
+// Tile k of the list; false (in the whole block): none.
+template <typename R>
+__device__ __forceinline__ bool listed_tile(const StepArgs<R>& a, int k, int& bx, int& by) {
+  if (k >= a.n_tiles) return false;
+  const unsigned code = a.tiles[k];
+  bx = (int)(code & 0xffffu);
+  by = (int)(code >> 16);
+  return bx < a.grid_x && by < a.grid_y;
+}
 
 // Writes the value of interior point (ii, jj) of a w x h array into each of
 // its ghost mirror images (pad layers per side): column images negated when
@@ -1197,7 +1219,7 @@ __device__ __forceinline__ void tile_lag_energy_dt(const StepArgs<R>& a, int bx,
     // the previous step: it keeps every energy, has no viscous stress, and
     // its cells' CFL candidates are those of the previous step, from the
     // same densities and energies -- its minimum then stands.
-    if (a.rest && a.cfl_tile) {
+    if (a.rest && a.cfl_tile && a.cfl_known) {
       const int nx = a.nx, ny = a.ny, pad = a.pad;
       const int cb = pad + bx * kCols, i0 = pad + by * a.rows;
       const int i1 = min(i0 + a.rows, ny - pad);
@@ -1739,10 +1761,7 @@ __device__ __forceinline__ void tile_mass_sweep_x(const StepArgs<R>& a, const Sw
       if (sk && !rest_cells(a, i0, i1, cb, min(cb + kCols - 1, a.nx - pad))) {
         sk = block_round_trip_exact(s.r_in, s.e_in, a.nx, i0, i1, jj, cell_ok);
       }
-      if (t == 0) {
-        store_flag(s.skip + (size_t)by * s.skip_tiles_x + bx, sk);
-        if (!sk && a.moving) atomicAdd(a.moving, 1ull);
-      }
+      if (t == 0) store_flag(s.skip + (size_t)by * s.skip_tiles_x + bx, sk);
       if (sk) {
         zero_flags();
         return;
@@ -2079,10 +2098,7 @@ __device__ __forceinline__ void tile_mass_sweep_y(const StepArgs<R>& a, const Sw
       if (sk && !rest_cells(a, i0, i1, cb, min(cb + kCols, a.nx - pad))) {
         sk = block_round_trip_exact(s.r_in, s.e_in, a.nx, i0, i1, jj, col_ok);
       }
-      if (threadIdx.x == 0) {
-        store_flag(s.skip + (size_t)by * s.skip_tiles_x + bx, sk);
-        if (!sk && a.moving) atomicAdd(a.moving, 1ull);
-      }
+      if (threadIdx.x == 0) store_flag(s.skip + (size_t)by * s.skip_tiles_x + bx, sk);
       if (sk) {
         zero_flags();
         return;
