@@ -356,20 +356,12 @@ __global__ void k_batch_finish_dt(const BatchDev<R> b, int first_step) {
   }
 }
 
-// Whether every spacing of an instance's mesh is a positive normal power of
-// two, one block per instance, into the flag its tiles read (mesh_pow2).
+// The mesh test of every instance, one block each (StepArgs::mesh).
 template <typename R>
-__global__ void __launch_bounds__(256) k_batch_mesh_pow2(const BatchDev<R> b) {
+__global__ void __launch_bounds__(256) k_batch_mesh_test(const BatchDev<R> b) {
   const StepArgs<R>& a = b.inst[blockIdx.x].a;
-  bool ok = true;
-  for (int j = threadIdx.x; j <= a.nx; j += blockDim.x) {
-    ok = ok && d_is_pow2(a.celldx[j]) && d_is_pow2(a.edgedx[j]);
-  }
-  for (int j = threadIdx.x; j <= a.ny; j += blockDim.x) {
-    ok = ok && d_is_pow2(a.celldy[j]) && d_is_pow2(a.edgedy[j]);
-  }
-  ok = __syncthreads_and(ok) != 0;
-  if (threadIdx.x == 0) *const_cast<unsigned long long*>(a.mesh_pow2) = ok ? 1ull : 0ull;
+  mesh_test_block(a.nx, a.ny, a.celldx, a.edgedx, a.celldy, a.edgedy,
+                  const_cast<double*>(a.mesh));
 }
 
 }  // namespace
@@ -486,7 +478,7 @@ Instance<R> make_instance(const BatchImpl& B, int i) {
   a.uF_x = Rp(L.uF_x); a.uF_y = Rp(L.uF_y); a.vF_x = Rp(L.vF_x); a.vF_y = Rp(L.vF_y);
   a.ra = D(L.ra);
   a.min_slot = reinterpret_cast<unsigned long long*>(D(L.ra) + kRaMinSlot);
-  a.mesh_pow2 = reinterpret_cast<const unsigned long long*>(D(L.ra) + kRaMeshPow2);
+  a.mesh = D(L.ra) + kRaMesh;
   a.dt_slot = D(L.ra) + kRaDt;
   a.max_dt = 10.0;
   a.rows = B.rows;
@@ -618,7 +610,7 @@ int launch_batch_phases(BatchImpl& B, cudaStream_t s, int tt) {
 // not change during the steps of a call).
 template <typename R>
 int launch_batch_mesh_test(BatchImpl& B, cudaStream_t s) {
-  k_batch_mesh_pow2<R><<<(unsigned)B.n, 256, 0, s>>>(batch_dev<R>(B));
+  k_batch_mesh_test<R><<<(unsigned)B.n, 256, 0, s>>>(batch_dev<R>(B));
   count_launches(1);
   return check_launch("gb300_batch_step: mesh test");
 }

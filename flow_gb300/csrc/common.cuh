@@ -30,13 +30,14 @@ constexpr double kCT = 0.3;
 //   [6] CFL minimum           running minimum of the fused step's CFL
 //                             candidates (uint64 bits of a non-negative
 //                             double: bit order = value order)
-//   [7] mesh power-of-two     1 when every mesh spacing is a power of two
-//                             (formed on the device at the start of a step)
-//   [8] minimum at rest       the CFL minimum over the shock-heating tiles
+//   [7] mesh uniform          1 (uint64) when the mesh is uniform, formed on
+//                             the device at the start of a run, with the
+//   [8 .. 11] spacings        dx, dy, 1/dx, 1/dy of a uniform mesh
+//   [12] minimum at rest      the CFL minimum over the shock-heating tiles
 //                             the next step need not visit (as [6])
-//   [9 .. 12] tile counts     lengths of the next step's tile lists (uint32,
+//   [13 .. 16] tile counts    lengths of the next step's tile lists (uint32,
 //                             128- and 127-column tiles of 2, 4, 8, 16 rows)
-//   [13 ...]                  per-block partials (2 doubles per block, at
+//   [17 ...]                  per-block partials (2 doubles per block, at
 //                             most kMaxReduceBlocks blocks)
 //   [kRaQFlags ...]           the fused step's tile flags, when the array
 //                             is large enough to hold them: per-tile CFL
@@ -52,10 +53,10 @@ enum : int {
   kRaEnergy = 4,
   kRaStatus = 5,
   kRaMinBits = 6,
-  kRaMeshPow2 = 7,
-  kRaRestMin = 8,
-  kRaTileCounts = 9,
-  kRaPartial = 13,
+  kRaMesh = 7,
+  kRaRestMin = 12,
+  kRaTileCounts = 13,
+  kRaPartial = 17,
 };
 constexpr int kMaxReduceBlocks = 1024;
 constexpr int kRaQFlags = kRaPartial + 2 * kMaxReduceBlocks;

@@ -27,35 +27,20 @@ __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" :::);
 }
 
-// Whether every mesh spacing (celldx, edgedx: 0 .. nx; celldy, edgedy: 0 ..
-// ny) is a positive normal power of two: one block, the first kernel of the
-// step.  The tiles then skip their own spacing tests (block_mesh_pow2).
-constexpr int kPow2Threads = 1024;
-// It also clears the CFL minimum slot and the block ticket for the step's
+// The mesh test (mesh_test_block): one block, the first kernel of a run.  It
+// also clears the CFL minimum slot and the block ticket for the step's
 // Lagrangian kernels.
-__global__ void __launch_bounds__(kPow2Threads)
-    k_mesh_pow2(int nx, int ny, const double* celldx, const double* edgedx,
-                const double* celldy, const double* edgedy, unsigned long long* flag,
-                double* ra) {
+constexpr int kMeshThreads = 1024;
+__global__ void __launch_bounds__(kMeshThreads)
+    k_mesh_test(int nx, int ny, const double* celldx, const double* edgedx, const double* celldy,
+                const double* edgedy, double* ra) {
   pdl_wait();
   pdl_trigger();
   if (threadIdx.x == 0) {
     *reinterpret_cast<unsigned long long*>(ra + kRaTicket) = 0ull;
     *reinterpret_cast<unsigned long long*>(ra + kRaMinBits) = ~0ull;
   }
-  // Every test is made (no short circuit), so that a thread's loads are
-  // independent and in flight together.
-  bool ok = true;
-#pragma unroll 4
-  for (int j = threadIdx.x; j <= nx; j += kPow2Threads) {
-    ok &= d_is_pow2(celldx[j]) & d_is_pow2(edgedx[j]);
-  }
-#pragma unroll 4
-  for (int i = threadIdx.x; i <= ny; i += kPow2Threads) {
-    ok &= d_is_pow2(celldy[i]) & d_is_pow2(edgedy[i]);
-  }
-  ok = __syncthreads_and(ok) != 0;
-  if (threadIdx.x == 0) *flag = ok ? 1ull : 0ull;
+  mesh_test_block(nx, ny, celldx, edgedx, celldy, edgedy, ra + kRaMesh);
 }
 
 // How a kernel of the step runs: without flags (a mesh too small for them),
@@ -356,8 +341,8 @@ __global__ void __launch_bounds__(lagf::kT, 4) k_lag_fused(const lagf::LagArgs a
   pdl_wait();
   pdl_trigger();
   lagf::CflBest cfl;
-  const lagf::TileGeom g = lagf::tile_geom(a, blockIdx.x, blockIdx.y);
-  const bool ok = lagf::tile_pow2(a, g)
+  const bool uniform = mesh_uniform(a.mesh);
+  const bool ok = uniform
                       ? lagf::lag_tile<true>(a, sm, blockIdx.x, blockIdx.y, cfl)
                       : lagf::lag_tile<false>(a, sm, blockIdx.x, blockIdx.y, cfl);
   if (!ok) {
@@ -369,6 +354,10 @@ __global__ void __launch_bounds__(lagf::kT, 4) k_lag_fused(const lagf::LagArgs a
   }
   unsigned long long best = ~0ull;
   if (cfl.kbest >= 0) best = (unsigned long long)dbits(cfl.c_best * d_rsqrt(cfl.s_best));
+  if (uniform) {
+    const UniformMesh um = uniform_mesh(a.mesh);
+    best = cfl.max.candidate(um.dx, um.dy);
+  }
   best = warp_min_u64(best);
   if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = best;
   __syncthreads();
@@ -689,9 +678,9 @@ void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
   // The whole-mesh spacing test the tiles read (one block, a few
   // microseconds), formed unless the previous step's still stands.
   if (!mesh_known) {
-    prof.mark("mesh_pow2");
-    launch_pdl_block(k_mesh_pow2, dim3(1), dim3(kPow2Threads), s, nx, ny, a.celldx, a.edgedx,
-                     a.celldy, a.edgedy, const_cast<unsigned long long*>(a.mesh_pow2), a.ra);
+    prof.mark("mesh_test");
+    launch_pdl_block(k_mesh_test, dim3(1), dim3(kMeshThreads), s, nx, ny, a.celldx, a.edgedx,
+                     a.celldy, a.edgedy, a.ra);
   }
   if (lag) {
     const int nty = (ny - 2 * pad + lag->rows - 1) / lag->rows;
@@ -775,7 +764,7 @@ int finish_step(cudaStream_t s, Mesh* mesh, double* ra, StepProfiler& prof,
     if (st != GB300_OK) return st;
   }
   // dt, dt_h (slots 0, 1), the status word (slot 5) and the lengths of the
-  // tile lists (slots 9 .. 12) in one copy.
+  // tile lists (slots 13 .. 16) in one copy.
   double head[kRaPartial];
   cudaMemcpyAsync(head, ra + kRaDt, sizeof(head), cudaMemcpyDeviceToHost, s);
   const cudaError_t err = cudaStreamSynchronize(s);
@@ -860,7 +849,7 @@ void fill_mesh_args(StepArgs<R>& a, const Mesh* mesh, int tt, double* ra) {
   a.celldy = mesh->celldy;
   a.ra = ra;
   a.min_slot = reinterpret_cast<unsigned long long*>(ra + kRaMinBits);
-  a.mesh_pow2 = reinterpret_cast<unsigned long long*>(ra + kRaMeshPow2);
+  a.mesh = ra + kRaMesh;
   a.dt_slot = ra + kRaDt;
   a.dt = mesh->dt;
   a.dt_h = mesh->dt_h;
@@ -1313,7 +1302,7 @@ int fused_solve(Mesh* mesh, int tt, double* P, double* rho, double* rho_old,
       lag.masks = reinterpret_cast<unsigned*>(rho_old);
       lag.ra = reduce_array;
       lag.min_slot = a.min_slot;
-      lag.mesh_pow2 = a.mesh_pow2;
+      lag.mesh = a.mesh;
       lag.dt_slot = a.dt_slot;
       lag.dt = a.dt; lag.dt_h = a.dt_h; lag.max_dt = a.max_dt;
       lag.first_step = a.first_step;

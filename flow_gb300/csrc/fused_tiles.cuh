@@ -75,9 +75,11 @@ struct StepArgs {
   R* vF_y;
   double* ra;                  // caller scratch (reduce_array)
   unsigned long long* min_slot;  // running CFL minimum (FP64 bit pattern)
-  // 1 when every mesh spacing is a positive normal power of two (formed on
-  // the device at the start of the step); null or 0: tested per tile.
-  const unsigned long long* mesh_pow2;
+  // The mesh test's result (formed on the device at the start of a run): [0]
+  // 1 (uint64) when the mesh is uniform -- every celldx and edgedx one number,
+  // every celldy and edgedy one number -- then [1], [2] the two spacings and
+  // [3], [4] their reciprocals.
+  const double* mesh;
   double* dt_slot;             // [0] dt, [1] dt_h for the advection phase
   double dt, dt_h, max_dt;     // Lagrangian-phase pair (host values), max_dt
   int first_step;
@@ -368,73 +370,102 @@ __device__ __forceinline__ bool tile_near_edge(int nx, int ny, int pad, int col0
            row0 + rows + 2 <= ny - 2 * pad);
 }
 
-// True when every mesh spacing (celldx, edgedx, celldy, edgedy) within two
-// entries of the block's columns [col0, col0 + kCols) and rows
-// [row0, row0 + rows) is a power of two -- the uniform power-of-two meshes of
-// the benchmark problems -- so that divisions by those spacings are exact as
-// multiplications by their reciprocals.  Block-uniform (barrier).
-template <typename R>
-__device__ __forceinline__ bool block_mesh_pow2(const StepArgs<R>& a, int col0, int row0) {
-  // The whole mesh (one cached word) before the tile's own spacings.
-  if (a.mesh_pow2 && *a.mesh_pow2 == 1ull) return true;
-  bool ok = true;
-  for (int j = col0 - 2 + (int)threadIdx.x; j < col0 + kCols + 2; j += kCols) {
-    if (j >= 0 && j <= a.nx) ok = ok && d_is_pow2(a.celldx[j]) && d_is_pow2(a.edgedx[j]);
-  }
-  for (int i = row0 - 2 + (int)threadIdx.x; i < row0 + a.rows + 2; i += kCols) {
-    if (i >= 0 && i <= a.ny) ok = ok && d_is_pow2(a.celldy[i]) && d_is_pow2(a.edgedy[i]);
-  }
-  return __syncthreads_and(ok) != 0;
+// A uniform mesh's spacings and their reciprocals (StepArgs::mesh).
+struct UniformMesh {
+  double dx, dy, ix, iy;
+};
+__device__ __forceinline__ bool mesh_uniform(const double* mesh) {
+  return *reinterpret_cast<const unsigned long long*>(mesh) == 1ull;
+}
+__device__ __forceinline__ UniformMesh uniform_mesh(const double* mesh) {
+  return UniformMesh{mesh[1], mesh[2], mesh[3], mesh[4]};
 }
 
-// Runs tile(kPow2) with kPow2 = true for FP64 tiles whose mesh spacings are
-// all powers of two.  (The mixed form's FP32 arithmetic gains nothing from
-// it; its mass sweeps, whose FP64 conservative update multiplies by the face
-// lengths, dispatch with FLOW_POW2_DISPATCH_ALL.)
-#define FLOW_POW2_DISPATCH(R, a, col0, row0, CALL_TRUE, CALL_FALSE)          \
-  do {                                                                      \
-    if constexpr (!Prec<R>::kMixed) {                                       \
-      if (block_mesh_pow2(a, col0, row0)) {                                 \
-        CALL_TRUE;                                                          \
-        return;                                                             \
-      }                                                                     \
-    }                                                                       \
-    CALL_FALSE;                                                             \
+// The mesh test, by one block (barrier): whether every celldx and edgedx
+// (entries 0 .. nx) is one positive normal number with a normal reciprocal,
+// and every celldy and edgedy (0 .. ny) likewise, written to mesh with the
+// spacings.  Every test is made (no short circuit), so that a thread's loads
+// are independent and in flight together.
+__device__ __forceinline__ void mesh_test_block(int nx, int ny, const double* celldx,
+                                                const double* edgedx, const double* celldy,
+                                                const double* edgedy, double* mesh) {
+  const double dx = celldx[0], dy = celldy[0];
+  const long long bx = dbits(dx), by = dbits(dy);
+  // (Exponents from 2^-1000 to 2^1000: the reciprocals are normal too.)
+  auto fine = [](long long b) {
+    return b > 0 && (b >> 52) - 23 >= 0 && (b >> 52) - 23 <= 2000;
+  };
+  bool ok = fine(bx) & fine(by);
+#pragma unroll 4
+  for (int j = threadIdx.x; j <= nx; j += blockDim.x) {
+    ok &= (dbits(celldx[j]) == bx) & (dbits(edgedx[j]) == bx);
+  }
+#pragma unroll 4
+  for (int i = threadIdx.x; i <= ny; i += blockDim.x) {
+    ok &= (dbits(celldy[i]) == by) & (dbits(edgedy[i]) == by);
+  }
+  ok = __syncthreads_and(ok) != 0;
+  if (threadIdx.x == 0) {
+    *reinterpret_cast<unsigned long long*>(mesh) = ok ? 1ull : 0ull;
+    mesh[1] = dx;
+    mesh[2] = dy;
+    mesh[3] = 1.0 / dx;
+    mesh[4] = 1.0 / dy;
+  }
+}
+
+// Runs the tile of a uniform mesh where the mesh is one (FP64 form; the mixed
+// form's FP32 arithmetic gains nothing from it, but for its mass sweeps, whose
+// FP64 conservative update does: FLOW_UNIFORM_DISPATCH_ALL).  On a uniform
+// mesh the FP64 form folds the spacings into the timestep once per tile --
+//   m - dt d / h as fma(-(dt / h), d, m), h -+ w dt_h times 1/h as
+//   fma(-+w, dt_h / h, 1), the face lengths and half widths of the fluxes into
+//   their updates' coefficients, a face density as half the sum --
+// so a momentum update is one FP64 instruction besides its difference where
+// the general tile takes four (a quotient corrected to the reference's
+// rounding), and a tile reads no spacing arrays.  Each folded product is
+// rounded once per step instead of once per cell.
+#define FLOW_UNIFORM_DISPATCH(R, a, CALL_TRUE, CALL_FALSE) \
+  do {                                                     \
+    if constexpr (!Prec<R>::kMixed) {                      \
+      if (mesh_uniform(a.mesh)) {                          \
+        CALL_TRUE;                                         \
+        return;                                            \
+      }                                                    \
+    }                                                      \
+    CALL_FALSE;                                            \
   } while (0)
-#define FLOW_POW2_DISPATCH_ALL(a, col0, row0, CALL_TRUE, CALL_FALSE)         \
-  do {                                                                      \
-    if (block_mesh_pow2(a, col0, row0)) {                                   \
-      CALL_TRUE;                                                            \
-      return;                                                               \
-    }                                                                       \
-    CALL_FALSE;                                                             \
+#define FLOW_UNIFORM_DISPATCH_ALL(a, CALL_TRUE, CALL_FALSE) \
+  do {                                                      \
+    if (mesh_uniform(a.mesh)) {                             \
+      CALL_TRUE;                                            \
+      return;                                               \
+    }                                                       \
+    CALL_FALSE;                                             \
   } while (0)
 
 // Spacing factors of a tile (mesh spacings, their reciprocals and ratios),
-// formed once per tile from the FP64 mesh arrays:
-//   FP64 form on a power-of-two tile (kP2): exact exponent arithmetic on the
-//     integer pipes (d_pow2_*), the same numbers as the IEEE expressions;
-//   FP64 form otherwise: the IEEE expressions 1/h, c/(2e), 1/(h*h);
-//   mixed form: FP32 arithmetic (IEEE division) on the spacings rounded to
-//     FP32 on the integer pipes -- an FP64->FP32 conversion instruction, like
-//     an FP64 division, occupies the FP64 pipe, and per tile these cost more
-//     than the arithmetic of a still cell.
+// formed once per tile from the FP64 mesh arrays: in the FP64 form the IEEE
+// expressions 1/h, c/(2e), 1/(h*h); in the mixed form FP32 arithmetic (IEEE
+// division) on the spacings rounded to FP32 on the integer pipes -- an
+// FP64->FP32 conversion instruction, like an FP64 division, occupies the FP64
+// pipe, and per tile these cost more than the arithmetic of a still cell.
 template <typename R>
 __device__ __forceinline__ R geo_v(double h) { return Prec<R>::from_d(h); }
-template <typename R, bool kP2>
+template <typename R>
 __device__ __forceinline__ R geo_rcp(double h) {
   if constexpr (Prec<R>::kMixed) {
     return __frcp_rn(f64_to_f32(h));
   } else {
-    return kP2 ? d_pow2_rcp(h) : 1.0 / h;
+    return 1.0 / h;
   }
 }
-template <typename R, bool kP2>
+template <typename R>
 __device__ __forceinline__ R geo_half_ratio(double c, double e) {
   if constexpr (Prec<R>::kMixed) {
     return __fdiv_rn(f64_to_f32(c), 2.0f * f64_to_f32(e));
   } else {
-    return kP2 ? d_pow2_half_ratio(c, e) : c / (2.0 * e);
+    return c / (2.0 * e);
   }
 }
 // h/2 in bulk precision (exact).
@@ -443,18 +474,13 @@ __device__ __forceinline__ R geo_half(double h) { return Prec<R>::from_d(d_half(
 // FP64 1/h for the coefficients of the FP64 conservative update: as geo_rcp
 // in the FP64 form; the MUFU reciprocal with two Newton steps in the mixed
 // form (whose fluxes are FP32).
-template <typename R, bool kP2>
+template <typename R>
 __device__ __forceinline__ double geo_rcp_d(double h) {
   if constexpr (Prec<R>::kMixed) {
-    return kP2 ? d_pow2_rcp(h) : d_rcp(h);
+    return d_rcp(h);
   } else {
-    return kP2 ? d_pow2_rcp(h) : 1.0 / h;
+    return 1.0 / h;
   }
-}
-// 1/(h*h), FP64 form only (CFL keys).
-template <bool kP2>
-__device__ __forceinline__ double geo_rcp_sq(double h) {
-  return kP2 ? d_pow2_rcp_sq(h) : 1.0 / (h * h);
 }
 
 // The FP64 quotient as a called function: a branch around five inline FP64
@@ -477,15 +503,25 @@ __device__ __forceinline__ R face_velocity(R mom, R rbar) {
 }
 
 // Volume-weighted face value a*wa + b*wb, rounded once after the product
-// b*wb (the reference's a*wa + b*wb contracted as in the fused kernels).  On
-// power-of-two meshes both weights are powers of two, both products exact
-// exponent adds, and the single rounding is that of the sum.
-template <typename R, bool kP2>
+// b*wb (the reference's a*wa + b*wb contracted as in the fused kernels).  On a
+// uniform mesh both weights are 1/2 and the rounding is that of the sum.
+template <typename R, bool kU>
 __device__ __forceinline__ R face_average(R a, R wa, R b, R wb) {
-  if constexpr (kP2 && !Prec<R>::kMixed) {
-    return Prec<R>::template mulp<true>(a, wa) + Prec<R>::template mulp<true>(b, wb);
+  if constexpr (kU) {
+    return Prec<R>::half(a + b);
   } else {
     return fma(a, wa, b * wb);
+  }
+}
+
+// A face momentum less dt * diff / h (inv_h = 1/h); on a uniform mesh k is
+// dt / h.
+template <typename R, bool kU>
+__device__ __forceinline__ R momentum_step(R m, R diff, R k, R dt, R h, R inv_h) {
+  if constexpr (kU) {
+    return fma(-k, diff, m);
+  } else {
+    return Prec<R>::dsub(m, dt * diff, h, inv_h);
   }
 }
 
@@ -497,7 +533,7 @@ __device__ __forceinline__ R face_average(R a, R wa, R b, R wb) {
 // shock-heating kernel reads it where a cell is compressed) and every interior
 // x/y face.  The reference's rho_old copy is not made: the first mass sweep
 // reads the density itself.  omp3/flow.c:55-70, 110-158.
-template <typename R, bool kP2, bool kFl>
+template <typename R, bool kU, bool kFl>
 __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int bx, int by) {
   using Pr = Prec<R>;
   __shared__ R sP[kCols + 1], sR[kCols + 1];
@@ -508,23 +544,29 @@ __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int
   const int i0 = by * a.rows;
   const bool edge = tile_near_edge(nx, ny, pad, bx * kCols, i0, a.rows);
   const R g1 = R(kG1);
-  if (t < a.rows) {
-    const int ii = i0 + t;
-    if (ii >= 1 && ii < ny) {
-      const double ey = a.edgedy[ii];
-      s_ey[t] = geo_v<R>(ey);
-      s_iey[t] = geo_rcp<R, kP2>(ey);
-      s_wy0[t] = geo_half_ratio<R, kP2>(a.celldy[ii], ey);
-      s_wy1[t] = geo_half_ratio<R, kP2>(a.celldy[ii - 1], ey);
+  R exr = R(0), iex = R(0), wx0 = R(0), wx1 = R(0), kx = R(0), ky = R(0);
+  if constexpr (kU) {
+    const UniformMesh um = uniform_mesh(a.mesh);
+    kx = a.dt * um.ix;
+    ky = a.dt * um.iy;
+  } else {
+    if (t < a.rows) {
+      const int ii = i0 + t;
+      if (ii >= 1 && ii < ny) {
+        const double ey = a.edgedy[ii];
+        s_ey[t] = geo_v<R>(ey);
+        s_iey[t] = geo_rcp<R>(ey);
+        s_wy0[t] = geo_half_ratio<R>(a.celldy[ii], ey);
+        s_wy1[t] = geo_half_ratio<R>(a.celldy[ii - 1], ey);
+      }
     }
-  }
-  R exr = R(0), iex = R(0), wx0 = R(0), wx1 = R(0);
-  if (jj >= 1 && jj < nx) {
-    const double ex = a.edgedx[jj];
-    exr = geo_v<R>(ex);
-    iex = geo_rcp<R, kP2>(ex);
-    wx0 = geo_half_ratio<R, kP2>(a.celldx[jj], ex);
-    wx1 = geo_half_ratio<R, kP2>(a.celldx[jj - 1], ex);
+    if (jj >= 1 && jj < nx) {
+      const double ex = a.edgedx[jj];
+      exr = geo_v<R>(ex);
+      iex = geo_rcp<R>(ex);
+      wx0 = geo_half_ratio<R>(a.celldx[jj], ex);
+      wx1 = geo_half_ratio<R>(a.celldx[jj - 1], ex);
+    }
   }
   const R dt = Pr::from_d(a.dt);
   R P_dn = R(0), r_dn = R(0);  // cell (ii-1, jj)
@@ -533,7 +575,7 @@ __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int
     r_dn = a.rho_r[c];
     P_dn = g1 * r_dn * a.e_r[c];
   }
-  __syncthreads();
+  if (!kU) __syncthreads();
   // Row ii+1's densities, energies and face momenta are loaded before row ii
   // is processed (its stores do not touch them).
   const bool u_col = jj >= pad && jj < nx + 1 - pad;
@@ -584,21 +626,19 @@ __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int
       R mom = mu_l;
       R rbar;
       bool dmom = false;  // the momentum changes (kFl: flagged as moving)
-      // FP64 form, power-of-two tile: a warp whose faces all have equal
-      // pressures, densities and weights either side keeps its momenta
-      // (dp = +0) and has the face density 2 (rc wx0) exactly, without FP64
-      // instructions.
-      if (kP2 && !Pr::kMixed &&
-          warp_all(lane_same(Pc, Pl) && lane_same(rc, rl) && lane_same(wx0, wx1))) {
-        rbar = Pr::twice(Pr::template mulp<true>(rc, wx0));
+      // FP64 form, uniform mesh: a warp whose faces all have equal pressures
+      // and densities either side keeps its momenta (dp = +0) and has that
+      // face density, without FP64 instructions.
+      if (kU && warp_all(lane_same(Pc, Pl) && lane_same(rc, rl))) {
+        rbar = rc;
       } else {
         const R dp = Pc - Pl;
         if (!Pr::zero_skip_mem(dp)) {
-          mom = Pr::template dsub<kP2>(mom, dt * dp, exr, iex);
+          mom = momentum_step<R, kU>(mom, dp, kx, dt, exr, iex);
           a.rho_u[f] = mom;
         }
         dmom = !Pr::is_zero(dp);
-        rbar = face_average<R, kP2>(rc, wx0, rl, wx1);
+        rbar = face_average<R, kU>(rc, wx0, rl, wx1);
       }
       const R vel = face_velocity(mom, rbar);
       a.u[f] = vel;
@@ -610,17 +650,17 @@ __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int
       R mom = mv_l;
       R rbar;
       bool dmom = false;
-      if (kP2 && !Pr::kMixed &&
-          warp_all(lane_same(Pc, P_dn) && lane_same(rc, r_dn) && lane_same(s_wy0[k], s_wy1[k]))) {
-        rbar = Pr::twice(Pr::template mulp<true>(rc, s_wy0[k]));
+      const R wy0 = kU ? R(0) : s_wy0[k], wy1 = kU ? R(0) : s_wy1[k];
+      if (kU && warp_all(lane_same(Pc, P_dn) && lane_same(rc, r_dn))) {
+        rbar = rc;
       } else {
         const R dp = Pc - P_dn;
         if (!Pr::zero_skip_mem(dp)) {
-          mom = Pr::template dsub<kP2>(mom, dt * dp, s_ey[k], s_iey[k]);
+          mom = momentum_step<R, kU>(mom, dp, ky, dt, kU ? R(0) : s_ey[k], kU ? R(0) : s_iey[k]);
           a.rho_v[c] = mom;
         }
         dmom = !Pr::is_zero(dp);
-        rbar = face_average<R, kP2>(rc, s_wy0[k], r_dn, s_wy1[k]);
+        rbar = face_average<R, kU>(rc, wy0, r_dn, wy1);
       }
       const R vel = face_velocity(mom, rbar);
       a.v[c] = vel;
@@ -649,9 +689,8 @@ __device__ __forceinline__ void tile_lag_pressure(const StepArgs<R>& a, int bx, 
     const int c0 = bx * kCols, i0 = by * a.rows;
     if (a.rest && rest_cells(a, i0 - 1, i0 + a.rows, c0 - 1, c0 + kCols)) return;
   }
-  FLOW_POW2_DISPATCH(R, a, bx * kCols, by * a.rows,
-                     (tile_lag_pressure_impl<R, true, kFl>(a, bx, by)),
-                     (tile_lag_pressure_impl<R, false, kFl>(a, bx, by)));
+  FLOW_UNIFORM_DISPATCH(R, a, (tile_lag_pressure_impl<R, true, kFl>(a, bx, by)),
+                        (tile_lag_pressure_impl<R, false, kFl>(a, bx, by)));
 }
 
 // Artificial viscous stresses on interior cells, omp3/flow.c:173-207.
@@ -784,7 +823,7 @@ __device__ __forceinline__ void tile_lag_viscosity(const StepArgs<R>& a, int bx,
 // the persistent batched kernel, whose register budget is spent across all
 // its phases).  With stress flags, a tile none of whose stresses can be
 // non-zero returns at once, and a stress flagged +0 is not loaded.
-template <typename R, bool kP2, bool kEarly, bool kFlags>
+template <typename R, bool kU, bool kEarly, bool kFlags>
 __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a, int bx, int by) {
   using Pr = Prec<R>;
   __shared__ R s_cy[kMaxRows], s_icy[kMaxRows], s_wy0[kMaxRows], s_wy1[kMaxRows];
@@ -795,13 +834,13 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
   const int jj = pad + bx * kCols + threadIdx.x;
   const int i0 = pad + by * a.rows;
   const bool edge = tile_near_edge(nx, ny, pad, pad + bx * kCols, i0, a.rows);
-  if (threadIdx.x < a.rows) {
+  if (!kU && threadIdx.x < a.rows) {
     const int ii = i0 + threadIdx.x;
     if (ii < ny) {
       s_cy[threadIdx.x] = geo_v<R>(a.celldy[ii]);
-      s_icy[threadIdx.x] = geo_rcp<R, kP2>(a.celldy[ii]);
-      s_wy0[threadIdx.x] = geo_half_ratio<R, kP2>(a.celldy[ii], a.edgedy[ii]);
-      s_wy1[threadIdx.x] = geo_half_ratio<R, kP2>(a.celldy[ii - 1], a.edgedy[ii]);
+      s_icy[threadIdx.x] = geo_rcp<R>(a.celldy[ii]);
+      s_wy0[threadIdx.x] = geo_half_ratio<R>(a.celldy[ii], a.edgedy[ii]);
+      s_wy1[threadIdx.x] = geo_half_ratio<R>(a.celldy[ii - 1], a.edgedy[ii]);
     }
   }
   const bool col_ok = jj < nx + 1 - pad;
@@ -857,14 +896,21 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
   // No stress gradient anywhere in the tile: momenta and velocities stand.
   if (!any_q || !col_ok) return;
   if (kEarly) prime();
-  const R cx = geo_v<R>(a.celldx[jj]);
-  const R icx = geo_rcp<R, kP2>(a.celldx[jj]);
   // Face-density weights (the pressure phase's): where a stress gradient
   // changes a face's momentum, the face density is formed again from the two
   // cell densities -- the same expression on the same values, so the same
   // number -- rather than stored for every face by the pressure phase.
-  const R wx0 = geo_half_ratio<R, kP2>(a.celldx[jj], a.edgedx[jj]);
-  const R wx1 = geo_half_ratio<R, kP2>(a.celldx[jj - 1], a.edgedx[jj]);
+  R cx = R(0), icx = R(0), wx0 = R(0), wx1 = R(0), kx = R(0), ky = R(0);
+  if constexpr (kU) {
+    const UniformMesh um = uniform_mesh(a.mesh);
+    kx = a.dt * um.ix;
+    ky = a.dt * um.iy;
+  } else {
+    cx = geo_v<R>(a.celldx[jj]);
+    icx = geo_rcp<R>(a.celldx[jj]);
+    wx0 = geo_half_ratio<R>(a.celldx[jj], a.edgedx[jj]);
+    wx1 = geo_half_ratio<R>(a.celldx[jj - 1], a.edgedx[jj]);
+  }
   const R dt = Pr::from_d(a.dt);
   if (!kEarly) prime();
   auto row = [&](int ii, R q1, R q0, R qy) {
@@ -876,10 +922,10 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
       if (!warp_same(q1, q0)) {  // equal stresses in the whole warp: dqx = +0
         const R dqx = q1 - q0;
         if (!Pr::zero_skip_mem(dqx)) {
-          const R mom = Pr::template dsub<kP2>(a.rho_u[f], dt * dqx, cx, icx);
+          const R mom = momentum_step<R, kU>(a.rho_u[f], dqx, kx, dt, cx, icx);
           const size_t c = cidx(nx, ii, jj);
           const R vel =
-              face_velocity(mom, face_average<R, kP2>(a.rho_r[c], wx0, a.rho_r[c - 1], wx1));
+              face_velocity(mom, face_average<R, kU>(a.rho_r[c], wx0, a.rho_r[c - 1], wx1));
           a.rho_u[f] = mom;
           a.u[f] = vel;
           mirror(edge, a.u, nx + 1, ny, pad, ii, jj, vel, true, false);
@@ -892,9 +938,11 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
       if (!warp_same(qy, qy_dn)) {
         const R dqy = qy - qy_dn;
         if (!Pr::zero_skip_mem(dqy)) {
-          const R mom = Pr::template dsub<kP2>(a.rho_v[c], dt * dqy, s_cy[k], s_icy[k]);
+          const R mom = momentum_step<R, kU>(a.rho_v[c], dqy, ky, dt, kU ? R(0) : s_cy[k],
+                                             kU ? R(0) : s_icy[k]);
           const R vel = face_velocity(
-              mom, face_average<R, kP2>(a.rho_r[c], s_wy0[k], a.rho_r[c - nx], s_wy1[k]));
+              mom, face_average<R, kU>(a.rho_r[c], kU ? R(0) : s_wy0[k], a.rho_r[c - nx],
+                                       kU ? R(0) : s_wy1[k]));
           a.rho_v[c] = mom;
           a.v[c] = vel;
           mirror(edge, a.v, nx, ny + 1, pad, ii, jj, vel, false, true);
@@ -948,9 +996,8 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
 
 template <typename R, bool kEarly = true, bool kFlags = false>
 __device__ __forceinline__ void tile_lag_viscous_accel(const StepArgs<R>& a, int bx, int by) {
-  FLOW_POW2_DISPATCH(R, a, a.pad + bx * kCols, a.pad + by * a.rows,
-                     (tile_lag_viscous_accel_impl<R, true, kEarly, kFlags>(a, bx, by)),
-                     (tile_lag_viscous_accel_impl<R, false, kEarly, kFlags>(a, bx, by)));
+  FLOW_UNIFORM_DISPATCH(R, a, (tile_lag_viscous_accel_impl<R, true, kEarly, kFlags>(a, bx, by)),
+                        (tile_lag_viscous_accel_impl<R, false, kEarly, kFlags>(a, bx, by)));
 }
 
 __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long x) {
@@ -962,18 +1009,72 @@ __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long x)
   return x;
 }
 
+__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long x) {
+  const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(x >> 32));
+  const unsigned lo = __reduce_max_sync(
+      0xffffffffu, (unsigned)(x >> 32) == hi ? (unsigned)x : 0u);
+  return ((unsigned long long)hi << 32) | lo;
+}
+
+// The largest S = c_s^2 + 2 Q / rho along x and y a thread has seen, as FP64
+// bit patterns plus one (0: none): on a uniform mesh the smallest candidate
+// h / sqrt(S) of each axis is that of its largest S, so no key is formed per
+// cell and one thread per block takes the two square roots.
+struct CflMax {
+  unsigned long long x = 0ull, y = 0ull;
+  // S of a cell (e_neg: its energy is negative).  In [+0, +inf] only: a
+  // negative or NaN S is a NaN candidate in the reference.
+  __device__ __forceinline__ void add(double sx, double sy, bool e_neg) {
+    const unsigned long long kx = (unsigned long long)dbits(sx);
+    const unsigned long long ky = (unsigned long long)dbits(sy);
+    if (!e_neg && kx <= 0x7ff0000000000000ULL && kx + 1 > x) x = kx + 1;
+    if (!e_neg && ky <= 0x7ff0000000000000ULL && ky + 1 > y) y = ky + 1;
+  }
+  // The smaller candidate, as a bit pattern.
+  __device__ __forceinline__ unsigned long long candidate(double dx, double dy) const {
+    unsigned long long b = ~0ull;
+    if (x) b = (unsigned long long)dbits(dx * d_rsqrt(dfrom((long long)(x - 1))));
+    if (y) {
+      const unsigned long long c =
+          (unsigned long long)dbits(dy * d_rsqrt(dfrom((long long)(y - 1))));
+      b = c < b ? c : b;
+    }
+    return b;
+  }
+};
+
+// The energy of one cell of a uniform mesh after shock heating and work
+// (omp3/flow.c:258-286), FP64 form: du, dv the differences of its face
+// velocities, kx, ky dt_h over the spacings, inv_r 1/rho (used only where q,
+// a stress of the warp is not zero).  The reference's p / rho is
+// (gamma - 1) e and its rho_c / rho is 1 / (1 + div dt_h): with those, and
+// products folded into FMAs, 15 FP64 instructions without stresses and 18 with
+// (and four for inv_r) in place of 26.
+__device__ __forceinline__ double shock_energy_uniform(double e, double du, double dv, double kx,
+                                                       double ky, bool q, double qx, double qy,
+                                                       double inv_r) {
+  const double dux = du * kx, dvy = dv * ky;
+  const double div = dux + dvy;
+  const double pr = kG1 * e;
+  double e_q = e;
+  if (q) e_q = fma(-fma(qx, dux, qy * dvy), inv_r, e);
+  const double e_c = fma(-pr, div, e_q);
+  const double x = fma(kG1 * e_c, d_rcp(1.0 + div), pr);
+  return fma(-d_half(div), x, e_q);
+}
+
 // Shock heating and work (omp3/flow.c:248-290) fused with the CFL minimum of
 // set_timestep (omp3/flow.c:73-106) on the updated energy.  One atomicMin per
 // block on the FP64 bit pattern of its smallest candidate; the last block to
 // finish applies the leapfrog dt/dt_h rule (finish_dt).  In the mixed form
 // the FP32 energy change is added to the FP64 energy.
-template <typename R, bool kP2, bool kRing, bool kFlags>
+template <typename R, bool kU, bool kRing, bool kFlags>
 __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, int bx, int by,
                                                         unsigned long long* tile_min) {
   using Pr = Prec<R>;
   __shared__ R s_icy[kMaxRows], s_cy[kMaxRows];
   __shared__ double s_icy2[kMaxRows];
-  __shared__ unsigned long long s_warp[kCols / 32];
+  __shared__ unsigned long long s_warp[kCols / 32], s_warp_y[kCols / 32];
   __shared__ unsigned s_qf[kMaxRows];  // stress-flag words of the tile's rows
   const int nx = a.nx, ny = a.ny, pad = a.pad;
   const int jj = pad + bx * kCols + threadIdx.x;
@@ -981,10 +1082,10 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
   const bool edge = tile_near_edge(nx, ny, pad, pad + bx * kCols, i0, a.rows);
   if (threadIdx.x < a.rows) {
     const int ii = i0 + threadIdx.x;
-    if (ii < ny) {
+    if (!kU && ii < ny) {
       s_cy[threadIdx.x] = geo_v<R>(a.celldy[ii]);
-      s_icy[threadIdx.x] = geo_rcp<R, kP2>(a.celldy[ii]);
-      if constexpr (!Pr::kMixed) s_icy2[threadIdx.x] = geo_rcp_sq<kP2>(a.celldy[ii]);
+      s_icy[threadIdx.x] = geo_rcp<R>(a.celldy[ii]);
+      if constexpr (!Pr::kMixed) s_icy2[threadIdx.x] = 1.0 / (a.celldy[ii] * a.celldy[ii]);
     }
     if (kFlags && ii < ny - pad) s_qf[threadIdx.x] = a.qmask[(size_t)(ii - pad) * a.qm_stride + bx];
   }
@@ -1005,10 +1106,19 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
   // FP64 form: the thread's largest 1/dt^2 key so far, with its S and spacing.
   long long kbest = -1;
   double s_best = 0.0, c_best = 0.0;
+  CflMax cfl;  // (uniform mesh)
   if (jj < nx - pad) {
-    const R cx = geo_v<R>(a.celldx[jj]);
-    const R icx = geo_rcp<R, kP2>(a.celldx[jj]);
-    const double icx2 = Pr::kMixed ? 0.0 : geo_rcp_sq<kP2>(a.celldx[jj]);
+    R cx = R(0), icx = R(0), kx = R(0), ky = R(0);
+    double icx2 = 0.0;
+    if constexpr (kU) {
+      const UniformMesh um = uniform_mesh(a.mesh);
+      kx = a.dt_h * um.ix;
+      ky = a.dt_h * um.iy;
+    } else {
+      cx = geo_v<R>(a.celldx[jj]);
+      icx = geo_rcp<R>(a.celldx[jj]);
+      if constexpr (!Pr::kMixed) icx2 = 1.0 / (a.celldx[jj] * a.celldx[jj]);
+    }
     const R dt_h = Pr::from_d(a.dt_h);
     const int i1 = min(i0 + a.rows, ny - pad);
     R v0 = vq ? R(0) : a.v[cidx(nx, i0, jj)];
@@ -1053,7 +1163,9 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
     // The CFL candidates of the cell in tile row k from S = c_s^2 + 2 Q / rho
     // along x and y (e_neg: its energy is negative).
     auto cfl_candidates = [&](int k, R sx, R sy, bool e_neg) {
-      if constexpr (Pr::kMixed) {
+      if constexpr (kU) {
+        cfl.add(sx, sy, e_neg);
+      } else if constexpr (Pr::kMixed) {
         const unsigned long long mx = (unsigned long long)dbits(Pr::to_d(cx * Pr::rsqrt(sx)));
         const unsigned long long my =
             (unsigned long long)dbits(Pr::to_d(s_cy[k] * Pr::rsqrt(sy)));
@@ -1064,15 +1176,15 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
         // is the smallest dt) and take the square root only for the
         // thread's winner after the loop.  Keys in [+0, +inf] only: a
         // negative or NaN S is a NaN candidate in the reference.
-        const long long kx = e_neg ? -1 : dbits(Prec<double>::mulp<kP2>(sx, icx2));
-        const long long ky = e_neg ? -1 : dbits(Prec<double>::mulp<kP2>(sy, s_icy2[k]));
-        if (kx >= 0 && kx <= 0x7ff0000000000000LL && kx > kbest) {
-          kbest = kx;
+        const long long qx = e_neg ? -1 : dbits(sx * icx2);
+        const long long qy = e_neg ? -1 : dbits(sy * s_icy2[k]);
+        if (qx >= 0 && qx <= 0x7ff0000000000000LL && qx > kbest) {
+          kbest = qx;
           s_best = sx;
           c_best = cx;
         }
-        if (ky >= 0 && ky <= 0x7ff0000000000000LL && ky > kbest) {
-          kbest = ky;
+        if (qy >= 0 && qy <= 0x7ff0000000000000LL && qy > kbest) {
+          kbest = qy;
           s_best = sy;
           c_best = s_cy[k];
         }
@@ -1114,14 +1226,27 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
       // FP64 form a warp whose cells all have equal opposite face velocities
       // (dudx = dvdy = +0) takes this without forming the differences.
       R inv_r = R(0);
+      // (uniform mesh) A stress of the warp is not zero.
+      bool q_any = false;
+      if constexpr (kU) {
+        q_any = !warp_all(Pr::is_zero(qx) && Pr::is_zero(qy));
+        if (q_any) inv_r = rz ? R(0) : Pr::rcp(r);
+      }
       double e_new;
       bool still;
       if (!Pr::kMixed && warp_all(lane_same(u1f, u0f) && lane_same(v1, v0))) {
         still = true;
         e_new = rz ? 0.0 : double(er);
+      } else if constexpr (kU) {
+        const R du = u1f - u0f, dv = v1 - v0;
+        still = Pr::zero_skip_coarse(du) && Pr::zero_skip_coarse(dv);
+        e_new = rz ? 0.0 : double(er);
+        if (!still && !rz) {
+          e_new = shock_energy_uniform(er, du, dv, kx, ky, q_any, qx, qy, inv_r);
+        }
       } else {
-        const R dudx = Pr::template mulp<kP2>(u1f - u0f, icx);
-        const R dvdy = Pr::template mulp<kP2>(v1 - v0, s_icy[k]);
+        const R dudx = (u1f - u0f) * icx;
+        const R dvdy = (v1 - v0) * s_icy[k];
         still = Pr::zero_skip_coarse(dudx) && Pr::zero_skip_coarse(dvdy);
         if (still) {
           // (Mixed form: the FP64 energy is not needed, as it is kept.)
@@ -1156,8 +1281,8 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
       const R e_nr = keep ? er : Pr::from_d(e_new);
       const R s2 = R(kGam * (kGam - 1.0)) * e_nr;
       R sx = s2, sy = s2;  // + 2 Q / rho, zero without viscous stress
-      if (!Pr::zero_skip_coarse(qx) || !Pr::zero_skip_coarse(qy)) {
-        if (still) inv_r = rz ? R(0) : Pr::rcp(r);
+      if (kU ? q_any : (!Pr::zero_skip_coarse(qx) || !Pr::zero_skip_coarse(qy))) {
+        if (!kU && still) inv_r = rz ? R(0) : Pr::rcp(r);
         const R two_inv_r = Pr::twice(inv_r);
         sx = fma(qx, two_inv_r, s2);
         sy = fma(qy, two_inv_r, s2);
@@ -1198,6 +1323,25 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
       }
     }
   }
+  if constexpr (kU) {
+    const unsigned long long wx = warp_max_u64(cfl.x), wy = warp_max_u64(cfl.y);
+    if ((threadIdx.x & 31) == 0) {
+      s_warp[threadIdx.x >> 5] = wx;
+      s_warp_y[threadIdx.x >> 5] = wy;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 0; w < kCols / 32; ++w) {
+        cfl.x = s_warp[w] > cfl.x ? s_warp[w] : cfl.x;
+        cfl.y = s_warp_y[w] > cfl.y ? s_warp_y[w] : cfl.y;
+      }
+      const UniformMesh um = uniform_mesh(a.mesh);
+      const unsigned long long b = cfl.candidate(um.dx, um.dy);
+      atomicMin(a.min_slot, b);
+      if (tile_min) *tile_min = b;
+    }
+    return;
+  }
   if (!Pr::kMixed && kbest >= 0) best = (unsigned long long)dbits(c_best * d_rsqrt(s_best));
   best = warp_min_u64(best);
   if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = best;
@@ -1234,9 +1378,8 @@ __device__ __forceinline__ void tile_lag_energy_dt(const StepArgs<R>& a, int bx,
       }
     }
   }
-  FLOW_POW2_DISPATCH(R, a, a.pad + bx * kCols, a.pad + by * a.rows,
-                     (tile_lag_energy_dt_impl<R, true, kRing, kFlags>(a, bx, by, tile_min)),
-                     (tile_lag_energy_dt_impl<R, false, kRing, kFlags>(a, bx, by, tile_min)));
+  FLOW_UNIFORM_DISPATCH(R, a, (tile_lag_energy_dt_impl<R, true, kRing, kFlags>(a, bx, by, tile_min)),
+                        (tile_lag_energy_dt_impl<R, false, kRing, kFlags>(a, bx, by, tile_min)));
 }
 
 // The leapfrog dt/dt_h rule of omp3/flow.c:103-105 applied to the finished
@@ -1266,26 +1409,44 @@ __device__ __forceinline__ void finish_dt(const StepArgs<R>& a) {
 // multiplication instead of three; halving, doubling and negation are exact
 // integer operations.  A zero slope (flat or extremal data) leaves the base
 // value, and the reconstruction arithmetic is skipped.
-template <typename R, bool kP2>
+template <typename R>
 __device__ __forceinline__ R mc_reconstruct(bool pos, R da, R db, R dc, R base, R inv_h, R h,
                                             R wdt) {
   using Pr = Prec<R>;
   const R m0 = Pr::minmod(Pr::minmod(Pr::half(da), Pr::twice(db)), Pr::twice(dc));
   if (Pr::zero_skip(m0)) return base;
-  const R mm = Pr::template mulp<kP2>(m0, inv_h);
+  const R mm = m0 * inv_h;
   const R w = h + (pos ? Pr::neg(wdt) : wdt);
   const R hm = Pr::half(pos ? mm : Pr::neg(mm));
   return Pr::madd(hm, w, base);
 }
 
+// The same on a uniform mesh (FP64 form), where h/h' is 1: base +- 0.5 m
+// (1 -+ wind dt_h / h), c the coefficient dt_h / h; two FP64 instructions after
+// the differences.
+__device__ __forceinline__ double mc_reconstruct_uniform(bool pos, double da, double db, double dc,
+                                                         double base, double wind, double c) {
+  const double m = d_minmod(d_minmod(d_half(da), d_twice(db)), d_twice(dc));
+  if (d_is_zero(m)) return base;
+  const double f = fma(pos ? d_neg(wind) : wind, c, 1.0);
+  return fma(d_half(pos ? m : d_neg(m)), f, base);
+}
+
 // The same from the four values themselves, selecting the operands before
 // subtracting so that each difference is one FP64 instruction.
-template <typename R, bool kP2>
+template <typename R>
 __device__ __forceinline__ R mc_face(bool pos, R m2, R m1, R p0, R p1, R inv_h, R h, R wdt) {
   const R a0 = pos ? p0 : p1;
   const R a1 = pos ? m2 : m1;
   const R base = pos ? m1 : p0;
-  return mc_reconstruct<R, kP2>(pos, a0 - a1, base - a1, a0 - base, base, inv_h, h, wdt);
+  return mc_reconstruct<R>(pos, a0 - a1, base - a1, a0 - base, base, inv_h, h, wdt);
+}
+__device__ __forceinline__ double mc_face_uniform(bool pos, double m2, double m1, double p0,
+                                                  double p1, double wind, double c) {
+  const double a0 = pos ? p0 : p1;
+  const double a1 = pos ? m2 : m1;
+  const double base = pos ? m1 : p0;
+  return mc_reconstruct_uniform(pos, a0 - a1, base - a1, a0 - base, base, wind, c);
 }
 
 // Four consecutive values of a column (m2, m1, p0, p1) with their one-step
@@ -1322,10 +1483,13 @@ struct ColWindow {
     D1 = D2; D2 = p1 - m1;
   }
   // mc_face of the window's face (between m1 and p0).
-  template <bool kP2>
   __device__ __forceinline__ R face(bool pos, R inv_h, R h, R wdt) const {
-    return mc_reconstruct<R, kP2>(pos, pos ? D1 : D2, pos ? d1 : d2, pos ? d2 : d3,
-                                  pos ? m1 : p0, inv_h, h, wdt);
+    return mc_reconstruct<R>(pos, pos ? D1 : D2, pos ? d1 : d2, pos ? d2 : d3,
+                             pos ? m1 : p0, inv_h, h, wdt);
+  }
+  __device__ __forceinline__ R face_uniform(bool pos, R wind, R c) const {
+    return mc_reconstruct_uniform(pos, pos ? D1 : D2, pos ? d1 : d2, pos ? d2 : d3,
+                                  pos ? m1 : p0, wind, c);
   }
 };
 
@@ -1360,7 +1524,7 @@ struct ColSteps {
 // side from v0 (the y sweep, omp3/flow.c:477) instead of the half-step
 // velocity.  A zero limiter (flat or extremal density) leaves the upwind
 // flux, and the second-order term is skipped.
-template <typename R, bool kSideV0, bool kP2, typename NumFn, typename EFaceFn>
+template <typename R, bool kSideV0, typename NumFn, typename EFaceFn>
 __device__ __forceinline__ void mass_energy_flux_core(R v0, R dv2, R dvm, R dvp, R rm1, R r0,
                                                       R jump, NumFn num_of, EFaceFn e_face_of,
                                                       R inv_h, R icd, R area, R dt, R dt_h,
@@ -1372,8 +1536,8 @@ __device__ __forceinline__ void mass_energy_flux_core(R v0, R dv2, R dvm, R dvp,
     return;
   }
   // minmod(0.5 (vp-vm)/h, 2 (v0-vm)/h, 2 (vp-v0)/h), scaled once (mc_reconstruct).
-  const R mm = Pr::template mulp<kP2>(
-      Pr::minmod(Pr::half(dv2), Pr::minmod(Pr::twice(dvm), Pr::twice(dvp))), inv_h);
+  const R mm =
+      Pr::minmod(Pr::half(dv2), Pr::minmod(Pr::twice(dvm), Pr::twice(dvp))) * inv_h;
   const R w_tc = Pr::msub(v0, Pr::half(v0) * dt, mm);
   R lim = R(0);
   if (!Pr::is_zero(jump)) {
@@ -1393,28 +1557,60 @@ __device__ __forceinline__ void mass_energy_flux_core(R v0, R dv2, R dvm, R dvp,
   } else {
     flux = Pr::madd(w_tc, rho_up,
                     Pr::half(Pr::abs(w_tc)) *
-                        (R(1) - Pr::abs(Pr::template mulp<kP2>(wdt, icd))) * lim * jump);
+                        (R(1) - Pr::abs(wdt * icd)) * lim * jump);
   }
   const R e_face = e_face_of(Pr::gt0(w_tc), wdt);
   *F_out = flux;
-  *eF_out = Pr::template mulp<kP2>(e_face, area) * flux;
+  *eF_out = e_face * area * flux;
+}
+
+// The same on a uniform mesh (FP64 form), with the timesteps over the spacing
+// along the sweep as coefficients (kd = dt / h, kh = dt_h / h); the energy
+// flux comes without the face length, which is in the update's coefficient.
+template <bool kSideV0, typename NumFn, typename EFaceFn>
+__device__ __forceinline__ void mass_energy_flux_uniform(double v0, double dv2, double dvm,
+                                                         double dvp, double rm1, double r0,
+                                                         double jump, NumFn num_of,
+                                                         EFaceFn e_face_of, double kd, double kh,
+                                                         double* F_out, double* eF_out) {
+  using Pr = Prec<double>;
+  if (d_is_zero(v0)) {  // a face at rest carries no mass and no energy
+    *F_out = 0.0;
+    *eF_out = 0.0;
+    return;
+  }
+  const double m = d_minmod(d_half(dv2), d_minmod(d_twice(dvm), d_twice(dvp)));
+  const double w = fma(-(d_half(v0) * m), kd, v0);
+  double lim = 0.0;  // half the Van Leer limiter
+  if (!d_is_zero(jump)) {
+    const bool up = kSideV0 ? d_ge0(v0) : d_ge0(w);
+    const double num = num_of(up);
+    if (Pr::same_sign_nz(num, jump)) lim = num * d_rcp(jump + num);
+  }
+  double flux = w * (d_ge0(w) ? rm1 : r0);
+  if (!d_is_zero(lim)) {
+    const double aw = d_abs(w);
+    flux = fma(aw * fma(-aw, kh, 1.0) * lim, jump, flux);
+  }
+  *F_out = flux;
+  *eF_out = e_face_of(d_gt0(w), w) * flux;
 }
 
 // The flux from the four cells straddling the face (m2, m1 | p0, p1) and
 // the face velocities vm, v0, vp (the x sweep); h_m/h_p are the cell widths
 // either side.
-template <typename R, bool kSideV0, bool kP2>
+template <typename R, bool kSideV0>
 __device__ __forceinline__ void mass_energy_flux(R vm, R v0, R vp, R rm2,
                                                  R rm1, R r0, R rp1, R em2,
                                                  R em1, R e0, R ep1, R inv_h,
                                                  R h_m, R h_p, R icd, R area,
                                                  R dt, R dt_h, R* F_out,
                                                  R* eF_out) {
-  mass_energy_flux_core<R, kSideV0, kP2>(
+  mass_energy_flux_core<R, kSideV0>(
       v0, vp - vm, v0 - vm, vp - v0, rm1, r0, r0 - rm1,
       [&](bool up) { return (up ? rm1 : rp1) - (up ? rm2 : r0); },
       [&](bool pos, R wdt) {
-        return mc_face<R, kP2>(pos, em2, em1, e0, ep1, inv_h, pos ? h_m : h_p, wdt);
+        return mc_face<R>(pos, em2, em1, e0, ep1, inv_h, pos ? h_m : h_p, wdt);
       },
       inv_h, icd, area, dt, dt_h, F_out, eF_out);
 }
@@ -1451,13 +1647,15 @@ static __device__ __noinline__ double still_energy(double r_old, double e_in, do
 
 // The fluxes arrive widened to FP64 (f0, f1 mass, ef0, ef1 energy; exact
 // for the mixed form's FP32 fluxes), each face's once.
-template <typename R, bool kFirst, bool kP2>
+// kU: a uniform mesh, with the coefficients kf, ke of the mass and energy flux
+// differences in the place of dt_h, vol, ivol and the face lengths.
+template <typename R, bool kFirst, bool kU>
 __device__ __forceinline__ void mass_energy_update(double r_in, double e_in,
                                                    double r_old, double dt_h,
                                                    double vol, double ivol, double a0,
                                                    double a1, double f0, double f1,
-                                                   double ef0, double ef1, double* r_out,
-                                                   double* e_out) {
+                                                   double ef0, double ef1, double kf, double ke,
+                                                   double* r_out, double* e_out) {
   using Pr = Prec<R>;
   // No mass or energy crosses any cell of the warp (a warp-uniform test): the
   // updates subtract zeros, the density stays and the energy takes the
@@ -1479,23 +1677,23 @@ __device__ __forceinline__ void mass_energy_update(double r_in, double e_in,
   }
   const double de = ef1 - ef0;
   double r_new, rho_e;
-  if (Pr::kMixed) {
-    const double coef = ivol;
-    // On power-of-two tiles the face-length products are exact exponent adds
-    // (the same numbers as the FMA below, which rounds once after them).
-    const double net = kP2 ? __dadd_rn(d_mul_pow2(f1, a1), -d_mul_pow2(f0, a0))
-                           : fma(a1, f1, -(a0 * f0));
-    r_new = fma(-coef, net, r_in);
-    rho_e = fma(-coef, de, r_old * e_in);
-  } else if (Pr::zero_skip(f0) && Pr::zero_skip(f1) && Pr::zero_skip(de)) {
+  if (!Pr::kMixed && Pr::zero_skip(f0) && Pr::zero_skip(f1) && Pr::zero_skip(de)) {
     // Nothing crosses the cell's faces: the updates subtract zeros.  (The
     // energy still takes the reference's rho_old*e/den round trip below.)
     r_new = r_in;
     rho_e = __dmul_rn(r_old, e_in);
+  } else if constexpr (kU) {
+    r_new = fma(-kf, f1 - f0, r_in);
+    rho_e = fma(-ke, de, __dmul_rn(r_old, e_in));
+  } else if constexpr (Pr::kMixed) {
+    const double coef = ivol;
+    const double net = fma(a1, f1, -(a0 * f0));
+    r_new = fma(-coef, net, r_in);
+    rho_e = fma(-coef, de, r_old * e_in);
   } else {
-    const double net = __dadd_rn(Prec<double>::mulp<kP2>(f1, a1), -Prec<double>::mulp<kP2>(f0, a0));
-    r_new = Prec<double>::dsub<kP2>(r_in, __dmul_rn(dt_h, net), vol, ivol);
-    rho_e = Prec<double>::dsub<kP2>(__dmul_rn(r_old, e_in), __dmul_rn(dt_h, de), vol, ivol);
+    const double net = __dadd_rn(f1 * a1, -__dmul_rn(f0, a0));
+    r_new = Prec<double>::dsub(r_in, __dmul_rn(dt_h, net), vol, ivol);
+    rho_e = Prec<double>::dsub(__dmul_rn(r_old, e_in), __dmul_rn(dt_h, de), vol, ivol);
   }
   const double den = kFirst ? r_old : r_new;
   *r_out = r_new;
@@ -1573,7 +1771,7 @@ __device__ __forceinline__ bool block_round_trip_exact(const double* rho, const 
 // kAlt (second sweep with flags): some tile near this one was skipped by the
 // first sweep (sk3, the skip marks of this band's y-sweep tiles tlo ..
 // tlo + 2); without it the loads need no selection.
-template <typename R, bool kFirst, bool kP2, bool kEarly, bool kFl, bool kAlt>
+template <typename R, bool kFirst, bool kU, bool kEarly, bool kFl, bool kAlt>
 __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
                                                        const SweepArgs<R>& s, int bx, int by,
                                                        unsigned sk3) {
@@ -1588,16 +1786,27 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
   const bool edge = tile_near_edge(nx, ny, pad, pad + bx * (kCols - 1), i0, a.rows);
   const double dt = a.dt_slot[0], dt_h = a.dt_slot[1];
   const int tlo = max(0, (bx * (kCols - 1) - 2) >> 7);
-  if (t < a.rows) {
+  constexpr bool kUd = kU && !Pr::kMixed;
+  // Uniform mesh: dt / dx and dt_h / dx, and the energy difference's
+  // coefficient (the FP64 form's energy fluxes leave out the face length).
+  double kd = 0.0, kh = 0.0, ke = 0.0;
+  if constexpr (kU) {
+    const UniformMesh um = uniform_mesh(a.mesh);
+    kd = dt * um.ix;
+    kh = dt_h * um.ix;
+    ke = kUd ? kh : kh * um.iy;
+  }
+  if (!kUd && t < a.rows) {
     const int ii = i0 + t;
     if (ii < ny - pad) {
-      // Row factor of the update: 1/celldy, times dt_h in the mixed form.
-      s_coef[t] = Pr::kMixed ? dt_h * geo_rcp_d<R, kP2>(a.celldy[ii])
-                             : geo_rcp_d<R, kP2>(a.celldy[ii]);
-      s_cyd[t] = a.celldy[ii];
-      s_ey0[t] = a.edgedy[ii];
       s_ey0r[t] = geo_v<R>(a.edgedy[ii]);
-      s_ey1[t] = a.edgedy[ii + 1];
+      if constexpr (!kU) {
+        // Row factor of the update: 1/celldy, times dt_h in the mixed form.
+        s_coef[t] = Pr::kMixed ? dt_h * geo_rcp_d<R>(a.celldy[ii]) : geo_rcp_d<R>(a.celldy[ii]);
+        s_cyd[t] = a.celldy[ii];
+        s_ey0[t] = a.edgedy[ii];
+        s_ey1[t] = a.edgedy[ii + 1];
+      }
     }
   }
   const bool face_ok = jj < nx + 1 - pad;
@@ -1605,11 +1814,11 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
   const bool face_owner = face_ok && (t < kCols - 1);
   R iex = R(0), cxm = R(0), cx0 = R(0), icx_r = R(0);
   double icx = 0.0;
-  if (face_ok) {
-    iex = geo_rcp<R, kP2>(a.edgedx[jj]);
+  if (!kUd && face_ok) {
+    iex = geo_rcp<R>(a.edgedx[jj]);
     cxm = geo_v<R>(a.celldx[jj - 1]);
     cx0 = geo_v<R>(a.celldx[jj]);
-    icx = geo_rcp_d<R, kP2>(a.celldx[jj]);
+    icx = geo_rcp_d<R>(a.celldx[jj]);
     icx_r = Pr::from_d(icx);
   }
   const R dt_r = Pr::from_d(dt), dt_h_r = Pr::from_d(dt_h);
@@ -1674,7 +1883,7 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
       cp_async_commit();
     }
   }
-  __syncthreads();
+  if (!kUd) __syncthreads();
   if (!kEarly && i0 < i1) load(i0);
   for (int ii = i0; ii < i1; ++ii) {
     const int k = ii - i0;
@@ -1707,9 +1916,20 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
       // skipped tile).
       auto rr = [&](int d) { return in_alt(jj + d) ? s.r_alt_r[c + d] : s.r_in_r[c + d]; };
       auto er = [&](int d) { return in_alt(jj + d) ? s.e_alt_r[c + d] : s.e_in_r[c + d]; };
-      mass_energy_flux<R, false, kP2>(a.u[f - 1], u0, a.u[f + 1], rr(-2), rr(-1), rr(0), rr(1),
-                                      er(-2), er(-1), er(0), er(1), iex, cxm, cx0, icx_r,
-                                      s_ey0r[k], dt_r, dt_h_r, &F, &eF);
+      if constexpr (kUd) {
+        const double vm = a.u[f - 1], vp = a.u[f + 1];
+        const double r2 = rr(-2), r1 = rr(-1), r0 = rr(0), q1 = rr(1);
+        const double e2 = er(-2), e1 = er(-1), e0 = er(0), p1 = er(1);
+        mass_energy_flux_uniform<false>(
+            u0, vp - vm, u0 - vm, vp - u0, r1, r0, r0 - r1,
+            [&](bool up) { return (up ? r1 : q1) - (up ? r2 : r0); },
+            [&](bool pos, double w) { return mc_face_uniform(pos, e2, e1, e0, p1, w, kh); }, kd,
+            kh, &F, &eF);
+      } else {
+        mass_energy_flux<R, false>(a.u[f - 1], u0, a.u[f + 1], rr(-2), rr(-1), rr(0), rr(1),
+                                   er(-2), er(-1), er(0), er(1), iex, cxm, cx0, icx_r,
+                                   s_ey0r[k], dt_r, dt_h_r, &F, &eF);
+      }
     }
     // kFl: a warp at rest stores only its flag (its fluxes are +0).
     if constexpr (kFl) {
@@ -1724,11 +1944,10 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
     __syncthreads();
     if (cell_ok) {
       double r_new, e_new;
-      mass_energy_update<R, kFirst, kP2>(r_in, e_in, r_old, dt_h,
-                                         a.celldx[jj] * s_cyd[k],
-                                         Prec<double>::mulp<kP2>(s_coef[k], icx),
-                                         s_ey0[k], s_ey1[k], sF[t],
-                                         sF[t + 1], seF[t], seF[t + 1], &r_new, &e_new);
+      mass_energy_update<R, kFirst, kU>(
+          r_in, e_in, r_old, dt_h, kU ? 0.0 : a.celldx[jj] * s_cyd[k], kU ? 0.0 : s_coef[k] * icx,
+          kU ? 0.0 : s_ey0[k], kU ? 0.0 : s_ey1[k], sF[t], sF[t + 1], seF[t], seF[t + 1], kh, ke,
+          &r_new, &e_new);
       // (A cell of a skipped tile is at rest and keeps its value, which rho
       // and e hold: storing it again writes the same value.)
       store_cell(edge, s.r_out, s.r_out_r, nx, ny, pad, ii, jj, r_new);
@@ -1781,17 +2000,15 @@ __device__ __forceinline__ void tile_mass_sweep_x(const StepArgs<R>& a, const Sw
         return;
       }
       if (__syncthreads_or(sk3 != 0u)) {
-        FLOW_POW2_DISPATCH_ALL(
-            a, a.pad + bx * (kCols - 1), a.pad + by * a.rows,
-            (tile_mass_sweep_x_impl<R, kFirst, true, kEarly, kFl, true>(a, s, bx, by, sk3)),
+        FLOW_UNIFORM_DISPATCH_ALL(
+            a, (tile_mass_sweep_x_impl<R, kFirst, true, kEarly, kFl, true>(a, s, bx, by, sk3)),
             (tile_mass_sweep_x_impl<R, kFirst, false, kEarly, kFl, true>(a, s, bx, by, sk3)));
-        return;  // (the dispatch returns only after its power-of-two branch)
+        return;  // (the dispatch returns only after its uniform branch)
       }
     }
   }
-  FLOW_POW2_DISPATCH_ALL(
-      a, a.pad + bx * (kCols - 1), a.pad + by * a.rows,
-      (tile_mass_sweep_x_impl<R, kFirst, true, kEarly, kFl, false>(a, s, bx, by, 0u)),
+  FLOW_UNIFORM_DISPATCH_ALL(
+      a, (tile_mass_sweep_x_impl<R, kFirst, true, kEarly, kFl, false>(a, s, bx, by, 0u)),
       (tile_mass_sweep_x_impl<R, kFirst, false, kEarly, kFl, false>(a, s, bx, by, 0u)));
 }
 
@@ -1800,7 +2017,7 @@ __device__ __forceinline__ void tile_mass_sweep_x(const StepArgs<R>& a, const Sw
 // kAlt (second sweep with flags): some tile near this one was skipped by the
 // first sweep (sk3, the skip marks of bands by - 1 .. by + 1 of this
 // column's x-sweep tile); without it the loads need no selection.
-template <typename R, bool kFirst, bool kP2, bool kEarly, bool kFl, bool kAlt>
+template <typename R, bool kFirst, bool kU, bool kEarly, bool kFl, bool kAlt>
 __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
                                                        const SweepArgs<R>& s, int bx, int by,
                                                        unsigned sk3) {
@@ -1813,19 +2030,29 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
   const bool edge = tile_near_edge(nx, ny, pad, pad + bx * kCols, i0, a.rows);
   const double dt = a.dt_slot[0], dt_h = a.dt_slot[1];
   constexpr bool kSkip2 = kFl && !kFirst && kAlt;
+  constexpr bool kUd = kU && !Pr::kMixed;
+  // Uniform mesh: dt / dy and dt_h / dy, and the energy difference's
+  // coefficient (the FP64 form's energy fluxes leave out the face length).
+  double kd = 0.0, kh = 0.0, ke = 0.0;
+  if constexpr (kU) {
+    const UniformMesh um = uniform_mesh(a.mesh);
+    kd = dt * um.iy;
+    kh = dt_h * um.iy;
+    ke = kUd ? kh : kh * um.ix;
+  }
   // Face rows i0 .. i0+a.rows, cell rows i0-1 .. i0+a.rows.
-  if (threadIdx.x < a.rows + 2) {
+  if (!kUd && threadIdx.x < a.rows + 2) {
     const int ii = i0 - 1 + threadIdx.x;
     if (ii < ny) s_cy[threadIdx.x] = geo_v<R>(a.celldy[ii]);
   }
-  if (threadIdx.x < a.rows + 1) {
+  if (!kUd && threadIdx.x < a.rows + 1) {
     const int ii = i0 + threadIdx.x;
     if (ii < ny) {
-      s_iey[threadIdx.x] = geo_rcp<R, kP2>(a.edgedy[ii]);
-      s_icy[threadIdx.x] = geo_rcp<R, kP2>(a.celldy[ii]);
-      if (threadIdx.x < a.rows) {
-        s_coef[threadIdx.x] = Pr::kMixed ? dt_h * geo_rcp_d<R, kP2>(a.celldy[ii])
-                                         : geo_rcp_d<R, kP2>(a.celldy[ii]);
+      s_iey[threadIdx.x] = geo_rcp<R>(a.edgedy[ii]);
+      s_icy[threadIdx.x] = geo_rcp<R>(a.celldy[ii]);
+      if (!kU && threadIdx.x < a.rows) {
+        s_coef[threadIdx.x] =
+            Pr::kMixed ? dt_h * geo_rcp_d<R>(a.celldy[ii]) : geo_rcp_d<R>(a.celldy[ii]);
         s_cyd[threadIdx.x] = a.celldy[ii];
       }
     }
@@ -1933,10 +2160,15 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
     }
     if (i0 < i1) load_upd(i0);
   }
-  __syncthreads();
+  if (!kUd) __syncthreads();
   if (!col_ok) return;
-  const double icx = geo_rcp_d<R, kP2>(a.celldx[jj]);
-  const double ex0 = a.edgedx[jj], ex1 = a.edgedx[jj + 1];
+  double icx = 0.0, ex0 = 0.0, ex1 = 0.0, cxd = 0.0;
+  if constexpr (!kUd) ex0 = a.edgedx[jj];
+  if constexpr (!kU) {
+    icx = geo_rcp_d<R>(a.celldx[jj]);
+    ex1 = a.edgedx[jj + 1];
+    cxd = a.celldx[jj];
+  }
   const R ex0_r = geo_v<R>(ex0), dt_r = Pr::from_d(dt), dt_h_r = Pr::from_d(dt_h);
   if (!kEarly) prime();
   auto refresh = [&]() {
@@ -1954,12 +2186,18 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
   // Face row f = i0 + k: inverse spacing s_iey[k], cell widths s_cy[k] below
   // and s_cy[k + 1] above, downstream inverse width s_icy[k].
   auto flux_at = [&](int k, R* F, R* eF) {
-    mass_energy_flux_core<R, true, kP2>(
-        v0, dv2, dvm, dvp, rw.m1, rw.p0, rw.d2, [&](bool up) { return up ? rw.d1 : rw.d3; },
-        [&](bool pos, R wdt) {
-          return ew.template face<kP2>(pos, s_iey[k], pos ? s_cy[k] : s_cy[k + 1], wdt);
-        },
-        s_iey[k], s_icy[k], ex0_r, dt_r, dt_h_r, F, eF);
+    if constexpr (kUd) {
+      mass_energy_flux_uniform<true>(
+          v0, dv2, dvm, dvp, rw.m1, rw.p0, rw.d2, [&](bool up) { return up ? rw.d1 : rw.d3; },
+          [&](bool pos, double w) { return ew.face_uniform(pos, w, kh); }, kd, kh, F, eF);
+    } else {
+      mass_energy_flux_core<R, true>(
+          v0, dv2, dvm, dvp, rw.m1, rw.p0, rw.d2, [&](bool up) { return up ? rw.d1 : rw.d3; },
+          [&](bool pos, R wdt) {
+            return ew.face(pos, s_iey[k], pos ? s_cy[k] : s_cy[k + 1], wdt);
+          },
+          s_iey[k], s_icy[k], ex0_r, dt_r, dt_h_r, F, eF);
+    }
   };
   // Stores the mass flux of face row f; kFl: only where the face row moves
   // somewhere in the warp (mv) -- a face row at rest carries +0 (the mixed
@@ -2053,10 +2291,9 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
     }
     double r_new, e_new;
     const double f1d = Pr::to_d(F1), ef1d = Pr::to_d(eF1);
-    mass_energy_update<R, kFirst, kP2>(r_in, e_in, r_old, dt_h,
-                                       a.celldx[jj] * s_cyd[k],
-                                       Prec<double>::mulp<kP2>(s_coef[k], icx), ex0, ex1,
-                                       f0d, f1d, ef0d, ef1d, &r_new, &e_new);
+    mass_energy_update<R, kFirst, kU>(r_in, e_in, r_old, dt_h, kU ? 0.0 : cxd * s_cyd[k],
+                                      kU ? 0.0 : s_coef[k] * icx, ex0, ex1, f0d, f1d, ef0d, ef1d,
+                                      kh, ke, &r_new, &e_new);
     // (A cell of a skipped tile is at rest and keeps its value, which rho and
     // e hold: storing it again writes the same value.)
     store_cell(edge, s.r_out, s.r_out_r, nx, ny, pad, ii, jj, r_new);
@@ -2121,17 +2358,15 @@ __device__ __forceinline__ void tile_mass_sweep_y(const StepArgs<R>& a, const Sw
         return;
       }
       if (__syncthreads_or(sk3 != 0u)) {
-        FLOW_POW2_DISPATCH_ALL(
-            a, a.pad + bx * kCols, a.pad + by * a.rows,
-            (tile_mass_sweep_y_impl<R, kFirst, true, kEarly, kFl, true>(a, s, bx, by, sk3)),
+        FLOW_UNIFORM_DISPATCH_ALL(
+            a, (tile_mass_sweep_y_impl<R, kFirst, true, kEarly, kFl, true>(a, s, bx, by, sk3)),
             (tile_mass_sweep_y_impl<R, kFirst, false, kEarly, kFl, true>(a, s, bx, by, sk3)));
-        return;  // (the dispatch returns only after its power-of-two branch)
+        return;  // (the dispatch returns only after its uniform branch)
       }
     }
   }
-  FLOW_POW2_DISPATCH_ALL(
-      a, a.pad + bx * kCols, a.pad + by * a.rows,
-      (tile_mass_sweep_y_impl<R, kFirst, true, kEarly, kFl, false>(a, s, bx, by, 0u)),
+  FLOW_UNIFORM_DISPATCH_ALL(
+      a, (tile_mass_sweep_y_impl<R, kFirst, true, kEarly, kFl, false>(a, s, bx, by, 0u)),
       (tile_mass_sweep_y_impl<R, kFirst, false, kEarly, kFl, false>(a, s, bx, by, 0u)));
 }
 
@@ -2140,12 +2375,17 @@ __device__ __forceinline__ void tile_mass_sweep_y(const StepArgs<R>& a, const Sw
 
 // MC-limited upwind value of a velocity at a flux point from its four
 // neighbours along the direction (m2, m1 | p0, p1): omp3/flow.c:791-820.
-template <typename R, bool kP2>
+// kU: a uniform mesh, with the coefficient c = dt_h / h.
+template <typename R, bool kU>
 __device__ __forceinline__ R momentum_upwind(R wind, R m2, R m1, R p0, R p1,
                                              R inv_h, R d_left, R d_right,
-                                             R dt_h) {
+                                             R dt_h, R c) {
   const bool pos = Prec<R>::gt0(wind);
-  return mc_face<R, kP2>(pos, m2, m1, p0, p1, inv_h, pos ? d_left : d_right, wind * dt_h);
+  if constexpr (kU) {
+    return mc_face_uniform(pos, m2, m1, p0, p1, wind, c);
+  } else {
+    return mc_face<R>(pos, m2, m1, p0, p1, inv_h, pos ? d_left : d_right, wind * dt_h);
+  }
 }
 
 // The momentum phase fuses each momentum flux with the update it feeds, so
@@ -2169,16 +2409,26 @@ __device__ __forceinline__ R momentum_upwind(R wind, R m2, R m1, R p0, R p1,
 // fluxes differ, stored; the momentum is read here unless kVel gave it.  A
 // call, so that the warps which skip it skip its FP64 instructions (if
 // converted to predicated code they would still take their FP64 issue
-// slots).
-template <bool kVel, bool kP2>
+// slots).  Uniform mesh: k times the difference (the fluxes leave out the half
+// width of their face, which is in k).
+template <bool kVel>
+static __device__ __noinline__ double momentum_change_uniform(double* mom, double m, double fa,
+                                                              double fb, double k) {
+  const double diff = fa - fb;
+  if (d_is_zero(diff)) return m;
+  if (!kVel) m = *mom;
+  m = fma(-k, diff, m);
+  *mom = m;
+  return m;
+}
+template <bool kVel>
 static __device__ __noinline__ double momentum_change(double* mom, double m, double fa, double fb,
                                                       double dt_h, double hx, double h,
                                                       double inv_h, double ihx) {
-  using Pr = Prec<double>;
   const double diff = fa - fb;
-  if (Pr::zero_skip_mem(diff)) return m;
+  if (d_is_zero(diff)) return m;
   if (!kVel) m = *mom;
-  m = Pr::template dsub<kP2>(m, dt_h * diff, hx * h, Pr::template mulp<kP2>(inv_h, ihx));
+  m = Prec<double>::dsub(m, dt_h * diff, hx * h, inv_h * ihx);
   *mom = m;
   return m;
 }
@@ -2189,9 +2439,10 @@ static __device__ __noinline__ double momentum_change(double* mom, double m, dou
 // h/inv_h: the divisor's row factor, hx/ihx its column factor; w0, w1 the
 // face-density weights, ra, rb the densities either side and m_in the
 // momentum (kVel; loaded by the caller, possibly a row ahead).
-template <typename R, bool kU, bool kVel, bool kP2>
+// kUm: a uniform mesh, with the update's coefficient k.
+template <typename R, bool kU, bool kVel, bool kUm>
 __device__ __forceinline__ void momentum_face_update(const StepArgs<R>& a, bool edge, int ii,
-                                                     int jj, R fa, R fb, R dt_h, R hx, R ihx,
+                                                     int jj, R fa, R fb, R k, R dt_h, R hx, R ihx,
                                                      R h, R inv_h, R w0, R w1, R m_in, R ra,
                                                      R rb, R* vout) {
   using Pr = Prec<R>;
@@ -2209,21 +2460,23 @@ __device__ __forceinline__ void momentum_face_update(const StepArgs<R>& a, bool 
       const R diff = fa - fb;
       if (!Pr::zero_skip_mem(diff)) {
         if (!kVel) m = *mom;
-        m = Pr::template dsub<kP2>(m, dt_h * diff, hx * h, Pr::template mulp<kP2>(inv_h, ihx));
+        m = Pr::dsub(m, dt_h * diff, hx * h, inv_h * ihx);
         *mom = m;
       }
+    } else if constexpr (kUm) {
+      m = momentum_change_uniform<kVel>(mom, m, fa, fb, k);
     } else {
-      m = momentum_change<kVel, kP2>(mom, m, fa, fb, dt_h, hx, h, inv_h, ihx);
+      m = momentum_change<kVel>(mom, m, fa, fb, dt_h, hx, h, inv_h, ihx);
     }
   }
   if (kVel) {
     R rbar;
-    // FP64 form, power-of-two tile: equal densities and weights either side
-    // in the whole warp give the face density 2 (ra w0) exactly.
-    if (kP2 && !Pr::kMixed && warp_all(lane_same(ra, rb) && lane_same(w0, w1))) {
-      rbar = Pr::twice(Pr::template mulp<true>(ra, w0));
+    // FP64 form, uniform mesh: equal densities either side in the whole warp
+    // are the face density.
+    if (kUm && warp_all(lane_same(ra, rb))) {
+      rbar = ra;
     } else {
-      rbar = face_average<R, kP2>(ra, w0, rb, w1);
+      rbar = face_average<R, kUm>(ra, w0, rb, w1);
     }
     const R vel = face_velocity(m, rbar);
     if (kU) {
@@ -2315,7 +2568,7 @@ __device__ __forceinline__ void copy_velocities(const StepArgs<R>& a, bool edge,
 //   kV = true (rho_v): thread t holds the vF_x of corner c0 + t (c0 = pad +
 //     127 bx) and, for t < 127, updates y-face c0 + t from corners c0 + t and
 //     c0 + t + 1.
-template <typename R, bool kV, bool kVel, bool kP2, bool kRing, bool kFl>
+template <typename R, bool kV, bool kVel, bool kU, bool kRing, bool kFl>
 __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, int by) {
   using Pr = Prec<R>;
   __shared__ R s_half[kMaxRows], s_h[kMaxRows], s_row[kMaxRows];
@@ -2355,16 +2608,16 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
       return;
     }
   }
-  if (t < a.rows) {
+  if (!kU && t < a.rows) {
     const int ii = i0 + t;
     if (ii < ny) {
       // Flux: edgedy/2 (uF_x) or celldy/2 (vF_x); update divisor: celldy.
       s_half[t] = geo_half<R>(kV ? a.celldy[ii] : a.edgedy[ii]);
       s_h[t] = geo_v<R>(a.celldy[ii]);
-      s_row[t] = geo_rcp<R, kP2>(a.celldy[ii]);
+      s_row[t] = geo_rcp<R>(a.celldy[ii]);
       if (kV && kVel) {
-        s_wy0[t] = geo_half_ratio<R, kP2>(a.celldy[ii], a.edgedy[ii]);
-        s_wy1[t] = geo_half_ratio<R, kP2>(a.celldy[ii - 1], a.edgedy[ii]);
+        s_wy0[t] = geo_half_ratio<R>(a.celldy[ii], a.edgedy[ii]);
+        s_wy1[t] = geo_half_ratio<R>(a.celldy[ii - 1], a.edgedy[ii]);
       }
     }
   }
@@ -2403,20 +2656,28 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
   const int js = kV ? j : (j < pad ? 2 * pad - 1 - j : (j >= nx - pad ? 2 * (nx - pad) - 1 - j : j));
   const bool upd = kV ? (t < kCols - 1 && j < nx - pad) : (t >= 1 && j < nx + 1 - pad);
   R iex = R(0), cxl = R(0), cxr = R(0), hx = R(0), ihx = R(0), wx0 = R(0), wx1 = R(0);
-  if (flux_ok) {
-    iex = geo_rcp<R, kP2>(a.edgedx[js]);
-    cxl = geo_v<R>(a.celldx[js - 1]);
-    cxr = geo_v<R>(a.celldx[js]);
-  }
-  if (upd) {
-    hx = geo_v<R>(a.edgedx[j]);
-    ihx = geo_rcp<R, kP2>(a.edgedx[j]);
-    if (!kV && kVel) {
-      wx0 = geo_half_ratio<R, kP2>(a.celldx[j], a.edgedx[j]);
-      wx1 = geo_half_ratio<R, kP2>(a.celldx[j - 1], a.edgedx[j]);
+  const R dt_h = Pr::from_d(a.dt_slot[1]);
+  // Uniform mesh: dt_h / dx, and half of it (the fluxes' half widths dy / 2
+  // over the updates' dx dy).
+  R kh = R(0), ku = R(0);
+  if constexpr (kU) {
+    kh = dt_h * uniform_mesh(a.mesh).ix;
+    ku = Pr::half(kh);
+  } else {
+    if (flux_ok) {
+      iex = geo_rcp<R>(a.edgedx[js]);
+      cxl = geo_v<R>(a.celldx[js - 1]);
+      cxr = geo_v<R>(a.celldx[js]);
+    }
+    if (upd) {
+      hx = geo_v<R>(a.edgedx[j]);
+      ihx = geo_rcp<R>(a.edgedx[j]);
+      if (!kV && kVel) {
+        wx0 = geo_half_ratio<R>(a.celldx[j], a.edgedx[j]);
+        wx1 = geo_half_ratio<R>(a.celldx[j - 1], a.edgedx[j]);
+      }
     }
   }
-  const R dt_h = Pr::from_d(a.dt_slot[1]);
   // Velocities the fluxes read: rho_u's uF_x reads u before its update when
   // this pair updates it, else after; rho_v's vF_x reads the advected u and
   // v before or after its own update likewise.
@@ -2507,23 +2768,23 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
           val = sum_zeros(Fa, Fb);
         } else {
           const R ua = uu[f], ub = uu[f + 1];
-          const R mass = Pr::template mulp<kP2>(Fa + Fb, s_half[k]);
+          const R mass = kU ? Fa + Fb : (Fa + Fb) * s_half[k];
           // No mass through the cell, no momentum flux.
           val = Pr::zero_skip_coarse(mass)
                     ? mass
-                    : mass * momentum_upwind<R, kP2>(Pr::half(ua + ub), uu[f - 1], ua, ub,
-                                                     uu[f + 2], iex, cxl, cxr, dt_h);
+                    : mass * momentum_upwind<R, kU>(Pr::half(ua + ub), uu[f - 1], ua, ub,
+                                                    uu[f + 2], iex, cxl, cxr, dt_h, kh);
         }
       } else {
         const size_t c = cidx(nx, ii, js);
         if (warp_zeros(Fa, F_dn)) {
           val = sum_zeros(Fa, F_dn);  // FP64 form: no mass through any corner of the warp
         } else {
-          const R mass = Pr::template mulp<kP2>(Fa + F_dn, s_half[k]);
+          const R mass = kU ? Fa + F_dn : (Fa + F_dn) * s_half[k];
           val = Pr::zero_skip_coarse(mass)
                     ? mass
-                    : mass * momentum_upwind<R, kP2>(Pr::half(u0 + u_dn), vv[c - 2], vv[c - 1],
-                                                     vv[c], vv[c + 1], iex, cxl, cxr, dt_h);
+                    : mass * momentum_upwind<R, kU>(Pr::half(u0 + u_dn), vv[c - 2], vv[c - 1],
+                                                    vv[c], vv[c + 1], iex, cxl, cxr, dt_h, kh);
         }
         F_dn = Fa;
         u_dn = u0;
@@ -2549,9 +2810,9 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
         ra = a.rho_r[c];
         rb = kV ? a.rho_r[c - nx] : a.rho_r[c - 1];
       }
-      momentum_face_update<R, !kV, kVel, kP2>(a, edge, ii, j, fa, fb, dt_h, hx, ihx, s_h[k],
-                                              s_row[k], kV ? s_wy0[k] : wx0,
-                                              kV ? s_wy1[k] : wx1, m, ra, rb, vout);
+      momentum_face_update<R, !kV, kVel, kU>(
+          a, edge, ii, j, fa, fb, ku, dt_h, hx, ihx, kU ? R(0) : s_h[k], kU ? R(0) : s_row[k],
+          kU ? R(0) : (kV ? s_wy0[k] : wx0), kU ? R(0) : (kV ? s_wy1[k] : wx1), m, ra, rb, vout);
     }
     __syncthreads();
   }
@@ -2567,7 +2828,7 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
 //     updates y-faces i0 .. i1-1 from cells ii-1, ii.
 // The windows form their differences only where mass moves in the warp
 // (FP64 form), as the y mass sweep does.
-template <typename R, bool kV, bool kVel, bool kP2, bool kRing, bool kFl>
+template <typename R, bool kV, bool kVel, bool kU, bool kRing, bool kFl>
 __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, int by) {
   using Pr = Prec<R>;
   // kVel and kRing (the fused kernels): the update inputs of a face stream
@@ -2610,20 +2871,20 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
   };
   // (Entries of a ghost flux row are never used: its flux is its mirror
   // source's.)
-  for (int q = threadIdx.x; q <= nfr; q += kCols) {
+  for (int q = kU ? nfr + 1 : (int)threadIdx.x; q <= nfr; q += kCols) {
     const int ci = fr0 + q;
-    if (q < nfr) s_iey[q] = geo_rcp<R, kP2>(a.edgedy[ci]);
+    if (q < nfr) s_iey[q] = geo_rcp<R>(a.edgedy[ci]);
     s_cy[q] = geo_v<R>(a.celldy[ci - 1]);
   }
-  if (threadIdx.x < a.rows) {
+  if (!kU && threadIdx.x < a.rows) {
     const int ii = i0 + threadIdx.x;
     if (ii < ny) {
       // Update divisor row factor: edgedy for both y pairs.
       s_h[threadIdx.x] = geo_v<R>(a.edgedy[ii]);
-      s_row[threadIdx.x] = geo_rcp<R, kP2>(a.edgedy[ii]);
+      s_row[threadIdx.x] = geo_rcp<R>(a.edgedy[ii]);
       if (kV && kVel) {
-        s_wy0[threadIdx.x] = geo_half_ratio<R, kP2>(a.celldy[ii], a.edgedy[ii]);
-        s_wy1[threadIdx.x] = geo_half_ratio<R, kP2>(a.celldy[ii - 1], a.edgedy[ii]);
+        s_wy0[threadIdx.x] = geo_half_ratio<R>(a.celldy[ii], a.edgedy[ii]);
+        s_wy1[threadIdx.x] = geo_half_ratio<R>(a.celldy[ii - 1], a.edgedy[ii]);
       }
     }
   }
@@ -2662,13 +2923,21 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
   };
   if (jj >= (kV ? nx - pad : nx + 1 - pad) || i0 >= i1) return;
   const R dt_h = Pr::from_d(a.dt_slot[1]);
-  const R hcol = geo_half<R>(kV ? a.celldx[jj] : a.edgedx[jj]);  // flux: celldx/2 or edgedx/2
-  const R hx = geo_v<R>(a.celldx[jj]);
-  const R ihx = geo_rcp<R, kP2>(a.celldx[jj]);
-  R wx0 = R(0), wx1 = R(0);
-  if (!kV && kVel) {
-    wx0 = geo_half_ratio<R, kP2>(a.celldx[jj], a.edgedx[jj]);
-    wx1 = geo_half_ratio<R, kP2>(a.celldx[jj - 1], a.edgedx[jj]);
+  R hcol = R(0), hx = R(0), ihx = R(0), wx0 = R(0), wx1 = R(0);
+  // Uniform mesh: dt_h / dy, and half of it (the fluxes' half widths dx / 2
+  // over the updates' dx dy).
+  R kh = R(0), ku = R(0);
+  if constexpr (kU) {
+    kh = dt_h * uniform_mesh(a.mesh).iy;
+    ku = Pr::half(kh);
+  } else {
+    hcol = geo_half<R>(kV ? a.celldx[jj] : a.edgedx[jj]);  // flux: celldx/2 or edgedx/2
+    hx = geo_v<R>(a.celldx[jj]);
+    ihx = geo_rcp<R>(a.celldx[jj]);
+    if (!kV && kVel) {
+      wx0 = geo_half_ratio<R>(a.celldx[jj], a.edgedx[jj]);
+      wx1 = geo_half_ratio<R>(a.celldx[jj - 1], a.edgedx[jj]);
+    }
   }
   // The window's velocity: before this pair's update when it recomputes it.
   const R* w = kV ? (kVel ? a.v : a.v_out) : (kVel ? a.u : a.u_out);
@@ -2700,11 +2969,15 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
     if (fresh) win.advance();
     else win.refresh();
     fresh = true;
-    const R mass = Pr::template mulp<kP2>(Fa + Fb, hcol);
+    const R mass = kU ? Fa + Fb : (Fa + Fb) * hcol;
     if (Pr::zero_skip_coarse(mass)) return mass;
     const R wind = kV ? Pr::half(win.m1 + win.p0) : Pr::half(vwind[c - 1] + vwind[c]);
     const bool pos = Pr::gt0(wind);
-    return mass * win.template face<kP2>(pos, s_iey[q], pos ? s_cy[q] : s_cy[q + 1], wind * dt_h);
+    if constexpr (kU) {
+      return mass * win.face_uniform(pos, wind, kh);
+    } else {
+      return mass * win.face(pos, s_iey[q], pos ? s_cy[q] : s_cy[q + 1], wind * dt_h);
+    }
   };
   // The mass fluxes of flux row ci and the value that moves the window there
   // from row ci-1, loaded a row ahead of their use.
@@ -2834,9 +3107,9 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
       rb = rb_n;
       if (ii + 1 < i1) load_upd(ii + 1);
     }
-    momentum_face_update<R, !kV, kVel, kP2>(a, edge, ii, jj, cur, prev, dt_h, hx, ihx, s_h[k],
-                                            s_row[k], kV ? s_wy0[k] : wx0, kV ? s_wy1[k] : wx1,
-                                            m, ra, rb, vout);
+    momentum_face_update<R, !kV, kVel, kU>(
+        a, edge, ii, jj, cur, prev, ku, dt_h, hx, ihx, kU ? R(0) : s_h[k], kU ? R(0) : s_row[k],
+        kU ? R(0) : (kV ? s_wy0[k] : wx0), kU ? R(0) : (kV ? s_wy1[k] : wx1), m, ra, rb, vout);
     prev = cur;
   }
   if constexpr (kUpdRing || kFluxRing) cp_async_wait<0>();
@@ -2844,15 +3117,13 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
 
 template <typename R, bool kV, bool kVel, bool kRing = true, bool kFl = false>
 __device__ __forceinline__ void tile_mom_x(const StepArgs<R>& a, int bx, int by) {
-  FLOW_POW2_DISPATCH(R, a, (kV ? a.pad : a.pad - 1) + bx * (kCols - 1), a.pad + by * a.rows,
-                     (tile_mom_x_impl<R, kV, kVel, true, kRing, kFl>(a, bx, by)),
-                     (tile_mom_x_impl<R, kV, kVel, false, kRing, kFl>(a, bx, by)));
+  FLOW_UNIFORM_DISPATCH(R, a, (tile_mom_x_impl<R, kV, kVel, true, kRing, kFl>(a, bx, by)),
+                        (tile_mom_x_impl<R, kV, kVel, false, kRing, kFl>(a, bx, by)));
 }
 template <typename R, bool kV, bool kVel, bool kRing = true, bool kFl = false>
 __device__ __forceinline__ void tile_mom_y(const StepArgs<R>& a, int bx, int by) {
-  FLOW_POW2_DISPATCH(R, a, a.pad + bx * kCols, a.pad + by * a.rows,
-                     (tile_mom_y_impl<R, kV, kVel, true, kRing, kFl>(a, bx, by)),
-                     (tile_mom_y_impl<R, kV, kVel, false, kRing, kFl>(a, bx, by)));
+  FLOW_UNIFORM_DISPATCH(R, a, (tile_mom_y_impl<R, kV, kVel, true, kRing, kFl>(a, bx, by)),
+                        (tile_mom_y_impl<R, kV, kVel, false, kRing, kFl>(a, bx, by)));
 }
 
 }  // namespace tiles

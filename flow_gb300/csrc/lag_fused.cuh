@@ -83,7 +83,7 @@ struct LagArgs {
   unsigned* masks;      // [(mask row * ntx + bx) * kMaskFields + field][kWarps]
   double* ra;           // reduce_array: ticket, status
   unsigned long long* min_slot;
-  const unsigned long long* mesh_pow2;
+  const double* mesh;  // the mesh test's result (StepArgs::mesh)
   double* dt_slot;
   double dt, dt_h, max_dt;
   int first_step;
@@ -201,25 +201,12 @@ __device__ __forceinline__ TileGeom tile_geom(const LagArgs& a, int bx, int by) 
   return g;
 }
 
-// True when every spacing the tile uses (columns cb-4 .. cb+kW+4, rows
-// r0-4 .. r1+4) is a positive normal power of two.  Block-uniform (barrier).
-__device__ __forceinline__ bool tile_pow2(const LagArgs& a, const TileGeom& g) {
-  if (a.mesh_pow2 && *a.mesh_pow2 == 1ull) return true;
-  bool ok = true;
-  for (int j = g.cb - 4 + (int)threadIdx.x; j <= g.cb + kW + 4; j += kT) {
-    if (j >= 0 && j <= a.nx) ok = ok && d_is_pow2(a.celldx[j]) && d_is_pow2(a.edgedx[j]);
-  }
-  for (int i = g.r0 - 4 + (int)threadIdx.x; i <= g.r1 + 4; i += kT) {
-    if (i >= 0 && i <= a.ny) ok = ok && d_is_pow2(a.celldy[i]) && d_is_pow2(a.edgedy[i]);
-  }
-  return __syncthreads_and(ok) != 0;
-}
-
 // The CFL result of a thread: its largest 1/dt^2 key with the S and spacing
 // that gave it (tile_lag_energy_dt_impl's ranking).
 struct CflBest {
   long long kbest = -1;
   double s_best = 0.0, c_best = 0.0;
+  tiles::CflMax max;  // uniform mesh: its largest S of each axis instead
 };
 
 // Ballot of pred over the warp, stored by lane 0 as the warp's mask word.
@@ -232,7 +219,7 @@ __device__ __forceinline__ void store_mask(const LagArgs& a, int row, int bx, in
 }
 
 // Shared memory of a tile (one allocation per kernel, shared by the
-// power-of-two and general variants of the tile).
+// uniform and general variants of the tile).
 struct __align__(16) LagSmem {
   double ring[kSlots][kPlanes][kSeg];    // staged input rows (TMA destinations)
   unsigned long long bar[kSlots];        // one mbarrier per ring slot
@@ -246,7 +233,7 @@ struct __align__(16) LagSmem {
 
 // One tile of the fused Lagrangian phase.  Returns false when a row copy was
 // lost (bounded wait); the caller then records the error.
-template <bool kP2>
+template <bool kU>
 __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, int by,
                                          CflBest& cfl) {
   using Pr = Prec<double>;
@@ -282,17 +269,24 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
   const double dt = a.dt, dt_h = a.dt_h;
 
   // ---- row factors of rows ia .. ib (y faces and cell rows)
-  if (t <= ib - ia) {
+  tiles::UniformMesh um{};
+  double kx = 0.0, ky = 0.0;
+  if constexpr (kU) {
+    um = tiles::uniform_mesh(a.mesh);
+    kx = dt * um.ix;
+    ky = dt * um.iy;
+  }
+  if (!kU && t <= ib - ia) {
     const int f = ia + t;
     if (f >= 1 && f <= ny) {
       const double ey = a.edgedy[f], cy = a.celldy[f];
       s_ey[t] = ey;
-      s_iey[t] = tiles::geo_rcp<double, kP2>(ey);
-      s_wy0[t] = tiles::geo_half_ratio<double, kP2>(cy, ey);
-      s_wy1[t] = tiles::geo_half_ratio<double, kP2>(a.celldy[f - 1], ey);
+      s_iey[t] = tiles::geo_rcp<double>(ey);
+      s_wy0[t] = tiles::geo_half_ratio<double>(cy, ey);
+      s_wy1[t] = tiles::geo_half_ratio<double>(a.celldy[f - 1], ey);
       s_cy[t] = cy;
-      s_icy[t] = tiles::geo_rcp<double, kP2>(cy);
-      s_icy2[t] = tiles::geo_rcp_sq<kP2>(cy);
+      s_icy[t] = tiles::geo_rcp<double>(cy);
+      s_icy2[t] = 1.0 / (cy * cy);
     }
   }
   // ---- roles of this thread's column
@@ -317,17 +311,17 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
   const bool uf_out = uf_role && c < cb + kW;
   const bool cell_out = c >= max(cb, pad) && c < min(cb + kW, nx - pad);  // shock, y faces
   double ex = 0.0, iex = 0.0, wx0 = 0.0, wx1 = 0.0;
-  if (fc >= 0) {
+  if (!kU && fc >= 0) {
     ex = a.edgedx[fc];
-    iex = tiles::geo_rcp<double, kP2>(ex);
-    wx0 = tiles::geo_half_ratio<double, kP2>(a.celldx[fc], ex);
-    wx1 = tiles::geo_half_ratio<double, kP2>(a.celldx[fc - 1], ex);
+    iex = tiles::geo_rcp<double>(ex);
+    wx0 = tiles::geo_half_ratio<double>(a.celldx[fc], ex);
+    wx1 = tiles::geo_half_ratio<double>(a.celldx[fc - 1], ex);
   }
   double cx = 0.0, icx = 0.0, icx2 = 0.0;
-  if (uf_role) {
+  if (!kU && uf_role) {
     cx = a.celldx[c];
-    icx = tiles::geo_rcp<double, kP2>(cx);
-    icx2 = tiles::geo_rcp_sq<kP2>(cx);
+    icx = tiles::geo_rcp<double>(cx);
+    icx2 = 1.0 / (cx * cx);
   }
   // First and last valid y face of the window (ghost faces included).
   const int fa = (r0 - 2 >= pad) ? r0 - 2 : pad - 1;
@@ -430,16 +424,16 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
         const int k = i - ia;
         double mom = mom_y;
         double rbar;
-        if (kP2 && warp_all(lane_same(P0, P1) && lane_same(R0, R1) &&
-                                   lane_same(s_wy0[k], s_wy1[k]))) {
-          rbar = Pr::twice(Pr::template mulp<true>(R0, s_wy0[k]));
+        if (kU && warp_all(lane_same(P0, P1) && lane_same(R0, R1))) {
+          rbar = R0;
         } else {
           const double dp = P0 - P1;
           if (!Pr::zero_skip_mem(dp)) {
-            mom = Pr::template dsub<kP2>(mom, dt * dp, s_ey[k], s_iey[k]);
+            mom = tiles::momentum_step<double, kU>(mom, dp, ky, dt, kU ? 0.0 : s_ey[k],
+                                                   kU ? 0.0 : s_iey[k]);
             chn = true;
           }
-          rbar = face_average<double, kP2>(R0, s_wy0[k], R1, s_wy1[k]);
+          rbar = face_average<double, kU>(R0, kU ? 0.0 : s_wy0[k], R1, kU ? 0.0 : s_wy1[k]);
         }
         vnew = face_velocity(mom, rbar);
         mvn = mom;
@@ -480,7 +474,8 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
           const double dqy = qy - qy_dn;
           if (!Pr::zero_skip_mem(dqy)) {
             const int k = fv - ia;
-            mom = Pr::template dsub<kP2>(mom, dt * dqy, s_cy[k], s_icy[k]);
+            mom = tiles::momentum_step<double, kU>(mom, dqy, ky, dt, kU ? 0.0 : s_cy[k],
+                                                   kU ? 0.0 : s_icy[k]);
             vel = face_velocity(mom, rb2);
             vf_changed = true;
           }
@@ -516,13 +511,25 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
         const double r = R3, er = E3, qx = s_Q[sb][t], qy = qyA;
         const bool rz = Pr::is_zero(r);
         double inv_r = 0.0, e_new;
-        bool still;
+        bool still, q_any = false;
+        if constexpr (kU) {
+          q_any = !warp_all(Pr::is_zero(qx) && Pr::is_zero(qy));
+          if (q_any) inv_r = rz ? 0.0 : Pr::rcp(r);
+        }
         if (warp_all(lane_same(u1f, u0f) && lane_same(v1, v0))) {
           still = true;
           e_new = rz ? 0.0 : er;
+        } else if constexpr (kU) {
+          const double du = u1f - u0f, dv = v1 - v0;
+          still = Pr::zero_skip_coarse(du) && Pr::zero_skip_coarse(dv);
+          e_new = rz ? 0.0 : er;
+          if (!still && !rz) {
+            e_new = tiles::shock_energy_uniform(er, du, dv, dt_h * um.ix, dt_h * um.iy, q_any, qx,
+                                                qy, inv_r);
+          }
         } else {
-          const double dudx = Pr::template mulp<kP2>(u1f - u0f, icx);
-          const double dvdy = Pr::template mulp<kP2>(v1 - v0, s_icy[k]);
+          const double dudx = (u1f - u0f) * icx;
+          const double dvdy = (v1 - v0) * s_icy[k];
           still = Pr::zero_skip_coarse(dudx) && Pr::zero_skip_coarse(dvdy);
           if (still) {
             e_new = rz ? 0.0 : er;
@@ -547,24 +554,28 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
         const double e_nr = keep ? er : e_new;
         const double s2 = double(kGam * (kGam - 1.0)) * e_nr;
         double sx = s2, sy = s2;
-        if (!Pr::zero_skip_coarse(qx) || !Pr::zero_skip_coarse(qy)) {
-          if (still) inv_r = rz ? 0.0 : Pr::rcp(r);
+        if (kU ? q_any : (!Pr::zero_skip_coarse(qx) || !Pr::zero_skip_coarse(qy))) {
+          if (!kU && still) inv_r = rz ? 0.0 : Pr::rcp(r);
           const double two_inv_r = Pr::twice(inv_r);
           sx = fma(qx, two_inv_r, s2);
           sy = fma(qy, two_inv_r, s2);
         }
         const bool e_neg = d_lt0(e_new);
-        const long long kx = e_neg ? -1 : dbits(Pr::template mulp<kP2>(sx, icx2));
-        const long long ky = e_neg ? -1 : dbits(Pr::template mulp<kP2>(sy, s_icy2[k]));
-        if (kx >= 0 && kx <= 0x7ff0000000000000LL && kx > cfl.kbest) {
-          cfl.kbest = kx;
-          cfl.s_best = sx;
-          cfl.c_best = cx;
-        }
-        if (ky >= 0 && ky <= 0x7ff0000000000000LL && ky > cfl.kbest) {
-          cfl.kbest = ky;
-          cfl.s_best = sy;
-          cfl.c_best = s_cy[k];
+        if constexpr (kU) {
+          cfl.max.add(sx, sy, e_neg);
+        } else {
+          const long long qkx = e_neg ? -1 : dbits(sx * icx2);
+          const long long qky = e_neg ? -1 : dbits(sy * s_icy2[k]);
+          if (qkx >= 0 && qkx <= 0x7ff0000000000000LL && qkx > cfl.kbest) {
+            cfl.kbest = qkx;
+            cfl.s_best = sx;
+            cfl.c_best = cx;
+          }
+          if (qky >= 0 && qky <= 0x7ff0000000000000LL && qky > cfl.kbest) {
+            cfl.kbest = qky;
+            cfl.s_best = sy;
+            cfl.c_best = s_cy[k];
+          }
         }
       }
       store_mask(a, ks, bx, kMaskE, e_changed);
@@ -582,7 +593,7 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
         if (!warp_same(q1, q0)) {
           const double dqx = q1 - q0;
           if (!Pr::zero_skip_mem(dqx)) {
-            mom = Pr::template dsub<kP2>(mom, dt * dqx, cx, icx);
+            mom = tiles::momentum_step<double, kU>(mom, dqx, kx, dt, cx, icx);
             vel = face_velocity(mom, rbx2);
             u_changed = true;
           }
@@ -613,15 +624,15 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
       const double Pc = s_P[b][tf], Pl = s_P[b][tf - 1];
       double mom = mom_x;
       double rbar;
-      if (kP2 && warp_all(lane_same(Pc, Pl) && lane_same(rc, rl) && lane_same(wx0, wx1))) {
-        rbar = Pr::twice(Pr::template mulp<true>(rc, wx0));
+      if (kU && warp_all(lane_same(Pc, Pl) && lane_same(rc, rl))) {
+        rbar = rc;
       } else {
         const double dp = Pc - Pl;
         if (!Pr::zero_skip_mem(dp)) {
-          mom = Pr::template dsub<kP2>(mom, dt * dp, ex, iex);
+          mom = tiles::momentum_step<double, kU>(mom, dp, kx, dt, ex, iex);
           cu0 = true;
         }
-        rbar = face_average<double, kP2>(rc, wx0, rl, wx1);
+        rbar = face_average<double, kU>(rc, wx0, rl, wx1);
       }
       const double vel = face_velocity(mom, rbar);
       s_U[b][t] = ghost ? d_neg(vel) : vel;
