@@ -791,7 +791,7 @@ int finish_step(cudaStream_t s, Mesh* mesh, double* ra, StepProfiler& prof,
 // arch layer allocates it); a mesh too small for them stores and reads every
 // stress and flux.  Offsets in 4-byte words: the per-tile CFL minima (two
 // words per shock-heating tile) and the conservation totals' tile partials
-// (four words per kConsTile^2 tile) first, 8-byte aligned; then the stress
+// (four words per tile) first, 8-byte aligned; then the stress
 // flags ((ny - 2 pad) x stride words), the y mass-flux flags
 // ((ny + 1 - 2 pad) x stride), the x mass-flux flags ((ny - 2 pad) x xtiles),
 // the velocity flags (ny x vtiles) and the skip marks of even and odd steps
@@ -799,10 +799,20 @@ int finish_step(cudaStream_t s, Mesh* mesh, double* ra, StepProfiler& prof,
 // own first sweep writes the other), and the tile lists that even and odd steps
 // leave (the step's last kernel forms its own while it reads the previous
 // step's).
-constexpr int kConsTile = 128;  // rows and columns of a conservation tile
+// Conservation tiles: 128 columns and the fewest rows, 16 times a power of two,
+// that leave at most kConsTiles of them.  128 rows a tile kept a 1024^2 mesh's
+// 64 blocks at their chain of loads and additions for 30 us; shorter tiles
+// spread it, and the last block adds at most 32 partials a thread.
+constexpr int kConsTile = 128, kConsTiles = 4096;
+inline int cons_rows(int cols, long long rows) {
+  const long long tx = (cols + kConsTile - 1) / kConsTile;
+  int h = 16;
+  while (tx * ((rows + h - 1) / h) > kConsTiles && h < (1 << 20)) h *= 2;
+  return h;
+}
 struct FlagLayout {
   bool fits = false;
-  int stride = 0, xtiles = 0, vtiles = 0, cons_tx = 0, cons_ty = 0;
+  int stride = 0, xtiles = 0, vtiles = 0, cons_tx = 0, cons_ty = 0, cons_h = 0;
   int list_tx[2] = {0, 0}, list_bands = 0;
   size_t cfl = 0, cons = 0, q = 0, fy = 0, fx = 0, v = 0, marks = 0, sk_words = 0, lists = 0,
          list_words[2] = {0, 0};
@@ -815,7 +825,8 @@ FlagLayout flag_layout(int nx, int ny, int pad) {
   const long long rows = ny - 2 * pad;
   if (L.stride <= 0 || rows <= 0) return L;
   L.cons_tx = (nx - 2 * pad + kConsTile - 1) / kConsTile;
-  L.cons_ty = (int)((rows + kConsTile - 1) / kConsTile);
+  L.cons_h = cons_rows(nx - 2 * pad, rows);
+  L.cons_ty = (int)((rows + L.cons_h - 1) / L.cons_h);
   const long long bands = (rows + kMinRowsFlags - 1) / kMinRowsFlags;  // tile bands, at most
   L.sk_words = ((size_t)bands * (L.xtiles > L.stride ? L.xtiles : L.stride) + 3) / 4;
   L.cfl = 0;
@@ -1074,7 +1085,7 @@ StepRows take_rest(StepArgs<R>& a, int tt, int form, const std::array<const void
 
 // ---------------------------------------------------------------------------
 // Conservation totals by tiles (the reference's print_conservation sums,
-// omp3/flow.c:976-994): each kConsTile x kConsTile tile of interior cells
+// omp3/flow.c:976-994): each tile of interior cells (cons_rows)
 // keeps its partial sums (sum rho, sum rho e; each thread down its column, the
 // warps and then the four warps of the block in a fixed order) in
 // reduce_array, and the last block adds the partials of all tiles in a fixed
@@ -1089,10 +1100,59 @@ struct ConsArgs {
   const double* e;
   double* ra;
   double* part;                // 2 doubles per tile: sum rho, sum rho e
-  int nx, ny, pad, tiles_x, tiles;
+  int nx, ny, pad, tiles_x, tiles, rows;
   const unsigned char* marks;  // the last step's skip marks, or null
   int mark_w, mark_tiles_x, mark_rows;
 };
+
+// The sum of eight doubles on the integer pipes, rounded once: their
+// mantissas, aligned to the largest exponent with 7 more bits, added as 64-bit
+// integers (60 bits and 3 for the sum).  Bits of a value more than 59 places
+// below the largest's leading one are dropped, well below the rounding of an
+// FP64 addition at that size.  About 85 integer instructions (two clocks of a
+// scheduler each) in place of eight additions of 64 clocks: the totals' two
+// FP64 instructions a cell bound them (16.4 M cells: 58 us of FP64 issue, 39
+// us of memory).  Infinities, NaNs and the ends of the exponent range take the
+// additions (a call, so that the others do not issue them).
+static __device__ __noinline__ double sum8_slow(double a, double b, double c, double d, double e,
+                                                double f, double g, double h) {
+  return ((a + b) + (c + d)) + ((e + f) + (g + h));
+}
+__device__ __forceinline__ double sum8_aligned(const double (&v)[8]) {
+  int emax = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int ex = (dhi(v[q]) >> 20) & 0x7ff;
+    emax = ex > emax ? ex : emax;
+  }
+  if (emax > 0x7f8 || emax < 64) {
+    return sum8_slow(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+  }
+  long long sum = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const long long b = dbits(v[q]);
+    const int ex = (int)((b >> 52) & 0x7ff);
+    const int sh = emax - ex;
+    // (A zero or subnormal, which has no leading one, lies below the alignment.)
+    const unsigned long long m =
+        (((unsigned long long)b & 0x000fffffffffffffULL) | 0x0010000000000000ULL) << 7;
+    const long long a = sh < 60 ? (long long)(m >> sh) : 0;
+    sum += b < 0 ? -a : a;
+  }
+  if (sum == 0) return 0.0;
+  const bool neg = sum < 0;
+  unsigned long long m = neg ? 0ull - (unsigned long long)sum : (unsigned long long)sum;
+  const int lz = __clzll((long long)m);  // leading one at bit 63 - lz
+  m <<= lz;
+  // Round to nearest even at bit 11.
+  const unsigned long long r = (m >> 11) + (((m & 0x7ffULL) + ((m >> 11) & 1ULL)) > 0x400ULL);
+  // m at bit 59 has the exponent emax; r holds the leading one at bit 52 (or
+  // carried to 53), which the sum adds to the exponent field below it.
+  const long long e = (long long)(emax + (63 - lz) - 59 - 1);
+  return dfrom((long long)((unsigned long long)(e << 52) + r) |
+               (neg ? (long long)0x8000000000000000ULL : 0LL));
+}
 
 __device__ __forceinline__ double block_sum_fixed(double x, double* s_w) {
 #pragma unroll
@@ -1112,8 +1172,8 @@ __global__ void __launch_bounds__(kCols) k_conservation_tiles(const ConsArgs c) 
   __shared__ bool s_last;
   const int bx = blockIdx.x % c.tiles_x, by = blockIdx.x / c.tiles_x;
   const int pad = c.pad;
-  const int c0 = pad + bx * kConsTile, r0 = pad + by * kConsTile;
-  const int c1 = min(c0 + kConsTile, c.nx - pad), r1 = min(r0 + kConsTile, c.ny - pad);
+  const int c0 = pad + bx * kConsTile, r0 = pad + by * c.rows;
+  const int c1 = min(c0 + kConsTile, c.nx - pad), r1 = min(r0 + c.rows, c.ny - pad);
   bool kept = false;
   if (c.marks) {
     const int b0 = (r0 - pad) / c.mark_rows, b1 = (r1 - 1 - pad) / c.mark_rows;
@@ -1139,13 +1199,10 @@ __global__ void __launch_bounds__(kCols) k_conservation_tiles(const ConsArgs c) 
           rv[q] = in ? c.rho[k] : 0.0;
           ev[q] = in ? c.e[k] : 0.0;
         }
+        // (Rows past the end hold zeros.)
+        ms = __dadd_rn(ms, sum8_aligned(rv));
 #pragma unroll
-        for (int q = 0; q < kB; ++q) {
-          if (ib + q < r1) {
-            ms = __dadd_rn(ms, rv[q]);
-            es = __fma_rn(rv[q], ev[q], es);
-          }
-        }
+        for (int q = 0; q < kB; ++q) es = __fma_rn(rv[q], ev[q], es);
       }
     }
     const double tm = block_sum_fixed(ms, s_w);
@@ -1209,6 +1266,7 @@ bool tile_conservation(int nx, int ny, int pad, const double* rho, const double*
   c.pad = pad;
   c.tiles_x = L.cons_tx;
   c.tiles = L.cons_tx * L.cons_ty;
+  c.rows = L.cons_h;
   c.marks = nullptr;
   const unsigned long long calls = mesh_calls();
   const RestRecord& p = t_rest;
@@ -1228,7 +1286,8 @@ bool tile_conservation(int nx, int ny, int pad, const double* rho, const double*
     c.mark_tiles_x = x_first ? L.xtiles : L.stride;
     c.mark_rows = p.rows.sweep;
   }
-  cudaMemsetAsync(ra + kRaTicket, 0, sizeof(double), s);
+  // (A fused step leaves the ticket at zero.)
+  if (!after_step) cudaMemsetAsync(ra + kRaTicket, 0, sizeof(double), s);
   k_conservation_tiles<<<(unsigned)c.tiles, kCols, 0, s>>>(c);
   count_launches(1);
   ConsRecord r;
