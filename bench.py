@@ -61,8 +61,9 @@ KERNEL_BYTES_PER_CELL = {
     "lag_fused": 8 * 6,          # one-kernel Lagrangian phase: rho, e, rho_u, rho_v in; u, v out
     "lag_apply": 0,
     "mass_sweep_x": 0, "mass_sweep_y": 0,
-    "mom_uFx": 0, "mom_uFy": 0, "mom_vFx": 0, "mom_vFy": 0,
-    "mesh_pow2": 0,
+    # The momentum pairs by launch (two pairs share one where independent).
+    "mom_uFx": 0, "mom_uFy_vFx": 0, "mom_vFy": 0, "mom_uFy_vFy": 0, "mom_uFx_vFx": 0,
+    "mesh_test": 0,
 }
 
 # ncu figures (DRAM bytes per cell of each kernel on the blast workload, FP64

@@ -98,29 +98,31 @@ __device__ __forceinline__ int shape_of(int ph) {
 // instance, their tiles ran slower.)  A call per tile costs nothing per cell.
 template <typename R, int kPh>
 __device__ __noinline__ void tile_call(const Instance<R>& __restrict__ I, int tx, int ty) {
+  const bool uni = mesh_uniform(I.a.mesh);
   switch (kPh) {
-    case kPhMomUxV: tile_mom_x<R, false, true, false>(I.a, tx, ty); break;
-    case kPhMomUx: tile_mom_x<R, false, false, false>(I.a, tx, ty); break;
-    case kPhMomUyV: tile_mom_y<R, false, true, false>(I.a, tx, ty); break;
-    case kPhMomUy: tile_mom_y<R, false, false, false>(I.a, tx, ty); break;
-    case kPhMomVxV: tile_mom_x<R, true, true, false>(I.a, tx, ty); break;
-    case kPhMomVx: tile_mom_x<R, true, false, false>(I.a, tx, ty); break;
-    case kPhMomVyV: tile_mom_y<R, true, true, false>(I.a, tx, ty); break;
-    default: tile_mom_y<R, true, false, false>(I.a, tx, ty); break;
+    case kPhMomUxV: tile_mom_x<R, false, true, false>(I.a, tx, ty, uni); break;
+    case kPhMomUx: tile_mom_x<R, false, false, false>(I.a, tx, ty, uni); break;
+    case kPhMomUyV: tile_mom_y<R, false, true, false>(I.a, tx, ty, uni); break;
+    case kPhMomUy: tile_mom_y<R, false, false, false>(I.a, tx, ty, uni); break;
+    case kPhMomVxV: tile_mom_x<R, true, true, false>(I.a, tx, ty, uni); break;
+    case kPhMomVx: tile_mom_x<R, true, false, false>(I.a, tx, ty, uni); break;
+    case kPhMomVyV: tile_mom_y<R, true, true, false>(I.a, tx, ty, uni); break;
+    default: tile_mom_y<R, true, false, false>(I.a, tx, ty, uni); break;
   }
 }
 
 template <typename R>
 __device__ __forceinline__ void run_tile(int ph, const Instance<R>& I, int tx, int ty) {
+  const bool uni = mesh_uniform(I.a.mesh);
   switch (ph) {
-    case kPhPressure: tile_lag_pressure(I.a, tx, ty); break;
+    case kPhPressure: tile_lag_pressure(I.a, tx, ty, uni); break;
     case kPhViscosity: tile_lag_viscosity(I.a, tx, ty); break;
-    case kPhAccel: tile_lag_viscous_accel<R, false>(I.a, tx, ty); break;
-    case kPhEnergy: tile_lag_energy_dt<R, false>(I.a, tx, ty); break;
-    case kPhSweepX1: tile_mass_sweep_x<R, true, false>(I.a, I.first, tx, ty); break;
-    case kPhSweepY1: tile_mass_sweep_y<R, true, false>(I.a, I.first, tx, ty); break;
-    case kPhSweepX2: tile_mass_sweep_x<R, false, false>(I.a, I.second, tx, ty); break;
-    case kPhSweepY2: tile_mass_sweep_y<R, false, false>(I.a, I.second, tx, ty); break;
+    case kPhAccel: tile_lag_viscous_accel<R, false>(I.a, tx, ty, uni); break;
+    case kPhEnergy: tile_lag_energy_dt<R, false>(I.a, tx, ty, uni); break;
+    case kPhSweepX1: tile_mass_sweep_x<R, true, false>(I.a, I.first, tx, ty, uni); break;
+    case kPhSweepY1: tile_mass_sweep_y<R, true, false>(I.a, I.first, tx, ty, uni); break;
+    case kPhSweepX2: tile_mass_sweep_x<R, false, false>(I.a, I.second, tx, ty, uni); break;
+    case kPhSweepY2: tile_mass_sweep_y<R, false, false>(I.a, I.second, tx, ty, uni); break;
     case kPhMomUxV: tile_call<R, kPhMomUxV>(I, tx, ty); break;
     case kPhMomUx: tile_call<R, kPhMomUx>(I, tx, ty); break;
     case kPhMomUyV: tile_call<R, kPhMomUyV>(I, tx, ty); break;
@@ -278,22 +280,23 @@ __host__ __device__ constexpr int phase_shape() {
 // (copy rings and early first loads on).
 template <typename R, int kPh>
 __device__ __forceinline__ void phase_tile(const Instance<R>& I, int tx, int ty) {
-  if constexpr (kPh == kPhPressure) tile_lag_pressure(I.a, tx, ty);
+  const bool uni = mesh_uniform(I.a.mesh);
+  if constexpr (kPh == kPhPressure) tile_lag_pressure(I.a, tx, ty, uni);
   else if constexpr (kPh == kPhViscosity) tile_lag_viscosity(I.a, tx, ty);
-  else if constexpr (kPh == kPhAccel) tile_lag_viscous_accel<R, true>(I.a, tx, ty);
-  else if constexpr (kPh == kPhEnergy) tile_lag_energy_dt<R, true>(I.a, tx, ty);
-  else if constexpr (kPh == kPhSweepX1) tile_mass_sweep_x<R, true, true>(I.a, I.first, tx, ty);
-  else if constexpr (kPh == kPhSweepY1) tile_mass_sweep_y<R, true, true>(I.a, I.first, tx, ty);
-  else if constexpr (kPh == kPhSweepX2) tile_mass_sweep_x<R, false, true>(I.a, I.second, tx, ty);
-  else if constexpr (kPh == kPhSweepY2) tile_mass_sweep_y<R, false, true>(I.a, I.second, tx, ty);
-  else if constexpr (kPh == kPhMomUxV) tile_mom_x<R, false, true, true>(I.a, tx, ty);
-  else if constexpr (kPh == kPhMomUx) tile_mom_x<R, false, false, true>(I.a, tx, ty);
-  else if constexpr (kPh == kPhMomUyV) tile_mom_y<R, false, true, true>(I.a, tx, ty);
-  else if constexpr (kPh == kPhMomUy) tile_mom_y<R, false, false, true>(I.a, tx, ty);
-  else if constexpr (kPh == kPhMomVxV) tile_mom_x<R, true, true, true>(I.a, tx, ty);
-  else if constexpr (kPh == kPhMomVx) tile_mom_x<R, true, false, true>(I.a, tx, ty);
-  else if constexpr (kPh == kPhMomVyV) tile_mom_y<R, true, true, true>(I.a, tx, ty);
-  else tile_mom_y<R, true, false, true>(I.a, tx, ty);
+  else if constexpr (kPh == kPhAccel) tile_lag_viscous_accel<R, true>(I.a, tx, ty, uni);
+  else if constexpr (kPh == kPhEnergy) tile_lag_energy_dt<R, true>(I.a, tx, ty, uni);
+  else if constexpr (kPh == kPhSweepX1) tile_mass_sweep_x<R, true, true>(I.a, I.first, tx, ty, uni);
+  else if constexpr (kPh == kPhSweepY1) tile_mass_sweep_y<R, true, true>(I.a, I.first, tx, ty, uni);
+  else if constexpr (kPh == kPhSweepX2) tile_mass_sweep_x<R, false, true>(I.a, I.second, tx, ty, uni);
+  else if constexpr (kPh == kPhSweepY2) tile_mass_sweep_y<R, false, true>(I.a, I.second, tx, ty, uni);
+  else if constexpr (kPh == kPhMomUxV) tile_mom_x<R, false, true, true>(I.a, tx, ty, uni);
+  else if constexpr (kPh == kPhMomUx) tile_mom_x<R, false, false, true>(I.a, tx, ty, uni);
+  else if constexpr (kPh == kPhMomUyV) tile_mom_y<R, false, true, true>(I.a, tx, ty, uni);
+  else if constexpr (kPh == kPhMomUy) tile_mom_y<R, false, false, true>(I.a, tx, ty, uni);
+  else if constexpr (kPh == kPhMomVxV) tile_mom_x<R, true, true, true>(I.a, tx, ty, uni);
+  else if constexpr (kPh == kPhMomVx) tile_mom_x<R, true, false, true>(I.a, tx, ty, uni);
+  else if constexpr (kPh == kPhMomVyV) tile_mom_y<R, true, true, true>(I.a, tx, ty, uni);
+  else tile_mom_y<R, true, false, true>(I.a, tx, ty, uni);
 }
 
 // Resident CTAs per SM of each phase kernel: those of the single-problem

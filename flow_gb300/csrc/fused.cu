@@ -80,7 +80,10 @@ __global__ void __launch_bounds__(kCols) k_lag_pressure(const StepArgs<R> a) {
     }
   }
   int bx, by;
-  if (block_tile<kMd>(a, bx, by)) tile_lag_pressure<R, (kMd != kNoFlags)>(a, bx, by);
+  const bool uni = mesh_uniform(a.mesh);
+  if (block_tile<kMd>(a, bx, by)) {
+    tile_lag_pressure<R, (kMd != kNoFlags), (kMd != kListed)>(a, bx, by, uni);
+  }
 }
 // With flags, the viscous-stress flags (a.qmask) are kept -- the viscosity
 // kernel stores only warp rows with a non-zero stress, and the two kernels
@@ -90,43 +93,44 @@ __global__ void __launch_bounds__(kCols) k_lag_viscosity(const StepArgs<R> a) {
   pdl_wait();
   pdl_trigger();
   int bx, by;
-  if (block_tile<kMd>(a, bx, by)) tile_lag_viscosity<R, (kMd != kNoFlags)>(a, bx, by);
+  if (block_tile<kMd>(a, bx, by)) {
+    tile_lag_viscosity<R, (kMd != kNoFlags), (kMd != kListed)>(a, bx, by);
+  }
 }
 template <typename R, int kMd>
 __global__ void __launch_bounds__(kCols) k_lag_viscous_accel(const StepArgs<R> a) {
   pdl_wait();
   pdl_trigger();
   int bx, by;
+  const bool uni = mesh_uniform(a.mesh);
   if (block_tile<kMd>(a, bx, by)) {
-    tile_lag_viscous_accel<R, true, (kMd != kNoFlags)>(a, bx, by);
+    tile_lag_viscous_accel<R, true, (kMd != kNoFlags)>(a, bx, by, uni);
   }
 }
-// Shock heating + CFL minimum; the last block to finish (ticket in
-// reduce_array) applies the dt rule.
+// Shock heating + CFL minimum (the first sweep applies the dt rule).
 template <typename R, int kMd>
 __global__ void __launch_bounds__(kCols) k_lag_energy_dt(const StepArgs<R> a) {
-  __shared__ bool s_last;
-  __shared__ unsigned long long s_tile_min;  // the tile's CFL minimum (kFlags)
+  __shared__ unsigned long long s_tile_min;  // the tile's CFL minimum (with flags)
   pdl_wait();
   pdl_trigger();
   int bx, by;
   constexpr bool kFlags = kMd != kNoFlags;
-  const bool tile = block_tile<kMd>(a, bx, by);
-  if (tile) tile_lag_energy_dt<R, true, kFlags>(a, bx, by, kFlags ? &s_tile_min : nullptr);
-  if (threadIdx.x == 0) {
-    // (Thread 0 wrote the minimum it stores here.)
-    if (kFlags && a.cfl_tile && tile) {
-      a.cfl_tile[(size_t)by * a.qm_stride + bx] = s_tile_min;
-    }
-    __threadfence();
-    unsigned long long* ticket = reinterpret_cast<unsigned long long*>(a.ra + kRaTicket);
-    s_last = (atomicAdd(ticket, 1ull) == (unsigned long long)gridDim.x * gridDim.y - 1);
+  const bool uni = mesh_uniform(a.mesh);
+  if (!block_tile<kMd>(a, bx, by)) return;
+  tile_lag_energy_dt<R, true, kFlags, (kMd != kListed)>(a, bx, by, uni,
+                                                       kFlags ? &s_tile_min : nullptr);
+  // (Thread 0 wrote the minimum it stores here.)
+  if (kFlags && a.cfl_tile && threadIdx.x == 0) {
+    a.cfl_tile[(size_t)by * a.qm_stride + bx] = s_tile_min;
   }
-  __syncthreads();
-  if (s_last && threadIdx.x == 0) {
-    __threadfence();
-    finish_dt(a);
-    *reinterpret_cast<unsigned long long*>(a.ra + kRaTicket) = 0ull;
+}
+// The first sweep's block 0 leaves the dt pair for the kernels after it.
+template <typename R, bool kFirst>
+__device__ __forceinline__ void store_dt(const StepArgs<R>& a) {
+  if (kFirst && a.dt_from_min && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    const DtPair p = dt_rule(a, *a.min_slot);
+    a.dt_slot[0] = p.dt;
+    a.dt_slot[1] = p.dt_h;
   }
 }
 // With flags, the mass-flux flags (a.fxflag, a.fyflag) are kept -- the sweeps store only warps with a non-zero mass flux, and the
@@ -137,9 +141,11 @@ __global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 8 : 7) k_mass_sweep_x
   pdl_wait();
   pdl_trigger();
   int bx, by;
+  const bool uni = mesh_uniform(a.mesh);
   if (block_tile<kMd>(a, bx, by)) {
-    tile_mass_sweep_x<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by);
+    tile_mass_sweep_x<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by, uni);
   }
+  store_dt<R, kFirst>(a);
 }
 template <typename R, bool kFirst, int kMd>
 __global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 7 : 6) k_mass_sweep_y(const StepArgs<R> a,
@@ -147,9 +153,11 @@ __global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 7 : 6) k_mass_sweep_y
   pdl_wait();
   pdl_trigger();
   int bx, by;
+  const bool uni = mesh_uniform(a.mesh);
   if (block_tile<kMd>(a, bx, by)) {
-    tile_mass_sweep_y<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by);
+    tile_mass_sweep_y<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by, uni);
   }
+  store_dt<R, kFirst>(a);
 }
 // ---------------------------------------------------------------------------
 // Tile lists: the tiles the next step has to visit.  A cell in a tile the
@@ -289,44 +297,55 @@ unsigned acts[kListHeights], all[kListHeights];
 
 // Momentum pairs (flux fused with its update): x pairs share a row's fluxes
 // through shared memory (127 faces per CTA), y pairs march down columns.
-// kLists: the step's last pair, whose last 2 l.blocks blocks form the next
-// step's tile lists beside it (the pair reads neither the marks nor the minima
-// they are formed from; on its own the list kernel took 7 to 20 us a step,
-// mostly latency).  Its grid is 1-D.
-template <int kMd, bool kLists, typename R>
-__device__ __forceinline__ bool pair_tile(const StepArgs<R>& a, const ListArgs& l, int& bx,
-                                          int& by) {
-  if constexpr (kLists) {
-    const int k = (int)blockIdx.x, n = (int)gridDim.x - 2 * l.blocks;
-    if (k >= n) {
-      tile_lists(l, k - n);
-      return false;
-    }
-    if constexpr (kMd == kListed) return listed_tile(a, k, bx, by);
+// One launch runs one pair, or two that do not read what the other writes
+// (launch_step): two dependent launches of a few microseconds each become one.
+enum : int { kNone = 0, kXU = 1, kXV = 2, kYU = 3, kYV = 4 };  // direction and momentum
+template <typename R, int kPair, bool kVel, int kMd>
+__device__ __forceinline__ void pair_tile(const StepArgs<R>& a, int bx, int by, bool uni) {
+  constexpr bool kFl = kMd != kNoFlags, kTest = kMd != kListed;
+  if constexpr (kPair == kXU) tile_mom_x<R, false, kVel, true, kFl, kTest>(a, bx, by, uni);
+  else if constexpr (kPair == kXV) tile_mom_x<R, true, kVel, true, kFl, kTest>(a, bx, by, uni);
+  else if constexpr (kPair == kYU) tile_mom_y<R, false, kVel, true, kFl, kTest>(a, bx, by, uni);
+  else if constexpr (kPair == kYV) tile_mom_y<R, true, kVel, true, kFl, kTest>(a, bx, by, uni);
+}
+// Block k of a 1-D launch over pair tiles.
+template <int kMd, typename R>
+__device__ __forceinline__ bool pair_block(const StepArgs<R>& a, int k, int& bx, int& by) {
+  if constexpr (kMd == kListed) {
+    return listed_tile(a, k, bx, by);
+  } else {
     by = k / a.grid_x;
     bx = k - by * a.grid_x;
     return true;
-  } else {
-    return block_tile<kMd>(a, bx, by);
   }
 }
-template <typename R, bool kV, bool kVel, int kMd, bool kLists>
-__global__ void __launch_bounds__(kCols) k_mom_x(const StepArgs<R> a, const ListArgs l) {
+// The tiles of pair A (blocks 0 .. na - 1), then those of pair B; then, in the
+// step's last launch (kLists), 2 l.blocks blocks that form the next step's
+// tile lists beside it (the pairs read neither the marks nor the minima they
+// are formed from; on its own the list kernel took 7 to 20 us a step, mostly
+// latency).
+template <typename R, int kA, bool kVelA, int kB, bool kVelB, int kMd, bool kLists>
+__global__ void __launch_bounds__(kCols) k_mom(const StepArgs<R> a, const StepArgs<R> b, int na,
+                                               const ListArgs l) {
   pdl_wait();
   pdl_trigger();
-  int bx, by;
-  if (pair_tile<kMd, kLists>(a, l, bx, by)) {
-    tile_mom_x<R, kV, kVel, true, (kMd != kNoFlags)>(a, bx, by);
+  const bool uni = mesh_uniform(a.mesh);
+  const int k = (int)blockIdx.x;
+  if constexpr (kLists) {
+    const int n = (int)gridDim.x - 2 * l.blocks;
+    if (k >= n) {
+      tile_lists(l, k - n);
+      return;
+    }
   }
-}
-template <typename R, bool kV, bool kVel, int kMd, bool kLists>
-__global__ void __launch_bounds__(kCols) k_mom_y(const StepArgs<R> a, const ListArgs l) {
-  pdl_wait();
-  pdl_trigger();
   int bx, by;
-  if (pair_tile<kMd, kLists>(a, l, bx, by)) {
-    tile_mom_y<R, kV, kVel, true, (kMd != kNoFlags)>(a, bx, by);
+  if constexpr (kB != kNone) {
+    if (k >= na) {
+      if (pair_block<kMd>(b, k - na, bx, by)) pair_tile<R, kB, kVelB, kMd>(b, bx, by, uni);
+      return;
+    }
   }
+  if (pair_block<kMd>(a, k, bx, by)) pair_tile<R, kA, kVelA, kMd>(a, bx, by, uni);
 }
 
 // The whole Lagrangian phase of the FP64 step in one kernel (lag_fused.cuh):
@@ -594,45 +613,37 @@ int step_mode(const StepArgs<R>& a) {
   return !a.qmask ? kNoFlags : a.tiles ? kListed : kWhole;
 }
 
-template <typename R, bool kV, bool kVel>
-void launch_mom_x(cudaStream_t s, const StepArgs<R>& a0, const StepRows& sr,
-                  const TileLists& tl, const ListArgs& l) {
+// The tiles of one momentum pair: x pairs have 127 faces per CTA; rho_u lives
+// on x-faces pad .. nx-pad, rho_v on y-faces pad .. nx-pad-1 of one more row.
+template <typename R, int kPair, bool kVel>
+StepArgs<R> pair_args(const StepArgs<R>& a0, const StepRows& sr, const TileLists& tl, int& tiles) {
+  constexpr bool kV = kPair == kXV || kPair == kYV, kX = kPair == kXU || kPair == kXV;
   StepArgs<R> a = with_rows(a0, kVel ? sr.mom_vel : sr.mom_flux);
   const int cols = kV ? (a.nx - 2 * a.pad) : (a.nx + 1 - 2 * a.pad);
   const int rows = kV ? (a.ny + 1 - 2 * a.pad) : (a.ny - 2 * a.pad);
-  dim3 g = tile_grid(a, tl, 1, strip_grid(cols, rows, a.rows, kCols - 1));
-  const int md = step_mode(a);
-  if constexpr (kV && !kVel) {  // the step's last pair
-    if (l.blocks) {
-      g = dim3(g.x * g.y + 2 * (unsigned)l.blocks);
-      if (md == kListed) launch_pdl(k_mom_x<R, kV, kVel, kListed, true>, g, s, a, l);
-      else launch_pdl(k_mom_x<R, kV, kVel, kWhole, true>, g, s, a, l);
-      return;
-    }
-  }
-  if (md == kNoFlags) launch_pdl(k_mom_x<R, kV, kVel, kNoFlags, false>, g, s, a, l);
-  else if (md == kWhole) launch_pdl(k_mom_x<R, kV, kVel, kWhole, false>, g, s, a, l);
-  else launch_pdl(k_mom_x<R, kV, kVel, kListed, false>, g, s, a, l);
+  const dim3 g = tile_grid(a, tl, kX ? 1 : 0, strip_grid(cols, rows, a.rows, kX ? kCols - 1 : kCols));
+  tiles = (int)(g.x * g.y);
+  return a;
 }
-template <typename R, bool kV, bool kVel>
-void launch_mom_y(cudaStream_t s, const StepArgs<R>& a0, const StepRows& sr,
-                  const TileLists& tl, const ListArgs& l) {
-  StepArgs<R> a = with_rows(a0, kVel ? sr.mom_vel : sr.mom_flux);
-  const int cols = kV ? (a.nx - 2 * a.pad) : (a.nx + 1 - 2 * a.pad);
-  const int rows = kV ? (a.ny + 1 - 2 * a.pad) : (a.ny - 2 * a.pad);
-  dim3 g = tile_grid(a, tl, 0, strip_grid(cols, rows, a.rows));
+template <typename R, int kA, bool kVelA, int kB, bool kVelB>
+void launch_mom(cudaStream_t s, const StepArgs<R>& a0, const StepRows& sr, const TileLists& tl,
+                const ListArgs* lists) {
+  int na = 0, nb = 0;
+  const StepArgs<R> a = pair_args<R, kA, kVelA>(a0, sr, tl, na);
+  const StepArgs<R> b = pair_args<R, kB, kVelB>(a0, sr, tl, nb);
+  if (kB == kNone) nb = 0;
   const int md = step_mode(a);
-  if constexpr (kV && !kVel) {  // the step's last pair
-    if (l.blocks) {
-      g = dim3(g.x * g.y + 2 * (unsigned)l.blocks);
-      if (md == kListed) launch_pdl(k_mom_y<R, kV, kVel, kListed, true>, g, s, a, l);
-      else launch_pdl(k_mom_y<R, kV, kVel, kWhole, true>, g, s, a, l);
-      return;
-    }
+  if (lists && lists->blocks) {
+    const dim3 g((unsigned)(na + nb + 2 * lists->blocks));
+    if (md == kListed) launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kListed, true>, g, s, a, b, na, *lists);
+    else launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kWhole, true>, g, s, a, b, na, *lists);
+    return;
   }
-  if (md == kNoFlags) launch_pdl(k_mom_y<R, kV, kVel, kNoFlags, false>, g, s, a, l);
-  else if (md == kWhole) launch_pdl(k_mom_y<R, kV, kVel, kWhole, false>, g, s, a, l);
-  else launch_pdl(k_mom_y<R, kV, kVel, kListed, false>, g, s, a, l);
+  const dim3 g((unsigned)(na + nb));
+  const ListArgs l{};
+  if (md == kNoFlags) launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kNoFlags, false>, g, s, a, b, na, l);
+  else if (md == kWhole) launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kWhole, false>, g, s, a, b, na, l);
+  else launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kListed, false>, g, s, a, b, na, l);
 }
 
 template <typename R>
@@ -714,7 +725,10 @@ void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
   // The advection phase reads velocity flags only when this step's
   // Lagrangian kernels wrote them (not the one-kernel phase).
   StepArgs<R> ad = a;
-  if (lag) ad.vflag = nullptr;
+  if (lag) {
+    ad.vflag = nullptr;
+    ad.dt_from_min = 0;  // (its last block has applied the dt rule)
+  }
   const StepArgs<R> as = with_rows(ad, sr.sweep);
   const bool x_first = (tt % 2 == 0);
   // With flags, the first sweep marks the tiles it skips (in its own grid);
@@ -735,25 +749,23 @@ void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
   launch_mass(s, as, x_first, false, sw2, tl);
 
   // Momentum: each flux fused with its update, in the reference order; the
-  // pair that recomputes a velocity comes first in each chain.
+  // pair that recomputes a velocity comes first in each chain.  Two pairs share
+  // a launch where neither reads what the other writes: the y pairs take the
+  // Lagrangian velocities as their wind, so both velocity pairs of an even
+  // step, whose flux pairs then read only the advected velocities; of an odd
+  // step the y flux pair of rho_u and the x velocity pair of rho_v.
   if (tt % 2) {
     prof.mark("mom_uFx");
-    launch_mom_x<R, false, true>(s, ad, sr, tl, lists);
-    prof.mark("mom_uFy");
-    launch_mom_y<R, false, false>(s, ad, sr, tl, lists);
-    prof.mark("mom_vFx");
-    launch_mom_x<R, true, true>(s, ad, sr, tl, lists);
+    launch_mom<R, kXU, true, kNone, false>(s, ad, sr, tl, nullptr);
+    prof.mark("mom_uFy_vFx");
+    launch_mom<R, kYU, false, kXV, true>(s, ad, sr, tl, nullptr);
     prof.mark("mom_vFy");
-    launch_mom_y<R, true, false>(s, ad, sr, tl, lists);
+    launch_mom<R, kYV, false, kNone, false>(s, ad, sr, tl, &lists);
   } else {
-    prof.mark("mom_uFy");
-    launch_mom_y<R, false, true>(s, ad, sr, tl, lists);
-    prof.mark("mom_uFx");
-    launch_mom_x<R, false, false>(s, ad, sr, tl, lists);
-    prof.mark("mom_vFy");
-    launch_mom_y<R, true, true>(s, ad, sr, tl, lists);
-    prof.mark("mom_vFx");
-    launch_mom_x<R, true, false>(s, ad, sr, tl, lists);
+    prof.mark("mom_uFy_vFy");
+    launch_mom<R, kYU, true, kYV, true>(s, ad, sr, tl, nullptr);
+    prof.mark("mom_uFx_vFx");
+    launch_mom<R, kXU, false, kXV, false>(s, ad, sr, tl, &lists);
   }
 }
 
@@ -883,6 +895,7 @@ void fill_mesh_args(StepArgs<R>& a, const Mesh* mesh, int tt, double* ra) {
   a.n_tiles = a.grid_x = a.grid_y = 0;
   a.rest_min = reinterpret_cast<unsigned long long*>(ra + kRaRestMin);
   a.from_rest_min = 0;
+  a.dt_from_min = 1;
   const FlagLayout L = flag_layout(a.nx, a.ny, a.pad);
   if (L.fits) {
     unsigned* base = reinterpret_cast<unsigned*>(ra + kRaQFlags);

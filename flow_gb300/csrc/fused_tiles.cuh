@@ -143,6 +143,8 @@ struct StepArgs {
   // and whether the step starts its own minimum from it.
   unsigned long long* rest_min;
   int from_rest_min;
+  // The first sweep forms the dt pair from the CFL minimum.
+  int dt_from_min;
 };
 
 // Tile k of the list; false (in the whole block): none.
@@ -425,23 +427,25 @@ __device__ __forceinline__ void mesh_test_block(int nx, int ny, const double* ce
 // the general tile takes four (a quotient corrected to the reference's
 // rounding), and a tile reads no spacing arrays.  Each folded product is
 // rounded once per step instead of once per cell.
-#define FLOW_UNIFORM_DISPATCH(R, a, CALL_TRUE, CALL_FALSE) \
-  do {                                                     \
-    if constexpr (!Prec<R>::kMixed) {                      \
-      if (mesh_uniform(a.mesh)) {                          \
-        CALL_TRUE;                                         \
-        return;                                            \
-      }                                                    \
-    }                                                      \
-    CALL_FALSE;                                            \
+// uni: mesh_uniform(a.mesh), which a kernel reads beside its tile's index, so
+// that the two loads are in flight together.
+#define FLOW_UNIFORM_DISPATCH(R, CALL_TRUE, CALL_FALSE) \
+  do {                                                  \
+    if constexpr (!Prec<R>::kMixed) {                   \
+      if (uni) {                                        \
+        CALL_TRUE;                                      \
+        return;                                         \
+      }                                                 \
+    }                                                   \
+    CALL_FALSE;                                         \
   } while (0)
-#define FLOW_UNIFORM_DISPATCH_ALL(a, CALL_TRUE, CALL_FALSE) \
-  do {                                                      \
-    if (mesh_uniform(a.mesh)) {                             \
-      CALL_TRUE;                                            \
-      return;                                               \
-    }                                                       \
-    CALL_FALSE;                                             \
+#define FLOW_UNIFORM_DISPATCH_ALL(CALL_TRUE, CALL_FALSE) \
+  do {                                                   \
+    if (uni) {                                           \
+      CALL_TRUE;                                         \
+      return;                                            \
+    }                                                    \
+    CALL_FALSE;                                          \
   } while (0)
 
 // Spacing factors of a tile (mesh spacings, their reciprocals and ratios),
@@ -677,9 +681,14 @@ __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int
   }
 }
 
-template <typename R, bool kFl = false>
-__device__ __forceinline__ void tile_lag_pressure(const StepArgs<R>& a, int bx, int by) {
-  if constexpr (kFl) {
+// kTest (here and in the other tiles): whether to look for what the tile may
+// leave out because its cells were at rest.  Off for listed tiles, most of
+// which move: each test is a load and a barrier ahead of the tile's own (about
+// a microsecond), and a tile at rest that takes the plain path stores the
+// values its arrays hold.
+template <typename R, bool kFl = false, bool kTest = true>
+__device__ __forceinline__ void tile_lag_pressure(const StepArgs<R>& a, int bx, int by, bool uni) {
+  if constexpr (kFl && kTest) {
     // A tile whose cells (and the row above and column left it reads) were
     // at rest through the previous step: its pressures, momenta, velocities
     // (with their ghost images) and velocity flags are what that step's
@@ -689,7 +698,7 @@ __device__ __forceinline__ void tile_lag_pressure(const StepArgs<R>& a, int bx, 
     const int c0 = bx * kCols, i0 = by * a.rows;
     if (a.rest && rest_cells(a, i0 - 1, i0 + a.rows, c0 - 1, c0 + kCols)) return;
   }
-  FLOW_UNIFORM_DISPATCH(R, a, (tile_lag_pressure_impl<R, true, kFl>(a, bx, by)),
+  FLOW_UNIFORM_DISPATCH(R, (tile_lag_pressure_impl<R, true, kFl>(a, bx, by)),
                         (tile_lag_pressure_impl<R, false, kFl>(a, bx, by)));
 }
 
@@ -724,7 +733,7 @@ __device__ __forceinline__ R visc_stress(R rho, const R* w, R mid, R hi) {
 
 // kFlags: a.qmask is set -- a warp row whose stresses are all +0 stores only
 // its flag (the single-problem kernels; the batched kernels keep no flags).
-template <typename R, bool kFlags = false>
+template <typename R, bool kFlags = false, bool kTest = true>
 __device__ __forceinline__ void tile_lag_viscosity(const StepArgs<R>& a, int bx, int by) {
   const int nx = a.nx, ny = a.ny, pad = a.pad;
   const int jj = pad + bx * kCols + threadIdx.x;
@@ -735,7 +744,7 @@ __device__ __forceinline__ void tile_lag_viscosity(const StepArgs<R>& a, int bx,
   // kFlags: a tile whose face velocities (with the stencil's reach) are all
   // +0 loads none of them; its stresses are +0 and nothing is stored.
   bool vq = false;
-  if constexpr (kFlags) {
+  if constexpr (kFlags && kTest) {
     const int cb = pad + bx * kCols;
     vq = tile_vel_still(a, i0 - 3, i1 + 4, cb - 3, cb + kCols + 3);
   }
@@ -995,8 +1004,9 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
 }
 
 template <typename R, bool kEarly = true, bool kFlags = false>
-__device__ __forceinline__ void tile_lag_viscous_accel(const StepArgs<R>& a, int bx, int by) {
-  FLOW_UNIFORM_DISPATCH(R, a, (tile_lag_viscous_accel_impl<R, true, kEarly, kFlags>(a, bx, by)),
+__device__ __forceinline__ void tile_lag_viscous_accel(const StepArgs<R>& a, int bx, int by,
+                                                       bool uni) {
+  FLOW_UNIFORM_DISPATCH(R, (tile_lag_viscous_accel_impl<R, true, kEarly, kFlags>(a, bx, by)),
                         (tile_lag_viscous_accel_impl<R, false, kEarly, kFlags>(a, bx, by)));
 }
 
@@ -1068,7 +1078,7 @@ __device__ __forceinline__ double shock_energy_uniform(double e, double du, doub
 // block on the FP64 bit pattern of its smallest candidate; the last block to
 // finish applies the leapfrog dt/dt_h rule (finish_dt).  In the mixed form
 // the FP32 energy change is added to the FP64 energy.
-template <typename R, bool kU, bool kRing, bool kFlags>
+template <typename R, bool kU, bool kRing, bool kFlags, bool kTest>
 __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, int bx, int by,
                                                         unsigned long long* tile_min) {
   using Pr = Prec<R>;
@@ -1093,7 +1103,7 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
   // kFlags: a tile whose face velocities are all +0 (velocity flags) loads
   // none of them: its cells are still, and take the still path on +0 values.
   bool vq = false;
-  if constexpr (kFlags) {
+  if constexpr (kFlags && kTest) {
     const int cb = pad + bx * kCols;
     vq = tile_vel_still(a, i0 - 2, min(i0 + a.rows, ny - pad) + 2, cb - 2, cb + kCols + 2);
   }
@@ -1355,10 +1365,10 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
 }
 
 // tile_min: where thread 0 also stores the tile's CFL minimum, or null.
-template <typename R, bool kRing = true, bool kFlags = false>
-__device__ __forceinline__ void tile_lag_energy_dt(const StepArgs<R>& a, int bx, int by,
+template <typename R, bool kRing = true, bool kFlags = false, bool kTest = true>
+__device__ __forceinline__ void tile_lag_energy_dt(const StepArgs<R>& a, int bx, int by, bool uni,
                                                    unsigned long long* tile_min = nullptr) {
-  if constexpr (kFlags) {
+  if constexpr (kFlags && kTest) {
     // A tile at rest now (velocity flags) whose cells were at rest through
     // the previous step: it keeps every energy, has no viscous stress, and
     // its cells' CFL candidates are those of the previous step, from the
@@ -1378,20 +1388,37 @@ __device__ __forceinline__ void tile_lag_energy_dt(const StepArgs<R>& a, int bx,
       }
     }
   }
-  FLOW_UNIFORM_DISPATCH(R, a, (tile_lag_energy_dt_impl<R, true, kRing, kFlags>(a, bx, by, tile_min)),
-                        (tile_lag_energy_dt_impl<R, false, kRing, kFlags>(a, bx, by, tile_min)));
+  FLOW_UNIFORM_DISPATCH(R, (tile_lag_energy_dt_impl<R, true, kRing, kFlags, kTest>(a, bx, by, tile_min)),
+                        (tile_lag_energy_dt_impl<R, false, kRing, kFlags, kTest>(a, bx, by, tile_min)));
 }
 
-// The leapfrog dt/dt_h rule of omp3/flow.c:103-105 applied to the finished
-// CFL minimum, in FP64 without contraction; resets the minimum slot.
+// The leapfrog dt/dt_h rule of omp3/flow.c:103-105 for the CFL minimum g, in
+// FP64 without contraction.
+struct DtPair {
+  double dt, dt_h;
+};
 template <typename R>
-__device__ __forceinline__ void finish_dt(const StepArgs<R>& a) {
-  const unsigned long long g = atomicExch(a.min_slot, ~0ull);
+__device__ __forceinline__ DtPair dt_rule(const StepArgs<R>& a, unsigned long long g) {
   const double cfl = d_min_pos(a.max_dt, dfrom((long long)g));
   const double limited = dmin(cfl, __dmul_rn(FLOW_C_M, a.dt_h));
   const double dt = __dmul_rn(0.5, __dadd_rn(__dmul_rn(kCT, limited), a.dt_h));
-  a.dt_slot[0] = dt;
-  a.dt_slot[1] = a.first_step ? dt : __dmul_rn(kCT, limited);
+  return DtPair{dt, a.first_step ? dt : __dmul_rn(kCT, limited)};
+}
+// The rule applied once, to the finished minimum; resets the minimum slot.
+template <typename R>
+__device__ __forceinline__ void finish_dt(const StepArgs<R>& a) {
+  const DtPair p = dt_rule(a, atomicExch(a.min_slot, ~0ull));
+  a.dt_slot[0] = p.dt;
+  a.dt_slot[1] = p.dt_h;
+}
+// The pair a sweep takes: the step's first one forms it from the minimum
+// (dt_from_min; every thread for itself, one of them storing it for the
+// kernels after), so that the shock-heating kernel needs no ticket and no last
+// block: an atomic on one address per block, and about 2 us at its end.
+template <typename R, bool kFirst>
+__device__ __forceinline__ DtPair sweep_dt(const StepArgs<R>& a) {
+  if (kFirst && a.dt_from_min) return dt_rule(a, *a.min_slot);
+  return DtPair{a.dt_slot[0], a.dt_slot[1]};
 }
 
 // ===========================================================================
@@ -1784,7 +1811,8 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
   const int jj = pad + bx * (kCols - 1) + t;  // face (and cell) column
   const int i0 = pad + by * a.rows;
   const bool edge = tile_near_edge(nx, ny, pad, pad + bx * (kCols - 1), i0, a.rows);
-  const double dt = a.dt_slot[0], dt_h = a.dt_slot[1];
+  const DtPair dtp = sweep_dt<R, kFirst>(a);
+  const double dt = dtp.dt, dt_h = dtp.dt_h;
   const int tlo = max(0, (bx * (kCols - 1) - 2) >> 7);
   constexpr bool kUd = kU && !Pr::kMixed;
   // Uniform mesh: dt / dx and dt_h / dx, and the energy difference's
@@ -1960,7 +1988,7 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
 
 template <typename R, bool kFirst, bool kEarly = true, bool kFl = false>
 __device__ __forceinline__ void tile_mass_sweep_x(const StepArgs<R>& a, const SweepArgs<R>& s,
-                                                  int bx, int by) {
+                                                  int bx, int by, bool uni) {
   if constexpr (kFl) {
     // Tile skips (SweepArgs::skip), decided before any other work.
     const int pad = a.pad, t = threadIdx.x;
@@ -2001,14 +2029,14 @@ __device__ __forceinline__ void tile_mass_sweep_x(const StepArgs<R>& a, const Sw
       }
       if (__syncthreads_or(sk3 != 0u)) {
         FLOW_UNIFORM_DISPATCH_ALL(
-            a, (tile_mass_sweep_x_impl<R, kFirst, true, kEarly, kFl, true>(a, s, bx, by, sk3)),
+            (tile_mass_sweep_x_impl<R, kFirst, true, kEarly, kFl, true>(a, s, bx, by, sk3)),
             (tile_mass_sweep_x_impl<R, kFirst, false, kEarly, kFl, true>(a, s, bx, by, sk3)));
         return;  // (the dispatch returns only after its uniform branch)
       }
     }
   }
   FLOW_UNIFORM_DISPATCH_ALL(
-      a, (tile_mass_sweep_x_impl<R, kFirst, true, kEarly, kFl, false>(a, s, bx, by, 0u)),
+      (tile_mass_sweep_x_impl<R, kFirst, true, kEarly, kFl, false>(a, s, bx, by, 0u)),
       (tile_mass_sweep_x_impl<R, kFirst, false, kEarly, kFl, false>(a, s, bx, by, 0u)));
 }
 
@@ -2028,7 +2056,8 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
   const int jj = pad + bx * kCols + threadIdx.x;
   const int i0 = pad + by * a.rows;
   const bool edge = tile_near_edge(nx, ny, pad, pad + bx * kCols, i0, a.rows);
-  const double dt = a.dt_slot[0], dt_h = a.dt_slot[1];
+  const DtPair dtp = sweep_dt<R, kFirst>(a);
+  const double dt = dtp.dt, dt_h = dtp.dt_h;
   constexpr bool kSkip2 = kFl && !kFirst && kAlt;
   constexpr bool kUd = kU && !Pr::kMixed;
   // Uniform mesh: dt / dy and dt_h / dy, and the energy difference's
@@ -2314,7 +2343,7 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
 
 template <typename R, bool kFirst, bool kEarly = true, bool kFl = false>
 __device__ __forceinline__ void tile_mass_sweep_y(const StepArgs<R>& a, const SweepArgs<R>& s,
-                                                  int bx, int by) {
+                                                  int bx, int by, bool uni) {
   if constexpr (kFl) {
     // Tile skips (SweepArgs::skip), decided before any other work.
     const int pad = a.pad;
@@ -2359,14 +2388,14 @@ __device__ __forceinline__ void tile_mass_sweep_y(const StepArgs<R>& a, const Sw
       }
       if (__syncthreads_or(sk3 != 0u)) {
         FLOW_UNIFORM_DISPATCH_ALL(
-            a, (tile_mass_sweep_y_impl<R, kFirst, true, kEarly, kFl, true>(a, s, bx, by, sk3)),
+            (tile_mass_sweep_y_impl<R, kFirst, true, kEarly, kFl, true>(a, s, bx, by, sk3)),
             (tile_mass_sweep_y_impl<R, kFirst, false, kEarly, kFl, true>(a, s, bx, by, sk3)));
         return;  // (the dispatch returns only after its uniform branch)
       }
     }
   }
   FLOW_UNIFORM_DISPATCH_ALL(
-      a, (tile_mass_sweep_y_impl<R, kFirst, true, kEarly, kFl, false>(a, s, bx, by, 0u)),
+      (tile_mass_sweep_y_impl<R, kFirst, true, kEarly, kFl, false>(a, s, bx, by, 0u)),
       (tile_mass_sweep_y_impl<R, kFirst, false, kEarly, kFl, false>(a, s, bx, by, 0u)));
 }
 
@@ -2568,7 +2597,7 @@ __device__ __forceinline__ void copy_velocities(const StepArgs<R>& a, bool edge,
 //   kV = true (rho_v): thread t holds the vF_x of corner c0 + t (c0 = pad +
 //     127 bx) and, for t < 127, updates y-face c0 + t from corners c0 + t and
 //     c0 + t + 1.
-template <typename R, bool kV, bool kVel, bool kU, bool kRing, bool kFl>
+template <typename R, bool kV, bool kVel, bool kU, bool kRing, bool kFl, bool kTest>
 __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, int by) {
   using Pr = Prec<R>;
   __shared__ R s_half[kMaxRows], s_h[kMaxRows], s_row[kMaxRows];
@@ -2595,7 +2624,7 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
   const int i0 = pad + by * a.rows;
   const bool edge = tile_near_edge(nx, ny, pad, c0, i0, a.rows);
   const int i1 = min(i0 + a.rows, kV ? ny + 1 - pad : ny - pad);
-  if constexpr (kVel && kFl) {
+  if constexpr (kVel && kFl && kTest) {
     // No mass moves around the tile's faces: the Lagrangian velocities stand.
     if (tile_mass_still(a, i0 - 1, i1, c0 - 1, c0 + kCols)) {
       const bool upd = kV ? (t < kCols - 1 && j < nx - pad) : (t >= 1 && j < nx + 1 - pad);
@@ -2828,7 +2857,7 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
 //     updates y-faces i0 .. i1-1 from cells ii-1, ii.
 // The windows form their differences only where mass moves in the warp
 // (FP64 form), as the y mass sweep does.
-template <typename R, bool kV, bool kVel, bool kU, bool kRing, bool kFl>
+template <typename R, bool kV, bool kVel, bool kU, bool kRing, bool kFl, bool kTest>
 __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, int by) {
   using Pr = Prec<R>;
   // kVel and kRing (the fused kernels): the update inputs of a face stream
@@ -2850,7 +2879,7 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
   const int i0 = pad + by * a.rows;
   const bool edge = tile_near_edge(nx, ny, pad, pad + bx * kCols, i0, a.rows);
   const int i1 = min(i0 + a.rows, kV ? ny + 1 - pad : ny - pad);
-  if constexpr (kVel && kFl) {
+  if constexpr (kVel && kFl && kTest) {
     // No mass moves around the tile's faces: the Lagrangian velocities stand.
     const int cb = pad + bx * kCols;
     if (tile_mass_still(a, i0 - 1, i1, cb - 1, cb + kCols)) {
@@ -3115,15 +3144,17 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
   if constexpr (kUpdRing || kFluxRing) cp_async_wait<0>();
 }
 
-template <typename R, bool kV, bool kVel, bool kRing = true, bool kFl = false>
-__device__ __forceinline__ void tile_mom_x(const StepArgs<R>& a, int bx, int by) {
-  FLOW_UNIFORM_DISPATCH(R, a, (tile_mom_x_impl<R, kV, kVel, true, kRing, kFl>(a, bx, by)),
-                        (tile_mom_x_impl<R, kV, kVel, false, kRing, kFl>(a, bx, by)));
+template <typename R, bool kV, bool kVel, bool kRing = true, bool kFl = false,
+          bool kTest = true>
+__device__ __forceinline__ void tile_mom_x(const StepArgs<R>& a, int bx, int by, bool uni) {
+  FLOW_UNIFORM_DISPATCH(R, (tile_mom_x_impl<R, kV, kVel, true, kRing, kFl, kTest>(a, bx, by)),
+                        (tile_mom_x_impl<R, kV, kVel, false, kRing, kFl, kTest>(a, bx, by)));
 }
-template <typename R, bool kV, bool kVel, bool kRing = true, bool kFl = false>
-__device__ __forceinline__ void tile_mom_y(const StepArgs<R>& a, int bx, int by) {
-  FLOW_UNIFORM_DISPATCH(R, a, (tile_mom_y_impl<R, kV, kVel, true, kRing, kFl>(a, bx, by)),
-                        (tile_mom_y_impl<R, kV, kVel, false, kRing, kFl>(a, bx, by)));
+template <typename R, bool kV, bool kVel, bool kRing = true, bool kFl = false,
+          bool kTest = true>
+__device__ __forceinline__ void tile_mom_y(const StepArgs<R>& a, int bx, int by, bool uni) {
+  FLOW_UNIFORM_DISPATCH(R, (tile_mom_y_impl<R, kV, kVel, true, kRing, kFl, kTest>(a, bx, by)),
+                        (tile_mom_y_impl<R, kV, kVel, false, kRing, kFl, kTest>(a, bx, by)));
 }
 
 }  // namespace tiles
