@@ -169,14 +169,44 @@ __device__ __forceinline__ double d_pow2_rcp_sq(double y) {
   return d_pow2_quot_slow(1.0, y, 2);
 }
 
-// 1/x for finite normal non-zero x: MUFU seed, two Newton-Raphson steps.
-__device__ __forceinline__ double d_rcp(double x) {
+// 1/x to ~2^-43 for finite normal non-zero x, off the FP64 pipe: the mantissa
+// as f + t 2^-23 in FP32 (f its first 24 bits, t the next 23), r0 the MUFU
+// reciprocal of f, the Newton correction r0 (e + e^2) with e = 1 - (f + t
+// 2^-23) r0 in FP32 FMAs, and r0 plus the correction (in units of 2^-43)
+// assembled on the integer pipes.  About 30 FP32 and integer instructions in
+// place of the two FP64 ones (128 clocks of a scheduler's FP64 issue) that
+// bring the FP64 MUFU seed (2^-20) as far.
+static __device__ __noinline__ double d_rcp_seed_slow(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  double e = fma(-x, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-x, r, 1.0);
-  return fma(r, e, r);
+  return fma(r, fma(-x, r, 1.0), r);
+}
+__device__ __forceinline__ double d_rcp_seed(double x) {
+  const int hi = dhi(x), lo = dlo(x);
+  const int ex = (hi >> 20) & 0x7ff;
+  // (The ends of the exponent range: the result would not be normal.)
+  if ((unsigned)(ex - 1) >= 2043u) return d_rcp_seed_slow(x);
+  const float f = __int_as_float(
+      (int)(__funnelshift_l((unsigned)lo, (unsigned)hi, 3) & 0x7fffffu) | 0x3f800000);
+  const float t = __int_as_float((int)(((unsigned)lo >> 6) & 0x7fffffu) | 0x3f800000) - 1.0f;
+  float r0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(f));
+  r0 = fminf(fmaxf(r0, 0.5f), 1.0f);  // (f lies in [1, 2); its last place aside, so does 1/r0)
+  float e = fmaf(-f, r0, 1.0f);
+  e = fmaf(-t, r0 * 1.1920928955078125e-7f, e);
+  const float r1 = r0 * fmaf(e, e, e);  // |r1| < 2^-21
+  constexpr float kMagic = 1.430511474609375e-6f;  // 1.5 2^-20: units of 2^-43
+  const int k = __float_as_int(r1 + kMagic) - __float_as_int(kMagic);
+  const unsigned b = (unsigned)__float_as_int(r0);
+  // r0 widened, its exponent less x's, plus k 2^-43 (r0's last place is 2^-53).
+  const long long m = ((long long)(int)((b >> 3) + (unsigned)((896 + 1023 - ex) << 20)) << 32) +
+                      (long long)(unsigned)(b << 29) + ((long long)k << 10);
+  return dfrom2((int)(m >> 32) ^ (hi & (int)0x80000000), (int)m);
+}
+// 1/x for finite normal non-zero x: the seed and one Newton step.
+__device__ __forceinline__ double d_rcp(double x) {
+  const double r = d_rcp_seed(x);
+  return fma(r, fma(-x, r, 1.0), r);
 }
 // 1/x to ~2^-40 (one Newton step on the MUFU seed) for a reciprocal that is
 // only ever used through a residual-corrected quotient (qdiv), which is then
@@ -186,15 +216,12 @@ __device__ __forceinline__ double d_rcp_for_qdiv(double x) {
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
   return fma(r, fma(-x, r, 1.0), r);
 }
-// n/d for finite normal non-zero d when 1/d itself is not needed: one Newton
-// step on the MUFU seed (relative error ~2^-20 measured -> ~2^-40), the
-// quotient from it, and one residual correction q + r (n - d q) (-> ~2^-80):
-// the correctly rounded quotient except in vanishingly rare near-ties, as
-// d_rcp followed by qdiv gives, in 5 FP64 instructions instead of 7.
+// n/d for finite normal non-zero d when 1/d itself is not needed: the quotient
+// from the seed and one residual correction q + r (n - d q) (2^-43 -> ~2^-86):
+// the correctly rounded quotient except in vanishingly rare near-ties, in 3
+// FP64 instructions (5 with a Newton step on the MUFU seed).
 __device__ __forceinline__ double d_div(double n, double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  r = fma(r, fma(-d, r, 1.0), r);
+  const double r = d_rcp_seed(d);
   const double q = n * r;
   return fma(r, fma(-d, q, n), q);
 }
