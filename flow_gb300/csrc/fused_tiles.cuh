@@ -1476,6 +1476,16 @@ __device__ __forceinline__ double mc_face_uniform(bool pos, double m2, double m1
   return mc_reconstruct_uniform(pos, a0 - a1, base - a1, a0 - base, base, wind, c);
 }
 
+// The value itself, as one the compiler cannot form again: under register
+// pressure it recomputed carried FP64 differences from the window's values
+// (six more FP64 instructions a cell in the first y sweep, three in a y
+// momentum pair), which costs more than the registers.
+template <typename R>
+__device__ __forceinline__ R carried(R x) {
+  if constexpr (!Prec<R>::kMixed) asm volatile("" : "+d"(x));
+  return x;
+}
+
 // Four consecutive values of a column (m2, m1, p0, p1) with their one-step
 // differences d1 = m1-m2, d2 = p0-m1, d3 = p1-p0 and two-step differences
 // D1 = p0-m2, D2 = p1-m1.  A tile marching down the column shifts the window
@@ -1498,7 +1508,7 @@ struct ColWindow {
     m2 = m1; m1 = p0; p0 = p1; p1 = next;
   }
   __device__ __forceinline__ void shift(R next) {
-    const R D2n = next - p0, d3n = next - p1;
+    const R D2n = carried(next - p0), d3n = carried(next - p1);
     m2 = m1; m1 = p0; p0 = p1; p1 = next;
     d1 = d2; d2 = d3; d3 = d3n;
     D1 = D2; D2 = D2n;
@@ -1506,8 +1516,8 @@ struct ColWindow {
   // After a push: the differences shift's would have given, from those of
   // the window one row before (same operands, same values).
   __device__ __forceinline__ void advance() {
-    d1 = d2; d2 = d3; d3 = p1 - p0;
-    D1 = D2; D2 = p1 - m1;
+    d1 = d2; d2 = d3; d3 = carried(p1 - p0);
+    D1 = D2; D2 = carried(p1 - m1);
   }
   // mc_face of the window's face (between m1 and p0).
   __device__ __forceinline__ R face(bool pos, R inv_h, R h, R wdt) const {
@@ -1519,6 +1529,14 @@ struct ColWindow {
                                   pos ? m1 : p0, wind, c);
   }
 };
+
+// The differences of a window that advance() takes from the row before.
+struct WindowSteps {
+  double d1, d2, D1;
+};
+static __device__ __noinline__ WindowSteps window_steps(double m2, double m1, double p0) {
+  return WindowSteps{m1 - m2, p0 - m1, p0 - m2};
+}
 
 // The one-step differences only (d1, d2, d3) of a marching column window.
 template <typename R>
@@ -1535,7 +1553,7 @@ struct ColSteps {
     m2 = m1; m1 = p0; p0 = p1; p1 = next;
   }
   __device__ __forceinline__ void shift(R next) {
-    const R d3n = next - p1;
+    const R d3n = carried(next - p1);
     m2 = m1; m1 = p0; p0 = p1; p1 = next;
     d1 = d2; d2 = d3; d3 = d3n;
   }
@@ -2296,7 +2314,7 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
       if (was_fresh) {
         rw.shift(rn);
         ew.shift(en);
-        const R dv2n = vn - v_prev0, dvpn = vn - v_prevp;
+        const R dv2n = carried(vn - v_prev0), dvpn = carried(vn - v_prevp);
         dvm = dvp;
         dvp = dvpn;
         dv2 = dv2n;
@@ -2995,8 +3013,20 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
     // that row moved, else all of them.  (A shift per row under a branch
     // would be predicated code, its FP64 subtractions taking FP64 issue
     // slots in every warp at rest.)
-    if (fresh) win.advance();
-    else win.refresh();
+    if constexpr (Pr::kMixed) {
+      if (fresh) win.advance();
+      else win.refresh();
+    } else {
+      // (A call: as a plain branch the three differences that a window which
+      // had stood still lacks were predicated, and issued in every row.)
+      win.advance();
+      if (!fresh) {
+        const WindowSteps w = window_steps(win.m2, win.m1, win.p0);
+        win.d1 = w.d1;
+        win.d2 = w.d2;
+        win.D1 = w.D1;
+      }
+    }
     fresh = true;
     const R mass = kU ? Fa + Fb : (Fa + Fb) * hcol;
     if (Pr::zero_skip_coarse(mass)) return mass;
