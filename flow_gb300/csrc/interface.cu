@@ -185,6 +185,18 @@ int st_boundary(int w, int h, const Mesh* mesh, double* arr, int invert) {
   return GB300_OK;
 }
 
+// The fills of two arrays that no kernel comes between: one launch on a
+// single-rank mesh.
+void st_boundary2(int w0, int h0, double* a0, int invert0, int w1, int h1, double* a1, int invert1,
+                  const Mesh* mesh) {
+  if (decomposed(mesh)) {
+    st_boundary(w0, h0, mesh, a0, invert0);
+    st_boundary(w1, h1, mesh, a1, invert1);
+    return;
+  }
+  launch_boundary2(current_stream(), w0, h0, a0, invert0, w1, h1, a1, invert1, mesh->pad);
+}
+
 int st_pressure_acceleration(int nx, int ny, Mesh* mesh, double dt,
                              double* rho_u, double* rho_v, double* u, double* v,
                              const double* P, const double* rho,
@@ -193,8 +205,7 @@ int st_pressure_acceleration(int nx, int ny, Mesh* mesh, double dt,
   cudaStream_t s = current_stream();
   launch_accelerate(s, false, nx, ny, mesh->pad, dt, rho_u, rho_v, u, v, P, P,
                     rho, m);
-  st_boundary(nx + 1, ny, mesh, u, kInvertX);
-  st_boundary(nx, ny + 1, mesh, v, kInvertY);
+  st_boundary2(nx + 1, ny, u, kInvertX, nx, ny + 1, v, kInvertY, mesh);
   return check_launch("pressure_acceleration");
 }
 
@@ -205,12 +216,10 @@ int st_artificial_viscosity(int nx, int ny, Mesh* mesh, double dt, double* Qxx,
   FLOW_TRY(check_mesh(mesh, nx, ny, "artificial_viscosity"));
   cudaStream_t s = current_stream();
   launch_viscous_stress(s, nx, ny, mesh->pad, Qxx, Qyy, u, v, rho);
-  st_boundary(nx, ny, mesh, Qxx, kNoInvert);
-  st_boundary(nx, ny, mesh, Qyy, kNoInvert);
+  st_boundary2(nx, ny, Qxx, kNoInvert, nx, ny, Qyy, kNoInvert, mesh);
   launch_accelerate(s, true, nx, ny, mesh->pad, dt, rho_u, rho_v, u, v, Qxx,
                     Qyy, rho, m);
-  st_boundary(nx + 1, ny, mesh, u, kInvertX);
-  st_boundary(nx, ny + 1, mesh, v, kInvertY);
+  st_boundary2(nx + 1, ny, u, kInvertX, nx, ny + 1, v, kInvertY, mesh);
   return check_launch("artificial_viscosity");
 }
 
@@ -295,8 +304,7 @@ int st_mass_energy_sweep(bool dir_y, int nx, int ny, int first, Mesh* mesh,
   }
   launch_mass_energy_update(s, dir_y, nx, ny, pad, first, dt_h, rho, rho_old,
                             e, F, eF, m);
-  st_boundary(nx, ny, mesh, rho, kNoInvert);
-  st_boundary(nx, ny, mesh, e, kNoInvert);
+  st_boundary2(nx, ny, rho, kNoInvert, nx, ny, e, kNoInvert, mesh);
   return check_launch(dir_y ? "y_mass_and_energy_flux" : "x_mass_and_energy_flux");
 }
 

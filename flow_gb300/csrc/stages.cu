@@ -14,6 +14,7 @@
 
 #include "common.cuh"
 #include "exact_math.cuh"
+#include "precision.cuh"
 #include "stages.h"
 
 namespace flow {
@@ -174,6 +175,98 @@ __device__ __forceinline__ void apply_dt_rule(double g, double dt_h_in, int firs
   ra[kRaDtH] = first_step ? dt : kCT * limited;
 }
 
+// The timestep candidates of one cell (omp3/flow.c:80-90).
+__device__ __forceinline__ double cfl_candidate(double e, double q, double rho, double h) {
+  const double sound = sqrt(kGam * (kGam - 1.0) * e);
+  return h / sqrt(sound * sound + 2.0 * q / rho);
+}
+
+// The smallest candidate of a block's cells, each thread's from its first cell
+// t on in strides: m where it is smaller, else m.  A candidate costs about 45
+// FP64 instructions (two square roots and two quotients), and nearly every one
+// is larger than the smallest by far, so a first pass ranks the cells in FP32
+// by S / h^2 = 1/dt^2 (S = c_s^2 + 2 Q / rho), and the second evaluates
+//   - among the cells without viscous stress, only the largest energy: every
+//     operation of the candidate rounds monotonically, so it is the smallest;
+//   - of the others those within 1e-4 of the block's largest FP32 rank, whose
+//     error is below 1e-5.
+// Returns false, with nothing done, for a block with a cell the ranks do not
+// hold for (negative, infinite or NaN energy or stress, a density that is not
+// positive and normal, ranks outside FP32's middle range, or spacings that are
+// not all one number): its cells are all evaluated.  (1280x1024: 224 us with
+// every cell evaluated, NNN with the ranks.)
+__device__ __forceinline__ bool ranked_min(int w, long long n, int nx, int pad, const double* Qxx,
+                                           const double* Qyy, const double* rho, const double* e,
+                                           const double* celldx, const double* celldy, double* m) {
+  __shared__ unsigned s_rank;
+  __shared__ unsigned long long s_ex, s_ey;
+  const double hx = celldx[pad], hy = celldy[pad];
+  const float ix = 1.0f / f64_to_f32(hx), iy = 1.0f / f64_to_f32(hy);
+  const float kx = ix * ix, ky = iy * iy;
+  const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  if (threadIdx.x == 0) {
+    s_rank = 0u;
+    s_ex = s_ey = 0ull;
+  }
+  // The larger rank of the cell, negative where the ranks do not hold; each
+  // axis's own in rx, ry.
+  auto rank = [&](double ec, double qx, double qy, double r, float& rx, float& ry) {
+    const long long be = dbits(ec), bx = dbits(qx), by = dbits(qy), br = dbits(r);
+    const float ef = f64_to_f32(ec), ir = 2.0f / f64_to_f32(r);
+    rx = fmaf(f64_to_f32(qx), ir, 0.56f * ef) * kx;
+    ry = fmaf(f64_to_f32(qy), ir, 0.56f * ef) * ky;
+    const bool ok = be >= 0 && be < ex::kInf && (bx >= 0 || (bx << 1) == 0) && bx < ex::kInf &&
+                    (by >= 0 || (by << 1) == 0) && by < ex::kInf &&
+                    (unsigned long long)br - 0x0010000000000000ULL < 0x7fe0000000000000ULL;
+    const float k = fmaxf(rx, ry);
+    return ok && k > 1e-30f && k < 1e30f && f64_to_f32(r) > 1e-30f && f64_to_f32(r) < 1e30f ? k
+                                                                                          : -1.0f;
+  };
+  bool ok = true;
+  float best = 0.0f;
+  for (long long t = t0; t < n; t += step) {
+    const int ii = pad + (int)(t / w), jj = pad + (int)(t % w);
+    const size_t c = cidx(nx, ii, jj);
+    float rx, ry;
+    const float k = rank(e[c], Qxx[c], Qyy[c], rho[c], rx, ry);
+    ok = ok && k >= 0.0f && dbits(celldx[jj]) == dbits(hx) && dbits(celldy[ii]) == dbits(hy);
+    best = fmaxf(best, k);
+  }
+  if (!__syncthreads_and(ok)) return false;
+  atomicMax(&s_rank, __float_as_uint(best));  // (non-negative: ordered as integers)
+  __syncthreads();
+  const float bound = __uint_as_float(s_rank) * 0.9999f;
+  unsigned long long ex_x = 0ull, ex_y = 0ull;  // bits of the largest energies, plus one
+  for (long long t = t0; t < n; t += step) {
+    const int ii = pad + (int)(t / w), jj = pad + (int)(t % w);
+    const size_t c = cidx(nx, ii, jj);
+    const double ec = e[c], qx = Qxx[c], qy = Qyy[c], r = rho[c];
+    float rx, ry;
+    rank(ec, qx, qy, r, rx, ry);
+    const unsigned long long be = (unsigned long long)dbits(ec) + 1ull;
+    if (d_is_zero(qx)) {
+      ex_x = be > ex_x ? be : ex_x;
+    } else if (rx >= bound) {
+      *m = dmin(*m, cfl_candidate(ec, qx, r, hx));
+    }
+    if (d_is_zero(qy)) {
+      ex_y = be > ex_y ? be : ex_y;
+    } else if (ry >= bound) {
+      *m = dmin(*m, cfl_candidate(ec, qy, r, hy));
+    }
+  }
+  if (ex_x) atomicMax(&s_ex, ex_x);
+  if (ex_y) atomicMax(&s_ey, ex_y);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // (Without stress 2 Q / rho is a zero.)
+    if (s_ex) *m = dmin(*m, cfl_candidate(dfrom((long long)(s_ex - 1)), 0.0, 1.0, hx));
+    if (s_ey) *m = dmin(*m, cfl_candidate(dfrom((long long)(s_ey - 1)), 0.0, 1.0, hy));
+  }
+  return true;
+}
+
 // local_only: a rank of a decomposed mesh keeps its minimum in ra[kRaMinBits]
 // (the caller reduces it over the ranks and applies the rule, k_dt_rule).
 __global__ void __launch_bounds__(kRedThreads)
@@ -184,17 +277,16 @@ __global__ void __launch_bounds__(kRedThreads)
   const int w = nx - 2 * pad;
   const long long n = (long long)w * (ny - 2 * pad);
   double m = max_dt;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int ii = pad + (int)(t / w);
-    const int jj = pad + (int)(t % w);
-    const size_t c = cidx(nx, ii, jj);
-    const double sound = sqrt(kGam * (kGam - 1.0) * e[c]);
-    const double cfl_x =
-        celldx[jj] / sqrt(sound * sound + 2.0 * Qxx[c] / rho[c]);
-    const double cfl_y =
-        celldy[ii] / sqrt(sound * sound + 2.0 * Qyy[c] / rho[c]);
-    m = dmin(m, dmin(cfl_x, cfl_y));
+  if (!ranked_min(w, n, nx, pad, Qxx, Qyy, rho, e, celldx, celldy, &m)) {
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
+         t += (long long)gridDim.x * blockDim.x) {
+      const int ii = pad + (int)(t / w);
+      const int jj = pad + (int)(t % w);
+      const size_t c = cidx(nx, ii, jj);
+      const double cfl_x = cfl_candidate(e[c], Qxx[c], rho[c], celldx[jj]);
+      const double cfl_y = cfl_candidate(e[c], Qyy[c], rho[c], celldy[ii]);
+      m = dmin(m, dmin(cfl_x, cfl_y));
+    }
   }
   __shared__ double s_part[kRedThreads / 32];
   __shared__ bool s_last;
@@ -621,9 +713,8 @@ __global__ void k_momentum_update(int nx, int ny, int pad, double dt_h,
 // interior, negated once per mirrored axis that is inverted; this equals
 // filling the x walls over the interior rows and then copying whole rows for
 // the y walls.  Needs at least `pad` interior points per axis.
-__global__ void k_boundary(int w, int h, int pad, double* arr, int flip_x,
-                           int flip_y) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+__device__ __forceinline__ void boundary_point(long long t, int w, int h, int pad, double* arr,
+                                               int flip_x, int flip_y) {
   const long long n_rows = 2LL * pad * w;
   const long long n_cols = 2LL * pad * (h - 2 * pad);
   if (t >= n_rows + n_cols) return;
@@ -647,6 +738,18 @@ __global__ void k_boundary(int w, int h, int pad, double* arr, int flip_x,
   else if (ii >= h - pad) { si = 2 * (h - pad) - 1 - ii; neg ^= (flip_y != 0); }
   const double val = arr[(size_t)si * w + sj];
   arr[(size_t)ii * w + jj] = neg ? -val : val;
+}
+
+__global__ void k_boundary(int w, int h, int pad, double* arr, int flip_x, int flip_y) {
+  boundary_point(blockIdx.x * (long long)blockDim.x + threadIdx.x, w, h, pad, arr, flip_x, flip_y);
+}
+// Two arrays in one launch (blockIdx.y): a fill of a few hundred KB takes 4 to 5
+// us, most of it the launch.
+__global__ void k_boundary2(int w0, int h0, double* a0, int flip_x0, int flip_y0, int w1, int h1,
+                            double* a1, int flip_x1, int flip_y1, int pad) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (blockIdx.y == 0) boundary_point(t, w0, h0, pad, a0, flip_x0, flip_y0);
+  else boundary_point(t, w1, h1, pad, a1, flip_x1, flip_y1);
 }
 
 // The x-wall part of the reflective fill (ghost columns of the interior rows)
@@ -899,6 +1002,18 @@ void launch_boundary(cudaStream_t s, int w, int h, int pad, double* arr,
   const int threads = 256;
   k_boundary<<<(unsigned)((n + threads - 1) / threads), threads, 0, s>>>(
       w, h, pad, arr, invert == kInvertX, invert == kInvertY);
+}
+
+void launch_boundary2(cudaStream_t s, int w0, int h0, double* a0, int invert0, int w1, int h1,
+                      double* a1, int invert1, int pad) {
+  const long long n0 = 2LL * pad * w0 + 2LL * pad * (h0 - 2 * pad);
+  const long long n1 = 2LL * pad * w1 + 2LL * pad * (h1 - 2 * pad);
+  const long long n = n0 > n1 ? n0 : n1;
+  if (n <= 0) return;
+  const int threads = 256;
+  k_boundary2<<<dim3((unsigned)((n + threads - 1) / threads), 2u), threads, 0, s>>>(
+      w0, h0, a0, invert0 == kInvertX, invert0 == kInvertY, w1, h1, a1, invert1 == kInvertX,
+      invert1 == kInvertY, pad);
 }
 
 void launch_copy(cudaStream_t s, size_t n, double* dst, const double* src) {

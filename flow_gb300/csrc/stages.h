@@ -80,6 +80,9 @@ void launch_momentum_update(cudaStream_t s, int which, int nx, int ny, int pad,
 // Reflective ghost fill of a w x h array; invert is 0, 1 (x) or 2 (y).
 void launch_boundary(cudaStream_t s, int w, int h, int pad, double* arr,
                      int invert);
+// The ghost fills of two arrays as one launch.
+void launch_boundary2(cudaStream_t s, int w0, int h0, double* a0, int invert0, int w1, int h1,
+                      double* a1, int invert1, int pad);
 void launch_copy(cudaStream_t s, size_t n, double* dst, const double* src);
 int reduce_blocks(int nx, int ny, int pad, int partials_per_block);
 

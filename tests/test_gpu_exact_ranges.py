@@ -57,3 +57,32 @@ def test_exact_steps_over_the_range(rho, e, width, nx, ny):
                     hm.mesh.dt, hm.mesh.dt_h = got
     finally:
         fg.set_mode(fg.MODE_FUSED)
+
+
+@pytest.mark.parametrize("stress", ["none", "some", "all", "one_axis"])
+@pytest.mark.parametrize("nx,ny", [(31, 5), (700, 640), (1024, 512)])
+def test_timestep_minimum_by_ranks(stress, nx, ny):
+    """The CFL minimum evaluates only the cells that FP32 ranks leave in
+    question; the mesh sizes give a thread no cell, one, and several."""
+    import torch
+
+    import flow_gb300 as fg
+    from flow_gb300 import problems
+    p = problems.sod(nx, ny)
+    rng = np.random.default_rng(nx + len(stress))
+    sim = fg.DeviceSim(p)
+    hm = O.HostMesh(nx, ny, dt=p.dt_param)
+    st = O.HostState(hm)
+    shape = (p.ny, p.nx)
+    e = np.round(rng.uniform(0.5, 2.5, shape), 2)  # (many equal energies)
+    keep = {"none": 0.0, "some": 0.3, "all": 1.0, "one_axis": 0.5}[stress]
+    q = [rng.uniform(0.0, 3.0, shape) * (rng.random(shape) < keep) for _ in range(2)]
+    if stress == "one_axis":
+        q[1][:] = 0.0
+    fields = {"rho": rng.uniform(0.1, 2.0, shape), "e": e, "Qxx": q[0], "Qyy": q[1]}
+    for k, a in fields.items():
+        sim.a[k].copy_(torch.from_numpy(np.ascontiguousarray(a).reshape(-1)))
+        np.asarray(st[k]).reshape(-1)[: a.size] = a.reshape(-1)
+    sim.initial_timestep()
+    O.initial_timestep(hm, st)
+    assert (sim.mesh.dt, sim.mesh.dt_h) == (hm.mesh.dt, hm.mesh.dt_h)
