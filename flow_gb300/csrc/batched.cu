@@ -98,7 +98,7 @@ __device__ __forceinline__ int shape_of(int ph) {
 // instance, their tiles ran slower.)  A call per tile costs nothing per cell.
 template <typename R, int kPh>
 __device__ __noinline__ void tile_call(const Instance<R>& __restrict__ I, int tx, int ty) {
-  const bool uni = mesh_uniform(I.a.mesh);
+  const bool uni = mesh_uniform<R>(I.a.mesh);
   switch (kPh) {
     case kPhMomUxV: tile_mom_x<R, false, true, false>(I.a, tx, ty, uni); break;
     case kPhMomUx: tile_mom_x<R, false, false, false>(I.a, tx, ty, uni); break;
@@ -113,7 +113,7 @@ __device__ __noinline__ void tile_call(const Instance<R>& __restrict__ I, int tx
 
 template <typename R>
 __device__ __forceinline__ void run_tile(int ph, const Instance<R>& I, int tx, int ty) {
-  const bool uni = mesh_uniform(I.a.mesh);
+  const bool uni = mesh_uniform<R>(I.a.mesh);
   switch (ph) {
     case kPhPressure: tile_lag_pressure(I.a, tx, ty, uni); break;
     case kPhViscosity: tile_lag_viscosity(I.a, tx, ty); break;
@@ -280,7 +280,7 @@ __host__ __device__ constexpr int phase_shape() {
 // (copy rings and early first loads on).
 template <typename R, int kPh>
 __device__ __forceinline__ void phase_tile(const Instance<R>& I, int tx, int ty) {
-  const bool uni = mesh_uniform(I.a.mesh);
+  const bool uni = mesh_uniform<R>(I.a.mesh);
   if constexpr (kPh == kPhPressure) tile_lag_pressure(I.a, tx, ty, uni);
   else if constexpr (kPh == kPhViscosity) tile_lag_viscosity(I.a, tx, ty);
   else if constexpr (kPh == kPhAccel) tile_lag_viscous_accel<R, true>(I.a, tx, ty, uni);

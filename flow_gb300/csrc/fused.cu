@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kCols) k_lag_pressure(const StepArgs<R> a) {
     }
   }
   int bx, by;
-  const bool uni = mesh_uniform(a.mesh);
+  const bool uni = mesh_uniform<R>(a.mesh);
   if (block_tile<kMd>(a, bx, by)) {
     tile_lag_pressure<R, (kMd != kNoFlags), (kMd != kListed)>(a, bx, by, uni);
   }
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kCols) k_lag_viscous_accel(const StepArgs<R> a
   pdl_wait();
   pdl_trigger();
   int bx, by;
-  const bool uni = mesh_uniform(a.mesh);
+  const bool uni = mesh_uniform<R>(a.mesh);
   if (block_tile<kMd>(a, bx, by)) {
     tile_lag_viscous_accel<R, true, (kMd != kNoFlags)>(a, bx, by, uni);
   }
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kCols) k_lag_energy_dt(const StepArgs<R> a) {
   pdl_trigger();
   int bx, by;
   constexpr bool kFlags = kMd != kNoFlags;
-  const bool uni = mesh_uniform(a.mesh);
+  const bool uni = mesh_uniform<R>(a.mesh);
   if (!block_tile<kMd>(a, bx, by)) return;
   tile_lag_energy_dt<R, true, kFlags, (kMd != kListed)>(a, bx, by, uni,
                                                        kFlags ? &s_tile_min : nullptr);
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 8 : 7) k_mass_sweep_x
   pdl_wait();
   pdl_trigger();
   int bx, by;
-  const bool uni = mesh_uniform(a.mesh);
+  const bool uni = mesh_uniform<R>(a.mesh);
   if (block_tile<kMd>(a, bx, by)) {
     tile_mass_sweep_x<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by, uni);
   }
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 7 : 6) k_mass_sweep_y
   pdl_wait();
   pdl_trigger();
   int bx, by;
-  const bool uni = mesh_uniform(a.mesh);
+  const bool uni = mesh_uniform<R>(a.mesh);
   if (block_tile<kMd>(a, bx, by)) {
     tile_mass_sweep_y<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by, uni);
   }
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kCols) k_mom(const StepArgs<R> a, const StepAr
                                                const ListArgs l) {
   pdl_wait();
   pdl_trigger();
-  const bool uni = mesh_uniform(a.mesh);
+  const bool uni = mesh_uniform<R>(a.mesh);
   const int k = (int)blockIdx.x;
   if constexpr (kLists) {
     const int n = (int)gridDim.x - 2 * l.blocks;
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(lagf::kT, 4) k_lag_fused(const lagf::LagArgs a
   pdl_wait();
   pdl_trigger();
   lagf::CflBest cfl;
-  const bool uniform = mesh_uniform(a.mesh);
+  const bool uniform = mesh_uniform<double>(a.mesh);
   const bool ok = uniform
                       ? lagf::lag_tile<true>(a, sm, blockIdx.x, blockIdx.y, cfl)
                       : lagf::lag_tile<false>(a, sm, blockIdx.x, blockIdx.y, cfl);

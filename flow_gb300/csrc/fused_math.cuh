@@ -203,6 +203,16 @@ __device__ __forceinline__ double d_rcp_seed(double x) {
                       (long long)(unsigned)(b << 29) + ((long long)k << 10);
   return dfrom2((int)(m >> 32) ^ (hi & (int)0x80000000), (int)m);
 }
+// 1/x for finite normal non-zero x: MUFU seed, two Newton-Raphson steps (the
+// mixed form's spacing factors, once per tile).
+__device__ __forceinline__ double d_rcp_newton(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  double e = fma(-x, r, 1.0);
+  r = fma(r, e, r);
+  e = fma(-x, r, 1.0);
+  return fma(r, e, r);
+}
 // 1/x for finite normal non-zero x: the seed and one Newton step.
 __device__ __forceinline__ double d_rcp(double x) {
   const double r = d_rcp_seed(x);

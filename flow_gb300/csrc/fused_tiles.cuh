@@ -76,9 +76,9 @@ struct StepArgs {
   double* ra;                  // caller scratch (reduce_array)
   unsigned long long* min_slot;  // running CFL minimum (FP64 bit pattern)
   // The mesh test's result (formed on the device at the start of a run): [0]
-  // 1 (uint64) when the mesh is uniform -- every celldx and edgedx one number,
-  // every celldy and edgedy one number -- then [1], [2] the two spacings and
-  // [3], [4] their reciprocals.
+  // non-zero (uint64) when the mesh is uniform -- every celldx and edgedx one
+  // number, every celldy and edgedy one number --, 3 when both are powers of
+  // two, then [1], [2] the two spacings and [3], [4] their reciprocals.
   const double* mesh;
   double* dt_slot;             // [0] dt, [1] dt_h for the advection phase
   double dt, dt_h, max_dt;     // Lagrangian-phase pair (host values), max_dt
@@ -376,8 +376,14 @@ __device__ __forceinline__ bool tile_near_edge(int nx, int ny, int pad, int col0
 struct UniformMesh {
   double dx, dy, ix, iy;
 };
+// Whether a form's tiles take the uniform variants: the mixed form's mass
+// sweeps (its others have none) only where the spacings are powers of two, so
+// that folding them rounds nothing.  An FP64 rounding there now and then turns
+// an FP32 one (the shadows of density and energy), which the timestep shows.
+template <typename R>
 __device__ __forceinline__ bool mesh_uniform(const double* mesh) {
-  return *reinterpret_cast<const unsigned long long*>(mesh) == 1ull;
+  const unsigned long long f = *reinterpret_cast<const unsigned long long*>(mesh);
+  return Prec<R>::kMixed ? f == 3ull : f != 0ull;
 }
 __device__ __forceinline__ UniformMesh uniform_mesh(const double* mesh) {
   return UniformMesh{mesh[1], mesh[2], mesh[3], mesh[4]};
@@ -408,7 +414,8 @@ __device__ __forceinline__ void mesh_test_block(int nx, int ny, const double* ce
   }
   ok = __syncthreads_and(ok) != 0;
   if (threadIdx.x == 0) {
-    *reinterpret_cast<unsigned long long*>(mesh) = ok ? 1ull : 0ull;
+    *reinterpret_cast<unsigned long long*>(mesh) =
+        !ok ? 0ull : (d_is_pow2(dx) && d_is_pow2(dy)) ? 3ull : 1ull;
     mesh[1] = dx;
     mesh[2] = dy;
     mesh[3] = 1.0 / dx;
@@ -427,7 +434,7 @@ __device__ __forceinline__ void mesh_test_block(int nx, int ny, const double* ce
 // the general tile takes four (a quotient corrected to the reference's
 // rounding), and a tile reads no spacing arrays.  Each folded product is
 // rounded once per step instead of once per cell.
-// uni: mesh_uniform(a.mesh), which a kernel reads beside its tile's index, so
+// uni: mesh_uniform<R>(a.mesh), which a kernel reads beside its tile's index, so
 // that the two loads are in flight together.
 #define FLOW_UNIFORM_DISPATCH(R, CALL_TRUE, CALL_FALSE) \
   do {                                                  \
@@ -481,7 +488,7 @@ __device__ __forceinline__ R geo_half(double h) { return Prec<R>::from_d(d_half(
 template <typename R>
 __device__ __forceinline__ double geo_rcp_d(double h) {
   if constexpr (Prec<R>::kMixed) {
-    return d_rcp(h);
+    return d_rcp_newton(h);
   } else {
     return 1.0 / h;
   }

