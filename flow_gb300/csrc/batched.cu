@@ -387,6 +387,7 @@ struct BatchImpl {
   void* d_inst = nullptr;
   size_t tables_off = 0;
   int rows = kDefaultRows;
+  bool rows_set = false;  // by the caller (else chosen from the instances' tiles)
   int ctas_per_sm = 0;  // 0 = as many as fit
   int order = 0;        // 0 largest first, 1 input order
   int grid = 0;
@@ -654,7 +655,32 @@ int choose_grid(BatchImpl& B) {
   return GB300_OK;
 }
 
+// The tile height with the least time on the busiest SM, as the single-problem
+// step chooses it (fused.cu): (rows + 1.5) * max(tiles / SMs, the tiles whose
+// latencies an SM hides behind one another).  An ensemble of five meshes of 90
+// to 300 a side left most SMs one tile of 16 rows: 204 us a mixed step.
+int pick_batch_rows(const BatchImpl& B) {
+  const double overlap = B.precision ? 6.0 : 3.0;
+  int best = kDefaultRows;
+  double best_cost = 0.0;
+  for (int rows = kDefaultRows; rows >= 1; rows /= 2) {
+    long long tiles = 0;
+    for (int i = 0; i < B.n; ++i) {
+      int tx = 0;
+      tiles += tiles_for(kShInterior, B.gnx[i] + 4, B.gny[i] + 4, rows, &tx);
+    }
+    const double per_sm = (double)((tiles + num_sms() - 1) / num_sms());
+    const double cost = (rows + 1.5) * (per_sm > overlap ? per_sm : overlap);
+    if (rows == kDefaultRows || cost < best_cost) {
+      best = rows;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 int retune(BatchImpl& B) {
+  if (!B.rows_set) B.rows = pick_batch_rows(B);
   B.perm.resize(B.n);
   std::iota(B.perm.begin(), B.perm.end(), 0);
   if (B.order == 0) {
@@ -866,6 +892,7 @@ int gb300_batch_set_tuning(GB300Batch* b, int rows, int ctas_per_sm, int order) 
   }
   BatchImpl& B = b->impl;
   B.rows = rows;
+  B.rows_set = true;
   B.ctas_per_sm = ctas_per_sm;
   B.order = order;
   return B.pool ? retune(B) : GB300_OK;
