@@ -769,16 +769,28 @@ void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
   }
 }
 
+// Copies the step's header (reduce_array before the partials) to page-locked
+// host memory.
+__global__ void k_step_head(const double* ra, double* host) {
+  pdl_wait();
+  if (threadIdx.x < kRaPartial) host[threadIdx.x] = ra[threadIdx.x];
+}
+
 int finish_step(cudaStream_t s, Mesh* mesh, double* ra, StepProfiler& prof,
                 const char* where, unsigned* counts) {
+  // dt, dt_h (slots 0, 1), the status word (slot 5) and the lengths of the
+  // tile lists (slots 13 .. 16) at once.
+  double local[kRaPartial];
+  double* head = pinned_head();
+  if (head) launch_pdl_block(k_step_head, dim3(1), dim3(32), s, ra, head);
   {
     const int st = check_launch(where);
     if (st != GB300_OK) return st;
   }
-  // dt, dt_h (slots 0, 1), the status word (slot 5) and the lengths of the
-  // tile lists (slots 13 .. 16) in one copy.
-  double head[kRaPartial];
-  cudaMemcpyAsync(head, ra + kRaDt, sizeof(head), cudaMemcpyDeviceToHost, s);
+  if (!head) {
+    head = local;
+    cudaMemcpyAsync(head, ra + kRaDt, sizeof(local), cudaMemcpyDeviceToHost, s);
+  }
   const cudaError_t err = cudaStreamSynchronize(s);
   if (err != cudaSuccess) {
     return record_error(GB300_ERR_CUDA, "%s: %s", where, cudaGetErrorString(err));
@@ -1112,6 +1124,7 @@ struct ConsArgs {
   const double* rho;
   const double* e;
   double* ra;
+  double* host;                // page-locked memory for the totals too, or null
   double* part;                // 2 doubles per tile: sum rho, sum rho e
   int nx, ny, pad, tiles_x, tiles, rows;
   const unsigned char* marks;  // the last step's skip marks, or null
@@ -1243,6 +1256,10 @@ __global__ void __launch_bounds__(kCols) k_conservation_tiles(const ConsArgs c) 
   if (threadIdx.x == 0) {
     c.ra[kRaMass] = ta;
     c.ra[kRaEnergy] = tb;
+    if (c.host) {
+      c.host[0] = ta;
+      c.host[1] = tb;
+    }
     *reinterpret_cast<unsigned long long*>(c.ra + kRaTicket) = 0ull;
   }
 }
@@ -1265,7 +1282,7 @@ thread_local ConsRecord t_cons;
 }  // namespace
 
 bool tile_conservation(int nx, int ny, int pad, const double* rho, const double* e,
-                       double* ra, cudaStream_t s) {
+                       double* ra, double* host, cudaStream_t s) {
   const FlagLayout L = flag_layout(nx, ny, pad);
   if (!L.fits) return false;
   unsigned* base = reinterpret_cast<unsigned*>(ra + kRaQFlags);
@@ -1273,6 +1290,7 @@ bool tile_conservation(int nx, int ny, int pad, const double* rho, const double*
   c.rho = rho;
   c.e = e;
   c.ra = ra;
+  c.host = host;
   c.part = reinterpret_cast<double*>(base + L.cons);
   c.nx = nx;
   c.ny = ny;

@@ -26,8 +26,11 @@ void note_state_write();
 // partial sums stay in reduce_array's flag region, kept across calls for tiles
 // at rest through the fused step between them; false (nothing launched) when
 // reduce_array is too small for the region.
+// host: page-locked memory for the two totals too, or null.
 bool tile_conservation(int nx, int ny, int pad, const double* rho, const double* e,
-                       double* ra, cudaStream_t s);
+                       double* ra, double* host, cudaStream_t s);
+// Page-locked doubles of this host thread (kRaPartial of them), or null.
+double* pinned_head();
 // Kernel launches issued by this library (the fused step's kernels and the
 // conservation totals), for gb300_launch_count.
 void count_launches(unsigned n);
