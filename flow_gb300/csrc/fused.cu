@@ -1215,20 +1215,30 @@ __global__ void __launch_bounds__(kCols) k_conservation_tiles(const ConsArgs c) 
     const int j = c0 + threadIdx.x;
     double ms = 0.0, es = 0.0;
     if (j < c1) {
+      // The next eight rows are in flight while these are summed.
       constexpr int kB = 8;
-      for (int ib = r0; ib < r1; ib += kB) {
-        double rv[kB], ev[kB];
+      double rv[kB], ev[kB];
+      auto load = [&](int ib) {
 #pragma unroll
         for (int q = 0; q < kB; ++q) {
-          const bool in = ib + q < r1;
+          const bool in = ib + q < r1;  // (rows past the end count as zeros)
           const size_t k = (size_t)(in ? ib + q : r0) * c.nx + j;
           rv[q] = in ? c.rho[k] : 0.0;
           ev[q] = in ? c.e[k] : 0.0;
         }
-        // (Rows past the end hold zeros.)
-        ms = __dadd_rn(ms, sum8_aligned(rv));
+      };
+      load(r0);
+      for (int ib = r0; ib < r1; ib += kB) {
+        double rc[kB], ec[kB];
 #pragma unroll
-        for (int q = 0; q < kB; ++q) es = __fma_rn(rv[q], ev[q], es);
+        for (int q = 0; q < kB; ++q) {
+          rc[q] = rv[q];
+          ec[q] = ev[q];
+        }
+        if (ib + kB < r1) load(ib + kB);
+        ms = __dadd_rn(ms, sum8_aligned(rc));
+#pragma unroll
+        for (int q = 0; q < kB; ++q) es = __fma_rn(rc[q], ec[q], es);
       }
     }
     const double tm = block_sum_fixed(ms, s_w);
@@ -1247,9 +1257,22 @@ __global__ void __launch_bounds__(kCols) k_conservation_tiles(const ConsArgs c) 
   if (!s_last) return;
   __threadfence();
   double a = 0.0, b = 0.0;
-  for (int k = threadIdx.x; k < c.tiles; k += blockDim.x) {
-    a = __dadd_rn(a, __ldcg(c.part + 2 * (size_t)k));
-    b = __dadd_rn(b, __ldcg(c.part + 2 * (size_t)k + 1));
+  // (Eight pairs in flight: one after another the loads took 20 us of a large
+  // mesh's call.  The partials are 8-byte aligned, as reduce_array is.)
+  constexpr int kP = 8;
+  for (int k0 = threadIdx.x; k0 < c.tiles; k0 += kP * kCols) {
+    double pm[kP], pe[kP];
+#pragma unroll
+    for (int q = 0; q < kP; ++q) {
+      const int k = k0 + q * kCols;
+      pm[q] = k < c.tiles ? __ldcg(c.part + 2 * (size_t)k) : 0.0;
+      pe[q] = k < c.tiles ? __ldcg(c.part + 2 * (size_t)k + 1) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < kP; ++q) {
+      a = __dadd_rn(a, pm[q]);
+      b = __dadd_rn(b, pe[q]);
+    }
   }
   const double ta = block_sum_fixed(a, s_w);
   const double tb = block_sum_fixed(b, s_w);
