@@ -79,6 +79,14 @@ __global__ void __launch_bounds__(kCols) k_lag_pressure(const StepArgs<R> a) {
       }
     }
   }
+  if constexpr (kMd == kListed) {
+    // The skip marks this step leaves: set for every tile, those the first
+    // sweep visits it writes itself.
+    unsigned* marks = reinterpret_cast<unsigned*>(a.skipf);
+    for (int q = blockIdx.x * kCols + threadIdx.x; q < a.skip_words; q += gridDim.x * kCols) {
+      marks[q] = 0x01010101u;
+    }
+  }
   int bx, by;
   const bool uni = mesh_uniform<R>(a.mesh);
   if (block_tile<kMd>(a, bx, by)) {
@@ -133,32 +141,6 @@ __device__ __forceinline__ void store_dt(const StepArgs<R>& a) {
     a.dt_slot[1] = p.dt_h;
   }
 }
-// With flags, the mass-flux flags (a.fxflag, a.fyflag) are kept -- the sweeps store only warps with a non-zero mass flux, and the
-// momentum pairs load only those.
-template <typename R, bool kFirst, int kMd>
-__global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 8 : 7) k_mass_sweep_x(const StepArgs<R> a,
-                                                        const SweepArgs<R> s) {
-  pdl_wait();
-  pdl_trigger();
-  int bx, by;
-  const bool uni = mesh_uniform<R>(a.mesh);
-  if (block_tile<kMd>(a, bx, by)) {
-    tile_mass_sweep_x<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by, uni);
-  }
-  store_dt<R, kFirst>(a);
-}
-template <typename R, bool kFirst, int kMd>
-__global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 7 : 6) k_mass_sweep_y(const StepArgs<R> a,
-                                                        const SweepArgs<R> s) {
-  pdl_wait();
-  pdl_trigger();
-  int bx, by;
-  const bool uni = mesh_uniform<R>(a.mesh);
-  if (block_tile<kMd>(a, bx, by)) {
-    tile_mass_sweep_y<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by, uni);
-  }
-  store_dt<R, kFirst>(a);
-}
 // ---------------------------------------------------------------------------
 // Tile lists: the tiles the next step has to visit.  A cell in a tile the
 // step's first sweep marked was at rest through the step (StepArgs::rest).  In
@@ -178,8 +160,6 @@ struct ListArgs {
   int nx, ny, pad;
   const unsigned char* marks;  // this step's skip marks
   int mark_w, mark_tiles_x, mark_rows;
-  unsigned* next_marks;        // the next step's half, filled with ones here
-  int next_words;
   int tx[2], bands;            // columns of 128- and 127-wide tiles, 16-row bands
   int blocks;                  // of each width (0: no lists)
   unsigned* list[2];           // [heights][tx * bands * 16 / height] each
@@ -202,9 +182,6 @@ __host__ __device__ inline size_t list_offset(int tx, int bands, int h) {
 __device__ __forceinline__ void tile_lists(const ListArgs& l, int block) {
   const int wd = block < l.blocks ? 0 : 1;  // the tile width
   const int t = (block - wd * l.blocks) * kCols + (int)threadIdx.x;
-  if (wd == 0) {
-    for (int q = t; q < l.next_words; q += l.blocks * kCols) l.next_marks[q] = 0x01010101u;
-  }
   constexpr int kSub = kListBand / 2;
   const int lane = threadIdx.x & 31, sub = lane & (kSub - 1), grp = lane & ~(kSub - 1);
   const int tx = l.tx[wd];
@@ -297,6 +274,62 @@ unsigned acts[kListHeights], all[kListHeights];
 
 // Momentum pairs (flux fused with its update): x pairs share a row's fluxes
 // through shared memory (127 faces per CTA), y pairs march down columns.
+// Tile k of a 1-D launch.
+template <int kMd, typename R>
+__device__ __forceinline__ bool line_tile(const StepArgs<R>& a, int k, int& bx, int& by) {
+  if constexpr (kMd == kListed) {
+    return listed_tile(a, k, bx, by);
+  } else {
+    by = k / a.grid_x;
+    bx = k - by * a.grid_x;
+    return true;
+  }
+}
+// kLists (a second sweep): the last 2 l.blocks blocks of the (1-D) launch form
+// the next step's tile lists beside the sweep, which reads neither the marks of
+// the tiles it visits later nor the minima the lists are formed from in a way
+// they change; as a kernel of their own the lists took 7 to 20 us a step, and
+// beside the step's last launch, which is short, 5.
+// With flags, the mass-flux flags (a.fxflag, a.fyflag) are kept -- the sweeps store only warps with a non-zero mass flux, and the
+// momentum pairs load only those.
+template <typename R, bool kFirst, int kMd, bool kLists>
+__global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 8 : 7) k_mass_sweep_x(
+    const StepArgs<R> a, const SweepArgs<R> s, const ListArgs l) {
+  pdl_wait();
+  pdl_trigger();
+  int bx, by;
+  const bool uni = mesh_uniform<R>(a.mesh);
+  if constexpr (kLists) {
+    const int n = (int)gridDim.x - 2 * l.blocks;
+    if ((int)blockIdx.x >= n) {
+      tile_lists(l, (int)blockIdx.x - n);
+      return;
+    }
+  }
+  if (kLists ? line_tile<kMd>(a, blockIdx.x, bx, by) : block_tile<kMd>(a, bx, by)) {
+    tile_mass_sweep_x<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by, uni);
+  }
+  store_dt<R, kFirst>(a);
+}
+template <typename R, bool kFirst, int kMd, bool kLists>
+__global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 7 : 6) k_mass_sweep_y(
+    const StepArgs<R> a, const SweepArgs<R> s, const ListArgs l) {
+  pdl_wait();
+  pdl_trigger();
+  int bx, by;
+  const bool uni = mesh_uniform<R>(a.mesh);
+  if constexpr (kLists) {
+    const int n = (int)gridDim.x - 2 * l.blocks;
+    if ((int)blockIdx.x >= n) {
+      tile_lists(l, (int)blockIdx.x - n);
+      return;
+    }
+  }
+  if (kLists ? line_tile<kMd>(a, blockIdx.x, bx, by) : block_tile<kMd>(a, bx, by)) {
+    tile_mass_sweep_y<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by, uni);
+  }
+  store_dt<R, kFirst>(a);
+}
 // One launch runs one pair, or two that do not read what the other writes
 // (launch_step): two dependent launches of a few microseconds each become one.
 enum : int { kNone = 0, kXU = 1, kXV = 2, kYU = 3, kYV = 4 };  // direction and momentum
@@ -308,44 +341,21 @@ __device__ __forceinline__ void pair_tile(const StepArgs<R>& a, int bx, int by, 
   else if constexpr (kPair == kYU) tile_mom_y<R, false, kVel, true, kFl, kTest>(a, bx, by, uni);
   else if constexpr (kPair == kYV) tile_mom_y<R, true, kVel, true, kFl, kTest>(a, bx, by, uni);
 }
-// Block k of a 1-D launch over pair tiles.
-template <int kMd, typename R>
-__device__ __forceinline__ bool pair_block(const StepArgs<R>& a, int k, int& bx, int& by) {
-  if constexpr (kMd == kListed) {
-    return listed_tile(a, k, bx, by);
-  } else {
-    by = k / a.grid_x;
-    bx = k - by * a.grid_x;
-    return true;
-  }
-}
-// The tiles of pair A (blocks 0 .. na - 1), then those of pair B; then, in the
-// step's last launch (kLists), 2 l.blocks blocks that form the next step's
-// tile lists beside it (the pairs read neither the marks nor the minima they
-// are formed from; on its own the list kernel took 7 to 20 us a step, mostly
-// latency).
-template <typename R, int kA, bool kVelA, int kB, bool kVelB, int kMd, bool kLists>
-__global__ void __launch_bounds__(kCols) k_mom(const StepArgs<R> a, const StepArgs<R> b, int na,
-                                               const ListArgs l) {
+// The tiles of pair A (blocks 0 .. na - 1), then those of pair B.
+template <typename R, int kA, bool kVelA, int kB, bool kVelB, int kMd>
+__global__ void __launch_bounds__(kCols) k_mom(const StepArgs<R> a, const StepArgs<R> b, int na) {
   pdl_wait();
   pdl_trigger();
   const bool uni = mesh_uniform<R>(a.mesh);
   const int k = (int)blockIdx.x;
-  if constexpr (kLists) {
-    const int n = (int)gridDim.x - 2 * l.blocks;
-    if (k >= n) {
-      tile_lists(l, k - n);
-      return;
-    }
-  }
   int bx, by;
   if constexpr (kB != kNone) {
     if (k >= na) {
-      if (pair_block<kMd>(b, k - na, bx, by)) pair_tile<R, kB, kVelB, kMd>(b, bx, by, uni);
+      if (line_tile<kMd>(b, k - na, bx, by)) pair_tile<R, kB, kVelB, kMd>(b, bx, by, uni);
       return;
     }
   }
-  if (pair_block<kMd>(a, k, bx, by)) pair_tile<R, kA, kVelA, kMd>(a, bx, by, uni);
+  if (line_tile<kMd>(a, k, bx, by)) pair_tile<R, kA, kVelA, kMd>(a, bx, by, uni);
 }
 
 // The whole Lagrangian phase of the FP64 step in one kernel (lag_fused.cuh):
@@ -626,44 +636,54 @@ StepArgs<R> pair_args(const StepArgs<R>& a0, const StepRows& sr, const TileLists
   return a;
 }
 template <typename R, int kA, bool kVelA, int kB, bool kVelB>
-void launch_mom(cudaStream_t s, const StepArgs<R>& a0, const StepRows& sr, const TileLists& tl,
-                const ListArgs* lists) {
+void launch_mom(cudaStream_t s, const StepArgs<R>& a0, const StepRows& sr, const TileLists& tl) {
   int na = 0, nb = 0;
   const StepArgs<R> a = pair_args<R, kA, kVelA>(a0, sr, tl, na);
   const StepArgs<R> b = pair_args<R, kB, kVelB>(a0, sr, tl, nb);
   if (kB == kNone) nb = 0;
-  const int md = step_mode(a);
-  if (lists && lists->blocks) {
-    const dim3 g((unsigned)(na + nb + 2 * lists->blocks));
-    if (md == kListed) launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kListed, true>, g, s, a, b, na, *lists);
-    else launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kWhole, true>, g, s, a, b, na, *lists);
-    return;
-  }
   const dim3 g((unsigned)(na + nb));
-  const ListArgs l{};
-  if (md == kNoFlags) launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kNoFlags, false>, g, s, a, b, na, l);
-  else if (md == kWhole) launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kWhole, false>, g, s, a, b, na, l);
-  else launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kListed, false>, g, s, a, b, na, l);
+  const int md = step_mode(a);
+  if (md == kNoFlags) launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kNoFlags>, g, s, a, b, na);
+  else if (md == kWhole) launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kWhole>, g, s, a, b, na);
+  else launch_pdl(k_mom<R, kA, kVelA, kB, kVelB, kListed>, g, s, a, b, na);
 }
 
-template <typename R>
-void launch_mass(cudaStream_t s, const StepArgs<R>& a0, bool dir_y, bool first,
-                 const SweepArgs<R>& sw, const TileLists& tl) {
+// lists: formed beside the step's second sweep (blocks 0: none).
+template <typename R, bool kY>
+void launch_sweep(cudaStream_t s, const StepArgs<R>& a0, bool first, const SweepArgs<R>& sw,
+                  const TileLists& tl, const ListArgs& lists) {
   StepArgs<R> a = a0;
   const int pad = a.pad;
-  if (dir_y) {
-    const dim3 g = tile_grid(a, tl, 0, strip_grid(a.nx - 2 * pad, a.ny - 2 * pad, a.rows));
-    const int md = step_mode(a);
-    if (first) FLOW_LAUNCH_MODE(md, g, s, (a, sw), k_mass_sweep_y, R, true);
-    else FLOW_LAUNCH_MODE(md, g, s, (a, sw), k_mass_sweep_y, R, false);
+  // The x sweep: faces pad .. nx-pad; every CTA advances 127 columns.
+  const dim3 g = tile_grid(a, tl, kY ? 0 : 1,
+                           kY ? strip_grid(a.nx - 2 * pad, a.ny - 2 * pad, a.rows)
+                              : strip_grid(a.nx + 1 - 2 * pad, a.ny - 2 * pad, a.rows, kCols - 1));
+  const int md = step_mode(a);
+#define FLOW_SWEEP(FIRST, MODE, LISTS, GRID)                                                  \
+  do {                                                                                        \
+    if constexpr (kY) launch_pdl(k_mass_sweep_y<R, FIRST, MODE, LISTS>, GRID, s, a, sw, lists); \
+    else launch_pdl(k_mass_sweep_x<R, FIRST, MODE, LISTS>, GRID, s, a, sw, lists);            \
+  } while (0)
+  if (first) {
+    if (md == kNoFlags) FLOW_SWEEP(true, kNoFlags, false, g);
+    else if (md == kWhole) FLOW_SWEEP(true, kWhole, false, g);
+    else FLOW_SWEEP(true, kListed, false, g);
+  } else if (lists.blocks) {
+    const dim3 line(g.x * g.y + 2 * (unsigned)lists.blocks);
+    if (md == kListed) FLOW_SWEEP(false, kListed, true, line);
+    else FLOW_SWEEP(false, kWhole, true, line);
   } else {
-    // Faces pad .. nx-pad; every CTA advances 127 columns.
-    const dim3 g =
-        tile_grid(a, tl, 1, strip_grid(a.nx + 1 - 2 * pad, a.ny - 2 * pad, a.rows, kCols - 1));
-    const int md = step_mode(a);
-    if (first) FLOW_LAUNCH_MODE(md, g, s, (a, sw), k_mass_sweep_x, R, true);
-    else FLOW_LAUNCH_MODE(md, g, s, (a, sw), k_mass_sweep_x, R, false);
+    if (md == kNoFlags) FLOW_SWEEP(false, kNoFlags, false, g);
+    else if (md == kWhole) FLOW_SWEEP(false, kWhole, false, g);
+    else FLOW_SWEEP(false, kListed, false, g);
   }
+#undef FLOW_SWEEP
+}
+template <typename R>
+void launch_mass(cudaStream_t s, const StepArgs<R>& a, bool dir_y, bool first,
+                 const SweepArgs<R>& sw, const TileLists& tl, const ListArgs& lists) {
+  if (dir_y) launch_sweep<R, true>(s, a, first, sw, tl, lists);
+  else launch_sweep<R, false>(s, a, first, sw, tl, lists);
 }
 
 // Blocks of k_lag_apply: one thread per (mask row, tile) pair, at most 8
@@ -744,9 +764,9 @@ void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
     sw2.e_alt_r = first.e_in_r;
   }
   prof.mark(x_first ? "mass_sweep_x" : "mass_sweep_y");
-  launch_mass(s, as, !x_first, true, sw1, tl);
+  launch_mass(s, as, !x_first, true, sw1, tl, lists);
   prof.mark(x_first ? "mass_sweep_y" : "mass_sweep_x");
-  launch_mass(s, as, x_first, false, sw2, tl);
+  launch_mass(s, as, x_first, false, sw2, tl, lists);
 
   // Momentum: each flux fused with its update, in the reference order; the
   // pair that recomputes a velocity comes first in each chain.  Two pairs share
@@ -756,16 +776,16 @@ void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
   // step the y flux pair of rho_u and the x velocity pair of rho_v.
   if (tt % 2) {
     prof.mark("mom_uFx");
-    launch_mom<R, kXU, true, kNone, false>(s, ad, sr, tl, nullptr);
+    launch_mom<R, kXU, true, kNone, false>(s, ad, sr, tl);
     prof.mark("mom_uFy_vFx");
-    launch_mom<R, kYU, false, kXV, true>(s, ad, sr, tl, nullptr);
+    launch_mom<R, kYU, false, kXV, true>(s, ad, sr, tl);
     prof.mark("mom_vFy");
-    launch_mom<R, kYV, false, kNone, false>(s, ad, sr, tl, &lists);
+    launch_mom<R, kYV, false, kNone, false>(s, ad, sr, tl);
   } else {
     prof.mark("mom_uFy_vFy");
-    launch_mom<R, kYU, true, kYV, true>(s, ad, sr, tl, nullptr);
+    launch_mom<R, kYU, true, kYV, true>(s, ad, sr, tl);
     prof.mark("mom_uFx_vFx");
-    launch_mom<R, kXU, false, kXV, false>(s, ad, sr, tl, &lists);
+    launch_mom<R, kXU, false, kXV, false>(s, ad, sr, tl);
   }
 }
 
@@ -899,6 +919,7 @@ void fill_mesh_args(StepArgs<R>& a, const Mesh* mesh, int tt, double* ra) {
   a.vflag = nullptr;
   a.vf_stride = 0;
   a.skipf = nullptr;
+  a.skip_words = 0;
   a.rest = nullptr;
   a.rest_w = a.rest_tiles_x = a.rest_rows = 0;
   a.cfl_tile = nullptr;
@@ -921,6 +942,7 @@ void fill_mesh_args(StepArgs<R>& a, const Mesh* mesh, int tt, double* ra) {
     a.vf_stride = 4 * L.vtiles;
     unsigned* marks = base + L.marks;
     a.skipf = reinterpret_cast<unsigned char*>(marks + (tt & 1) * L.sk_words);
+    a.skip_words = (int)L.sk_words;
     // The previous step's half, described; take_rest keeps it only when
     // that step was a flagged step on these arrays, and sets its tile height.
     a.rest = reinterpret_cast<unsigned char*>(marks + ((tt + 1) & 1) * L.sk_words);
@@ -1070,8 +1092,6 @@ StepRows take_rest(StepArgs<R>& a, int tt, int form, const std::array<const void
     la.mark_w = x_first ? kCols - 1 : kCols;
     la.mark_tiles_x = x_first ? L.xtiles : L.stride;
     la.mark_rows = rows.sweep;
-    la.next_marks = base + L.marks + ((tt + 1) & 1) * L.sk_words;
-    la.next_words = (int)L.sk_words;
     la.bands = L.list_bands;
     const int tx = L.list_tx[0] > L.list_tx[1] ? L.list_tx[0] : L.list_tx[1];
     la.blocks = (int)(((long long)tx * L.list_bands * (kListBand / 2) + kCols - 1) / kCols);

@@ -113,8 +113,9 @@ struct StepArgs {
   int vf_stride;               // bytes per row: 4 ceil(nx / 128)
   // The sweeps' tile-skip marks (SweepArgs::skip), set with the flags: one
   // byte per sweep tile, ceil((ny - 2 pad) / the sweeps' rows) bands of
-  // max(ceil((nx + 1 - 2 pad) / 127), qm_stride) tiles.
+  // max(ceil((nx + 1 - 2 pad) / 127), qm_stride) tiles, in skip_words words.
   unsigned char* skipf;
+  int skip_words;
   // The skip marks the previous step's first sweep left (its own half of the
   // two mark buffers), or null when this step does not directly follow a
   // flagged step on the same arrays.  Mark x of band b covers the interior
