@@ -27,7 +27,32 @@ inline dim3 grid_for(int rows, int cols) {
   return dim3((unsigned)((cols + kBX - 1) / kBX),
               (unsigned)((rows + kBY - 1) / kBY));
 }
+// The stage kernels are launched with programmatic stream serialisation: a
+// kernel's blocks start while its predecessor's last ones run, and wait here
+// for it to complete before they touch memory (after any other predecessor the
+// wait returns at once).  A step is some thirty launches, most of them of a few
+// microseconds: 3.63 -> 3.35 ms for eight steps at 1280x1024.  Every
+// predecessor of a waiting kernel has itself waited, so the order is the
+// stream's.
+__device__ __forceinline__ void stage_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" :::);
+}
+template <typename... KArgs, typename... Args>
+void launch_stage(void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
+}
 #define FLOW_POINT(i0, i1, j0, j1)                                   \
+  stage_begin();                                                     \
   const int jj = (j0) + (int)(blockIdx.x * blockDim.x + threadIdx.x); \
   const int ii = (i0) + (int)(blockIdx.y * blockDim.y + threadIdx.y); \
   if (ii >= (i1) || jj >= (j1)) return;
@@ -741,12 +766,14 @@ __device__ __forceinline__ void boundary_point(long long t, int w, int h, int pa
 }
 
 __global__ void k_boundary(int w, int h, int pad, double* arr, int flip_x, int flip_y) {
+  stage_begin();
   boundary_point(blockIdx.x * (long long)blockDim.x + threadIdx.x, w, h, pad, arr, flip_x, flip_y);
 }
 // Two arrays in one launch (blockIdx.y): a fill of a few hundred KB takes 4 to 5
 // us, most of it the launch.
 __global__ void k_boundary2(int w0, int h0, double* a0, int flip_x0, int flip_y0, int w1, int h1,
                             double* a1, int flip_x1, int flip_y1, int pad) {
+  stage_begin();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (blockIdx.y == 0) boundary_point(t, w0, h0, pad, a0, flip_x0, flip_y0);
   else boundary_point(t, w1, h1, pad, a1, flip_x1, flip_y1);
@@ -793,6 +820,7 @@ __global__ void k_reflect_y(int w, int h, int pad, double* arr, int flip_y, int 
 }
 
 __global__ void k_copy(size_t n, double* dst, const double* src) {
+  stage_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     dst[i] = src[i];
@@ -807,7 +835,7 @@ __global__ void k_copy(size_t n, double* dst, const double* src) {
 #define FLOW_LAUNCH2D(kern, rows, cols, ...)                         \
   do {                                                               \
     if ((rows) > 0 && (cols) > 0) {                                  \
-      kern<<<grid_for((rows), (cols)), dim3(kBX, kBY), 0, s>>>(__VA_ARGS__); \
+      launch_stage(kern, grid_for((rows), (cols)), dim3(kBX, kBY), s, __VA_ARGS__); \
     }                                                                \
   } while (0)
 
@@ -1000,8 +1028,8 @@ void launch_boundary(cudaStream_t s, int w, int h, int pad, double* arr,
   const long long n = 2LL * pad * w + 2LL * pad * (h - 2 * pad);
   if (n <= 0) return;
   const int threads = 256;
-  k_boundary<<<(unsigned)((n + threads - 1) / threads), threads, 0, s>>>(
-      w, h, pad, arr, invert == kInvertX, invert == kInvertY);
+  launch_stage(k_boundary, dim3((unsigned)((n + threads - 1) / threads)), dim3(threads), s, w, h,
+               pad, arr, invert == kInvertX, invert == kInvertY);
 }
 
 void launch_boundary2(cudaStream_t s, int w0, int h0, double* a0, int invert0, int w1, int h1,
@@ -1011,16 +1039,16 @@ void launch_boundary2(cudaStream_t s, int w0, int h0, double* a0, int invert0, i
   const long long n = n0 > n1 ? n0 : n1;
   if (n <= 0) return;
   const int threads = 256;
-  k_boundary2<<<dim3((unsigned)((n + threads - 1) / threads), 2u), threads, 0, s>>>(
-      w0, h0, a0, invert0 == kInvertX, invert0 == kInvertY, w1, h1, a1, invert1 == kInvertX,
-      invert1 == kInvertY, pad);
+  launch_stage(k_boundary2, dim3((unsigned)((n + threads - 1) / threads), 2u), dim3(threads), s,
+               w0, h0, a0, invert0 == kInvertX, invert0 == kInvertY, w1, h1, a1,
+               invert1 == kInvertX, invert1 == kInvertY, pad);
 }
 
 void launch_copy(cudaStream_t s, size_t n, double* dst, const double* src) {
   if (n == 0) return;
   size_t blocks = (n + 255) / 256;
   if (blocks > 8192) blocks = 8192;
-  k_copy<<<(unsigned)blocks, 256, 0, s>>>(n, dst, src);
+  launch_stage(k_copy, dim3((unsigned)blocks), dim3(256), s, n, dst, src);
 }
 
 }  // namespace flow
