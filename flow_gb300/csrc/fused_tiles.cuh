@@ -1448,7 +1448,7 @@ template <typename R>
 __device__ __forceinline__ R mc_reconstruct(bool pos, R da, R db, R dc, R base, R inv_h, R h,
                                             R wdt) {
   using Pr = Prec<R>;
-  const R m0 = Pr::minmod(Pr::minmod(Pr::half(da), Pr::twice(db)), Pr::twice(dc));
+  const R m0 = Pr::minmod(Pr::half(da), Pr::twice(db), Pr::twice(dc));
   if (Pr::zero_skip(m0)) return base;
   const R mm = m0 * inv_h;
   const R w = h + (pos ? Pr::neg(wdt) : wdt);
@@ -1590,7 +1590,7 @@ __device__ __forceinline__ void mass_energy_flux_core(R v0, R dv2, R dvm, R dvp,
   }
   // minmod(0.5 (vp-vm)/h, 2 (v0-vm)/h, 2 (vp-v0)/h), scaled once (mc_reconstruct).
   const R mm =
-      Pr::minmod(Pr::half(dv2), Pr::minmod(Pr::twice(dvm), Pr::twice(dvp))) * inv_h;
+      Pr::minmod(Pr::twice(dvm), Pr::twice(dvp), Pr::half(dv2)) * inv_h;
   const R w_tc = Pr::msub(v0, Pr::half(v0) * dt, mm);
   R lim = R(0);
   if (!Pr::is_zero(jump)) {

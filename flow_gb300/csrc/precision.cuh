@@ -42,7 +42,9 @@ struct Prec<double> {
   }
   __device__ static __forceinline__ double abs(double x) { return d_abs(x); }
   __device__ static __forceinline__ double min0(double x) { return d_min0(x); }
-  __device__ static __forceinline__ double minmod(double a, double b) { return d_minmod(a, b); }
+  __device__ static __forceinline__ double minmod(double a, double b, double c) {
+    return d_minmod(d_minmod(a, b), c);
+  }
   __device__ static __forceinline__ double rcp(double x) { return d_rcp(x); }
   // A reciprocal used only through qdiv (which corrects the quotient).
   __device__ static __forceinline__ double rcp_q(double x) { return d_rcp_for_qdiv(x); }
@@ -77,27 +79,27 @@ struct Prec<double> {
 };
 
 __device__ __forceinline__ double f32_to_f64(float f) {
-  const unsigned b = __float_as_uint(f);
-  const unsigned sign = b & 0x80000000u;
-  const unsigned ex = (b >> 23) & 0xffu;
-  if (ex == 0u) return __hiloint2double((int)sign, 0);
-  const unsigned hi = sign | ((ex + 896u) << 20) | ((b & 0x7fffffu) >> 3);
-  const unsigned lo = b << 29;
-  return __hiloint2double((int)hi, (int)lo);
+  const int b = __float_as_int(f);
+  const bool tiny = (b & 0x7f800000) == 0;  // zero, or below the smallest normal: signed zero
+  // The arithmetic shift leaves the sign in bit 31 and its copies in bits
+  // 28..30, where the exponent's three new bits are zero.
+  const int hi = ((b >> 3) & (int)0x8fffffffu) + (896 << 20);
+  return __hiloint2double(tiny ? b & (int)0x80000000u : hi, tiny ? 0 : b << 29);
 }
 
+// The nearest FP32 value (ties to even): half a unit of the last place kept,
+// less one where that bit is even, carries into it; the bits then move up by
+// three and the exponent is rebased (896 << 23 modulo 2^32).
 __device__ __forceinline__ float f64_to_f32(double x) {
   const unsigned hi = (unsigned)__double2hiint(x);
   const unsigned lo = (unsigned)__double2loint(x);
-  const unsigned sign = hi & 0x80000000u;
-  const int ex = (int)((hi >> 20) & 0x7ffu) - 896;
-  if (ex <= 0) return __uint_as_float(sign);
-  if (ex >= 255) return __uint_as_float(sign | 0x7f800000u);
-  const unsigned mant = ((hi & 0xfffffu) << 3) | (lo >> 29);
-  const unsigned rest = lo & 0x1fffffffu;
-  unsigned f = sign | ((unsigned)ex << 23) | mant;
-  f += (rest > 0x10000000u) || (rest == 0x10000000u && (mant & 1u));
-  return __uint_as_float(f);
+  const unsigned mag = hi & 0x7fffffffu;
+  const unsigned long long r =
+      (((unsigned long long)mag << 32) | lo) + (0x0fffffffu + ((lo >> 29) & 1u));
+  unsigned f = (unsigned)(r >> 29) - 0xc0000000u;
+  if (mag < 0x38100000u) f = 0u;            // below the smallest normal
+  if (mag >= 0x47f00000u) f = 0x7f800000u;  // above the largest
+  return __uint_as_float(f | (hi & 0x80000000u));
 }
 
 template <>
@@ -123,11 +125,16 @@ struct Prec<float> {
   }
   __device__ static __forceinline__ float abs(float x) { return fabsf(x); }
   __device__ static __forceinline__ float min0(float x) { return (x > 0.0f) ? 0.0f : x; }
-  __device__ static __forceinline__ float minmod(float a, float b) {
-    if ((a > 0.0f && b > 0.0f) || (a < 0.0f && b < 0.0f)) {
-      return (fabsf(a) < fabsf(b)) ? a : b;
-    }
-    return 0.0f;
+  // The argument nearest to zero where all three share a sign, else +0 (a NaN
+  // anywhere gives +0 too): the positive part of the least plus the negative
+  // part of the greatest, one of which is zero.  Four minimum / maximum
+  // instructions and a sum for the fourteen of two nested comparisons (with
+  // the conversions above, a step of a smooth 2048x2048 field: 545 -> 518 us).
+  __device__ static __forceinline__ float minmod(float a, float b, float c) {
+    float lo, hi;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(lo) : "f"(a), "f"(b), "f"(c));
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(hi) : "f"(a), "f"(b), "f"(c));
+    return fmaxf(lo, 0.0f) + fminf(hi, 0.0f);
   }
   __device__ static __forceinline__ float rcp(float x) {
     float r;
