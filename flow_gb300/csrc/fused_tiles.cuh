@@ -1,6 +1,5 @@
 // fused_tiles.cuh -- the tile-level device code of the fused timestep, shared
-// by the single-problem kernels (fused.cu) and the persistent batched kernel
-// (batched.cu).  Each tile_* function processes one CTA-sized tile (bx, by)
+// by the single-problem kernels (fused.cu) and the batched ones (batched.cu).  Each tile_* function processes one CTA-sized tile (bx, by)
 // of one phase of the timestep for one problem described by StepArgs; a
 // thread may return early, but no tile function has a barrier after such a
 // return, so consecutive tiles can run back to back in one CTA.
@@ -21,11 +20,14 @@
 //     (mirror), replacing the 19 ghost-fill launches per step;
 //   * comparisons, selections and minmod run on the integer pipes, divisions
 //     by the mesh spacing become multiplications by per-column / per-row
-//     reciprocals (exact on power-of-two meshes), data divisions start from a
-//     MUFU reciprocal with an FMA correction;
-//   * the momentum/velocity chain and the conservative updates keep the
-//     reference's evaluation order in the FP64 form, with correctly rounded
-//     quotients (precision.cuh msub/madd/qdiv/dsub);
+//     reciprocals, data divisions start from an FP32 reciprocal with one
+//     Newton step and an FMA correction;
+//   * on a uniform mesh (one spacing a direction, tested once a run) the FP64
+//     form folds the timestep, the spacings and the constant factors into one
+//     coefficient per phase (the kU variants); on other meshes the momentum /
+//     velocity chain and the conservative updates keep the reference's
+//     evaluation order, with correctly rounded quotients (precision.cuh
+//     msub/madd/qdiv/dsub);
 //   * the CFL minimum and dt/dt_h stay on the device (dt_slot).
 // Every tile is a column strip: 128 threads own 128 consecutive columns and
 // march a.rows rows (at most kMaxRows), carrying the values of previous rows

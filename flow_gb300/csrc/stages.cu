@@ -31,7 +31,7 @@ inline dim3 grid_for(int rows, int cols) {
 // kernel's blocks start while its predecessor's last ones run, and wait here
 // for it to complete before they touch memory (after any other predecessor the
 // wait returns at once).  A step is some thirty launches, most of them of a few
-// microseconds: 3.63 -> 3.35 ms for eight steps at 1280x1024.  Every
+// microseconds: 3.63 -> 3.35 ms for four steps at 1280x1024.  Every
 // predecessor of a waiting kernel has itself waited, so the order is the
 // stream's.
 __device__ __forceinline__ void stage_begin() {

@@ -207,8 +207,9 @@ int gb300_synchronize(void);
  * tiles of the mesh were at rest, and does not recompute them while they stay
  * so.  It trusts that record only for the step that directly follows (tt one
  * more, the same arrays and reduce_array, no other call of this library that
- * takes a mesh in between).  A caller that writes the state arrays by other
- * means (its own copies or kernels) between two such steps calls this first.
+ * takes a mesh in between).  A caller that writes the state arrays or the mesh
+ * spacing arrays by other means (its own copies or kernels) between two such
+ * steps calls this first.
  * No reference counterpart (the reference recomputes every cell). */
 int gb300_state_changed(void);
 
@@ -223,7 +224,8 @@ int gb300_solve_hydro_2d(Mesh* mesh, int tt, double* P, double* rho,
 /* Interior totals: out[0] = sum rho, out[1] = sum rho*e (host array).  With
  * sync = 0 the totals stay in reduce_array[3..4] and out is not written.
  * Where reduce_array holds the fused step's flag region the sums are formed by
- * 128x128 tiles whose partial sums stay there; a call directly after a fused
+ * tiles (128 columns, 16 rows or more by the size of the mesh) whose partial
+ * sums stay there; a call directly after a fused
  * step keeps the partials of the tiles that step left at rest (see
  * gb300_state_changed).  The totals depend only on the cells. */
 int gb300_conservation(int nx, int ny, int pad, const double* rho,
