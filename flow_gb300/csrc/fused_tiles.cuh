@@ -1700,16 +1700,17 @@ static __device__ __noinline__ double still_energy(double r_old, double e_in, do
 // The FP64 form keeps the reference's evaluation order; the mixed form
 // contracts into FMAs.
 
-// The fluxes arrive widened to FP64 (f0, f1 mass, ef0, ef1 energy; exact
-// for the mixed form's FP32 fluxes), each face's once.
+// The fluxes (f0, f1 mass, ef0, ef1 energy) arrive in bulk precision; the
+// mixed form takes their differences to FP64 on the other pipes (diff_d: two of
+// the eight FP64 instructions of a cell, which bound its sweeps).
 // kU: a uniform mesh, with the coefficients kf, ke of the mass and energy flux
 // differences in the place of dt_h, vol, ivol and the face lengths.
 template <typename R, bool kFirst, bool kU>
 __device__ __forceinline__ void mass_energy_update(double r_in, double e_in,
                                                    double r_old, double dt_h,
                                                    double vol, double ivol, double a0,
-                                                   double a1, double f0, double f1,
-                                                   double ef0, double ef1, double kf, double ke,
+                                                   double a1, R f0, R f1, R ef0, R ef1,
+                                                   double kf, double ke,
                                                    double* r_out, double* e_out) {
   using Pr = Prec<R>;
   // No mass or energy crosses any cell of the warp (a warp-uniform test): the
@@ -1718,8 +1719,8 @@ __device__ __forceinline__ void mass_energy_update(double r_in, double e_in,
   // product rho_old*e is exact and den is rho_old, as in the still background
   // of a blast (a power-of-two density: settled without FP64 instructions).
   // The FP64 form takes the per-lane skip below otherwise.
-  const bool none = warp_all(d_is_zero(f0) && d_is_zero(f1) &&
-                             (Pr::kMixed || (d_is_zero(ef0) && d_is_zero(ef1))));
+  const bool none = warp_all(Pr::zero_d(f0) && Pr::zero_d(f1) &&
+                             (Pr::kMixed || (Pr::zero_d(ef0) && Pr::zero_d(ef1))));
   if (none) {
     const double den = kFirst ? r_old : r_in;
     *r_out = r_in;
@@ -1730,7 +1731,7 @@ __device__ __forceinline__ void mass_energy_update(double r_in, double e_in,
     }
     return;
   }
-  const double de = ef1 - ef0;
+  const double de = Pr::diff_d(ef1, ef0);
   double r_new, rho_e;
   if (!Pr::kMixed && Pr::zero_skip(f0) && Pr::zero_skip(f1) && Pr::zero_skip(de)) {
     // Nothing crosses the cell's faces: the updates subtract zeros.  (The
@@ -1738,11 +1739,11 @@ __device__ __forceinline__ void mass_energy_update(double r_in, double e_in,
     r_new = r_in;
     rho_e = __dmul_rn(r_old, e_in);
   } else if constexpr (kU) {
-    r_new = fma(-kf, f1 - f0, r_in);
+    r_new = fma(-kf, Pr::diff_d(f1, f0), r_in);
     rho_e = fma(-ke, de, __dmul_rn(r_old, e_in));
   } else if constexpr (Pr::kMixed) {
     const double coef = ivol;
-    const double net = fma(a1, f1, -(a0 * f0));
+    const double net = fma(a1, Pr::to_d(f1), -(a0 * Pr::to_d(f0)));
     r_new = fma(-coef, net, r_in);
     rho_e = fma(-coef, de, r_old * e_in);
   } else {
@@ -1832,7 +1833,7 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
                                                        unsigned sk3) {
   using Pr = Prec<R>;
   __shared__ R s_ey0r[kMaxRows];
-  __shared__ double sF[kCols], seF[kCols];  // the row's face fluxes, widened once
+  __shared__ R sF[kCols], seF[kCols];  // the row's face fluxes
   __shared__ double s_coef[kMaxRows], s_cyd[kMaxRows], s_ey0[kMaxRows], s_ey1[kMaxRows];
   const int nx = a.nx, ny = a.ny, pad = a.pad;
   const int t = threadIdx.x;
@@ -1995,8 +1996,8 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
       a.F_x[fidx(nx, ii, jj)] = F;
       mirror(edge, a.F_x, nx + 1, ny, pad, ii, jj, F, true, false);
     }
-    sF[t] = Pr::to_d(F);
-    seF[t] = Pr::to_d(eF);
+    sF[t] = F;
+    seF[t] = eF;
     __syncthreads();
     if (cell_ok) {
       double r_new, e_new;
@@ -2275,8 +2276,6 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
   R F0 = R(0), eF0 = R(0);
   if (fresh) flux_at(0, &F0, &eF0);
   store_fy(i0, F0, fresh);
-  // The fluxes of the face below, widened once and carried to the next row.
-  double f0d = Pr::to_d(F0), ef0d = Pr::to_d(eF0);
   if (!kEarly && i0 < i1) load(i0);
   for (int ii = i0; ii < i1; ++ii) {
     const int k = ii - i0;
@@ -2347,16 +2346,15 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
       store_fy(ii + 1, F1, fresh);
     }
     double r_new, e_new;
-    const double f1d = Pr::to_d(F1), ef1d = Pr::to_d(eF1);
     mass_energy_update<R, kFirst, kU>(r_in, e_in, r_old, dt_h, kU ? 0.0 : cxd * s_cyd[k],
-                                      kU ? 0.0 : s_coef[k] * icx, ex0, ex1, f0d, f1d, ef0d, ef1d,
+                                      kU ? 0.0 : s_coef[k] * icx, ex0, ex1, F0, F1, eF0, eF1,
                                       kh, ke, &r_new, &e_new);
     // (A cell of a skipped tile is at rest and keeps its value, which rho and
     // e hold: storing it again writes the same value.)
     store_cell(edge, s.r_out, s.r_out_r, nx, ny, pad, ii, jj, r_new);
     store_cell(edge, s.e_out, s.e_out_r, nx, ny, pad, ii, jj, e_new);
-    f0d = f1d;
-    ef0d = ef1d;
+    F0 = F1;
+    eF0 = eF1;
   }
   if constexpr (kFl) {
     // Face rows i0 .. i1 - 1, and the north boundary row in the last tile.

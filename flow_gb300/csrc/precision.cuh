@@ -50,6 +50,8 @@ struct Prec<double> {
   __device__ static __forceinline__ double rcp_q(double x) { return d_rcp_for_qdiv(x); }
   __device__ static __forceinline__ double rsqrt(double x) { return d_rsqrt(x); }
   __device__ static __forceinline__ double to_d(double x) { return x; }
+  __device__ static __forceinline__ double diff_d(double a, double b) { return a - b; }
+  __device__ static __forceinline__ bool zero_d(double x) { return d_is_zero(x); }
   __device__ static __forceinline__ double from_d(double x) { return x; }
   // m - t*s and b + h*w with the product rounded before the sum, as the
   // reference evaluates them (no contraction into an FMA).
@@ -102,6 +104,31 @@ __device__ __forceinline__ float f64_to_f32(double x) {
   return __uint_as_float(f | (hi & 0x80000000u));
 }
 
+// f32_to_f64(a) - f32_to_f64(b), rounded to nearest, off the FP64 pipe: the
+// FP32 difference and its rounding error (exact: Knuth's two-sum), the error in
+// units of the last FP64 place of the difference added to its bits.  Where the
+// exponent is near an end of the range, or the difference is a power of two
+// (below which the unit is half as large), the FP64 instruction itself, a call.
+// (Two of the eight FP64 instructions of a mixed sweep's cell, which kept the
+// FP64 pipe busy for two thirds of a sweep: a step of a smooth 2048x2048 field
+// 518 -> 506 us.)
+static __device__ __noinline__ double f32_diff_slow(float a, float b) {
+  return f32_to_f64(a) - f32_to_f64(b);
+}
+__device__ __forceinline__ double f32_diff(float a, float b) {
+  const float d = __fsub_rn(a, b);
+  const float bb = __fsub_rn(d, a);
+  const float lo = __fsub_rn(__fsub_rn(a, __fsub_rn(d, bb)), __fadd_rn(b, bb));
+  const unsigned bits = __float_as_uint(d), ex = (bits >> 23) & 0xffu;
+  if (d != 0.0f && (ex - 60u > 190u || ((bits & 0x7fffffu) == 0u && lo != 0.0f))) {
+    return f32_diff_slow(a, b);
+  }
+  // 2^(52 - exponent), signed as d (any finite value where d is zero: lo is too).
+  const float unit = __uint_as_float((bits & 0x80000000u) | ((306u - max(ex, 60u)) << 23));
+  const long long k = __float2int_rn(lo * unit);
+  return dfrom(dbits(f32_to_f64(d)) + k);
+}
+
 template <>
 struct Prec<float> {
   static constexpr bool kMixed = true;
@@ -143,6 +170,11 @@ struct Prec<float> {
   }
   __device__ static __forceinline__ float rsqrt(float x) { return rsqrtf(x); }
   __device__ static __forceinline__ double to_d(float x) { return f32_to_f64(x); }
+  // to_d(a) - to_d(b), and whether to_d(x) is a zero.
+  __device__ static __forceinline__ double diff_d(float a, float b) { return f32_diff(a, b); }
+  __device__ static __forceinline__ bool zero_d(float x) {
+    return (__float_as_uint(x) & 0x7f800000u) == 0u;
+  }
   __device__ static __forceinline__ float from_d(double x) { return f64_to_f32(x); }
   __device__ static __forceinline__ float msub(float m, float t, float s) { return fmaf(-t, s, m); }
   __device__ static __forceinline__ float madd(float h, float w, float b) { return fmaf(h, w, b); }
