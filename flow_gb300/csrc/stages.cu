@@ -235,18 +235,27 @@ __device__ __forceinline__ bool ranked_min(int w, long long n, int nx, int pad, 
     s_ex = s_ey = 0ull;
   }
   // The larger rank of the cell, negative where the ranks do not hold; each
-  // axis's own in rx, ry.
+  // axis's own in rx, ry.  The narrowing turns a stress below 2^-126 into zero,
+  // which takes up to 2^-126 ir from the cell's S: less than 1e-5 of an S above
+  // 1.2e-33 ir.  (A stress of 1e-39 sets the timestep where the density is
+  // 1e-25 and the energy 1e-15.)  S and the squares of the reciprocal spacings
+  // are normal FP32 numbers too, so that no step but the narrowing loses bits.
+  const bool mid = kx > 1e-30f && kx < 1e30f && ky > 1e-30f && ky < 1e30f;
   auto rank = [&](double ec, double qx, double qy, double r, float& rx, float& ry) {
     const long long be = dbits(ec), bx = dbits(qx), by = dbits(qy), br = dbits(r);
-    const float ef = f64_to_f32(ec), ir = 2.0f / f64_to_f32(r);
-    rx = fmaf(f64_to_f32(qx), ir, 0.56f * ef) * kx;
-    ry = fmaf(f64_to_f32(qy), ir, 0.56f * ef) * ky;
+    const float ef = f64_to_f32(ec), rf = f64_to_f32(r), ir = 2.0f / rf;
+    const float sx = fmaf(f64_to_f32(qx), ir, 0.56f * ef);
+    const float sy = fmaf(f64_to_f32(qy), ir, 0.56f * ef);
+    rx = sx * kx;
+    ry = sy * ky;
     const bool ok = be >= 0 && be < ex::kInf && (bx >= 0 || (bx << 1) == 0) && bx < ex::kInf &&
                     (by >= 0 || (by << 1) == 0) && by < ex::kInf &&
                     (unsigned long long)br - 0x0010000000000000ULL < 0x7fe0000000000000ULL;
     const float k = fmaxf(rx, ry);
-    return ok && k > 1e-30f && k < 1e30f && f64_to_f32(r) > 1e-30f && f64_to_f32(r) < 1e30f ? k
-                                                                                          : -1.0f;
+    return ok && mid && k > 1e-30f && k < 1e30f && rf > 1e-30f && rf < 1e30f &&
+                   fminf(sx, sy) > fmaxf(1e-30f, 2e-33f * ir)
+               ? k
+               : -1.0f;
   };
   bool ok = true;
   float best = 0.0f;
