@@ -33,6 +33,28 @@ __device__ __forceinline__ double minmod(double a, double b) {
   return ok ? (ma < mb ? a : b) : 0.0;
 }
 
+// The limited slope minmod(minmod(0.5 k a, 2 k b), 2 k c) of three differences,
+// k = 1/h, with the products formed as the reference does, (0.5 k) a.  Where
+// halving and doubling are exact for a, b, c and k the scaling can follow the
+// selection: (0.5 k) a and k (0.5 a) then round the same number, and rounding
+// keeps the order of the magnitudes.  Near the ends of the exponent range
+// (half of a subnormal difference rounds, twice a large one overflows) the
+// products are formed one by one.
+static __device__ __noinline__ double slope_ieee(double a, double b, double c, double k) {
+  const double h = __dmul_rn(0.5, k), t = __dmul_rn(2.0, k);
+  return minmod(minmod(__dmul_rn(h, a), __dmul_rn(t, b)), __dmul_rn(t, c));
+}
+// Exponent fields 4 .. 2043.
+__device__ __forceinline__ bool mid_range(double x) {
+  return (unsigned)(dhi(x) & 0x7fffffff) - 0x00400000u < 0x7f800000u;
+}
+__device__ __forceinline__ double slope(double a, double b, double c, double k) {
+  const bool ok = mid_range(k) && (mid_range(a) || d_is_zero(a)) &&
+                  (mid_range(b) || d_is_zero(b)) && (mid_range(c) || d_is_zero(c));
+  if (!ok) return slope_ieee(a, b, c, k);
+  return __dmul_rn(minmod(minmod(d_half(a), d_twice(b)), d_twice(c)), k);
+}
+
 // n / d.  The quotient from the 2^-43 seed with one residual correction, then
 // its exact residual t = n - d q: q is the correctly rounded quotient when |t|
 // is less than |d| times half a unit of q's last place (no quotient of two

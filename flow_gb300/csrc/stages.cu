@@ -554,11 +554,7 @@ __global__ void k_mass_energy_flux(int nx, int ny, int pad, double dt,
   const ptrdiff_t sc = kDirY ? nx : 1;             // cell stride
   const double invd = Spacing(kDirY ? edgedy[ii] : edgedx[jj]).rcp();
   const double wm = vel[fv - sv], w0 = vel[fv], wp = vel[fv + sv];
-  // 0.5 invd a, 2 invd b, 2 invd c: scaling by a power of two is exact, and
-  // scaling by invd > 0 after the selection gives the selected product (the
-  // rounding is monotonic, so it keeps the order of the magnitudes).
-  const double slope =
-      ex::minmod(d_half(wp - wm), ex::minmod(d_twice(w0 - wm), d_twice(wp - w0))) * invd;
+  const double slope = ex::slope(wp - wm, w0 - wm, wp - w0, invd);
   const double w_tc = w0 - d_half(w0) * dt * slope;
 
   const double r_m2 = rho[c - 2 * sc], r_m1 = rho[c - sc], r_0 = rho[c],
@@ -586,8 +582,7 @@ __global__ void k_mass_energy_flux(int nx, int ny, int pad, double dt,
                e_p1 = e[c + sc];
   // The side the wind comes from: the reference evaluates both.
   const double base = pos ? e_m1 : e_0, far = pos ? e_m2 : e_m1, near = pos ? e_0 : e_p1;
-  const double m = ex::minmod(ex::minmod(d_half(near - far), d_twice(base - far)),
-                              d_twice(near - base)) * invd;
+  const double m = ex::slope(near - far, base - far, near - base, invd);
   const double hs = d_half(m) * (pos ? hm - wdt : h0.h + wdt);
   const double e_face = pos ? base + hs : base - hs;
   const double area = kDirY ? edgedx[jj] : edgedy[ii];
@@ -626,13 +621,11 @@ __device__ __forceinline__ double mc_upwind(double wind, double m2, double m1,
                                             double p0, double p1, double invd,
                                             double d_left, double d_right,
                                             double dt_h, double lm, double rp) {
-  // The side the wind comes from (the reference evaluates both), the slope
-  // scaled after its selection (k_mass_energy_flux).
+  // The side the wind comes from (the reference evaluates both).
   const bool pos = ex::gt0(wind);
   const double base = pos ? lm : rp, far = pos ? m2 : m1, mid = pos ? m1 : p0,
                near = pos ? p0 : p1;
-  const double m = ex::minmod(ex::minmod(d_half(near - far), d_twice(mid - far)),
-                              d_twice(near - mid)) * invd;
+  const double m = ex::slope(near - far, mid - far, near - mid, invd);
   const double wdt = wind * dt_h;
   const double hs = d_half(m) * (pos ? d_left - wdt : d_right + wdt);
   return pos ? base + hs : base - hs;
