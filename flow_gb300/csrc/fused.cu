@@ -191,8 +191,8 @@ __device__ __forceinline__ void tile_lists(const ListArgs& l, int block) {
   const int pad = l.pad, D = kReach + pad;
   const int w = wd ? kCols - 1 : kCols;
   // The tile's columns and rows (clamped next to the walls: a ghost cell's
-  // mirror source lies within pad of them) with the reach around them: at most
-  // three columns of marks.
+  // mirror source lies within pad of them) with the reach around them: three
+  // columns of marks at most, where the ghost layers are no wider than 57.
   const int c0 = min(pad + bx * w, l.nx - 2 * pad);
   const int x0 = (max(c0 - D, pad) - pad) / l.mark_w;
   const int x1 = (min(c0 + w + D, l.nx - pad) - 1 - pad) / l.mark_w;
@@ -211,6 +211,11 @@ __device__ __forceinline__ void tile_lists(const ListArgs& l, int block) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) m[q][c] = l.marks[row + min(x0 + c, x1)];
   }
+  for (int c = x0 + 3; c <= x1; ++c) {  // (wider ghost layers)
+    for (int q = 0; q < kRounds; ++q) {
+      m[q][0] &= l.marks[(size_t)min(b0 + q * kSub + sub, b1) * l.mark_tiles_x + c];
+    }
+  }
 #pragma unroll
   for (int q = 0; q < kRounds; ++q) {
     const bool rest = (m[q][0] & m[q][1] & m[q][2]) != 0 || b0 + q * kSub + sub > b1;
@@ -219,9 +224,9 @@ __device__ __forceinline__ void tile_lists(const ListArgs& l, int block) {
   }
   for (int q = kRounds * kSub; b0 + q <= b1; ++q) {  // (wide ghost layers)
     const size_t row = (size_t)(b0 + q) * l.mark_tiles_x;
-    if ((l.marks[row + x0] & l.marks[row + min(x0 + 1, x1)] & l.marks[row + x1]) == 0) {
-      moved |= 1ull << min(q, 63);
-    }
+    unsigned char rest = 1;
+    for (int c = x0; c <= x1; ++c) rest &= l.marks[row + c];
+    if (!rest) moved |= 1ull << min(q, 63);
   }
   const int s0 = r0 + 2 * sub;
   const int p0 = (max(min(s0, l.ny - 2 * pad) - D, pad) - pad) / l.mark_rows - b0;
@@ -231,7 +236,7 @@ __device__ __forceinline__ void tile_lists(const ListArgs& l, int block) {
   // The tiles of height 2, then 4, 8 and 16: bit i of act, the group's i-th.
   unsigned act = (__ballot_sync(0xffffffffu, in && (moved & window) != 0ull) >> grp) &
                  ((1u << kSub) - 1);
-unsigned acts[kListHeights], all[kListHeights];
+  unsigned acts[kListHeights], all[kListHeights];
 #pragma unroll
   for (int h = 0; h < kListHeights; ++h) {
     const int per = kSub >> h;
