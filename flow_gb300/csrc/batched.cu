@@ -363,8 +363,11 @@ __global__ void k_batch_finish_dt(const BatchDev<R> b, int first_step) {
 template <typename R>
 __global__ void __launch_bounds__(256) k_batch_mesh_test(const BatchDev<R> b) {
   const StepArgs<R>& a = b.inst[blockIdx.x].a;
-  mesh_test_block(a.nx, a.ny, a.celldx, a.edgedx, a.celldy, a.edgedy,
-                  const_cast<double*>(a.mesh));
+  const unsigned r = mesh_test_part(a.nx, a.ny, a.celldx, a.edgedx, a.celldy, a.edgedy,
+                                    const_cast<double*>(a.mesh), 0, 1);
+  if (threadIdx.x == 0) {
+    *reinterpret_cast<unsigned long long*>(const_cast<double*>(a.mesh)) = kMeshBytes * r;
+  }
 }
 
 }  // namespace

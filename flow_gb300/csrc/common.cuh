@@ -30,9 +30,10 @@ constexpr double kCT = 0.3;
 //   [6] CFL minimum           running minimum of the fused step's CFL
 //                             candidates (uint64 bits of a non-negative
 //                             double: bit order = value order)
-//   [7] mesh uniform          1 (uint64) when the mesh is uniform, 3 when its
-//                             spacings are powers of two, formed on the
-//                             device at the start of a run, with the
+//   [7] mesh uniform          eight bytes, each 1 where a part of the mesh
+//                             test found it uniform, 3 where its spacings are
+//                             powers of two too (StepArgs::mesh), formed on
+//                             the device at the start of a step, with the
 //   [8 .. 11] spacings        dx, dy, 1/dx, 1/dy of a uniform mesh
 //   [12] minimum at rest      the CFL minimum over the shock-heating tiles
 //                             the next step need not visit (as [6])

@@ -27,20 +27,25 @@ __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" :::);
 }
 
-// The mesh test (mesh_test_block): one block, the first kernel of a run.  It
-// also clears the CFL minimum slot and the block ticket for the step's
-// Lagrangian kernels.
-constexpr int kMeshThreads = 1024;
+// The mesh test (mesh_test_part), the first kernel of a step: a block per part
+// (one block alone took 1 us of a step longer on a 4096^2 mesh, whose 131 KB of
+// spacings it read through one SM).  It also clears the CFL minimum slot and the
+// block ticket for the step's Lagrangian kernels.
+constexpr int kMeshThreads = 512;
 __global__ void __launch_bounds__(kMeshThreads)
     k_mesh_test(int nx, int ny, const double* celldx, const double* edgedx, const double* celldy,
                 const double* edgedy, double* ra) {
   pdl_wait();
   pdl_trigger();
-  if (threadIdx.x == 0) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     *reinterpret_cast<unsigned long long*>(ra + kRaTicket) = 0ull;
     *reinterpret_cast<unsigned long long*>(ra + kRaMinBits) = ~0ull;
   }
-  mesh_test_block(nx, ny, celldx, edgedx, celldy, edgedy, ra + kRaMesh);
+  const unsigned r = mesh_test_part(nx, ny, celldx, edgedx, celldy, edgedy, ra + kRaMesh,
+                                    (int)blockIdx.x, kMeshParts);
+  if (threadIdx.x == 0) {
+    reinterpret_cast<unsigned char*>(ra + kRaMesh)[blockIdx.x] = (unsigned char)r;
+  }
 }
 
 // How a kernel of the step runs: without flags (a mesh too small for them),
@@ -702,22 +707,20 @@ inline int apply_blocks(const lagf::LagArgs& l) {
 // One timestep of either form; first/second are the two mass sweeps' buffers.
 // lag: the FP64 form's one-kernel Lagrangian phase (k_lag_fused +
 // k_lag_apply), or null for the four separate Lagrangian kernels.
-// mesh_known: the step directly follows a step on the same mesh arrays (no
-// mesh call between), whose spacing test reduce_array still holds.
 template <typename R>
 void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
                  const SweepArgs<R>& first, const SweepArgs<R>& second,
-                 StepProfiler& prof, const StepRows& sr, bool mesh_known,
+                 StepProfiler& prof, const StepRows& sr,
                  const TileLists& tl, const ListArgs& lists,
                  const lagf::LagArgs* lag = nullptr) {
   const int nx = a.nx, ny = a.ny, pad = a.pad;
-  // The whole-mesh spacing test the tiles read (one block, a few
-  // microseconds), formed unless the previous step's still stands.
-  if (!mesh_known) {
-    prof.mark("mesh_test");
-    launch_pdl_block(k_mesh_test, dim3(1), dim3(kMeshThreads), s, nx, ny, a.celldx, a.edgedx,
-                     a.celldy, a.edgedy, a.ra);
-  }
+  // The whole-mesh spacing test the tiles read, formed by every step: the
+  // caller may have written the spacing arrays since the last.  (A launch more,
+  // about 2 us of a step: 1024^2 with a box 139 -> 141 us with the totals,
+  // 4096^2 with a blast 135 -> 137.)
+  prof.mark("mesh_test");
+  launch_pdl_block(k_mesh_test, dim3(kMeshParts), dim3(kMeshThreads), s, nx, ny, a.celldx, a.edgedx,
+                   a.celldy, a.edgedy, a.ra);
   if (lag) {
     const int nty = (ny - 2 * pad + lag->rows - 1) / lag->rows;
     prof.mark("lag_fused");
@@ -1454,7 +1457,7 @@ int fused_solve(Mesh* mesh, int tt, double* P, double* rho, double* rho_old,
                 a.skipf != nullptr && lagp == nullptr, rho, e, reduce_array, tl, la);
   StepProfiler prof;
   prof.begin(s);
-  launch_step(s, a, tt, first, second, prof, sr, a.rest != nullptr, tl, la, lagp);
+  launch_step(s, a, tt, first, second, prof, sr, tl, la, lagp);
   const int st = finish_step(s, mesh, reduce_array, prof, "solve_hydro_2d (fused)", t_rest.counts);
   if (st != GB300_OK) t_rest.valid = false;
   return st;
@@ -1527,7 +1530,7 @@ int mixed_solve(Mesh* mesh, int tt, double* rho, double* e, float* rho_u,
                 a.skipf != nullptr, rho, e, reduce_array, tl, la);
   StepProfiler prof;
   prof.begin(s);
-  launch_step(s, a, tt, first, second, prof, sr, a.rest != nullptr, tl, la);
+  launch_step(s, a, tt, first, second, prof, sr, tl, la);
   const int st = finish_step(s, mesh, reduce_array, prof, "gb300_mixed_solve", t_rest.counts);
   if (st != GB300_OK) t_rest.valid = false;
   return st;

@@ -22,7 +22,7 @@
 //     by the mesh spacing become multiplications by per-column / per-row
 //     reciprocals, data divisions start from an FP32 reciprocal with one
 //     Newton step and an FMA correction;
-//   * on a uniform mesh (one spacing a direction, tested once a run) the FP64
+//   * on a uniform mesh (one spacing a direction, tested every step) the FP64
 //     form folds the timestep, the spacings and the constant factors into one
 //     coefficient per phase (the kU variants); on other meshes the momentum /
 //     velocity chain and the conservative updates keep the reference's
@@ -77,10 +77,11 @@ struct StepArgs {
   R* vF_y;
   double* ra;                  // caller scratch (reduce_array)
   unsigned long long* min_slot;  // running CFL minimum (FP64 bit pattern)
-  // The mesh test's result (formed on the device at the start of a run): [0]
-  // non-zero (uint64) when the mesh is uniform -- every celldx and edgedx one
-  // number, every celldy and edgedy one number --, 3 when both are powers of
-  // two, then [1], [2] the two spacings and [3], [4] their reciprocals.
+  // The mesh test's result (formed on the device at the start of a step): [0]
+  // holds eight bytes, the results of its kMeshParts parts -- each 1 when the
+  // mesh is uniform there (every celldx and edgedx one number, every celldy and
+  // edgedy one number), 3 when both are powers of two --, then [1], [2] the two
+  // spacings and [3], [4] their reciprocals.
   const double* mesh;
   double* dt_slot;             // [0] dt, [1] dt_h for the advection phase
   double dt, dt_h, max_dt;     // Lagrangian-phase pair (host values), max_dt
@@ -379,6 +380,9 @@ __device__ __forceinline__ bool tile_near_edge(int nx, int ny, int pad, int col0
 struct UniformMesh {
   double dx, dy, ix, iy;
 };
+// Parts of the mesh test, each with a byte of its result's first word.
+constexpr int kMeshParts = 8;
+constexpr unsigned long long kMeshBytes = 0x0101010101010101ull;
 // Whether a form's tiles take the uniform variants: the mixed form's mass
 // sweeps (its others have none) only where the spacings are powers of two, so
 // that folding them rounds nothing.  An FP64 rounding there now and then turns
@@ -386,20 +390,24 @@ struct UniformMesh {
 template <typename R>
 __device__ __forceinline__ bool mesh_uniform(const double* mesh) {
   const unsigned long long f = *reinterpret_cast<const unsigned long long*>(mesh);
-  return Prec<R>::kMixed ? f == 3ull : f != 0ull;
+  return Prec<R>::kMixed ? f == kMeshBytes * 3 : (f & kMeshBytes) == kMeshBytes;
 }
 __device__ __forceinline__ UniformMesh uniform_mesh(const double* mesh) {
   return UniformMesh{mesh[1], mesh[2], mesh[3], mesh[4]};
 }
 
-// The mesh test, by one block (barrier): whether every celldx and edgedx
-// (entries 0 .. nx) is one positive normal number with a normal reciprocal,
-// and every celldy and edgedy (0 .. ny) likewise, written to mesh with the
-// spacings.  Every test is made (no short circuit), so that a thread's loads
-// are independent and in flight together.
-__device__ __forceinline__ void mesh_test_block(int nx, int ny, const double* celldx,
-                                                const double* edgedx, const double* celldy,
-                                                const double* edgedy, double* mesh) {
+// Block `part` of `parts` of the mesh test (barrier): whether every celldx and
+// edgedx (entries 0 .. nx) is one positive normal number with a normal
+// reciprocal, and every celldy and edgedy (0 .. ny) likewise, for its share of
+// the entries.  Returns 1 if so, 3 when both numbers are powers of two too, else
+// 0; part 0 writes the spacings to mesh.  Every test is made (no short circuit)
+// and the four arrays are read together, so that a thread's loads are in flight
+// at once, and the reciprocals are formed meanwhile.
+__device__ __forceinline__ unsigned mesh_test_part(int nx, int ny, const double* celldx,
+                                                   const double* edgedx, const double* celldy,
+                                                   const double* edgedy, double* mesh, int part,
+                                                   int parts) {
+  constexpr int kB = 2;
   const double dx = celldx[0], dy = celldy[0];
   const long long bx = dbits(dx), by = dbits(dy);
   // (Exponents from 2^-1000 to 2^1000: the reciprocals are normal too.)
@@ -407,23 +415,34 @@ __device__ __forceinline__ void mesh_test_block(int nx, int ny, const double* ce
     return b > 0 && (b >> 52) - 23 >= 0 && (b >> 52) - 23 <= 2000;
   };
   bool ok = fine(bx) & fine(by);
-#pragma unroll 4
-  for (int j = threadIdx.x; j <= nx; j += blockDim.x) {
-    ok &= (dbits(celldx[j]) == bx) & (dbits(edgedx[j]) == bx);
+  const int n = max(nx, ny), stride = parts * (int)blockDim.x;
+  for (int j0 = part * (int)blockDim.x + (int)threadIdx.x; j0 <= n; j0 += kB * stride) {
+    double v[kB][4];
+#pragma unroll
+    for (int q = 0; q < kB; ++q) {
+      const int j = j0 + q * stride;
+      const bool x = j <= nx, y = j <= ny;
+      v[q][0] = x ? celldx[j] : dx;
+      v[q][1] = x ? edgedx[j] : dx;
+      v[q][2] = y ? celldy[j] : dy;
+      v[q][3] = y ? edgedy[j] : dy;
+    }
+#pragma unroll
+    for (int q = 0; q < kB; ++q) {
+      ok &= (dbits(v[q][0]) == bx) & (dbits(v[q][1]) == bx);
+      ok &= (dbits(v[q][2]) == by) & (dbits(v[q][3]) == by);
+    }
   }
-#pragma unroll 4
-  for (int i = threadIdx.x; i <= ny; i += blockDim.x) {
-    ok &= (dbits(celldy[i]) == by) & (dbits(edgedy[i]) == by);
-  }
-  ok = __syncthreads_and(ok) != 0;
-  if (threadIdx.x == 0) {
-    *reinterpret_cast<unsigned long long*>(mesh) =
-        !ok ? 0ull : (d_is_pow2(dx) && d_is_pow2(dy)) ? 3ull : 1ull;
+  if (part == 0 && threadIdx.x == 0) {
     mesh[1] = dx;
-    mesh[2] = dy;
     mesh[3] = 1.0 / dx;
+  }
+  if (part == 0 && threadIdx.x == 32) {
+    mesh[2] = dy;
     mesh[4] = 1.0 / dy;
   }
+  ok = __syncthreads_and(ok) != 0;
+  return !ok ? 0u : (d_is_pow2(dx) && d_is_pow2(dy)) ? 3u : 1u;
 }
 
 // Runs the tile of a uniform mesh where the mesh is one (FP64 form; the mixed

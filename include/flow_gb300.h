@@ -207,9 +207,11 @@ int gb300_synchronize(void);
  * tiles of the mesh were at rest, and does not recompute them while they stay
  * so.  It trusts that record only for the step that directly follows (tt one
  * more, the same arrays and reduce_array, no other call of this library that
- * takes a mesh in between).  A caller that writes the state arrays or the mesh
- * spacing arrays by other means (its own copies or kernels) between two such
- * steps calls this first.
+ * takes a mesh in between).  A caller that writes the state arrays by other
+ * means (its own copies or kernels) between two such steps calls this first.
+ * Every step takes the mesh spacing arrays as they are then; only the timestep
+ * candidates of tiles at rest stand from the step that formed them, so a caller
+ * that writes new spacings where tiles are at rest calls this too.
  * No reference counterpart (the reference recomputes every cell). */
 int gb300_state_changed(void);
 
