@@ -30,10 +30,11 @@ constexpr double kCT = 0.3;
 //   [6] CFL minimum           running minimum of the fused step's CFL
 //                             candidates (uint64 bits of a non-negative
 //                             double: bit order = value order)
-//   [7] mesh uniform          eight bytes, each 1 where a part of the mesh
-//                             test found it uniform, 3 where its spacings are
-//                             powers of two too (StepArgs::mesh), formed on
-//                             the device at the start of a step, with the
+//   [7] mesh                  eight bytes, one of each part of the mesh test:
+//                             bit 0 uniform, bit 1 spacings all powers of two,
+//                             bits 2 and 3 some of them (StepArgs::mesh),
+//                             formed on the device at the start of a step,
+//                             with the
 //   [8 .. 11] spacings        dx, dy, 1/dx, 1/dy of a uniform mesh
 //   [12] minimum at rest      the CFL minimum over the shock-heating tiles
 //                             the next step need not visit (as [6])

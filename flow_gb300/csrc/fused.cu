@@ -66,7 +66,7 @@ __device__ __forceinline__ bool block_tile(const StepArgs<R>& a, int& bx, int& b
 }
 
 template <typename R, int kMd>
-__global__ void __launch_bounds__(kCols) k_lag_pressure(const StepArgs<R> a) {
+__global__ void __launch_bounds__(kCols, 8) k_lag_pressure(const StepArgs<R> a) {
   pdl_wait();
   pdl_trigger();
   // The first kernel of the step clears the CFL minimum and the block ticket
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kCols) k_lag_pressure(const StepArgs<R> a) {
   int bx, by;
   const bool uni = mesh_uniform<R>(a.mesh);
   if (block_tile<kMd>(a, bx, by)) {
-    tile_lag_pressure<R, (kMd != kNoFlags), (kMd != kListed)>(a, bx, by, uni);
+    tile_lag_pressure<R, (kMd != kNoFlags), (kMd != kListed), (kMd != kListed)>(a, bx, by, uni);
   }
 }
 // With flags, the viscous-stress flags (a.qmask) are kept -- the viscosity
@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(kCols) k_lag_energy_dt(const StepArgs<R> a) {
   constexpr bool kFlags = kMd != kNoFlags;
   const bool uni = mesh_uniform<R>(a.mesh);
   if (!block_tile<kMd>(a, bx, by)) return;
-  tile_lag_energy_dt<R, true, kFlags, (kMd != kListed)>(a, bx, by, uni,
-                                                       kFlags ? &s_tile_min : nullptr);
+  tile_lag_energy_dt<R, true, kFlags, (kMd != kListed), (kMd != kListed)>(
+      a, bx, by, uni, kFlags ? &s_tile_min : nullptr);
   // (Thread 0 wrote the minimum it stores here.)
   if (kFlags && a.cfl_tile && threadIdx.x == 0) {
     a.cfl_tile[(size_t)by * a.qm_stride + bx] = s_tile_min;
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 8 : 7) k_mass_sweep_x
     }
   }
   if (kLists ? line_tile<kMd>(a, blockIdx.x, bx, by) : block_tile<kMd>(a, bx, by)) {
-    tile_mass_sweep_x<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by, uni);
+    tile_mass_sweep_x<R, kFirst, true, (kMd != kNoFlags), (kMd != kListed)>(a, s, bx, by, uni);
   }
   store_dt<R, kFirst>(a);
 }
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 7 : 6) k_mass_sweep_y
     }
   }
   if (kLists ? line_tile<kMd>(a, blockIdx.x, bx, by) : block_tile<kMd>(a, bx, by)) {
-    tile_mass_sweep_y<R, kFirst, true, (kMd != kNoFlags)>(a, s, bx, by, uni);
+    tile_mass_sweep_y<R, kFirst, true, (kMd != kNoFlags), (kMd != kListed)>(a, s, bx, by, uni);
   }
   store_dt<R, kFirst>(a);
 }
@@ -346,10 +346,10 @@ enum : int { kNone = 0, kXU = 1, kXV = 2, kYU = 3, kYV = 4 };  // direction and 
 template <typename R, int kPair, bool kVel, int kMd>
 __device__ __forceinline__ void pair_tile(const StepArgs<R>& a, int bx, int by, bool uni) {
   constexpr bool kFl = kMd != kNoFlags, kTest = kMd != kListed;
-  if constexpr (kPair == kXU) tile_mom_x<R, false, kVel, true, kFl, kTest>(a, bx, by, uni);
-  else if constexpr (kPair == kXV) tile_mom_x<R, true, kVel, true, kFl, kTest>(a, bx, by, uni);
-  else if constexpr (kPair == kYU) tile_mom_y<R, false, kVel, true, kFl, kTest>(a, bx, by, uni);
-  else if constexpr (kPair == kYV) tile_mom_y<R, true, kVel, true, kFl, kTest>(a, bx, by, uni);
+  if constexpr (kPair == kXU) tile_mom_x<R, false, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
+  else if constexpr (kPair == kXV) tile_mom_x<R, true, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
+  else if constexpr (kPair == kYU) tile_mom_y<R, false, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
+  else if constexpr (kPair == kYV) tile_mom_y<R, true, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
 }
 // The tiles of pair A (blocks 0 .. na - 1), then those of pair B.
 template <typename R, int kA, bool kVelA, int kB, bool kVelB, int kMd>

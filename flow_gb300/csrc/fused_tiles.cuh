@@ -1,8 +1,9 @@
 // fused_tiles.cuh -- the tile-level device code of the fused timestep, shared
-// by the single-problem kernels (fused.cu) and the batched ones (batched.cu).  Each tile_* function processes one CTA-sized tile (bx, by)
-// of one phase of the timestep for one problem described by StepArgs; a
-// thread may return early, but no tile function has a barrier after such a
-// return, so consecutive tiles can run back to back in one CTA.
+// by the single-problem kernels (fused.cu) and the batched ones (batched.cu).
+// Each tile_* function processes one CTA-sized tile (bx, by) of one phase of the
+// timestep for one problem described by StepArgs; a thread may return early, but
+// no tile function has a barrier after such a return, so consecutive tiles can
+// run one after another in one CTA (with a barrier between two).
 //
 // Two precision forms share the code (precision.cuh):
 //   R = double  the FP64 form behind solve_hydro_2d (GB300_MODE_FUSED);
@@ -24,10 +25,10 @@
 //     Newton step and an FMA correction;
 //   * on a uniform mesh (one spacing a direction, tested every step) the FP64
 //     form folds the timestep, the spacings and the constant factors into one
-//     coefficient per phase (the kU variants); on other meshes the momentum /
+//     coefficient per phase (kMeshUniform); on other meshes the momentum /
 //     velocity chain and the conservative updates keep the reference's
 //     evaluation order, with correctly rounded quotients (precision.cuh
-//     msub/madd/qdiv/dsub);
+//     msub/madd/qdiv/dsub), exponent adds where spacings are powers of two;
 //   * the CFL minimum and dt/dt_h stay on the device (dt_slot).
 // Every tile is a column strip: 128 threads own 128 consecutive columns and
 // march a.rows rows (at most kMaxRows), carrying the values of previous rows
@@ -78,10 +79,11 @@ struct StepArgs {
   double* ra;                  // caller scratch (reduce_array)
   unsigned long long* min_slot;  // running CFL minimum (FP64 bit pattern)
   // The mesh test's result (formed on the device at the start of a step): [0]
-  // holds eight bytes, the results of its kMeshParts parts -- each 1 when the
-  // mesh is uniform there (every celldx and edgedx one number, every celldy and
-  // edgedy one number), 3 when both are powers of two --, then [1], [2] the two
-  // spacings and [3], [4] their reciprocals.
+  // holds eight bytes, the results of its kMeshParts parts -- bit 0 of each set
+  // when the mesh is uniform there (every celldx and edgedx one number, every
+  // celldy and edgedy one number), bit 1 when every spacing is a power of two,
+  // bits 2 and 3 when a run of them along x and along y is --, then [1], [2] the
+  // two spacings (of a uniform mesh) and [3], [4] their reciprocals.
   const double* mesh;
   double* dt_slot;             // [0] dt, [1] dt_h for the advection phase
   double dt, dt_h, max_dt;     // Lagrangian-phase pair (host values), max_dt
@@ -225,13 +227,23 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(n) : "memory");
 }
 // The shared-memory slots of an asynchronous-copy ring, [slots][planes][cols]
-// of T.  Declared here rather than in the tile: a tile's power-of-two and
-// general variants are both compiled into its kernel, and shared arrays
-// declared in each would be allocated twice; this function's array is one
+// of T.  Declared here rather than in the tile: a tile's variants (kMeshUniform
+// and the others) are all compiled into its kernel, and shared arrays
+// declared in each would be allocated once for each; this function's array is one
 // allocation per kernel for each (T, shape, tag).
 template <typename T, int kSlotsN, int kPlanes, int kColsN, int kTag>
 __device__ __forceinline__ T (*ring_slots())[kPlanes][kColsN] {
   __shared__ T buf[kSlotsN][kPlanes][kColsN];
+  return buf;
+}
+
+// Shared table kTag of a tile (kN entries of T), one allocation per kernel like
+// ring_slots, for the variants of its tile and for every tile it may run: a
+// block runs one at a time (batched.cu's persistent kernel with a barrier
+// between two).
+template <typename T, int kN, int kTag>
+__device__ __forceinline__ T* tile_table() {
+  __shared__ T buf[kN];
   return buf;
 }
 
@@ -390,7 +402,7 @@ constexpr unsigned long long kMeshBytes = 0x0101010101010101ull;
 template <typename R>
 __device__ __forceinline__ bool mesh_uniform(const double* mesh) {
   const unsigned long long f = *reinterpret_cast<const unsigned long long*>(mesh);
-  return Prec<R>::kMixed ? f == kMeshBytes * 3 : (f & kMeshBytes) == kMeshBytes;
+  return Prec<R>::kMixed ? (f & 3 * kMeshBytes) == 3 * kMeshBytes : (f & kMeshBytes) == kMeshBytes;
 }
 __device__ __forceinline__ UniformMesh uniform_mesh(const double* mesh) {
   return UniformMesh{mesh[1], mesh[2], mesh[3], mesh[4]};
@@ -399,8 +411,9 @@ __device__ __forceinline__ UniformMesh uniform_mesh(const double* mesh) {
 // Block `part` of `parts` of the mesh test (barrier): whether every celldx and
 // edgedx (entries 0 .. nx) is one positive normal number with a normal
 // reciprocal, and every celldy and edgedy (0 .. ny) likewise, for its share of
-// the entries.  Returns 1 if so, 3 when both numbers are powers of two too, else
-// 0; part 0 writes the spacings to mesh.  Every test is made (no short circuit)
+// the entries: bit 0 of the result.  Bit 1: all of them are positive normal
+// powers of two; bits 2, 3: 32 consecutive entries along x, along y are.  Part 0
+// writes the spacings to mesh.  Every test is made (no short circuit)
 // and the four arrays are read together, so that a thread's loads are in flight
 // at once, and the reciprocals are formed meanwhile.
 __device__ __forceinline__ unsigned mesh_test_part(int nx, int ny, const double* celldx,
@@ -414,9 +427,10 @@ __device__ __forceinline__ unsigned mesh_test_part(int nx, int ny, const double*
   auto fine = [](long long b) {
     return b > 0 && (b >> 52) - 23 >= 0 && (b >> 52) - 23 <= 2000;
   };
-  bool ok = fine(bx) & fine(by);
+  bool ok = fine(bx) & fine(by), p2 = true, run_x = false, run_y = false;
   const int n = max(nx, ny), stride = parts * (int)blockDim.x;
-  for (int j0 = part * (int)blockDim.x + (int)threadIdx.x; j0 <= n; j0 += kB * stride) {
+  for (int b = part * (int)blockDim.x; b <= n; b += kB * stride) {  // (whole warps)
+    const int j0 = b + (int)threadIdx.x;
     double v[kB][4];
 #pragma unroll
     for (int q = 0; q < kB; ++q) {
@@ -431,6 +445,12 @@ __device__ __forceinline__ unsigned mesh_test_part(int nx, int ny, const double*
     for (int q = 0; q < kB; ++q) {
       ok &= (dbits(v[q][0]) == bx) & (dbits(v[q][1]) == bx);
       ok &= (dbits(v[q][2]) == by) & (dbits(v[q][3]) == by);
+      const bool px = d_is_pow2(v[q][0]) & d_is_pow2(v[q][1]);
+      const bool py = d_is_pow2(v[q][2]) & d_is_pow2(v[q][3]);
+      const int first = b + q * stride + ((int)threadIdx.x & ~31);
+      run_x |= (__all_sync(0xffffffffu, px) != 0) & (first <= nx);
+      run_y |= (__all_sync(0xffffffffu, py) != 0) & (first <= ny);
+      p2 &= px & py;
     }
   }
   if (part == 0 && threadIdx.x == 0) {
@@ -441,40 +461,87 @@ __device__ __forceinline__ unsigned mesh_test_part(int nx, int ny, const double*
     mesh[2] = dy;
     mesh[4] = 1.0 / dy;
   }
-  ok = __syncthreads_and(ok) != 0;
-  return !ok ? 0u : (d_is_pow2(dx) && d_is_pow2(dy)) ? 3u : 1u;
+  return (__syncthreads_and(ok) ? 1u : 0u) | (__syncthreads_and(p2) ? 2u : 0u) |
+         (__syncthreads_or(run_x) ? 4u : 0u) | (__syncthreads_or(run_y) ? 8u : 0u);
 }
 
-// Runs the tile of a uniform mesh where the mesh is one (FP64 form; the mixed
-// form's FP32 arithmetic gains nothing from it, but for its mass sweeps, whose
-// FP64 conservative update does: FLOW_UNIFORM_DISPATCH_ALL).  On a uniform
-// mesh the FP64 form folds the spacings into the timestep once per tile --
-//   m - dt d / h as fma(-(dt / h), d, m), h -+ w dt_h times 1/h as
-//   fma(-+w, dt_h / h, 1), the face lengths and half widths of the fluxes into
-//   their updates' coefficients, a face density as half the sum --
-// so a momentum update is one FP64 instruction besides its difference where
-// the general tile takes four (a quotient corrected to the reference's
-// rounding), and a tile reads no spacing arrays.  Each folded product is
-// rounded once per step instead of once per cell.
+// Whether every spacing of the mesh is a power of two, and whether a tile of a
+// mesh where not tests its own: not where the mesh test saw no run of powers of
+// two along an axis, nor in tiles of fewer than eight rows, which a step takes
+// where an SM has a few tiles and waits for their latencies -- the test's loads
+// and barrier then cost more than the FP64 instructions it saves (a field in
+// motion on a mesh of two halves, 256x256: 162 us a step without, 168 with;
+// 2048x2048: 2430 without, 1974 with).
+template <typename R>
+__device__ __forceinline__ bool mesh_all_pow2(const StepArgs<R>& a) {
+  const unsigned long long f = *reinterpret_cast<const unsigned long long*>(a.mesh);
+  return (f & 2 * kMeshBytes) == 2 * kMeshBytes;
+}
+template <typename R>
+__device__ __forceinline__ bool mesh_some_pow2(const StepArgs<R>& a) {
+  const unsigned long long f = *reinterpret_cast<const unsigned long long*>(a.mesh);
+  return a.rows >= 8 && (f & 4 * kMeshBytes) != 0ull && (f & 8 * kMeshBytes) != 0ull;
+}
+// True when every mesh spacing (celldx, edgedx, celldy, edgedy) within two
+// entries of the block's columns [col0, col0 + kCols) and rows
+// [row0, row0 + rows) is a power of two (by the rule above, false where the
+// tile does not look).  Block-uniform (barrier).
+template <typename R>
+__device__ __forceinline__ bool block_mesh_pow2(const StepArgs<R>& a, int col0, int row0) {
+  if (mesh_all_pow2(a)) return true;
+  if (!mesh_some_pow2(a)) return false;
+  bool ok = true;
+  for (int j = col0 - 2 + (int)threadIdx.x; j < col0 + kCols + 2; j += kCols) {
+    if (j >= 0 && j <= a.nx) ok = ok && d_is_pow2(a.celldx[j]) && d_is_pow2(a.edgedx[j]);
+  }
+  for (int i = row0 - 2 + (int)threadIdx.x; i < row0 + a.rows + 2; i += kCols) {
+    if (i >= 0 && i <= a.ny) ok = ok && d_is_pow2(a.celldy[i]) && d_is_pow2(a.edgedy[i]);
+  }
+  return __syncthreads_and(ok) != 0;
+}
+
+// The variants of a tile by the mesh's spacings:
+//   kMeshUniform  the whole mesh is uniform (uni).  The FP64 form folds the
+//     spacings into the timestep once per tile --
+//       m - dt d / h as fma(-(dt / h), d, m), h -+ w dt_h times 1/h as
+//       fma(-+w, dt_h / h, 1), the face lengths and half widths of the fluxes
+//       into their updates' coefficients, a face density as half the sum --
+//     so a momentum update is one FP64 instruction besides its difference where
+//     the general tile takes four (a quotient corrected to the reference's
+//     rounding), and a tile reads no spacing arrays.  Each folded product is
+//     rounded once per step instead of once per cell.
+//   kMeshPow2  every spacing the tile uses is a power of two: the general
+//     tile's numbers with the products and quotients by a spacing as exponent
+//     adds.  FP64 form, in the kernels over a whole mesh (kP2T): a 2048x2048
+//     field in motion on a mesh of two halves of different widths takes 2430 us
+//     a step with the general tiles and 1974 with these.
+//   kMeshGeneral  any other; the mixed form's only one but for its mass sweeps
+//     (FLOW_MESH_DISPATCH_ALL), whose FP64 conservative update gains from the
+//     uniform one, as its FP32 arithmetic does not.
 // uni: mesh_uniform<R>(a.mesh), which a kernel reads beside its tile's index, so
 // that the two loads are in flight together.
-#define FLOW_UNIFORM_DISPATCH(R, CALL_TRUE, CALL_FALSE) \
-  do {                                                  \
-    if constexpr (!Prec<R>::kMixed) {                   \
-      if (uni) {                                        \
-        CALL_TRUE;                                      \
-        return;                                         \
-      }                                                 \
-    }                                                   \
-    CALL_FALSE;                                         \
+enum : int { kMeshGeneral = 0, kMeshPow2 = 1, kMeshUniform = 2 };
+#define FLOW_MESH_DISPATCH_ALL(R, kP2T, POW2, CALL_UNIFORM, CALL_POW2, CALL_GENERAL) \
+  do {                                                                                       \
+    if (uni) {                                                                               \
+      CALL_UNIFORM;                                                                          \
+      return;                                                                                \
+    }                                                                                        \
+    if constexpr (!Prec<R>::kMixed && kP2T) {                                                \
+      if (POW2) {                                                                            \
+        CALL_POW2;                                                                           \
+        return;                                                                              \
+      }                                                                                      \
+    }                                                                                        \
+    CALL_GENERAL;                                                                            \
   } while (0)
-#define FLOW_UNIFORM_DISPATCH_ALL(CALL_TRUE, CALL_FALSE) \
-  do {                                                   \
-    if (uni) {                                           \
-      CALL_TRUE;                                         \
-      return;                                            \
-    }                                                    \
-    CALL_FALSE;                                          \
+#define FLOW_MESH_DISPATCH(R, kP2T, POW2, CALL_UNIFORM, CALL_POW2, CALL_GENERAL) \
+  do {                                                                                   \
+    if constexpr (!Prec<R>::kMixed) {                                                    \
+      FLOW_MESH_DISPATCH_ALL(R, kP2T, POW2, CALL_UNIFORM, CALL_POW2, CALL_GENERAL);      \
+    } else {                                                                             \
+      CALL_GENERAL;                                                                      \
+    }                                                                                    \
   } while (0)
 
 // Spacing factors of a tile (mesh spacings, their reciprocals and ratios),
@@ -485,20 +552,20 @@ __device__ __forceinline__ unsigned mesh_test_part(int nx, int ny, const double*
 // pipe, and per tile these cost more than the arithmetic of a still cell.
 template <typename R>
 __device__ __forceinline__ R geo_v(double h) { return Prec<R>::from_d(h); }
-template <typename R>
+template <typename R, bool kP2 = false>
 __device__ __forceinline__ R geo_rcp(double h) {
   if constexpr (Prec<R>::kMixed) {
     return __frcp_rn(f64_to_f32(h));
   } else {
-    return 1.0 / h;
+    return kP2 ? d_pow2_rcp(h) : 1.0 / h;
   }
 }
-template <typename R>
+template <typename R, bool kP2 = false>
 __device__ __forceinline__ R geo_half_ratio(double c, double e) {
   if constexpr (Prec<R>::kMixed) {
     return __fdiv_rn(f64_to_f32(c), 2.0f * f64_to_f32(e));
   } else {
-    return c / (2.0 * e);
+    return kP2 ? d_pow2_half_ratio(c, e) : c / (2.0 * e);
   }
 }
 // h/2 in bulk precision (exact).
@@ -507,13 +574,18 @@ __device__ __forceinline__ R geo_half(double h) { return Prec<R>::from_d(d_half(
 // FP64 1/h for the coefficients of the FP64 conservative update: as geo_rcp
 // in the FP64 form; the MUFU reciprocal with two Newton steps in the mixed
 // form (whose fluxes are FP32).
-template <typename R>
+template <typename R, bool kP2 = false>
 __device__ __forceinline__ double geo_rcp_d(double h) {
   if constexpr (Prec<R>::kMixed) {
     return d_rcp_newton(h);
   } else {
-    return 1.0 / h;
+    return kP2 ? d_pow2_rcp(h) : 1.0 / h;
   }
+}
+// 1/(h*h), FP64 form only (CFL keys).
+template <bool kP2>
+__device__ __forceinline__ double geo_rcp_sq(double h) {
+  return kP2 ? d_pow2_rcp_sq(h) : 1.0 / (h * h);
 }
 
 // The FP64 quotient as a called function: a branch around five inline FP64
@@ -537,11 +609,14 @@ __device__ __forceinline__ R face_velocity(R mom, R rbar) {
 
 // Volume-weighted face value a*wa + b*wb, rounded once after the product
 // b*wb (the reference's a*wa + b*wb contracted as in the fused kernels).  On a
-// uniform mesh both weights are 1/2 and the rounding is that of the sum.
-template <typename R, bool kU>
+// uniform mesh both weights are 1/2 and the rounding is that of the sum; with
+// power-of-two weights both products are exact exponent adds.
+template <typename R, int kM>
 __device__ __forceinline__ R face_average(R a, R wa, R b, R wb) {
-  if constexpr (kU) {
+  if constexpr (kM == kMeshUniform) {
     return Prec<R>::half(a + b);
+  } else if constexpr (kM == kMeshPow2) {
+    return Prec<R>::template mulp<true>(a, wa) + Prec<R>::template mulp<true>(b, wb);
   } else {
     return fma(a, wa, b * wb);
   }
@@ -549,12 +624,12 @@ __device__ __forceinline__ R face_average(R a, R wa, R b, R wb) {
 
 // A face momentum less dt * diff / h (inv_h = 1/h); on a uniform mesh k is
 // dt / h.
-template <typename R, bool kU>
+template <typename R, int kM>
 __device__ __forceinline__ R momentum_step(R m, R diff, R k, R dt, R h, R inv_h) {
-  if constexpr (kU) {
+  if constexpr (kM == kMeshUniform) {
     return fma(-k, diff, m);
   } else {
-    return Prec<R>::dsub(m, dt * diff, h, inv_h);
+    return Prec<R>::template dsub<kM == kMeshPow2>(m, dt * diff, h, inv_h);
   }
 }
 
@@ -566,11 +641,16 @@ __device__ __forceinline__ R momentum_step(R m, R diff, R k, R dt, R h, R inv_h)
 // shock-heating kernel reads it where a cell is compressed) and every interior
 // x/y face.  The reference's rho_old copy is not made: the first mass sweep
 // reads the density itself.  omp3/flow.c:55-70, 110-158.
-template <typename R, bool kU, bool kFl>
+template <typename R, int kM, bool kFl>
 __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int bx, int by) {
+  constexpr bool kU = kM == kMeshUniform, kP2 = kM == kMeshPow2;
   using Pr = Prec<R>;
-  __shared__ R sP[kCols + 1], sR[kCols + 1];
-  __shared__ R s_ey[kMaxRows], s_iey[kMaxRows], s_wy0[kMaxRows], s_wy1[kMaxRows];
+  R* const sP = tile_table<R, kCols + 1, 0>();
+  R* const sR = tile_table<R, kCols + 1, 1>();
+  R* const s_ey = tile_table<R, kMaxRows + 3, 0>();
+  R* const s_iey = tile_table<R, kMaxRows + 3, 1>();
+  R* const s_wy0 = tile_table<R, kMaxRows + 3, 2>();
+  R* const s_wy1 = tile_table<R, kMaxRows + 3, 3>();
   const int nx = a.nx, ny = a.ny, pad = a.pad;
   const int t = threadIdx.x;
   const int jj = bx * kCols + t;
@@ -588,17 +668,17 @@ __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int
       if (ii >= 1 && ii < ny) {
         const double ey = a.edgedy[ii];
         s_ey[t] = geo_v<R>(ey);
-        s_iey[t] = geo_rcp<R>(ey);
-        s_wy0[t] = geo_half_ratio<R>(a.celldy[ii], ey);
-        s_wy1[t] = geo_half_ratio<R>(a.celldy[ii - 1], ey);
+        s_iey[t] = geo_rcp<R, kP2>(ey);
+        s_wy0[t] = geo_half_ratio<R, kP2>(a.celldy[ii], ey);
+        s_wy1[t] = geo_half_ratio<R, kP2>(a.celldy[ii - 1], ey);
       }
     }
     if (jj >= 1 && jj < nx) {
       const double ex = a.edgedx[jj];
       exr = geo_v<R>(ex);
-      iex = geo_rcp<R>(ex);
-      wx0 = geo_half_ratio<R>(a.celldx[jj], ex);
-      wx1 = geo_half_ratio<R>(a.celldx[jj - 1], ex);
+      iex = geo_rcp<R, kP2>(ex);
+      wx0 = geo_half_ratio<R, kP2>(a.celldx[jj], ex);
+      wx1 = geo_half_ratio<R, kP2>(a.celldx[jj - 1], ex);
     }
   }
   const R dt = Pr::from_d(a.dt);
@@ -664,14 +744,16 @@ __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int
       // face density, without FP64 instructions.
       if (kU && warp_all(lane_same(Pc, Pl) && lane_same(rc, rl))) {
         rbar = rc;
+      } else if (kP2 && warp_all(lane_same(Pc, Pl) && lane_same(rc, rl) && lane_same(wx0, wx1))) {
+        rbar = Pr::twice(Pr::template mulp<true>(rc, wx0));
       } else {
         const R dp = Pc - Pl;
         if (!Pr::zero_skip_mem(dp)) {
-          mom = momentum_step<R, kU>(mom, dp, kx, dt, exr, iex);
+          mom = momentum_step<R, kM>(mom, dp, kx, dt, exr, iex);
           a.rho_u[f] = mom;
         }
         dmom = !Pr::is_zero(dp);
-        rbar = face_average<R, kU>(rc, wx0, rl, wx1);
+        rbar = face_average<R, kM>(rc, wx0, rl, wx1);
       }
       const R vel = face_velocity(mom, rbar);
       a.u[f] = vel;
@@ -686,14 +768,17 @@ __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int
       const R wy0 = kU ? R(0) : s_wy0[k], wy1 = kU ? R(0) : s_wy1[k];
       if (kU && warp_all(lane_same(Pc, P_dn) && lane_same(rc, r_dn))) {
         rbar = rc;
+      } else if (kP2 && warp_all(lane_same(Pc, P_dn) && lane_same(rc, r_dn) &&
+                                 lane_same(wy0, wy1))) {
+        rbar = Pr::twice(Pr::template mulp<true>(rc, wy0));
       } else {
         const R dp = Pc - P_dn;
         if (!Pr::zero_skip_mem(dp)) {
-          mom = momentum_step<R, kU>(mom, dp, ky, dt, kU ? R(0) : s_ey[k], kU ? R(0) : s_iey[k]);
+          mom = momentum_step<R, kM>(mom, dp, ky, dt, kU ? R(0) : s_ey[k], kU ? R(0) : s_iey[k]);
           a.rho_v[c] = mom;
         }
         dmom = !Pr::is_zero(dp);
-        rbar = face_average<R, kU>(rc, wy0, r_dn, wy1);
+        rbar = face_average<R, kM>(rc, wy0, r_dn, wy1);
       }
       const R vel = face_velocity(mom, rbar);
       a.v[c] = vel;
@@ -715,7 +800,7 @@ __device__ __forceinline__ void tile_lag_pressure_impl(const StepArgs<R>& a, int
 // which move: each test is a load and a barrier ahead of the tile's own (about
 // a microsecond), and a tile at rest that takes the plain path stores the
 // values its arrays hold.
-template <typename R, bool kFl = false, bool kTest = true>
+template <typename R, bool kFl = false, bool kTest = true, bool kP2T = false>
 __device__ __forceinline__ void tile_lag_pressure(const StepArgs<R>& a, int bx, int by, bool uni) {
   if constexpr (kFl && kTest) {
     // A tile whose cells (and the row above and column left it reads) were
@@ -727,8 +812,10 @@ __device__ __forceinline__ void tile_lag_pressure(const StepArgs<R>& a, int bx, 
     const int c0 = bx * kCols, i0 = by * a.rows;
     if (a.rest && rest_cells(a, i0 - 1, i0 + a.rows, c0 - 1, c0 + kCols)) return;
   }
-  FLOW_UNIFORM_DISPATCH(R, (tile_lag_pressure_impl<R, true, kFl>(a, bx, by)),
-                        (tile_lag_pressure_impl<R, false, kFl>(a, bx, by)));
+  FLOW_MESH_DISPATCH(R, kP2T, block_mesh_pow2(a, bx * kCols, by * a.rows),
+                     (tile_lag_pressure_impl<R, kMeshUniform, kFl>(a, bx, by)),
+                     (tile_lag_pressure_impl<R, kMeshPow2, kFl>(a, bx, by)),
+                     (tile_lag_pressure_impl<R, kMeshGeneral, kFl>(a, bx, by)));
 }
 
 // Artificial viscous stresses on interior cells, omp3/flow.c:173-207.
@@ -861,10 +948,14 @@ __device__ __forceinline__ void tile_lag_viscosity(const StepArgs<R>& a, int bx,
 // the persistent batched kernel, whose register budget is spent across all
 // its phases).  With stress flags, a tile none of whose stresses can be
 // non-zero returns at once, and a stress flagged +0 is not loaded.
-template <typename R, bool kU, bool kEarly, bool kFlags>
+template <typename R, int kM, bool kEarly, bool kFlags>
 __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a, int bx, int by) {
+  constexpr bool kU = kM == kMeshUniform, kP2 = kM == kMeshPow2;
   using Pr = Prec<R>;
-  __shared__ R s_cy[kMaxRows], s_icy[kMaxRows], s_wy0[kMaxRows], s_wy1[kMaxRows];
+  R* const s_cy = tile_table<R, kMaxRows + 3, 0>();
+  R* const s_icy = tile_table<R, kMaxRows + 3, 1>();
+  R* const s_wy0 = tile_table<R, kMaxRows + 3, 2>();
+  R* const s_wy1 = tile_table<R, kMaxRows + 3, 3>();
   // Stress flags (a.qmask) of rows i0 - 1 .. i1 - 1, each row taken at its
   // mirror source: the words of column tiles bx - 1 and bx.
   __shared__ unsigned s_qf[kMaxRows + 1][2];
@@ -876,9 +967,9 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
     const int ii = i0 + threadIdx.x;
     if (ii < ny) {
       s_cy[threadIdx.x] = geo_v<R>(a.celldy[ii]);
-      s_icy[threadIdx.x] = geo_rcp<R>(a.celldy[ii]);
-      s_wy0[threadIdx.x] = geo_half_ratio<R>(a.celldy[ii], a.edgedy[ii]);
-      s_wy1[threadIdx.x] = geo_half_ratio<R>(a.celldy[ii - 1], a.edgedy[ii]);
+      s_icy[threadIdx.x] = geo_rcp<R, kP2>(a.celldy[ii]);
+      s_wy0[threadIdx.x] = geo_half_ratio<R, kP2>(a.celldy[ii], a.edgedy[ii]);
+      s_wy1[threadIdx.x] = geo_half_ratio<R, kP2>(a.celldy[ii - 1], a.edgedy[ii]);
     }
   }
   const bool col_ok = jj < nx + 1 - pad;
@@ -945,9 +1036,9 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
     ky = a.dt * um.iy;
   } else {
     cx = geo_v<R>(a.celldx[jj]);
-    icx = geo_rcp<R>(a.celldx[jj]);
-    wx0 = geo_half_ratio<R>(a.celldx[jj], a.edgedx[jj]);
-    wx1 = geo_half_ratio<R>(a.celldx[jj - 1], a.edgedx[jj]);
+    icx = geo_rcp<R, kP2>(a.celldx[jj]);
+    wx0 = geo_half_ratio<R, kP2>(a.celldx[jj], a.edgedx[jj]);
+    wx1 = geo_half_ratio<R, kP2>(a.celldx[jj - 1], a.edgedx[jj]);
   }
   const R dt = Pr::from_d(a.dt);
   if (!kEarly) prime();
@@ -960,10 +1051,10 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
       if (!warp_same(q1, q0)) {  // equal stresses in the whole warp: dqx = +0
         const R dqx = q1 - q0;
         if (!Pr::zero_skip_mem(dqx)) {
-          const R mom = momentum_step<R, kU>(a.rho_u[f], dqx, kx, dt, cx, icx);
+          const R mom = momentum_step<R, kM>(a.rho_u[f], dqx, kx, dt, cx, icx);
           const size_t c = cidx(nx, ii, jj);
           const R vel =
-              face_velocity(mom, face_average<R, kU>(a.rho_r[c], wx0, a.rho_r[c - 1], wx1));
+              face_velocity(mom, face_average<R, kM>(a.rho_r[c], wx0, a.rho_r[c - 1], wx1));
           a.rho_u[f] = mom;
           a.u[f] = vel;
           mirror(edge, a.u, nx + 1, ny, pad, ii, jj, vel, true, false);
@@ -976,10 +1067,10 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
       if (!warp_same(qy, qy_dn)) {
         const R dqy = qy - qy_dn;
         if (!Pr::zero_skip_mem(dqy)) {
-          const R mom = momentum_step<R, kU>(a.rho_v[c], dqy, ky, dt, kU ? R(0) : s_cy[k],
+          const R mom = momentum_step<R, kM>(a.rho_v[c], dqy, ky, dt, kU ? R(0) : s_cy[k],
                                              kU ? R(0) : s_icy[k]);
           const R vel = face_velocity(
-              mom, face_average<R, kU>(a.rho_r[c], kU ? R(0) : s_wy0[k], a.rho_r[c - nx],
+              mom, face_average<R, kM>(a.rho_r[c], kU ? R(0) : s_wy0[k], a.rho_r[c - nx],
                                        kU ? R(0) : s_wy1[k]));
           a.rho_v[c] = mom;
           a.v[c] = vel;
@@ -1035,8 +1126,10 @@ __device__ __forceinline__ void tile_lag_viscous_accel_impl(const StepArgs<R>& a
 template <typename R, bool kEarly = true, bool kFlags = false>
 __device__ __forceinline__ void tile_lag_viscous_accel(const StepArgs<R>& a, int bx, int by,
                                                        bool uni) {
-  FLOW_UNIFORM_DISPATCH(R, (tile_lag_viscous_accel_impl<R, true, kEarly, kFlags>(a, bx, by)),
-                        (tile_lag_viscous_accel_impl<R, false, kEarly, kFlags>(a, bx, by)));
+  FLOW_MESH_DISPATCH(R, false, false,
+                     (tile_lag_viscous_accel_impl<R, kMeshUniform, kEarly, kFlags>(a, bx, by)),
+                     (void)0,
+                     (tile_lag_viscous_accel_impl<R, kMeshGeneral, kEarly, kFlags>(a, bx, by)));
 }
 
 __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long x) {
@@ -1107,12 +1200,14 @@ __device__ __forceinline__ double shock_energy_uniform(double e, double du, doub
 // block on the FP64 bit pattern of its smallest candidate; the last block to
 // finish applies the leapfrog dt/dt_h rule (finish_dt).  In the mixed form
 // the FP32 energy change is added to the FP64 energy.
-template <typename R, bool kU, bool kRing, bool kFlags, bool kTest>
+template <typename R, int kM, bool kRing, bool kFlags, bool kTest>
 __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, int bx, int by,
                                                         unsigned long long* tile_min) {
+  constexpr bool kU = kM == kMeshUniform, kP2 = kM == kMeshPow2;
   using Pr = Prec<R>;
-  __shared__ R s_icy[kMaxRows], s_cy[kMaxRows];
-  __shared__ double s_icy2[kMaxRows];
+  R* const s_icy = tile_table<R, kMaxRows + 3, 0>();
+  R* const s_cy = tile_table<R, kMaxRows + 3, 1>();
+  double* const s_icy2 = tile_table<double, kMaxRows + 3, 2>();
   __shared__ unsigned long long s_warp[kCols / 32], s_warp_y[kCols / 32];
   __shared__ unsigned s_qf[kMaxRows];  // stress-flag words of the tile's rows
   const int nx = a.nx, ny = a.ny, pad = a.pad;
@@ -1123,8 +1218,8 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
     const int ii = i0 + threadIdx.x;
     if (!kU && ii < ny) {
       s_cy[threadIdx.x] = geo_v<R>(a.celldy[ii]);
-      s_icy[threadIdx.x] = geo_rcp<R>(a.celldy[ii]);
-      if constexpr (!Pr::kMixed) s_icy2[threadIdx.x] = 1.0 / (a.celldy[ii] * a.celldy[ii]);
+      s_icy[threadIdx.x] = geo_rcp<R, kP2>(a.celldy[ii]);
+      if constexpr (!Pr::kMixed) s_icy2[threadIdx.x] = geo_rcp_sq<kP2>(a.celldy[ii]);
     }
     if (kFlags && ii < ny - pad) s_qf[threadIdx.x] = a.qmask[(size_t)(ii - pad) * a.qm_stride + bx];
   }
@@ -1155,8 +1250,8 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
       ky = a.dt_h * um.iy;
     } else {
       cx = geo_v<R>(a.celldx[jj]);
-      icx = geo_rcp<R>(a.celldx[jj]);
-      if constexpr (!Pr::kMixed) icx2 = 1.0 / (a.celldx[jj] * a.celldx[jj]);
+      icx = geo_rcp<R, kP2>(a.celldx[jj]);
+      if constexpr (!Pr::kMixed) icx2 = geo_rcp_sq<kP2>(a.celldx[jj]);
     }
     const R dt_h = Pr::from_d(a.dt_h);
     const int i1 = min(i0 + a.rows, ny - pad);
@@ -1215,8 +1310,8 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
         // is the smallest dt) and take the square root only for the
         // thread's winner after the loop.  Keys in [+0, +inf] only: a
         // negative or NaN S is a NaN candidate in the reference.
-        const long long qx = e_neg ? -1 : dbits(sx * icx2);
-        const long long qy = e_neg ? -1 : dbits(sy * s_icy2[k]);
+        const long long qx = e_neg ? -1 : dbits(Prec<double>::mulp<kP2>(sx, icx2));
+        const long long qy = e_neg ? -1 : dbits(Prec<double>::mulp<kP2>(sy, s_icy2[k]));
         if (qx >= 0 && qx <= 0x7ff0000000000000LL && qx > kbest) {
           kbest = qx;
           s_best = sx;
@@ -1284,8 +1379,8 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
           e_new = shock_energy_uniform(er, du, dv, kx, ky, q_any, qx, qy, inv_r);
         }
       } else {
-        const R dudx = (u1f - u0f) * icx;
-        const R dvdy = (v1 - v0) * s_icy[k];
+        const R dudx = Pr::template mulp<kP2>(u1f - u0f, icx);
+        const R dvdy = Pr::template mulp<kP2>(v1 - v0, s_icy[k]);
         still = Pr::zero_skip_coarse(dudx) && Pr::zero_skip_coarse(dvdy);
         if (still) {
           // (Mixed form: the FP64 energy is not needed, as it is kept.)
@@ -1394,7 +1489,7 @@ __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, in
 }
 
 // tile_min: where thread 0 also stores the tile's CFL minimum, or null.
-template <typename R, bool kRing = true, bool kFlags = false, bool kTest = true>
+template <typename R, bool kRing = true, bool kFlags = false, bool kTest = true, bool kP2T = false>
 __device__ __forceinline__ void tile_lag_energy_dt(const StepArgs<R>& a, int bx, int by, bool uni,
                                                    unsigned long long* tile_min = nullptr) {
   if constexpr (kFlags && kTest) {
@@ -1417,8 +1512,11 @@ __device__ __forceinline__ void tile_lag_energy_dt(const StepArgs<R>& a, int bx,
       }
     }
   }
-  FLOW_UNIFORM_DISPATCH(R, (tile_lag_energy_dt_impl<R, true, kRing, kFlags, kTest>(a, bx, by, tile_min)),
-                        (tile_lag_energy_dt_impl<R, false, kRing, kFlags, kTest>(a, bx, by, tile_min)));
+  FLOW_MESH_DISPATCH(
+      R, kP2T, block_mesh_pow2(a, a.pad + bx * kCols, a.pad + by * a.rows),
+      (tile_lag_energy_dt_impl<R, kMeshUniform, kRing, kFlags, kTest>(a, bx, by, tile_min)),
+      (tile_lag_energy_dt_impl<R, kMeshPow2, kRing, kFlags, kTest>(a, bx, by, tile_min)),
+      (tile_lag_energy_dt_impl<R, kMeshGeneral, kRing, kFlags, kTest>(a, bx, by, tile_min)));
 }
 
 // The leapfrog dt/dt_h rule of omp3/flow.c:103-105 for the CFL minimum g, in
@@ -1465,13 +1563,13 @@ __device__ __forceinline__ DtPair sweep_dt(const StepArgs<R>& a) {
 // multiplication instead of three; halving, doubling and negation are exact
 // integer operations.  A zero slope (flat or extremal data) leaves the base
 // value, and the reconstruction arithmetic is skipped.
-template <typename R>
+template <typename R, bool kP2>
 __device__ __forceinline__ R mc_reconstruct(bool pos, R da, R db, R dc, R base, R inv_h, R h,
                                             R wdt) {
   using Pr = Prec<R>;
   const R m0 = Pr::minmod(Pr::half(da), Pr::twice(db), Pr::twice(dc));
   if (Pr::zero_skip(m0)) return base;
-  const R mm = m0 * inv_h;
+  const R mm = Pr::template mulp<kP2>(m0, inv_h);
   const R w = h + (pos ? Pr::neg(wdt) : wdt);
   const R hm = Pr::half(pos ? mm : Pr::neg(mm));
   return Pr::madd(hm, w, base);
@@ -1490,12 +1588,12 @@ __device__ __forceinline__ double mc_reconstruct_uniform(bool pos, double da, do
 
 // The same from the four values themselves, selecting the operands before
 // subtracting so that each difference is one FP64 instruction.
-template <typename R>
+template <typename R, bool kP2>
 __device__ __forceinline__ R mc_face(bool pos, R m2, R m1, R p0, R p1, R inv_h, R h, R wdt) {
   const R a0 = pos ? p0 : p1;
   const R a1 = pos ? m2 : m1;
   const R base = pos ? m1 : p0;
-  return mc_reconstruct<R>(pos, a0 - a1, base - a1, a0 - base, base, inv_h, h, wdt);
+  return mc_reconstruct<R, kP2>(pos, a0 - a1, base - a1, a0 - base, base, inv_h, h, wdt);
 }
 __device__ __forceinline__ double mc_face_uniform(bool pos, double m2, double m1, double p0,
                                                   double p1, double wind, double c) {
@@ -1549,9 +1647,10 @@ struct ColWindow {
     D1 = D2; D2 = carried(p1 - m1);
   }
   // mc_face of the window's face (between m1 and p0).
+  template <bool kP2>
   __device__ __forceinline__ R face(bool pos, R inv_h, R h, R wdt) const {
-    return mc_reconstruct<R>(pos, pos ? D1 : D2, pos ? d1 : d2, pos ? d2 : d3,
-                             pos ? m1 : p0, inv_h, h, wdt);
+    return mc_reconstruct<R, kP2>(pos, pos ? D1 : D2, pos ? d1 : d2, pos ? d2 : d3,
+                                  pos ? m1 : p0, inv_h, h, wdt);
   }
   __device__ __forceinline__ R face_uniform(bool pos, R wind, R c) const {
     return mc_reconstruct_uniform(pos, pos ? D1 : D2, pos ? d1 : d2, pos ? d2 : d3,
@@ -1598,7 +1697,7 @@ struct ColSteps {
 // side from v0 (the y sweep, omp3/flow.c:477) instead of the half-step
 // velocity.  A zero limiter (flat or extremal density) leaves the upwind
 // flux, and the second-order term is skipped.
-template <typename R, bool kSideV0, typename NumFn, typename EFaceFn>
+template <typename R, bool kSideV0, bool kP2, typename NumFn, typename EFaceFn>
 __device__ __forceinline__ void mass_energy_flux_core(R v0, R dv2, R dvm, R dvp, R rm1, R r0,
                                                       R jump, NumFn num_of, EFaceFn e_face_of,
                                                       R inv_h, R icd, R area, R dt, R dt_h,
@@ -1610,8 +1709,8 @@ __device__ __forceinline__ void mass_energy_flux_core(R v0, R dv2, R dvm, R dvp,
     return;
   }
   // minmod(0.5 (vp-vm)/h, 2 (v0-vm)/h, 2 (vp-v0)/h), scaled once (mc_reconstruct).
-  const R mm =
-      Pr::minmod(Pr::twice(dvm), Pr::twice(dvp), Pr::half(dv2)) * inv_h;
+  const R mm = Pr::template mulp<kP2>(
+      Pr::minmod(Pr::twice(dvm), Pr::twice(dvp), Pr::half(dv2)), inv_h);
   const R w_tc = Pr::msub(v0, Pr::half(v0) * dt, mm);
   R lim = R(0);
   if (!Pr::is_zero(jump)) {
@@ -1631,11 +1730,11 @@ __device__ __forceinline__ void mass_energy_flux_core(R v0, R dv2, R dvm, R dvp,
   } else {
     flux = Pr::madd(w_tc, rho_up,
                     Pr::half(Pr::abs(w_tc)) *
-                        (R(1) - Pr::abs(wdt * icd)) * lim * jump);
+                        (R(1) - Pr::abs(Pr::template mulp<kP2>(wdt, icd))) * lim * jump);
   }
   const R e_face = e_face_of(Pr::gt0(w_tc), wdt);
   *F_out = flux;
-  *eF_out = e_face * area * flux;
+  *eF_out = Pr::template mulp<kP2>(e_face, area) * flux;
 }
 
 // The same on a uniform mesh (FP64 form), with the timesteps over the spacing
@@ -1673,18 +1772,18 @@ __device__ __forceinline__ void mass_energy_flux_uniform(double v0, double dv2, 
 // The flux from the four cells straddling the face (m2, m1 | p0, p1) and
 // the face velocities vm, v0, vp (the x sweep); h_m/h_p are the cell widths
 // either side.
-template <typename R, bool kSideV0>
+template <typename R, bool kSideV0, bool kP2>
 __device__ __forceinline__ void mass_energy_flux(R vm, R v0, R vp, R rm2,
                                                  R rm1, R r0, R rp1, R em2,
                                                  R em1, R e0, R ep1, R inv_h,
                                                  R h_m, R h_p, R icd, R area,
                                                  R dt, R dt_h, R* F_out,
                                                  R* eF_out) {
-  mass_energy_flux_core<R, kSideV0>(
+  mass_energy_flux_core<R, kSideV0, kP2>(
       v0, vp - vm, v0 - vm, vp - v0, rm1, r0, r0 - rm1,
       [&](bool up) { return (up ? rm1 : rp1) - (up ? rm2 : r0); },
       [&](bool pos, R wdt) {
-        return mc_face<R>(pos, em2, em1, e0, ep1, inv_h, pos ? h_m : h_p, wdt);
+        return mc_face<R, kP2>(pos, em2, em1, e0, ep1, inv_h, pos ? h_m : h_p, wdt);
       },
       inv_h, icd, area, dt, dt_h, F_out, eF_out);
 }
@@ -1722,9 +1821,9 @@ static __device__ __noinline__ double still_energy(double r_old, double e_in, do
 // The fluxes (f0, f1 mass, ef0, ef1 energy) arrive in bulk precision; the
 // mixed form takes their differences to FP64 on the other pipes (diff_d: two of
 // the eight FP64 instructions of a cell, which bound its sweeps).
-// kU: a uniform mesh, with the coefficients kf, ke of the mass and energy flux
+// kM: on a uniform mesh with the coefficients kf, ke of the mass and energy flux
 // differences in the place of dt_h, vol, ivol and the face lengths.
-template <typename R, bool kFirst, bool kU>
+template <typename R, bool kFirst, int kM>
 __device__ __forceinline__ void mass_energy_update(double r_in, double e_in,
                                                    double r_old, double dt_h,
                                                    double vol, double ivol, double a0,
@@ -1757,7 +1856,7 @@ __device__ __forceinline__ void mass_energy_update(double r_in, double e_in,
     // energy still takes the reference's rho_old*e/den round trip below.)
     r_new = r_in;
     rho_e = __dmul_rn(r_old, e_in);
-  } else if constexpr (kU) {
+  } else if constexpr (kM == kMeshUniform) {
     r_new = fma(-kf, Pr::diff_d(f1, f0), r_in);
     rho_e = fma(-ke, de, __dmul_rn(r_old, e_in));
   } else if constexpr (Pr::kMixed) {
@@ -1766,9 +1865,11 @@ __device__ __forceinline__ void mass_energy_update(double r_in, double e_in,
     r_new = fma(-coef, net, r_in);
     rho_e = fma(-coef, de, r_old * e_in);
   } else {
-    const double net = __dadd_rn(f1 * a1, -__dmul_rn(f0, a0));
-    r_new = Prec<double>::dsub(r_in, __dmul_rn(dt_h, net), vol, ivol);
-    rho_e = Prec<double>::dsub(__dmul_rn(r_old, e_in), __dmul_rn(dt_h, de), vol, ivol);
+    constexpr bool kP2 = kM == kMeshPow2;
+    const double net = kP2 ? __dadd_rn(d_mul_pow2(f1, a1), -d_mul_pow2(f0, a0))
+                           : __dadd_rn(f1 * a1, -__dmul_rn(f0, a0));
+    r_new = Prec<double>::dsub<kP2>(r_in, __dmul_rn(dt_h, net), vol, ivol);
+    rho_e = Prec<double>::dsub<kP2>(__dmul_rn(r_old, e_in), __dmul_rn(dt_h, de), vol, ivol);
   }
   const double den = kFirst ? r_old : r_new;
   *r_out = r_new;
@@ -1846,14 +1947,20 @@ __device__ __forceinline__ bool block_round_trip_exact(const double* rho, const 
 // kAlt (second sweep with flags): some tile near this one was skipped by the
 // first sweep (sk3, the skip marks of this band's y-sweep tiles tlo ..
 // tlo + 2); without it the loads need no selection.
-template <typename R, bool kFirst, bool kU, bool kEarly, bool kFl, bool kAlt>
+template <typename R, bool kFirst, int kM, bool kEarly, bool kFl, bool kAlt>
 __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
                                                        const SweepArgs<R>& s, int bx, int by,
                                                        unsigned sk3) {
+  constexpr bool kU = kM == kMeshUniform, kP2 = kM == kMeshPow2;
   using Pr = Prec<R>;
-  __shared__ R s_ey0r[kMaxRows];
-  __shared__ R sF[kCols], seF[kCols];  // the row's face fluxes
-  __shared__ double s_coef[kMaxRows], s_cyd[kMaxRows], s_ey0[kMaxRows], s_ey1[kMaxRows];
+  R* const s_ey0r = tile_table<R, kMaxRows + 3, 0>();
+  // The row's face fluxes.
+  R* const sF = tile_table<R, kCols, 0>();
+  R* const seF = tile_table<R, kCols, 1>();
+  double* const s_coef = tile_table<double, kMaxRows + 3, 1>();
+  double* const s_cyd = tile_table<double, kMaxRows + 3, 2>();
+  double* const s_ey0 = tile_table<double, kMaxRows + 3, 3>();
+  double* const s_ey1 = tile_table<double, kMaxRows + 3, 4>();
   const int nx = a.nx, ny = a.ny, pad = a.pad;
   const int t = threadIdx.x;
   const int jj = pad + bx * (kCols - 1) + t;  // face (and cell) column
@@ -1878,7 +1985,8 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
       s_ey0r[t] = geo_v<R>(a.edgedy[ii]);
       if constexpr (!kU) {
         // Row factor of the update: 1/celldy, times dt_h in the mixed form.
-        s_coef[t] = Pr::kMixed ? dt_h * geo_rcp_d<R>(a.celldy[ii]) : geo_rcp_d<R>(a.celldy[ii]);
+        const double ih = geo_rcp_d<R, kP2>(a.celldy[ii]);
+        s_coef[t] = Pr::kMixed ? dt_h * ih : ih;
         s_cyd[t] = a.celldy[ii];
         s_ey0[t] = a.edgedy[ii];
         s_ey1[t] = a.edgedy[ii + 1];
@@ -1891,10 +1999,10 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
   R iex = R(0), cxm = R(0), cx0 = R(0), icx_r = R(0);
   double icx = 0.0;
   if (!kUd && face_ok) {
-    iex = geo_rcp<R>(a.edgedx[jj]);
+    iex = geo_rcp<R, kP2>(a.edgedx[jj]);
     cxm = geo_v<R>(a.celldx[jj - 1]);
     cx0 = geo_v<R>(a.celldx[jj]);
-    icx = geo_rcp_d<R>(a.celldx[jj]);
+    icx = geo_rcp_d<R, kP2>(a.celldx[jj]);
     icx_r = Pr::from_d(icx);
   }
   const R dt_r = Pr::from_d(dt), dt_h_r = Pr::from_d(dt_h);
@@ -2002,9 +2110,9 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
             [&](bool pos, double w) { return mc_face_uniform(pos, e2, e1, e0, p1, w, kh); }, kd,
             kh, &F, &eF);
       } else {
-        mass_energy_flux<R, false>(a.u[f - 1], u0, a.u[f + 1], rr(-2), rr(-1), rr(0), rr(1),
-                                   er(-2), er(-1), er(0), er(1), iex, cxm, cx0, icx_r,
-                                   s_ey0r[k], dt_r, dt_h_r, &F, &eF);
+        mass_energy_flux<R, false, kP2>(a.u[f - 1], u0, a.u[f + 1], rr(-2), rr(-1), rr(0), rr(1),
+                                        er(-2), er(-1), er(0), er(1), iex, cxm, cx0, icx_r,
+                                        s_ey0r[k], dt_r, dt_h_r, &F, &eF);
       }
     }
     // kFl: a warp at rest stores only its flag (its fluxes are +0).
@@ -2020,10 +2128,10 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
     __syncthreads();
     if (cell_ok) {
       double r_new, e_new;
-      mass_energy_update<R, kFirst, kU>(
-          r_in, e_in, r_old, dt_h, kU ? 0.0 : a.celldx[jj] * s_cyd[k], kU ? 0.0 : s_coef[k] * icx,
-          kU ? 0.0 : s_ey0[k], kU ? 0.0 : s_ey1[k], sF[t], sF[t + 1], seF[t], seF[t + 1], kh, ke,
-          &r_new, &e_new);
+      mass_energy_update<R, kFirst, kM>(
+          r_in, e_in, r_old, dt_h, kU ? 0.0 : a.celldx[jj] * s_cyd[k],
+          kU ? 0.0 : Prec<double>::mulp<kP2>(s_coef[k], icx), kU ? 0.0 : s_ey0[k],
+          kU ? 0.0 : s_ey1[k], sF[t], sF[t + 1], seF[t], seF[t + 1], kh, ke, &r_new, &e_new);
       // (A cell of a skipped tile is at rest and keeps its value, which rho
       // and e hold: storing it again writes the same value.)
       store_cell(edge, s.r_out, s.r_out_r, nx, ny, pad, ii, jj, r_new);
@@ -2034,7 +2142,7 @@ __device__ __forceinline__ void tile_mass_sweep_x_impl(const StepArgs<R>& a,
   if constexpr (kEarly) cp_async_wait<0>();
 }
 
-template <typename R, bool kFirst, bool kEarly = true, bool kFl = false>
+template <typename R, bool kFirst, bool kEarly = true, bool kFl = false, bool kP2T = false>
 __device__ __forceinline__ void tile_mass_sweep_x(const StepArgs<R>& a, const SweepArgs<R>& s,
                                                   int bx, int by, bool uni) {
   if constexpr (kFl) {
@@ -2076,16 +2184,21 @@ __device__ __forceinline__ void tile_mass_sweep_x(const StepArgs<R>& a, const Sw
         return;
       }
       if (__syncthreads_or(sk3 != 0u)) {
-        FLOW_UNIFORM_DISPATCH_ALL(
-            (tile_mass_sweep_x_impl<R, kFirst, true, kEarly, kFl, true>(a, s, bx, by, sk3)),
-            (tile_mass_sweep_x_impl<R, kFirst, false, kEarly, kFl, true>(a, s, bx, by, sk3)));
+        FLOW_MESH_DISPATCH_ALL(
+            R, false, false,
+            (tile_mass_sweep_x_impl<R, kFirst, kMeshUniform, kEarly, kFl, true>(a, s, bx, by, sk3)),
+            (void)0,
+            (tile_mass_sweep_x_impl<R, kFirst, kMeshGeneral, kEarly, kFl, true>(a, s, bx, by,
+                                                                                sk3)));
         return;  // (the dispatch returns only after its uniform branch)
       }
     }
   }
-  FLOW_UNIFORM_DISPATCH_ALL(
-      (tile_mass_sweep_x_impl<R, kFirst, true, kEarly, kFl, false>(a, s, bx, by, 0u)),
-      (tile_mass_sweep_x_impl<R, kFirst, false, kEarly, kFl, false>(a, s, bx, by, 0u)));
+  FLOW_MESH_DISPATCH_ALL(
+      R, kP2T, block_mesh_pow2(a, a.pad + bx * (kCols - 1), a.pad + by * a.rows),
+      (tile_mass_sweep_x_impl<R, kFirst, kMeshUniform, kEarly, kFl, false>(a, s, bx, by, 0u)),
+      (tile_mass_sweep_x_impl<R, kFirst, kMeshPow2, kEarly, kFl, false>(a, s, bx, by, 0u)),
+      (tile_mass_sweep_x_impl<R, kFirst, kMeshGeneral, kEarly, kFl, false>(a, s, bx, by, 0u)));
 }
 
 // y sweep: each thread marches down its column; face row ii+1 is computed
@@ -2093,13 +2206,17 @@ __device__ __forceinline__ void tile_mass_sweep_x(const StepArgs<R>& a, const Sw
 // kAlt (second sweep with flags): some tile near this one was skipped by the
 // first sweep (sk3, the skip marks of bands by - 1 .. by + 1 of this
 // column's x-sweep tile); without it the loads need no selection.
-template <typename R, bool kFirst, bool kU, bool kEarly, bool kFl, bool kAlt>
+template <typename R, bool kFirst, int kM, bool kEarly, bool kFl, bool kAlt>
 __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
                                                        const SweepArgs<R>& s, int bx, int by,
                                                        unsigned sk3) {
+  constexpr bool kU = kM == kMeshUniform, kP2 = kM == kMeshPow2;
   using Pr = Prec<R>;
-  __shared__ R s_iey[kMaxRows + 1], s_cy[kMaxRows + 2], s_icy[kMaxRows + 1];
-  __shared__ double s_coef[kMaxRows], s_cyd[kMaxRows];
+  R* const s_iey = tile_table<R, kMaxRows + 3, 0>();
+  R* const s_cy = tile_table<R, kMaxRows + 3, 1>();
+  R* const s_icy = tile_table<R, kMaxRows + 3, 2>();
+  double* const s_coef = tile_table<double, kMaxRows + 3, 3>();
+  double* const s_cyd = tile_table<double, kMaxRows + 3, 4>();
   const int nx = a.nx, ny = a.ny, pad = a.pad;
   const int jj = pad + bx * kCols + threadIdx.x;
   const int i0 = pad + by * a.rows;
@@ -2125,11 +2242,11 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
   if (!kUd && threadIdx.x < a.rows + 1) {
     const int ii = i0 + threadIdx.x;
     if (ii < ny) {
-      s_iey[threadIdx.x] = geo_rcp<R>(a.edgedy[ii]);
-      s_icy[threadIdx.x] = geo_rcp<R>(a.celldy[ii]);
+      s_iey[threadIdx.x] = geo_rcp<R, kP2>(a.edgedy[ii]);
+      s_icy[threadIdx.x] = geo_rcp<R, kP2>(a.celldy[ii]);
       if (!kU && threadIdx.x < a.rows) {
         s_coef[threadIdx.x] =
-            Pr::kMixed ? dt_h * geo_rcp_d<R>(a.celldy[ii]) : geo_rcp_d<R>(a.celldy[ii]);
+            Pr::kMixed ? dt_h * geo_rcp_d<R, kP2>(a.celldy[ii]) : geo_rcp_d<R, kP2>(a.celldy[ii]);
         s_cyd[threadIdx.x] = a.celldy[ii];
       }
     }
@@ -2242,7 +2359,7 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
   double icx = 0.0, ex0 = 0.0, ex1 = 0.0, cxd = 0.0;
   if constexpr (!kUd) ex0 = a.edgedx[jj];
   if constexpr (!kU) {
-    icx = geo_rcp_d<R>(a.celldx[jj]);
+    icx = geo_rcp_d<R, kP2>(a.celldx[jj]);
     ex1 = a.edgedx[jj + 1];
     cxd = a.celldx[jj];
   }
@@ -2268,10 +2385,10 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
           v0, dv2, dvm, dvp, rw.m1, rw.p0, rw.d2, [&](bool up) { return up ? rw.d1 : rw.d3; },
           [&](bool pos, double w) { return ew.face_uniform(pos, w, kh); }, kd, kh, F, eF);
     } else {
-      mass_energy_flux_core<R, true>(
+      mass_energy_flux_core<R, true, kP2>(
           v0, dv2, dvm, dvp, rw.m1, rw.p0, rw.d2, [&](bool up) { return up ? rw.d1 : rw.d3; },
           [&](bool pos, R wdt) {
-            return ew.face(pos, s_iey[k], pos ? s_cy[k] : s_cy[k + 1], wdt);
+            return ew.template face<kP2>(pos, s_iey[k], pos ? s_cy[k] : s_cy[k + 1], wdt);
           },
           s_iey[k], s_icy[k], ex0_r, dt_r, dt_h_r, F, eF);
     }
@@ -2365,9 +2482,9 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
       store_fy(ii + 1, F1, fresh);
     }
     double r_new, e_new;
-    mass_energy_update<R, kFirst, kU>(r_in, e_in, r_old, dt_h, kU ? 0.0 : cxd * s_cyd[k],
-                                      kU ? 0.0 : s_coef[k] * icx, ex0, ex1, F0, F1, eF0, eF1,
-                                      kh, ke, &r_new, &e_new);
+    mass_energy_update<R, kFirst, kM>(r_in, e_in, r_old, dt_h, kU ? 0.0 : cxd * s_cyd[k],
+                                      kU ? 0.0 : Prec<double>::mulp<kP2>(s_coef[k], icx), ex0,
+                                      ex1, F0, F1, eF0, eF1, kh, ke, &r_new, &e_new);
     // (A cell of a skipped tile is at rest and keeps its value, which rho and
     // e hold: storing it again writes the same value.)
     store_cell(edge, s.r_out, s.r_out_r, nx, ny, pad, ii, jj, r_new);
@@ -2386,7 +2503,7 @@ __device__ __forceinline__ void tile_mass_sweep_y_impl(const StepArgs<R>& a,
   if constexpr (kEarly) cp_async_wait<0>();
 }
 
-template <typename R, bool kFirst, bool kEarly = true, bool kFl = false>
+template <typename R, bool kFirst, bool kEarly = true, bool kFl = false, bool kP2T = false>
 __device__ __forceinline__ void tile_mass_sweep_y(const StepArgs<R>& a, const SweepArgs<R>& s,
                                                   int bx, int by, bool uni) {
   if constexpr (kFl) {
@@ -2432,16 +2549,21 @@ __device__ __forceinline__ void tile_mass_sweep_y(const StepArgs<R>& a, const Sw
         return;
       }
       if (__syncthreads_or(sk3 != 0u)) {
-        FLOW_UNIFORM_DISPATCH_ALL(
-            (tile_mass_sweep_y_impl<R, kFirst, true, kEarly, kFl, true>(a, s, bx, by, sk3)),
-            (tile_mass_sweep_y_impl<R, kFirst, false, kEarly, kFl, true>(a, s, bx, by, sk3)));
+        FLOW_MESH_DISPATCH_ALL(
+            R, false, false,
+            (tile_mass_sweep_y_impl<R, kFirst, kMeshUniform, kEarly, kFl, true>(a, s, bx, by, sk3)),
+            (void)0,
+            (tile_mass_sweep_y_impl<R, kFirst, kMeshGeneral, kEarly, kFl, true>(a, s, bx, by,
+                                                                                sk3)));
         return;  // (the dispatch returns only after its uniform branch)
       }
     }
   }
-  FLOW_UNIFORM_DISPATCH_ALL(
-      (tile_mass_sweep_y_impl<R, kFirst, true, kEarly, kFl, false>(a, s, bx, by, 0u)),
-      (tile_mass_sweep_y_impl<R, kFirst, false, kEarly, kFl, false>(a, s, bx, by, 0u)));
+  FLOW_MESH_DISPATCH_ALL(
+      R, kP2T, block_mesh_pow2(a, a.pad + bx * kCols, a.pad + by * a.rows),
+      (tile_mass_sweep_y_impl<R, kFirst, kMeshUniform, kEarly, kFl, false>(a, s, bx, by, 0u)),
+      (tile_mass_sweep_y_impl<R, kFirst, kMeshPow2, kEarly, kFl, false>(a, s, bx, by, 0u)),
+      (tile_mass_sweep_y_impl<R, kFirst, kMeshGeneral, kEarly, kFl, false>(a, s, bx, by, 0u)));
 }
 
 // ===========================================================================
@@ -2449,16 +2571,17 @@ __device__ __forceinline__ void tile_mass_sweep_y(const StepArgs<R>& a, const Sw
 
 // MC-limited upwind value of a velocity at a flux point from its four
 // neighbours along the direction (m2, m1 | p0, p1): omp3/flow.c:791-820.
-// kU: a uniform mesh, with the coefficient c = dt_h / h.
-template <typename R, bool kU>
+// c: on a uniform mesh, dt_h / h.
+template <typename R, int kM>
 __device__ __forceinline__ R momentum_upwind(R wind, R m2, R m1, R p0, R p1,
                                              R inv_h, R d_left, R d_right,
                                              R dt_h, R c) {
   const bool pos = Prec<R>::gt0(wind);
-  if constexpr (kU) {
+  if constexpr (kM == kMeshUniform) {
     return mc_face_uniform(pos, m2, m1, p0, p1, wind, c);
   } else {
-    return mc_face<R>(pos, m2, m1, p0, p1, inv_h, pos ? d_left : d_right, wind * dt_h);
+    return mc_face<R, kM == kMeshPow2>(pos, m2, m1, p0, p1, inv_h, pos ? d_left : d_right,
+                                       wind * dt_h);
   }
 }
 
@@ -2495,14 +2618,15 @@ static __device__ __noinline__ double momentum_change_uniform(double* mom, doubl
   *mom = m;
   return m;
 }
-template <bool kVel>
+template <bool kVel, bool kP2>
 static __device__ __noinline__ double momentum_change(double* mom, double m, double fa, double fb,
                                                       double dt_h, double hx, double h,
                                                       double inv_h, double ihx) {
   const double diff = fa - fb;
   if (d_is_zero(diff)) return m;
   if (!kVel) m = *mom;
-  m = Prec<double>::dsub(m, dt_h * diff, hx * h, inv_h * ihx);
+  using Pr = Prec<double>;
+  m = Pr::dsub<kP2>(m, dt_h * diff, hx * h, Pr::mulp<kP2>(inv_h, ihx));
   *mom = m;
   return m;
 }
@@ -2513,8 +2637,8 @@ static __device__ __noinline__ double momentum_change(double* mom, double m, dou
 // h/inv_h: the divisor's row factor, hx/ihx its column factor; w0, w1 the
 // face-density weights, ra, rb the densities either side and m_in the
 // momentum (kVel; loaded by the caller, possibly a row ahead).
-// kUm: a uniform mesh, with the update's coefficient k.
-template <typename R, bool kU, bool kVel, bool kUm>
+// k: on a uniform mesh, the update's coefficient.
+template <typename R, bool kU, bool kVel, int kM>
 __device__ __forceinline__ void momentum_face_update(const StepArgs<R>& a, bool edge, int ii,
                                                      int jj, R fa, R fb, R k, R dt_h, R hx, R ihx,
                                                      R h, R inv_h, R w0, R w1, R m_in, R ra,
@@ -2537,20 +2661,23 @@ __device__ __forceinline__ void momentum_face_update(const StepArgs<R>& a, bool 
         m = Pr::dsub(m, dt_h * diff, hx * h, inv_h * ihx);
         *mom = m;
       }
-    } else if constexpr (kUm) {
+    } else if constexpr (kM == kMeshUniform) {
       m = momentum_change_uniform<kVel>(mom, m, fa, fb, k);
     } else {
-      m = momentum_change<kVel>(mom, m, fa, fb, dt_h, hx, h, inv_h, ihx);
+      m = momentum_change<kVel, kM == kMeshPow2>(mom, m, fa, fb, dt_h, hx, h, inv_h, ihx);
     }
   }
   if (kVel) {
     R rbar;
     // FP64 form, uniform mesh: equal densities either side in the whole warp
-    // are the face density.
-    if (kUm && warp_all(lane_same(ra, rb))) {
+    // are the face density; with power-of-two weights, equal too, it is
+    // 2 (ra w0), exactly.
+    if (kM == kMeshUniform && warp_all(lane_same(ra, rb))) {
       rbar = ra;
+    } else if (kM == kMeshPow2 && warp_all(lane_same(ra, rb) && lane_same(w0, w1))) {
+      rbar = Pr::twice(Pr::template mulp<true>(ra, w0));
     } else {
-      rbar = face_average<R, kUm>(ra, w0, rb, w1);
+      rbar = face_average<R, kM>(ra, w0, rb, w1);
     }
     const R vel = face_velocity(m, rbar);
     if (kU) {
@@ -2642,12 +2769,16 @@ __device__ __forceinline__ void copy_velocities(const StepArgs<R>& a, bool edge,
 //   kV = true (rho_v): thread t holds the vF_x of corner c0 + t (c0 = pad +
 //     127 bx) and, for t < 127, updates y-face c0 + t from corners c0 + t and
 //     c0 + t + 1.
-template <typename R, bool kV, bool kVel, bool kU, bool kRing, bool kFl, bool kTest>
+template <typename R, bool kV, bool kVel, int kM, bool kRing, bool kFl>
 __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, int by) {
+  constexpr bool kU = kM == kMeshUniform, kP2 = kM == kMeshPow2;
   using Pr = Prec<R>;
-  __shared__ R s_half[kMaxRows], s_h[kMaxRows], s_row[kMaxRows];
-  __shared__ R s_wy0[kMaxRows], s_wy1[kMaxRows];
-  __shared__ R sF[kCols];
+  R* const s_half = tile_table<R, kMaxRows + 3, 0>();
+  R* const s_h = tile_table<R, kMaxRows + 3, 1>();
+  R* const s_row = tile_table<R, kMaxRows + 3, 2>();
+  R* const s_wy0 = tile_table<R, kMaxRows + 3, 3>();
+  R* const s_wy1 = tile_table<R, kMaxRows + 3, 4>();
+  R* const sF = tile_table<R, kCols, 0>();
   // kVel and kRing (the fused kernels): the update inputs of a face (its
   // momentum and the densities either side) stream through a per-thread
   // ring of asynchronous copies, kAhead rows ahead (no registers held for
@@ -2669,29 +2800,16 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
   const int i0 = pad + by * a.rows;
   const bool edge = tile_near_edge(nx, ny, pad, c0, i0, a.rows);
   const int i1 = min(i0 + a.rows, kV ? ny + 1 - pad : ny - pad);
-  if constexpr (kVel && kFl && kTest) {
-    // No mass moves around the tile's faces: the Lagrangian velocities stand.
-    if (tile_mass_still(a, i0 - 1, i1, c0 - 1, c0 + kCols)) {
-      const bool upd = kV ? (t < kCols - 1 && j < nx - pad) : (t >= 1 && j < nx + 1 - pad);
-      const bool zero = tile_vel_still(a, i0 - 2, i1 + 2, c0 - 2, c0 + kCols + 2);
-      // Velocities all +0 whose cells were at rest through the previous
-      // step, when this pair stored (or kept) +0 for each of them: they stand.
-      if (zero && rest_cells(a, i0 - 1, i1, c0 - 1, c0 + kCols)) return;
-      copy_velocities<R, !kV>(a, edge, kV ? a.v : a.u, kV ? a.v_out : a.u_out, i0, i1, j, upd,
-                              zero);
-      return;
-    }
-  }
   if (!kU && t < a.rows) {
     const int ii = i0 + t;
     if (ii < ny) {
       // Flux: edgedy/2 (uF_x) or celldy/2 (vF_x); update divisor: celldy.
       s_half[t] = geo_half<R>(kV ? a.celldy[ii] : a.edgedy[ii]);
       s_h[t] = geo_v<R>(a.celldy[ii]);
-      s_row[t] = geo_rcp<R>(a.celldy[ii]);
+      s_row[t] = geo_rcp<R, kP2>(a.celldy[ii]);
       if (kV && kVel) {
-        s_wy0[t] = geo_half_ratio<R>(a.celldy[ii], a.edgedy[ii]);
-        s_wy1[t] = geo_half_ratio<R>(a.celldy[ii - 1], a.edgedy[ii]);
+        s_wy0[t] = geo_half_ratio<R, kP2>(a.celldy[ii], a.edgedy[ii]);
+        s_wy1[t] = geo_half_ratio<R, kP2>(a.celldy[ii - 1], a.edgedy[ii]);
       }
     }
   }
@@ -2739,16 +2857,16 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
     ku = Pr::half(kh);
   } else {
     if (flux_ok) {
-      iex = geo_rcp<R>(a.edgedx[js]);
+      iex = geo_rcp<R, kP2>(a.edgedx[js]);
       cxl = geo_v<R>(a.celldx[js - 1]);
       cxr = geo_v<R>(a.celldx[js]);
     }
     if (upd) {
       hx = geo_v<R>(a.edgedx[j]);
-      ihx = geo_rcp<R>(a.edgedx[j]);
+      ihx = geo_rcp<R, kP2>(a.edgedx[j]);
       if (!kV && kVel) {
-        wx0 = geo_half_ratio<R>(a.celldx[j], a.edgedx[j]);
-        wx1 = geo_half_ratio<R>(a.celldx[j - 1], a.edgedx[j]);
+        wx0 = geo_half_ratio<R, kP2>(a.celldx[j], a.edgedx[j]);
+        wx1 = geo_half_ratio<R, kP2>(a.celldx[j - 1], a.edgedx[j]);
       }
     }
   }
@@ -2842,11 +2960,11 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
           val = sum_zeros(Fa, Fb);
         } else {
           const R ua = uu[f], ub = uu[f + 1];
-          const R mass = kU ? Fa + Fb : (Fa + Fb) * s_half[k];
+          const R mass = kU ? Fa + Fb : Pr::template mulp<kP2>(Fa + Fb, s_half[k]);
           // No mass through the cell, no momentum flux.
           val = Pr::zero_skip_coarse(mass)
                     ? mass
-                    : mass * momentum_upwind<R, kU>(Pr::half(ua + ub), uu[f - 1], ua, ub,
+                    : mass * momentum_upwind<R, kM>(Pr::half(ua + ub), uu[f - 1], ua, ub,
                                                     uu[f + 2], iex, cxl, cxr, dt_h, kh);
         }
       } else {
@@ -2854,10 +2972,10 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
         if (warp_zeros(Fa, F_dn)) {
           val = sum_zeros(Fa, F_dn);  // FP64 form: no mass through any corner of the warp
         } else {
-          const R mass = kU ? Fa + F_dn : (Fa + F_dn) * s_half[k];
+          const R mass = kU ? Fa + F_dn : Pr::template mulp<kP2>(Fa + F_dn, s_half[k]);
           val = Pr::zero_skip_coarse(mass)
                     ? mass
-                    : mass * momentum_upwind<R, kU>(Pr::half(u0 + u_dn), vv[c - 2], vv[c - 1],
+                    : mass * momentum_upwind<R, kM>(Pr::half(u0 + u_dn), vv[c - 2], vv[c - 1],
                                                     vv[c], vv[c + 1], iex, cxl, cxr, dt_h, kh);
         }
         F_dn = Fa;
@@ -2884,7 +3002,7 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
         ra = a.rho_r[c];
         rb = kV ? a.rho_r[c - nx] : a.rho_r[c - 1];
       }
-      momentum_face_update<R, !kV, kVel, kU>(
+      momentum_face_update<R, !kV, kVel, kM>(
           a, edge, ii, j, fa, fb, ku, dt_h, hx, ihx, kU ? R(0) : s_h[k], kU ? R(0) : s_row[k],
           kU ? R(0) : (kV ? s_wy0[k] : wx0), kU ? R(0) : (kV ? s_wy1[k] : wx1), m, ra, rb, vout);
     }
@@ -2902,8 +3020,9 @@ __device__ __forceinline__ void tile_mom_x_impl(const StepArgs<R>& a, int bx, in
 //     updates y-faces i0 .. i1-1 from cells ii-1, ii.
 // The windows form their differences only where mass moves in the warp
 // (FP64 form), as the y mass sweep does.
-template <typename R, bool kV, bool kVel, bool kU, bool kRing, bool kFl, bool kTest>
+template <typename R, bool kV, bool kVel, int kM, bool kRing, bool kFl>
 __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, int by) {
+  constexpr bool kU = kM == kMeshUniform, kP2 = kM == kMeshPow2;
   using Pr = Prec<R>;
   // kVel and kRing (the fused kernels): the update inputs of a face stream
   // through a per-thread ring of asynchronous copies, kAhead rows ahead (as
@@ -2917,24 +3036,17 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
   auto s_flux = ring_slots<R, kFluxRing ? kSlots : 1, 3, kFluxRing ? kCols : 1, 5>();
   // Flux tables over flux rows q = ci - fr0 (fr0 the first flux row): 1/edgedy
   // of the row, celldy of the row below (s_cy[q]) and of the row (s_cy[q + 1]).
-  __shared__ R s_iey[kMaxRows + 2], s_cy[kMaxRows + 3];
-  __shared__ R s_h[kMaxRows], s_row[kMaxRows], s_wy0[kMaxRows], s_wy1[kMaxRows];
+  R* const s_iey = tile_table<R, kMaxRows + 3, 0>();
+  R* const s_cy = tile_table<R, kMaxRows + 3, 1>();
+  R* const s_h = tile_table<R, kMaxRows + 3, 2>();
+  R* const s_row = tile_table<R, kMaxRows + 3, 3>();
+  R* const s_wy0 = tile_table<R, kMaxRows + 3, 4>();
+  R* const s_wy1 = tile_table<R, kMaxRows + 3, 5>();
   const int nx = a.nx, ny = a.ny, pad = a.pad;
   const int jj = pad + bx * kCols + threadIdx.x;
   const int i0 = pad + by * a.rows;
   const bool edge = tile_near_edge(nx, ny, pad, pad + bx * kCols, i0, a.rows);
   const int i1 = min(i0 + a.rows, kV ? ny + 1 - pad : ny - pad);
-  if constexpr (kVel && kFl && kTest) {
-    // No mass moves around the tile's faces: the Lagrangian velocities stand.
-    const int cb = pad + bx * kCols;
-    if (tile_mass_still(a, i0 - 1, i1, cb - 1, cb + kCols)) {
-      const bool zero = tile_vel_still(a, i0 - 2, i1 + 2, cb - 2, cb + kCols + 2);
-      if (zero && rest_cells(a, i0 - 1, i1, cb - 1, cb + kCols)) return;
-      copy_velocities<R, !kV>(a, edge, kV ? a.v : a.u, kV ? a.v_out : a.u_out, i0, i1, jj,
-                              jj < (kV ? nx - pad : nx + 1 - pad), zero);
-      return;
-    }
-  }
   // Flux rows: corners i0 .. i1 (rho_u); cells i0-1 .. i1-1 (rho_v), a ghost
   // row computed at its mirror source.
   const int fr0 = kV ? i0 - 1 : i0;
@@ -2947,7 +3059,7 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
   // source's.)
   for (int q = kU ? nfr + 1 : (int)threadIdx.x; q <= nfr; q += kCols) {
     const int ci = fr0 + q;
-    if (q < nfr) s_iey[q] = geo_rcp<R>(a.edgedy[ci]);
+    if (q < nfr) s_iey[q] = geo_rcp<R, kP2>(a.edgedy[ci]);
     s_cy[q] = geo_v<R>(a.celldy[ci - 1]);
   }
   if (!kU && threadIdx.x < a.rows) {
@@ -2955,10 +3067,10 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
     if (ii < ny) {
       // Update divisor row factor: edgedy for both y pairs.
       s_h[threadIdx.x] = geo_v<R>(a.edgedy[ii]);
-      s_row[threadIdx.x] = geo_rcp<R>(a.edgedy[ii]);
+      s_row[threadIdx.x] = geo_rcp<R, kP2>(a.edgedy[ii]);
       if (kV && kVel) {
-        s_wy0[threadIdx.x] = geo_half_ratio<R>(a.celldy[ii], a.edgedy[ii]);
-        s_wy1[threadIdx.x] = geo_half_ratio<R>(a.celldy[ii - 1], a.edgedy[ii]);
+        s_wy0[threadIdx.x] = geo_half_ratio<R, kP2>(a.celldy[ii], a.edgedy[ii]);
+        s_wy1[threadIdx.x] = geo_half_ratio<R, kP2>(a.celldy[ii - 1], a.edgedy[ii]);
       }
     }
   }
@@ -3007,10 +3119,10 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
   } else {
     hcol = geo_half<R>(kV ? a.celldx[jj] : a.edgedx[jj]);  // flux: celldx/2 or edgedx/2
     hx = geo_v<R>(a.celldx[jj]);
-    ihx = geo_rcp<R>(a.celldx[jj]);
+    ihx = geo_rcp<R, kP2>(a.celldx[jj]);
     if (!kV && kVel) {
-      wx0 = geo_half_ratio<R>(a.celldx[jj], a.edgedx[jj]);
-      wx1 = geo_half_ratio<R>(a.celldx[jj - 1], a.edgedx[jj]);
+      wx0 = geo_half_ratio<R, kP2>(a.celldx[jj], a.edgedx[jj]);
+      wx1 = geo_half_ratio<R, kP2>(a.celldx[jj - 1], a.edgedx[jj]);
     }
   }
   // The window's velocity: before this pair's update when it recomputes it.
@@ -3055,14 +3167,14 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
       }
     }
     fresh = true;
-    const R mass = kU ? Fa + Fb : (Fa + Fb) * hcol;
+    const R mass = kU ? Fa + Fb : Pr::template mulp<kP2>(Fa + Fb, hcol);
     if (Pr::zero_skip_coarse(mass)) return mass;
     const R wind = kV ? Pr::half(win.m1 + win.p0) : Pr::half(vwind[c - 1] + vwind[c]);
     const bool pos = Pr::gt0(wind);
     if constexpr (kU) {
       return mass * win.face_uniform(pos, wind, kh);
     } else {
-      return mass * win.face(pos, s_iey[q], pos ? s_cy[q] : s_cy[q + 1], wind * dt_h);
+      return mass * win.template face<kP2>(pos, s_iey[q], pos ? s_cy[q] : s_cy[q + 1], wind * dt_h);
     }
   };
   // The mass fluxes of flux row ci and the value that moves the window there
@@ -3193,7 +3305,7 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
       rb = rb_n;
       if (ii + 1 < i1) load_upd(ii + 1);
     }
-    momentum_face_update<R, !kV, kVel, kU>(
+    momentum_face_update<R, !kV, kVel, kM>(
         a, edge, ii, jj, cur, prev, ku, dt_h, hx, ihx, kU ? R(0) : s_h[k], kU ? R(0) : s_row[k],
         kU ? R(0) : (kV ? s_wy0[k] : wx0), kU ? R(0) : (kV ? s_wy1[k] : wx1), m, ra, rb, vout);
     prev = cur;
@@ -3201,17 +3313,63 @@ __device__ __forceinline__ void tile_mom_y_impl(const StepArgs<R>& a, int bx, in
   if constexpr (kUpdRing || kFluxRing) cp_async_wait<0>();
 }
 
+// A velocity pair's tile around whose faces no mass moves (kX: of an x pair):
+// the Lagrangian velocities stand, and are copied.  Block-uniform (barrier);
+// tested before the tile's variant is chosen.
+template <typename R, bool kV, bool kX>
+__device__ __forceinline__ bool mom_still(const StepArgs<R>& a, int bx, int by) {
+  const int nx = a.nx, ny = a.ny, pad = a.pad, t = threadIdx.x;
+  const int c0 = kX ? (kV ? pad : pad - 1) + bx * (kCols - 1) : pad + bx * kCols;
+  const int j = c0 + t;
+  const int i0 = pad + by * a.rows;
+  const int i1 = min(i0 + a.rows, kV ? ny + 1 - pad : ny - pad);
+  if (!tile_mass_still(a, i0 - 1, i1, c0 - 1, c0 + kCols)) return false;
+  const bool upd = (kV ? j < nx - pad : j < nx + 1 - pad) &&
+                   (!kX || (kV ? t < kCols - 1 : t >= 1));
+  const bool zero = tile_vel_still(a, i0 - 2, i1 + 2, c0 - 2, c0 + kCols + 2);
+  // Velocities all +0 whose cells were at rest through the previous step, when
+  // this pair stored (or kept) +0 for each of them: they stand.
+  if (zero && rest_cells(a, i0 - 1, i1, c0 - 1, c0 + kCols)) return true;
+  copy_velocities<R, !kV>(a, tile_near_edge(nx, ny, pad, c0, i0, a.rows), kV ? a.v : a.u,
+                          kV ? a.v_out : a.u_out, i0, i1, j, upd, zero);
+  return true;
+}
+// Whether a momentum pair's tile takes the kMeshPow2 variant: not where no mass
+// moves around it, which the tile itself finds next (a velocity pair's has been
+// looked at) and leaves.
+template <bool kFl, typename R>
+__device__ __forceinline__ bool mom_pow2(const StepArgs<R>& a, int col0, int row0) {
+  if (kFl && !mesh_all_pow2(a) && mesh_some_pow2(a) &&
+      tile_mass_still(a, row0 - 1, row0 + a.rows, col0 - 1, col0 + kCols)) {
+    return false;
+  }
+  return block_mesh_pow2(a, col0, row0);
+}
+
 template <typename R, bool kV, bool kVel, bool kRing = true, bool kFl = false,
-          bool kTest = true>
+          bool kTest = true, bool kP2T = false>
 __device__ __forceinline__ void tile_mom_x(const StepArgs<R>& a, int bx, int by, bool uni) {
-  FLOW_UNIFORM_DISPATCH(R, (tile_mom_x_impl<R, kV, kVel, true, kRing, kFl, kTest>(a, bx, by)),
-                        (tile_mom_x_impl<R, kV, kVel, false, kRing, kFl, kTest>(a, bx, by)));
+  if constexpr (kVel && kFl && kTest) {
+    if (mom_still<R, kV, true>(a, bx, by)) return;
+  }
+  const int col0 = (kV ? a.pad : a.pad - 1) + bx * (kCols - 1), row0 = a.pad + by * a.rows;
+  FLOW_MESH_DISPATCH(
+      R, kP2T, (mom_pow2<kFl && !kVel>(a, col0, row0)),
+      (tile_mom_x_impl<R, kV, kVel, kMeshUniform, kRing, kFl>(a, bx, by)),
+      (tile_mom_x_impl<R, kV, kVel, kMeshPow2, kRing, kFl>(a, bx, by)),
+      (tile_mom_x_impl<R, kV, kVel, kMeshGeneral, kRing, kFl>(a, bx, by)));
 }
 template <typename R, bool kV, bool kVel, bool kRing = true, bool kFl = false,
-          bool kTest = true>
+          bool kTest = true, bool kP2T = false>
 __device__ __forceinline__ void tile_mom_y(const StepArgs<R>& a, int bx, int by, bool uni) {
-  FLOW_UNIFORM_DISPATCH(R, (tile_mom_y_impl<R, kV, kVel, true, kRing, kFl, kTest>(a, bx, by)),
-                        (tile_mom_y_impl<R, kV, kVel, false, kRing, kFl, kTest>(a, bx, by)));
+  if constexpr (kVel && kFl && kTest) {
+    if (mom_still<R, kV, false>(a, bx, by)) return;
+  }
+  FLOW_MESH_DISPATCH(
+      R, kP2T, (mom_pow2<kFl && !kVel>(a, a.pad + bx * kCols, a.pad + by * a.rows)),
+      (tile_mom_y_impl<R, kV, kVel, kMeshUniform, kRing, kFl>(a, bx, by)),
+      (tile_mom_y_impl<R, kV, kVel, kMeshPow2, kRing, kFl>(a, bx, by)),
+      (tile_mom_y_impl<R, kV, kVel, kMeshGeneral, kRing, kFl>(a, bx, by)));
 }
 
 }  // namespace tiles

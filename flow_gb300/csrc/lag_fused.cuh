@@ -237,6 +237,7 @@ template <bool kU>
 __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, int by,
                                          CflBest& cfl) {
   using Pr = Prec<double>;
+  constexpr int kM = kU ? tiles::kMeshUniform : tiles::kMeshGeneral;
   using tiles::face_average;
   using tiles::face_velocity;
   using tiles::lane_same;
@@ -429,11 +430,11 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
         } else {
           const double dp = P0 - P1;
           if (!Pr::zero_skip_mem(dp)) {
-            mom = tiles::momentum_step<double, kU>(mom, dp, ky, dt, kU ? 0.0 : s_ey[k],
+            mom = tiles::momentum_step<double, kM>(mom, dp, ky, dt, kU ? 0.0 : s_ey[k],
                                                    kU ? 0.0 : s_iey[k]);
             chn = true;
           }
-          rbar = face_average<double, kU>(R0, kU ? 0.0 : s_wy0[k], R1, kU ? 0.0 : s_wy1[k]);
+          rbar = face_average<double, kM>(R0, kU ? 0.0 : s_wy0[k], R1, kU ? 0.0 : s_wy1[k]);
         }
         vnew = face_velocity(mom, rbar);
         mvn = mom;
@@ -474,7 +475,7 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
           const double dqy = qy - qy_dn;
           if (!Pr::zero_skip_mem(dqy)) {
             const int k = fv - ia;
-            mom = tiles::momentum_step<double, kU>(mom, dqy, ky, dt, kU ? 0.0 : s_cy[k],
+            mom = tiles::momentum_step<double, kM>(mom, dqy, ky, dt, kU ? 0.0 : s_cy[k],
                                                    kU ? 0.0 : s_icy[k]);
             vel = face_velocity(mom, rb2);
             vf_changed = true;
@@ -593,7 +594,7 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
         if (!warp_same(q1, q0)) {
           const double dqx = q1 - q0;
           if (!Pr::zero_skip_mem(dqx)) {
-            mom = tiles::momentum_step<double, kU>(mom, dqx, kx, dt, cx, icx);
+            mom = tiles::momentum_step<double, kM>(mom, dqx, kx, dt, cx, icx);
             vel = face_velocity(mom, rbx2);
             u_changed = true;
           }
@@ -629,10 +630,10 @@ __device__ __forceinline__ bool lag_tile(const LagArgs& a, LagSmem& sm, int bx, 
       } else {
         const double dp = Pc - Pl;
         if (!Pr::zero_skip_mem(dp)) {
-          mom = tiles::momentum_step<double, kU>(mom, dp, kx, dt, ex, iex);
+          mom = tiles::momentum_step<double, kM>(mom, dp, kx, dt, ex, iex);
           cu0 = true;
         }
-        rbar = face_average<double, kU>(rc, wx0, rl, wx1);
+        rbar = face_average<double, kM>(rc, wx0, rl, wx1);
       }
       const double vel = face_velocity(mom, rbar);
       s_U[b][t] = ghost ? d_neg(vel) : vel;

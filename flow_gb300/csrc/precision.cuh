@@ -71,8 +71,15 @@ struct Prec<double> {
   __device__ static __forceinline__ double div(double n, double d) { return d_div(n, d); }
   // m - t/d with the quotient rounded before the difference, as the
   // reference evaluates a momentum or mass update by a mesh spacing d.
+  // kPow2: d is a power of two, so t*inv is the quotient, an exponent add.
+  template <bool kPow2 = false>
   __device__ static __forceinline__ double dsub(double m, double t, double d, double inv) {
-    return __dadd_rn(m, -qdiv(t, d, inv));
+    return __dadd_rn(m, -(kPow2 ? d_mul_pow2(t, inv) : qdiv(t, d, inv)));
+  }
+  // x * p; kPow2: p is a power of two and the product an exponent add.
+  template <bool kPow2>
+  __device__ static __forceinline__ double mulp(double x, double p) {
+    return kPow2 ? d_mul_pow2(x, p) : x * p;
   }
   // x * 0.5 and x * 2, exact, on the integer pipes.
   __device__ static __forceinline__ double half(double x) { return d_half(x); }
@@ -181,9 +188,12 @@ struct Prec<float> {
   __device__ static __forceinline__ float qdiv(float n, float, float inv) { return n * inv; }
   __device__ static __forceinline__ float rcp_q(float x) { return rcp(x); }
   __device__ static __forceinline__ float div(float n, float d) { return n * rcp(d); }
+  template <bool kPow2 = false>
   __device__ static __forceinline__ float dsub(float m, float t, float, float inv) {
     return fmaf(-t, inv, m);
   }
+  template <bool kPow2>
+  __device__ static __forceinline__ float mulp(float x, float p) { return x * p; }
   __device__ static __forceinline__ float half(float x) { return 0.5f * x; }
   __device__ static __forceinline__ float neg(float x) { return -x; }
   __device__ static __forceinline__ float twice(float x) { return x + x; }
