@@ -29,6 +29,15 @@ def _torch():
     return torch
 
 
+def totals_call():
+    """gb300_conservation taking addresses: a cast to double* per array and
+    call takes as long as the reduction on a small mesh."""
+    fn = lib()["gb300_conservation"]  # (a function object of its own)
+    fn.restype = ctypes.c_int
+    fn.argtypes = [ctypes.c_int] * 3 + [ctypes.c_void_p] * 4 + [ctypes.c_int]
+    return fn
+
+
 class DeviceSim:
     """All arrays of one problem on one GPU plus its ``Mesh``."""
 
@@ -63,8 +72,7 @@ class DeviceSim:
         self._mesh_ref = ctypes.byref(m)
         self._solve = lib().gb300_solve_hydro_2d
         self._args = None
-        self._conservation = lib().gb300_conservation
-        self._totals = None
+        self._conservation = totals_call()
         self.tt = 0
         if prob.box_list is not None:
             self.fill_boxes(prob.box_list)
@@ -139,16 +147,10 @@ class DeviceSim:
             self.step()
 
     def conservation(self) -> tuple[float, float]:
-        # The call's arguments are formed again only when an array moved (the
-        # casts take as long as the reduction on a small mesh).
-        key = tuple(self.a[f].data_ptr() for f in ("rho", "e", "reduce"))
-        if self._totals is None or self._totals[0] != key:
-            out = (ctypes.c_double * 2)()
-            self._totals = (key, out, (self.nx, self.ny, PAD, dptr(self.a["rho"]),
-                                       dptr(self.a["e"]), dptr(self.a["reduce"]),
-                                       ctypes.cast(out, ctypes.POINTER(ctypes.c_double)), 1))
-        _, out, args = self._totals
-        if self._conservation(*args) != GB300_OK:
+        a = self.a
+        out = (ctypes.c_double * 2)()
+        if self._conservation(self.nx, self.ny, PAD, a["rho"].data_ptr(), a["e"].data_ptr(),
+                              a["reduce"].data_ptr(), out, 1) != GB300_OK:
             check()
         return float(out[0]), float(out[1])
 
