@@ -82,13 +82,4 @@ __device__ __forceinline__ double dmin(double a, double b) {
   return (a < b) ? a : b;
 }
 
-// Slope limiter: the argument of smaller magnitude when both are non-zero and
-// of the same sign (the second on a tie), else 0.
-__device__ __forceinline__ double minmod(double a, double b) {
-  if ((a > 0.0 && b > 0.0) || (a < 0.0 && b < 0.0)) {
-    return (fabs(a) < fabs(b)) ? a : b;
-  }
-  return 0.0;
-}
-
 }  // namespace flow

@@ -25,7 +25,8 @@ __device__ __forceinline__ bool ge0(double x) {
 __device__ __forceinline__ bool nz(double x) { return !d_is_zero(x); }
 // (0.0 < x) ? 0.0 : x
 __device__ __forceinline__ double min0(double x) { return gt0(x) ? 0.0 : x; }
-// minmod of common.cuh (+0.0 where either argument is a NaN).
+// Slope limiter: the argument of smaller magnitude when both are non-zero and
+// of the same sign (the second on a tie), else +0.0 (also for a NaN).
 __device__ __forceinline__ double minmod(double a, double b) {
   const long long ia = dbits(a), ib = dbits(b);
   const long long ma = ia & 0x7fffffffffffffffLL, mb = ib & 0x7fffffffffffffffLL;
@@ -87,10 +88,6 @@ __device__ __forceinline__ double div_h(double n, double h, double ih, bool p2) 
 }
 __device__ __forceinline__ double mul_h(double x, double h, bool p2) {
   return p2 ? d_mul_pow2(x, h) : __dmul_rn(x, h);
-}
-// 1 / h
-__device__ __forceinline__ double rcp_h(double h, bool p2) {
-  return p2 ? d_pow2_rcp(h) : div(1.0, h);
 }
 
 }  // namespace ex

@@ -1159,55 +1159,6 @@ struct ConsArgs {
   int mark_w, mark_tiles_x, mark_rows;
 };
 
-// The sum of eight doubles on the integer pipes, rounded once: their
-// mantissas, aligned to the largest exponent with 7 more bits, added as 64-bit
-// integers (60 bits and 3 for the sum).  Bits of a value more than 59 places
-// below the largest's leading one are dropped, well below the rounding of an
-// FP64 addition at that size.  About 85 integer instructions (two clocks of a
-// scheduler each) in place of eight additions of 64 clocks: the totals' two
-// FP64 instructions a cell bound them (16.4 M cells: 58 us of FP64 issue, 39
-// us of memory).  Infinities, NaNs and the ends of the exponent range take the
-// additions (a call, so that the others do not issue them).
-static __device__ __noinline__ double sum8_slow(double a, double b, double c, double d, double e,
-                                                double f, double g, double h) {
-  return ((a + b) + (c + d)) + ((e + f) + (g + h));
-}
-__device__ __forceinline__ double sum8_aligned(const double (&v)[8]) {
-  int emax = 0;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int ex = (dhi(v[q]) >> 20) & 0x7ff;
-    emax = ex > emax ? ex : emax;
-  }
-  if (emax > 0x7f8 || emax < 64) {
-    return sum8_slow(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
-  }
-  long long sum = 0;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const long long b = dbits(v[q]);
-    const int ex = (int)((b >> 52) & 0x7ff);
-    const int sh = emax - ex;
-    // (A zero or subnormal, which has no leading one, lies below the alignment.)
-    const unsigned long long m =
-        (((unsigned long long)b & 0x000fffffffffffffULL) | 0x0010000000000000ULL) << 7;
-    const long long a = sh < 60 ? (long long)(m >> sh) : 0;
-    sum += b < 0 ? -a : a;
-  }
-  if (sum == 0) return 0.0;
-  const bool neg = sum < 0;
-  unsigned long long m = neg ? 0ull - (unsigned long long)sum : (unsigned long long)sum;
-  const int lz = __clzll((long long)m);  // leading one at bit 63 - lz
-  m <<= lz;
-  // Round to nearest even at bit 11.
-  const unsigned long long r = (m >> 11) + (((m & 0x7ffULL) + ((m >> 11) & 1ULL)) > 0x400ULL);
-  // m at bit 59 has the exponent emax; r holds the leading one at bit 52 (or
-  // carried to 53), which the sum adds to the exponent field below it.
-  const long long e = (long long)(emax + (63 - lz) - 59 - 1);
-  return dfrom((long long)((unsigned long long)(e << 52) + r) |
-               (neg ? (long long)0x8000000000000000ULL : 0LL));
-}
-
 __device__ __forceinline__ double block_sum_fixed(double x, double* s_w) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
@@ -1264,7 +1215,7 @@ __global__ void __launch_bounds__(kCols) k_conservation_tiles(const ConsArgs c) 
           ec[q] = ev[q];
         }
         if (ib + kB < r1) load(ib + kB);
-        ms = __dadd_rn(ms, sum8_aligned(rc));
+        ms = __dadd_rn(ms, d_sum8(rc));
 #pragma unroll
         for (int q = 0; q < kB; ++q) es = __fma_rn(rc[q], ec[q], es);
       }

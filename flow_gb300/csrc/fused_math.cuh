@@ -55,9 +55,6 @@ __device__ __forceinline__ bool d_ge0(double x) { return !d_lt0(x); }
 __device__ __forceinline__ double d_abs(double x) {
   return dfrom(dbits(x) & 0x7fffffffffffffffLL);
 }
-__device__ __forceinline__ double d_neg_if(double x, bool neg) {
-  return dfrom(dbits(x) ^ (neg ? (long long)0x8000000000000000ULL : 0LL));
-}
 // min(0.0, x) with the ordinary-minimum rule (first argument when smaller):
 // 0.0 when x > 0, else x itself.
 __device__ __forceinline__ double d_min0(double x) { return d_gt0(x) ? 0.0 : x; }
@@ -218,14 +215,6 @@ __device__ __forceinline__ double d_rcp(double x) {
   const double r = d_rcp_seed(x);
   return fma(r, fma(-x, r, 1.0), r);
 }
-// 1/x to ~2^-40 (one Newton step on the MUFU seed) for a reciprocal that is
-// only ever used through a residual-corrected quotient (qdiv), which is then
-// still correctly rounded: the correction squares the error.
-__device__ __forceinline__ double d_rcp_for_qdiv(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  return fma(r, fma(-x, r, 1.0), r);
-}
 // n/d for finite normal non-zero d when 1/d itself is not needed: the quotient
 // from the seed and one residual correction q + r (n - d q) (2^-43 -> ~2^-86):
 // the correctly rounded quotient except in vanishingly rare near-ties, in 3
@@ -269,6 +258,55 @@ __device__ __forceinline__ void mirror_store(double* a, int w, int h, int pad,
     a[(size_t)mr[r] * w + jj] = vy;
     for (int k = 0; k < nc; ++k) a[(size_t)mr[r] * w + mc[k]] = vxy;
   }
+}
+
+// The sum of eight doubles on the integer pipes, rounded once: their
+// mantissas, aligned to the largest exponent with 7 more bits, added as 64-bit
+// integers (60 bits and 3 for the sum).  Bits of a value more than 59 places
+// below the largest's leading one are dropped, well below the rounding of an
+// FP64 addition at that size.  About 85 integer instructions (two clocks of a
+// scheduler each) in place of eight additions of 64 clocks: the totals' two
+// FP64 instructions a cell bound them (16.4 M cells: 58 us of FP64 issue, 39
+// us of memory).  Infinities, NaNs and the ends of the exponent range take the
+// additions (a call, so that the others do not issue them).
+static __device__ __noinline__ double d_sum8_slow(double a, double b, double c, double d, double e,
+                                                  double f, double g, double h) {
+  return ((a + b) + (c + d)) + ((e + f) + (g + h));
+}
+__device__ __forceinline__ double d_sum8(const double (&v)[8]) {
+  int emax = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int ex = (dhi(v[q]) >> 20) & 0x7ff;
+    emax = ex > emax ? ex : emax;
+  }
+  if (emax > 0x7f8 || emax < 64) {
+    return d_sum8_slow(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+  }
+  long long sum = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const long long b = dbits(v[q]);
+    const int ex = (int)((b >> 52) & 0x7ff);
+    const int sh = emax - ex;
+    // (A zero or subnormal, which has no leading one, lies below the alignment.)
+    const unsigned long long m =
+        (((unsigned long long)b & 0x000fffffffffffffULL) | 0x0010000000000000ULL) << 7;
+    const long long a = sh < 60 ? (long long)(m >> sh) : 0;
+    sum += b < 0 ? -a : a;
+  }
+  if (sum == 0) return 0.0;
+  const bool neg = sum < 0;
+  unsigned long long m = neg ? 0ull - (unsigned long long)sum : (unsigned long long)sum;
+  const int lz = __clzll((long long)m);  // leading one at bit 63 - lz
+  m <<= lz;
+  // Round to nearest even at bit 11.
+  const unsigned long long r = (m >> 11) + (((m & 0x7ffULL) + ((m >> 11) & 1ULL)) > 0x400ULL);
+  // m at bit 59 has the exponent emax; r holds the leading one at bit 52 (or
+  // carried to 53), which the sum adds to the exponent field below it.
+  const long long e = (long long)(emax + (63 - lz) - 59 - 1);
+  return dfrom((long long)((unsigned long long)(e << 52) + r) |
+               (neg ? (long long)0x8000000000000000ULL : 0LL));
 }
 
 }  // namespace flow

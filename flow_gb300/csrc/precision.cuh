@@ -1,8 +1,8 @@
 // precision.cuh -- arithmetic policies of the fused timestep kernels.
 //
 // Prec<double>: the FP64 form.  Comparisons and selections run on the IEEE
-//   bit pattern with integer instructions; reciprocal and reciprocal square
-//   root start from the MUFU approximation (fused_math.cuh).
+//   bit pattern with integer instructions; reciprocals start from an FP32 seed,
+//   reciprocal square roots from the FP64 MUFU approximation (fused_math.cuh).
 // Prec<float>:  the bulk arithmetic of the mixed form.  FP32 compares are
 //   full-rate, so the native operations are used; reciprocals are the MUFU
 //   approximations.
@@ -46,8 +46,6 @@ struct Prec<double> {
     return d_minmod(d_minmod(a, b), c);
   }
   __device__ static __forceinline__ double rcp(double x) { return d_rcp(x); }
-  // A reciprocal used only through qdiv (which corrects the quotient).
-  __device__ static __forceinline__ double rcp_q(double x) { return d_rcp_for_qdiv(x); }
   __device__ static __forceinline__ double rsqrt(double x) { return d_rsqrt(x); }
   __device__ static __forceinline__ double to_d(double x) { return x; }
   __device__ static __forceinline__ double diff_d(double a, double b) { return a - b; }
@@ -186,7 +184,6 @@ struct Prec<float> {
   __device__ static __forceinline__ float msub(float m, float t, float s) { return fmaf(-t, s, m); }
   __device__ static __forceinline__ float madd(float h, float w, float b) { return fmaf(h, w, b); }
   __device__ static __forceinline__ float qdiv(float n, float, float inv) { return n * inv; }
-  __device__ static __forceinline__ float rcp_q(float x) { return rcp(x); }
   __device__ static __forceinline__ float div(float n, float d) { return n * rcp(d); }
   template <bool kPow2 = false>
   __device__ static __forceinline__ float dsub(float m, float t, float, float inv) {

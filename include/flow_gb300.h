@@ -387,15 +387,31 @@ int gb300_measure_fp64_fma_rate(double* fma_per_s);
  *   counts[0]  x*0.5 on the integer pipes != IEEE x*0.5 (every bit pattern)
  *   counts[1]  x*2 on the integer pipes != IEEE x*2
  *   counts[2]  power-of-two test wrong
- *   counts[3]  one-Newton-step quotient with one correction != IEEE n/d
- *   counts[4]  one-Newton-step reciprocal, then a corrected quotient != IEEE n/d
+ *   counts[3]  quotient from the reciprocal seed with one correction != IEEE n/d
+ *   counts[4]  reciprocal, then a corrected quotient != IEEE n/d
  *   counts[5]  x times a power of two on the integer pipes != IEEE product
  *   counts[6]  1/p, x/(2p), 1/(p*p) of powers of two x, p from their
  *              exponent fields != the IEEE expressions
  * max_ulp[0..1]: the largest gaps of counts[3..4] in units in the last
- * place; max_seed_rel_err: the largest |rcp.approx(d) * d - 1|. */
+ * place; max_seed_rel_err: the largest |seed(d) * d - 1| (exponents -60 to 60). */
 int gb300_check_fp64_helpers(long long n, unsigned long long seed, long long* counts,
                              long long* max_ulp, double* max_seed_rel_err);
+
+/* The same for the rest of the kernels' arithmetic, over the whole exponent
+ * range:
+ *   counts[0]  the bit-exact mode's quotient != IEEE n/d
+ *   counts[1]  the bit-exact mode's limited slope != the reference's products
+ *              (zeros of either sign alike)
+ *   counts[2]  FP32 flux difference widened to FP64 != the FP64 difference
+ *   counts[3]  FP64 / FP32 conversions on the integer pipes != the conversions
+ *              (FP32's normal range)
+ *   counts[4]  sum of eight doubles on the integer pipes further off than the
+ *              bits it drops and its rounding, or of another class
+ *   counts[5]  reciprocal != IEEE 1/x (a rare last place)
+ * max_rcp_ulp: the largest gap of counts[5]; max_seed_rel_err: the largest
+ * |seed(x) * x - 1| over all normal x with a normal reciprocal. */
+int gb300_check_kernel_math(long long n, unsigned long long seed, long long* counts,
+                            long long* max_rcp_ulp, double* max_seed_rel_err);
 
 #ifdef __cplusplus
 }
