@@ -137,9 +137,11 @@ class Batch:
                     return {"cached": True, **got}
             except (OSError, ValueError):
                 pass
+        # (The height in use, chosen from the ensemble's tiles unless set, too.)
+        heights = sorted({8, 16, 32, self.tuning()["rows"]})
         candidates = candidates or (
-            [(BATCH_PHASES, r, 0, o) for r in (8, 16, 32) for o in (0, 1)]
-            + [(BATCH_PERSISTENT, r, c, o) for r in (8, 16, 32) for c in (0, 2) for o in (0, 1)])
+            [(BATCH_PHASES, r, 0, o) for r in heights for o in (0, 1)]
+            + [(BATCH_PERSISTENT, r, c, o) for r in heights for c in (0, 2) for o in (0, 1)])
         results = []
         for (sc, r, c, o) in candidates:
             self.set_schedule(sc)
