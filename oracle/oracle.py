@@ -58,7 +58,7 @@ REF_DIR = os.environ.get("FLOW_REF_DIR", "/root/reference")
 def build() -> None:
     """Compiles the C restatement (and the reference, where its sources exist)."""
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
-    if os.path.isdir(REF_DIR):
+    if os.path.isfile(os.path.join(REF_DIR, "omp3", "flow.c")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF_DIR={REF_DIR}"], check=True)
 
 
