@@ -69,12 +69,11 @@ template <typename R, int kMd>
 __global__ void __launch_bounds__(kCols, 8) k_lag_pressure(const StepArgs<R> a) {
   pdl_wait();
   pdl_trigger();
-  // The first kernel of the step clears the CFL minimum and the block ticket
-  // of the shock-heating kernel (three kernels later, which waits for it).
+  // The phase's first block clears the block ticket (for the conservation totals
+  // after the step), starts the CFL minimum from the tiles the step does not
+  // visit, and clears what the second sweep's list blocks accumulate.
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
     *reinterpret_cast<unsigned long long*>(a.ra + kRaTicket) = 0ull;
-    // (and starts the minimum from the tiles the step does not visit), and
-    // what the step's last kernel accumulates.
     *a.min_slot = a.from_rest_min ? *a.rest_min : ~0ull;
     if constexpr (kMd != kNoFlags) {
       *a.rest_min = ~0ull;
@@ -295,13 +294,13 @@ __device__ __forceinline__ bool line_tile(const StepArgs<R>& a, int k, int& bx, 
     return true;
   }
 }
+// With flags, the mass-flux flags (a.fxflag, a.fyflag) are kept -- the sweeps
+// store only warps with a non-zero mass flux, and the momentum pairs load only
+// those.
 // kLists (a second sweep): the last 2 l.blocks blocks of the (1-D) launch form
-// the next step's tile lists beside the sweep, which reads neither the marks of
-// the tiles it visits later nor the minima the lists are formed from in a way
-// they change; as a kernel of their own the lists took 7 to 20 us a step, and
-// beside the step's last launch, which is short, 5.
-// With flags, the mass-flux flags (a.fxflag, a.fyflag) are kept -- the sweeps store only warps with a non-zero mass flux, and the
-// momentum pairs load only those.
+// the next step's tile lists beside the sweep, which changes neither the marks
+// nor the minima they are formed from; as a kernel of their own the lists took 7
+// to 20 us a step, and beside the step's last launch, which is short, 5.
 template <typename R, bool kFirst, int kMd, bool kLists>
 __global__ void __launch_bounds__(kCols, Prec<R>::kMixed ? 8 : 7) k_mass_sweep_x(
     const StepArgs<R> a, const SweepArgs<R> s, const ListArgs l) {
@@ -347,9 +346,12 @@ template <typename R, int kPair, bool kVel, int kMd>
 __device__ __forceinline__ void pair_tile(const StepArgs<R>& a, int bx, int by, bool uni) {
   constexpr bool kFl = kMd != kNoFlags, kTest = kMd != kListed;
   if constexpr (kPair == kXU) tile_mom_x<R, false, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
-  else if constexpr (kPair == kXV) tile_mom_x<R, true, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
-  else if constexpr (kPair == kYU) tile_mom_y<R, false, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
-  else if constexpr (kPair == kYV) tile_mom_y<R, true, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
+  else if constexpr (kPair == kXV)
+    tile_mom_x<R, true, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
+  else if constexpr (kPair == kYU)
+    tile_mom_y<R, false, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
+  else if constexpr (kPair == kYV)
+    tile_mom_y<R, true, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
 }
 // The tiles of pair A (blocks 0 .. na - 1), then those of pair B.
 template <typename R, int kA, bool kVelA, int kB, bool kVelB, int kMd>
@@ -641,7 +643,8 @@ StepArgs<R> pair_args(const StepArgs<R>& a0, const StepRows& sr, const TileLists
   StepArgs<R> a = with_rows(a0, kVel ? sr.mom_vel : sr.mom_flux);
   const int cols = kV ? (a.nx - 2 * a.pad) : (a.nx + 1 - 2 * a.pad);
   const int rows = kV ? (a.ny + 1 - 2 * a.pad) : (a.ny - 2 * a.pad);
-  const dim3 g = tile_grid(a, tl, kX ? 1 : 0, strip_grid(cols, rows, a.rows, kX ? kCols - 1 : kCols));
+  const dim3 g =
+      tile_grid(a, tl, kX ? 1 : 0, strip_grid(cols, rows, a.rows, kX ? kCols - 1 : kCols));
   tiles = (int)(g.x * g.y);
   return a;
 }
@@ -1083,7 +1086,8 @@ StepRows take_rest(StepArgs<R>& a, int tt, int form, const std::array<const void
     a.from_rest_min = a.cfl_known;
     for (int w = 0; w < 2; ++w) {
       for (int h = 0; h < kListHeights; ++h) {
-        tl.list[w][h] = lists + (w ? L.list_words[0] : 0) + list_offset(L.list_tx[w], L.list_bands, h);
+        tl.list[w][h] =
+            lists + (w ? L.list_words[0] : 0) + list_offset(L.list_tx[w], L.list_bands, h);
         tl.n[w][h] = (int)p.counts[w * kListHeights + h];
       }
     }

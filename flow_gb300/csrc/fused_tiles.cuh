@@ -1197,9 +1197,10 @@ __device__ __forceinline__ double shock_energy_uniform(double e, double du, doub
 
 // Shock heating and work (omp3/flow.c:248-290) fused with the CFL minimum of
 // set_timestep (omp3/flow.c:73-106) on the updated energy.  One atomicMin per
-// block on the FP64 bit pattern of its smallest candidate; the last block to
-// finish applies the leapfrog dt/dt_h rule (finish_dt).  In the mixed form
-// the FP32 energy change is added to the FP64 energy.
+// block on the FP64 bit pattern of its smallest candidate; the step's first sweep
+// applies the leapfrog dt/dt_h rule to the finished minimum (sweep_dt; a kernel
+// or phase of its own in the batched form).  In the mixed form the FP32 energy
+// change is added to the FP64 energy.
 template <typename R, int kM, bool kRing, bool kFlags, bool kTest>
 __device__ __forceinline__ void tile_lag_energy_dt_impl(const StepArgs<R>& a, int bx, int by,
                                                         unsigned long long* tile_min) {
