@@ -354,8 +354,11 @@ __device__ __forceinline__ void pair_tile(const StepArgs<R>& a, int bx, int by, 
     tile_mom_y<R, true, kVel, true, kFl, kTest, kTest>(a, bx, by, uni);
 }
 // The tiles of pair A (blocks 0 .. na - 1), then those of pair B.
+// (Two FP64 velocity pairs: six CTAs an SM; left to itself the compiler takes 86
+// registers, which hold five -- 253 us for 244 at 2048x2048 in motion.)
 template <typename R, int kA, bool kVelA, int kB, bool kVelB, int kMd>
-__global__ void __launch_bounds__(kCols) k_mom(const StepArgs<R> a, const StepArgs<R> b, int na) {
+__global__ void __launch_bounds__(kCols, (kVelA && kVelB && !Prec<R>::kMixed ? 6 : 0))
+    k_mom(const StepArgs<R> a, const StepArgs<R> b, int na) {
   pdl_wait();
   pdl_trigger();
   const bool uni = mesh_uniform<R>(a.mesh);
