@@ -791,6 +791,7 @@ def run_gpu(args):
     traffic = tb * cells if tb is not None else None
     step_gbs = value / world * B_ALG_FP64 / 1e9
     step_bpc = (figures or {}).get("dram_bytes_per_cell_step")
+    dram_gbs = value / world * step_bpc / 1e9 if step_bpc is not None else None
 
     cpu = None
     if host_legs:
@@ -817,17 +818,22 @@ def run_gpu(args):
                 "h2d_bytes_per_step": h2d / args.steps, "d2h_bytes_per_step": d2h / args.steps + 32,
                 "what": "initial state H2D from pinned host, K timesteps + conservation readback "
                         "through the C ABI, final state D2H"},
-        # The step as the unit (its 64 algorithmic bytes per cell-step: rho,
-        # e, rho_u, rho_v read and written once), timed live with CUDA
-        # events; traffic: the DRAM bytes ncu measured per step on this
-        # workload.  kernel: the dominant kernel, on the DRAM bytes per cell
-        # ncu measured for it on this workload over its live duration.
-        "roofline": {"bound": "hbm", "kernel": "timestep", "achieved": step_gbs, "peak": peak,
-                     "unit": "GB/s", "frac": step_gbs / peak,
+        # The step as the unit, timed live with CUDA events: the DRAM bytes
+        # ncu measured per step on this workload (traffic; null when the
+        # committed figures are of other sources) over its time.  Tiles at
+        # rest are not touched, so the bound of this workload is the latency
+        # of its moving tiles, not the bandwidth; whole_state is the rate at
+        # which a step that read and wrote rho, e, rho_u, rho_v everywhere (64
+        # B per cell-step) would have to move them, and may exceed the peak.
+        # dominant_kernel: on the DRAM bytes per cell ncu measured for it on
+        # this workload over its live duration.
+        "roofline": {"bound": "latency", "kernel": "timestep", "achieved": dram_gbs, "peak": peak,
+                     "unit": "GB/s", "frac": dram_gbs / peak if dram_gbs is not None else None,
                      "traffic": step_bpc * cells if step_bpc is not None else None,
                      "peak_kind": peak_kind,
-                     "what": "cell-steps/s x 64 B (rho, e, rho_u, rho_v read and written once "
-                             "per step) over the measured copy bandwidth",
+                     "what": "DRAM bytes per step (ncu) over the step's live time, of the "
+                             "measured copy bandwidth",
+                     "whole_state": {"gbs": step_gbs, "over_peak": step_gbs / peak},
                      "dram_bytes_per_cell_step": step_bpc,
                      "dominant_kernel": {"name": name, "achieved": achieved,
                                          "frac": achieved / peak, "traffic": traffic,
