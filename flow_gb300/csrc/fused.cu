@@ -66,7 +66,8 @@ __device__ __forceinline__ bool block_tile(const StepArgs<R>& a, int& bx, int& b
 }
 
 template <typename R, int kMd>
-__global__ void __launch_bounds__(kCols, 8) k_lag_pressure(const StepArgs<R> a) {
+__global__ void __launch_bounds__(kCols, (Prec<R>::kMixed ? 0 : 8))
+    k_lag_pressure(const StepArgs<R> a) {
   pdl_wait();
   pdl_trigger();
   // The phase's first block clears the block ticket (for the conservation totals
