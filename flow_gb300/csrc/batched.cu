@@ -300,13 +300,15 @@ __device__ __forceinline__ void phase_tile(const Instance<R>& I, int tx, int ty)
 }
 
 // Resident CTAs per SM of each phase kernel: those of the single-problem
-// kernels (fused.cu), which only the sweeps set -- one fewer for the y sweeps,
-// whose tile spills at the single-problem budget once the instance lookup
-// takes its registers (60-70 bytes per thread, measured with -Xptxas -v).
+// kernels (fused.cu), which only the sweeps set -- one fewer for the FP64 y
+// sweeps, whose tile spills at the single-problem budget once the instance
+// lookup takes its registers (60-70 bytes per thread, measured with -Xptxas
+// -v); the mixed ones fit (with six the second takes 76 registers, and eight
+// smooth meshes take 339 us a step for 335).
 template <typename R, int kPh>
 __host__ __device__ constexpr int phase_min_ctas() {
   return (kPh == kPhSweepX1 || kPh == kPhSweepX2) ? (Prec<R>::kMixed ? 8 : 7)
-       : (kPh == kPhSweepY1 || kPh == kPhSweepY2) ? (Prec<R>::kMixed ? 6 : 5)
+       : (kPh == kPhSweepY1 || kPh == kPhSweepY2) ? (Prec<R>::kMixed ? 7 : 5)
        : 1;
 }
 
