@@ -366,7 +366,7 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_batch_mesh_test(const BatchDev<R> b) {
   const StepArgs<R>& a = b.inst[blockIdx.x].a;
   const unsigned r = mesh_test_part(a.nx, a.ny, a.celldx, a.edgedx, a.celldy, a.edgedy,
-                                    const_cast<double*>(a.mesh), 0, 1);
+                                    const_cast<double*>(a.mesh), 0, 1, false);
   if (threadIdx.x == 0) {
     *reinterpret_cast<unsigned long long*>(const_cast<double*>(a.mesh)) = kMeshBytes * r;
   }

@@ -30,19 +30,21 @@ __device__ __forceinline__ void pdl_trigger() {
 // The mesh test (mesh_test_part), the first kernel of a step: a block per part
 // (one block alone took 1 us of a step longer on a 4096^2 mesh, whose 131 KB of
 // spacings it read through one SM).  It also clears the CFL minimum slot and the
-// block ticket for the step's Lagrangian kernels.
+// block ticket for the step's Lagrangian kernels.  It does not let the pressure
+// phase's blocks start early: while its own hold eight SMs they were spread
+// unevenly, which the next kernels' blocks inherit (611x389 in motion: the
+// viscosity phase 15.7 us for 11.4).
 constexpr int kMeshThreads = 512;
 __global__ void __launch_bounds__(kMeshThreads)
     k_mesh_test(int nx, int ny, const double* celldx, const double* edgedx, const double* celldy,
-                const double* edgedy, double* ra) {
+                const double* edgedy, double* ra, int known) {
   pdl_wait();
-  pdl_trigger();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *reinterpret_cast<unsigned long long*>(ra + kRaTicket) = 0ull;
     *reinterpret_cast<unsigned long long*>(ra + kRaMinBits) = ~0ull;
   }
   const unsigned r = mesh_test_part(nx, ny, celldx, edgedx, celldy, edgedy, ra + kRaMesh,
-                                    (int)blockIdx.x, kMeshParts);
+                                    (int)blockIdx.x, kMeshParts, known != 0);
   if (threadIdx.x == 0) {
     reinterpret_cast<unsigned char*>(ra + kRaMesh)[blockIdx.x] = (unsigned char)r;
   }
@@ -723,11 +725,11 @@ void launch_step(cudaStream_t s, const StepArgs<R>& a, int tt,
   const int nx = a.nx, ny = a.ny, pad = a.pad;
   // The whole-mesh spacing test the tiles read, formed by every step: the
   // caller may have written the spacing arrays since the last.  (A launch more,
-  // about 2 us of a step: 1024^2 with a box 139 -> 141 us with the totals,
-  // 4096^2 with a blast 135 -> 137.)
+  // 1 to 2 us of a step: 611x389 in motion 217.5 -> 219 us, a box on 1024^2 with
+  // the totals 137 -> 138.5, a blast on 4096^2 136 -> 137.5.)
   prof.mark("mesh_test");
   launch_pdl_block(k_mesh_test, dim3(kMeshParts), dim3(kMeshThreads), s, nx, ny, a.celldx, a.edgedx,
-                   a.celldy, a.edgedy, a.ra);
+                   a.celldy, a.edgedy, a.ra, a.rest != nullptr ? 1 : 0);
   if (lag) {
     const int nty = (ny - 2 * pad + lag->rows - 1) / lag->rows;
     prof.mark("lag_fused");

@@ -415,34 +415,34 @@ __device__ __forceinline__ UniformMesh uniform_mesh(const double* mesh) {
 // powers of two; bits 2, 3: 32 consecutive entries along x, along y are.  Part 0
 // writes the spacings to mesh.  Every test is made (no short circuit)
 // and the four arrays are read together, so that a thread's loads are in flight
-// at once, and the reciprocals are formed meanwhile.
+// at once.  known: mesh holds an earlier step's spacings and reciprocals; those
+// that are the same still are left as they are (0.2 us for the quotients).
 __device__ __forceinline__ unsigned mesh_test_part(int nx, int ny, const double* celldx,
                                                    const double* edgedx, const double* celldy,
                                                    const double* edgedy, double* mesh, int part,
-                                                   int parts) {
+                                                   int parts, bool known) {
   constexpr int kB = 2;
   const double dx = celldx[0], dy = celldy[0];
-  const long long bx = dbits(dx), by = dbits(dy);
-  // (Exponents from 2^-1000 to 2^1000: the reciprocals are normal too.)
-  auto fine = [](long long b) {
-    return b > 0 && (b >> 52) - 23 >= 0 && (b >> 52) - 23 <= 2000;
-  };
-  bool ok = fine(bx) & fine(by), p2 = true, run_x = false, run_y = false;
+  // (The one thread that keeps the spacing of each axis.)
+  const int keeps = part == 0 ? (threadIdx.x == 0 ? 1 : threadIdx.x == 32 ? 2 : 0) : 0;
+  const double was = known && keeps ? mesh[keeps] : 0.0;
+  bool ok = true, p2 = true, run_x = false, run_y = false;
   const int n = max(nx, ny), stride = parts * (int)blockDim.x;
   for (int b = part * (int)blockDim.x; b <= n; b += kB * stride) {  // (whole warps)
     const int j0 = b + (int)threadIdx.x;
     double v[kB][4];
 #pragma unroll
     for (int q = 0; q < kB; ++q) {
-      const int j = j0 + q * stride;
-      const bool x = j <= nx, y = j <= ny;
-      v[q][0] = x ? celldx[j] : dx;
-      v[q][1] = x ? edgedx[j] : dx;
-      v[q][2] = y ? celldy[j] : dy;
-      v[q][3] = y ? edgedy[j] : dy;
+      // (Past an axis's end its last entry again: no load waits for another.)
+      const int jx = min(j0 + q * stride, nx), jy = min(j0 + q * stride, ny);
+      v[q][0] = celldx[jx];
+      v[q][1] = edgedx[jx];
+      v[q][2] = celldy[jy];
+      v[q][3] = edgedy[jy];
     }
 #pragma unroll
     for (int q = 0; q < kB; ++q) {
+      const long long bx = dbits(dx), by = dbits(dy);  // (used after the loads above only)
       ok &= (dbits(v[q][0]) == bx) & (dbits(v[q][1]) == bx);
       ok &= (dbits(v[q][2]) == by) & (dbits(v[q][3]) == by);
       const bool px = d_is_pow2(v[q][0]) & d_is_pow2(v[q][1]);
@@ -453,16 +453,24 @@ __device__ __forceinline__ unsigned mesh_test_part(int nx, int ny, const double*
       p2 &= px & py;
     }
   }
-  if (part == 0 && threadIdx.x == 0) {
-    mesh[1] = dx;
-    mesh[3] = 1.0 / dx;
+  // (Exponents from 2^-1000 to 2^1000: the reciprocals are normal too.)
+  auto fine = [](long long b) {
+    return b > 0 && (b >> 52) - 23 >= 0 && (b >> 52) - 23 <= 2000;
+  };
+  ok &= fine(dbits(dx)) & fine(dbits(dy));
+  if (keeps) {
+    const double h = keeps == 1 ? dx : dy;
+    if (!known || dbits(was) != dbits(h)) {
+      mesh[keeps] = h;
+      mesh[keeps + 2] = 1.0 / h;
+    }
   }
-  if (part == 0 && threadIdx.x == 32) {
-    mesh[2] = dy;
-    mesh[4] = 1.0 / dy;
+  if (__syncthreads_and(ok)) {
+    const bool px = d_is_pow2(dx), py = d_is_pow2(dy);
+    return 1u | (px && py ? 2u : 0u) | (px ? 4u : 0u) | (py ? 8u : 0u);
   }
-  return (__syncthreads_and(ok) ? 1u : 0u) | (__syncthreads_and(p2) ? 2u : 0u) |
-         (__syncthreads_or(run_x) ? 4u : 0u) | (__syncthreads_or(run_y) ? 8u : 0u);
+  return (__syncthreads_and(p2) ? 2u : 0u) | (__syncthreads_or(run_x) ? 4u : 0u) |
+         (__syncthreads_or(run_y) ? 8u : 0u);
 }
 
 // Whether every spacing of the mesh is a power of two, and whether a tile of a
